@@ -295,11 +295,14 @@ int necg_fp64_peak(int iters, double *tflops, void *stream);
 /* Human-readable text for a status code. */
 const char *necg_status_string(int code);
 
-/* Algorithmic FP64 operation count of one (k, l, P) term (FMA = 2, add/mul = 1,
- * div/sqrt/rsqrt/exp = 1 each): which = 0 energy kernel, 1 ordered gradient
- * kernel, 2 one unordered term of the symmetric gradient pass (bra and ket
- * gradients), 3 one unordered term of the fused pass (H and S elements, bra
- * and ket gradients of H and of S); *special receives the div/sqrt/exp part. */
+/* FP64 operation counts of one (k, l, P) term (FMA = 2, add/mul = 1,
+ * div/sqrt/rsqrt/exp = 1 each).  which = 0 energy, 1 ordered gradient, 2 one
+ * unordered term of the symmetric gradient pass (bra and ket gradients), 3 one
+ * unordered term of the fused pass (H and S elements, bra and ket gradients of
+ * H and of S), in the direct formulation, where every term forms its own
+ * complete gradients: the fixed measure of a term's work by which rates are
+ * quoted.  which = 4 .. 7: the operations the kernels execute for the same
+ * terms.  *special receives the div/sqrt/exp part. */
 long long necg_term_flops(int n, int which, long long *special);
 
 #ifdef __cplusplus

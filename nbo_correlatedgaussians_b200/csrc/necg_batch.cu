@@ -50,7 +50,7 @@ struct InstDesc {
     int npc;             // one-warp fused kernel: symmetry terms split npc ways per tile
     double *psym;
     double *Hp, *Sp;     // npc > 1: the splits' H, S sums (npc K x K each)
-    KetMap kmap;
+    RawMap kmap;
     double cs[kConstsDoubles];
 };
 
@@ -95,13 +95,13 @@ __device__ __forceinline__ void flag_inst(int *status, int flags, int pair) {
     atomicMin(status + 1, pair);
 }
 
-#define BATCH_SWITCH(n, body)                          \
+#define BATCH_SWITCH(n, ...)                           \
     switch (n) {                                       \
-    case 1: { constexpr int N = 1; body; } break;      \
-    case 2: { constexpr int N = 2; body; } break;      \
-    case 3: { constexpr int N = 3; body; } break;      \
-    case 4: { constexpr int N = 4; body; } break;      \
-    case 5: { constexpr int N = 5; body; } break;      \
+    case 1: { constexpr int N = 1; __VA_ARGS__; } break; \
+    case 2: { constexpr int N = 2; __VA_ARGS__; } break; \
+    case 3: { constexpr int N = 3; __VA_ARGS__; } break; \
+    case 4: { constexpr int N = 4; __VA_ARGS__; } break; \
+    case 5: { constexpr int N = 5; __VA_ARGS__; } break; \
     default: break;                                    \
     }
 
@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(32) batch_energy_kernel(PlanPtrs p) {
 // device tile list.  Shared memory is sized for n = kMaxN.
 __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
     __shared__ double sacc[2 * Part<kMaxN>::size * 32];
-    __shared__ double krow[2 * 16 * 33];
+    __shared__ double krow[ket_table<kMaxN>(2)];
     __shared__ double kred[64];
     const int lane = threadIdx.x & 31;
     const int nf = p.hdr->nf;
@@ -203,20 +203,20 @@ __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
 // meet only at the group's barriers (no barrier per term, as the single-
 // instance variant 248).  Shared memory is sized for n = kMaxN.
 template <int N> __host__ __device__ constexpr int bfused_warp_smem() {
-    return 2 * Part<N>::size * 32 + 2 * 16 * 33 + 64 + 2 * KetLayout<N>::size;
+    return 2 * Part<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
 }
-constexpr int kBatchFusedSmem = (8 * bfused_warp_smem<kMaxN>() + BraLayout<kMaxN>::size * 32) * 8;
+constexpr int kBatchFusedSmem = (8 * bfused_warp_smem<kMaxN>() + BraLayout<kMaxN>::term * 32) * 8;
 
 template <int N>
 __device__ __forceinline__ void batch_fused_group(const InstDesc &d, int2 gr, double *smem) {
     constexpr int PS = Part<N>::size;
     constexpr int PER_WARP = bfused_warp_smem<N>();
-    constexpr int BS = BraLayout<N>::size;
+    constexpr int BS = BraLayout<N>::term;
+    constexpr int TBL = ket_table<N>(2);
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
     double *sbra = smem + 8 * PER_WARP;
-    const FusedSmem sm{base, base + 2 * PS * 32, base + 2 * PS * 32 + 2 * 16 * 33,
-                       base + 2 * PS * 32 + 2 * 16 * 33 + 64};
+    const FusedSmem sm{base, base + 2 * PS * 32, base + 2 * PS * 32 + TBL, base + 2 * PS * 32 + TBL + 64};
     const int K = d.K, kb = gr.x, lc = gr.y + w;
     const int last = min(kb * 32 + 31, K - 1);
     const bool idle = lc * d.lc_s > last;
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256) batch_hs_reduce_kernel(PlanPtrs p) {
     }
 }
 
-// g_H - E g_S of every instance into its part (field-major, chunk 0).
+// The per-basis sums of every instance (put_sums) into its part.
 __global__ void __launch_bounds__(256) batch_fsum_kernel(PlanPtrs p) {
     const int ninst = p.hdr->ninst;
     const int total = p.pref_sum[ninst];
@@ -278,13 +278,19 @@ __global__ void __launch_bounds__(256) batch_fsum_kernel(PlanPtrs p) {
         const InstDesc &d = p.inst[q];
         const int id = i - p.pref_sum[q];
         const int f = id / d.K, m = id - f * d.K;
-        const size_t PSd = (size_t)(tri(d.n) + 1 + 3 * d.n);
+        const int PS = tri(d.n) + 1 + 3 * d.n;
         const int npc = d.npc > 1 ? d.npc : 1;
-        const double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * npc * 2 * PSd * 32;
-        double v = 0.0;
-        BATCH_SWITCH(d.n, v = fsym_sum_one<N>(d.stile_start, d.lc_s, d.K, f, m, part_b, part_k, d.scal[0], 0,
-                                              0x7fffffff, npc));
-        d.part[(size_t)f * d.K + m] = v;
+        const double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * npc * 2 * PS * 32;
+        const int kb = m >> 5, lane = m & 31;
+        double bH = 0.0, bS = 0.0, kH = 0.0, kS = 0.0;
+        const int sa = d.stile_start[kb] * npc, sb = d.stile_start[kb + 1] * npc;
+        for (int t = sa; t < sb; ++t) {
+            bH += part_b[(((size_t)t * 2 + 0) * PS + f) * 32 + lane];
+            bS += part_b[(((size_t)t * 2 + 1) * PS + f) * 32 + lane];
+        }
+        BATCH_SWITCH(d.n, (ket_partials<N, true>(d.stile_start, d.lc_s, d.K, f, m, part_k, 0, 0x7fffffff, npc, 0, 1,
+                                                 kH, kS)));
+        put_sums(d.part, PS, d.K, f, m, bH, bS, kH, kS, 2.0 * d.scal[0], d.kmap.fold);
     }
 }
 
@@ -373,6 +379,7 @@ __global__ void __launch_bounds__(256) batch_finalize_kernel(PlanPtrs p) {
 }
 
 __global__ void __launch_bounds__(32) batch_grad_kernel(PlanPtrs p) {
+    __shared__ double sacc[2 * Part<kMaxN>::size * 32];
     const int lane = threadIdx.x & 31;
     const int ng = p.hdr->ng;
     for (;;) {
@@ -387,10 +394,12 @@ __global__ void __launch_bounds__(32) batch_grad_kernel(PlanPtrs p) {
         const int w = e.z * nkb + e.y;  // (kb, lc) as the single-instance kernel numbers it
         if (grad_lane_range(w, lane, nkb, d.lc_g, d.K, k, lc, l0, l1)) {
             bool ok = true;
-            BATCH_SWITCH(d.n, ok = (grad_lane<N, double>(BraRef{d.bra + k, (size_t)d.K}, DevKetB{d.ket}, l0, l1,
-                                                         d.nst, consts_of<N>(d), 1.0, d.scal[0],
-                                                         d.part + (size_t)lc * Part<N>::size * d.K + k,
-                                                         (size_t)d.K)));
+            BATCH_SWITCH(d.n, {
+                SmemAcc<N> accH{sacc + lane}, accS{sacc + Part<N>::size * 32 + lane};
+                ok = grad_lane<N, double>(BraRef{d.bra + k, (size_t)d.K}, DevKetB{d.ket}, l0, l1, d.nst,
+                                          consts_of<N>(d), 1.0, d.scal[0],
+                                          d.part + (size_t)lc * Part<N>::size * d.K + k, (size_t)d.K, accH, accS);
+            });
             if (!ok) flag_inst(d.status, 1, k * d.K + l0);
         }
     }
@@ -410,7 +419,8 @@ __global__ void __launch_bounds__(256) batch_sum_kernel(PlanPtrs p) {
     }
 }
 
-__global__ void __launch_bounds__(128) batch_reduce_kernel(PlanPtrs p) {
+// GRADA of every instance: from its per-basis sums (FUSED) or from its gradient fields.
+template <bool FUSED> __global__ void __launch_bounds__(128) batch_reduce_kernel(PlanPtrs p) {
     const int ninst = p.hdr->ninst;
     const int total = p.pref_bra[ninst];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -419,7 +429,15 @@ __global__ void __launch_bounds__(128) batch_reduce_kernel(PlanPtrs p) {
         const int k = i - p.pref_bra[q];
         const double sc = d.scal[1] * d.C[k];
         bool fin = true;
-        BATCH_SWITCH(d.n, fin = grad_reduce_one<N>(d.part, 1, d.K, d.bra, sc, d.g, k));
+        if (FUSED) {
+            BATCH_SWITCH(d.n, {
+                double o[Part<N>::size];
+                finish_one<N>(d.part, d.K, d.bra, consts_of<N>(d), d.kmap.fold, k, o);
+                fin = fields_to_grad<N>(o, d.bra, d.K, sc, d.g, k);
+            });
+        } else {
+            BATCH_SWITCH(d.n, fin = grad_reduce_one<N>(d.part, 1, d.K, d.bra, sc, d.g, k));
+        }
         if (!fin) atomicOr(d.status, 2);
     }
 }
@@ -512,14 +530,15 @@ void launch_step(necg_batch *b, cudaStream_t st, int mode) {
         batch_rows_kernel<<<g * 4, 256, 0, st>>>(p);
         batch_finalize_kernel<<<g, 256, 0, st>>>(p);
         batch_fsum_kernel<<<g * 4, 256, 0, st>>>(p);
+        batch_reduce_kernel<true><<<g * 2, 128, 0, st>>>(p);
     } else {
         batch_energy_kernel<<<g * b->occ_energy, 32, 0, st>>>(p);
         batch_rows_kernel<<<g * 4, 256, 0, st>>>(p);
         batch_finalize_kernel<<<g, 256, 0, st>>>(p);
         batch_grad_kernel<<<g * b->occ_grad, 32, 0, st>>>(p);
         batch_sum_kernel<<<g * 4, 256, 0, st>>>(p);
+        batch_reduce_kernel<false><<<g * 2, 128, 0, st>>>(p);
     }
-    batch_reduce_kernel<<<g * 2, 128, 0, st>>>(p);
     batch_status_kernel<<<1, 256, 0, st>>>(p);
 }
 
@@ -614,7 +633,7 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
     std::vector<double> fcost(count > 0 ? count : 1, 0.0);
     static const std::vector<long long> flops_fused = [] {
         std::vector<long long> v(kMaxN + 1, 0);
-        for (int n = 1; n <= kMaxN; ++n) v[n] = necg_term_flops(n, 3, nullptr);
+        for (int n = 1; n <= kMaxN; ++n) v[n] = necg_term_flops(n, 7, nullptr);
         return v;
     }();
     hp.pref_bra[0] = hp.pref_ket[0] = hp.pref_sum[0] = 0;
@@ -661,7 +680,7 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
             d.pinv = h->d_pinv;
             d.stile_start = h->d_stile_start;
             d.psym = h->d_psym;
-            d.kmap = KetMap{h->d_kcnt, h->d_ksrc, h->d_kcoef, h->kmaxnz};
+            d.kmap = RawMap{h->d_kcnt, h->d_ksrc, h->d_kcoef, h->kmaxnz, h->kfold};
             d.stiles = h->d_stiles;
             d.bgroups = h->d_bgroups;
             d.nbgroups = h->nbgroups;
@@ -678,7 +697,7 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
             fcost[q] = (double)flops_fused[n] * h->nst * d.lc_s;
             continue;
         }
-        const long long fe = necg_term_flops(n, 0, nullptr), fg = necg_term_flops(n, 1, nullptr);
+        const long long fe = necg_term_flops(n, 4, nullptr), fg = necg_term_flops(n, 5, nullptr);
         for (int kb = 0; kb < nkb; ++kb)
             for (int lc = 0; lc * d.lc_e <= kb * 32 + 31 && lc * d.lc_e < K; ++lc)
                 et.push_back({(double)fe * h->nst * d.lc_e, make_int4(q, kb, lc, 0)});

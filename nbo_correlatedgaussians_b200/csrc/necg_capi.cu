@@ -168,13 +168,12 @@ int ensure_tiles(necg_handle *h, int K, cudaStream_t st) {
 
 // Lower-triangle tiles of chunk LC for the symmetric pass, plus the first tile
 // of each 32-row block; the partial buffer grows here if this K and LC need more.
-// mult = 2 for the fused pass (H and S partials kept apart), 1 otherwise; the
-// fused pass with npc splits needs npc partial slots per tile and npc K x K
+// The fused pass with npc splits needs npc partial slots per tile and npc K x K
 // buffers for H and S.
-int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, int mult) {
+int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
     const int PS = necg::part_stride(h->n);
     const int gw = necg::fused_block_warps(h->minb_s);  // tiles per group of the lockstep-block pass
-    const int npc = mult == 2 ? necg::fused_splits(h) : 1;
+    const int npc = fused ? necg::fused_splits(h) : 1;
     const size_t hp_need = npc > 1 ? (size_t)npc * K * K : 0;
     if (hp_need > h->hp_cap) {
         pool_free(h, h->d_Hp, st);
@@ -188,7 +187,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, int mult) {
         h->hp_cap = hp_need;
     }
     if (h->stiles_K == K && h->stiles_lc == h->lc_s && h->sgroups_w == gw &&
-        (size_t)h->nstiles * PS * (32 + h->lc_s) * mult * npc <= h->psym_cap)
+        (size_t)h->nstiles * PS * (32 + h->lc_s) * 2 * npc <= h->psym_cap)
         return NECG_OK;
     std::vector<int2> t;
     std::vector<int> start;
@@ -206,7 +205,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, int mult) {
         h->stiles_cap = (int)t.size();
     }
     if (!h->d_stile_start) CK(pool_alloc(h, &h->d_stile_start, ((h->K_max + 31) / 32 + 2) * sizeof(int), st));
-    const size_t need = t.size() * (size_t)PS * (32 + LC) * mult * npc;
+    const size_t need = t.size() * (size_t)PS * (32 + LC) * 2 * npc;
     if (need > h->psym_cap) {
         pool_free(h, h->d_psym, st);
         h->d_psym = nullptr;
@@ -312,7 +311,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, int mult) {
 int necg::prepare_fused(necg_handle *h, int K, cudaStream_t st) {
     if (!h || !h->sym_ok) return NECG_ERR_UNSUPPORTED;
     CK(cudaSetDevice(h->device));
-    return ensure_sym_tiles(h, K, st, 2);
+    return ensure_sym_tiles(h, K, st, true);
 }
 
 namespace {
@@ -343,8 +342,21 @@ int setup_symmetric(necg_handle *h) {
         }
     for (int p = 0; p < nst; ++p)
         if (pinv[p] < 0) return NECG_OK;  // not closed under inverse: ordered pass only
-    const int T = n * (n + 1) / 2, PS = T + 1 + m;
-    std::vector<std::vector<std::pair<int, double>>> rows((size_t)nst * PS);
+    // e' = A' s' maps as e = A s does when each shift map is that of its coordinate
+    // map, sms = kron(sml^-1, I3), i.e. sms kron(sml, I3) = 1; the kets' raw sums
+    // are then mapped and summed as they are, else folded in P's frame first
+    bool fold = false;
+    for (int p = 0; p < nst && !fold; ++p)
+        for (int r = 0; r < m && !fold; ++r)
+            for (int j = 0; j < n && !fold; ++j)
+                for (int c = 0; c < 3 && !fold; ++c) {  // column (j, c) of sms kron(sml, I3)
+                    double v = 0.0;
+                    for (int k = 0; k < n; ++k) v += h->sms[(size_t)p * m * m + r * m + 3 * k + c] * h->sml[(size_t)p * n * n + k * n + j];
+                    fold = fabs(v - (r == 3 * j + c ? 1.0 : 0.0)) > 1e-12;
+                }
+    const int T = n * (n + 1) / 2, SL = necg::ket_slots(n);
+    std::vector<std::vector<std::pair<int, double>>> rows((size_t)nst * SL);
+    auto slot = [n](int f) { return necg::ket_slot(n, f); };
     for (int p = 0; p < nst; ++p) {
         const double *P = &h->sml[(size_t)p * n * n];
         const double *Sm = &h->sms[(size_t)p * m * m];
@@ -353,15 +365,20 @@ int setup_symmetric(necg_handle *h) {
                 std::vector<double> coef(T, 0.0);
                 for (int cc = 0; cc < n; ++cc)
                     for (int d = 0; d < n; ++d) coef[necg::sx(cc, d)] += P[a * n + cc] * P[b * n + d];
-                auto &row = rows[(size_t)p * PS + necg::sx(a, b)];
+                auto &row = rows[(size_t)p * SL + slot(necg::sx(a, b))];
                 for (int s = 0; s < T; ++s)
-                    if (coef[s] != 0.0) row.push_back({s, coef[s]});
+                    if (coef[s] != 0.0) row.push_back({slot(s), coef[s]});
             }
-        rows[(size_t)p * PS + T].push_back({T, 1.0});
-        for (int r = 0; r < m; ++r) {  // (sms^T g')_r
-            auto &row = rows[(size_t)p * PS + T + 1 + r];
-            for (int cc = 0; cc < m; ++cc)
-                if (Sm[cc * m + r] != 0.0) row.push_back({T + 1 + cc, Sm[cc * m + r]});
+        rows[(size_t)p * SL + slot(T)].push_back({slot(T), 1.0});
+        for (int r = 0; r < m; ++r) {
+            auto &row = rows[(size_t)p * SL + slot(T + 1 + r)];
+            if (fold) {  // dF/ds: (sms^T g')_r
+                for (int cc = 0; cc < m; ++cc)
+                    if (Sm[cc * m + r] != 0.0) row.push_back({slot(T + 1 + cc), Sm[cc * m + r]});
+            } else {  // dF/de: (sml g')_r
+                for (int k = 0; k < n; ++k)
+                    if (P[(r / 3) * n + k] != 0.0) row.push_back({slot(T + 1 + 3 * k + r % 3), P[(r / 3) * n + k]});
+            }
         }
     }
     int maxnz = 1;
@@ -388,6 +405,7 @@ int setup_symmetric(necg_handle *h) {
     CK(cudaMemcpyAsync(h->d_kcoef, coef.data(), coef.size() * sizeof(double), cudaMemcpyHostToDevice, ls));
     CK(cudaStreamSynchronize(ls));  // the host vectors above end with this scope
     h->kmaxnz = maxnz;
+    h->kfold = fold ? 1 : 0;
     h->sym_ok = true;
     h->grad_mode = 1;
     return NECG_OK;
@@ -419,12 +437,17 @@ LaunchArgs base_args(necg_handle *h, int K) {
     a.status = h->d_status;
     a.lam = 1.0;
     a.pinv = h->d_pinv;
-    a.kmap = necg::KetMap{h->d_kcnt, h->d_ksrc, h->d_kcoef, h->kmaxnz};
+    a.kmap = necg::RawMap{h->d_kcnt, h->d_ksrc, h->d_kcoef, h->kmaxnz, h->kfold};
+    a.minb_s = h->minb_s;
+    return a;
+}
+
+// The tile lists and buffers of the symmetric passes, as ensure_sym_tiles left them.
+void sym_args(const necg_handle *h, LaunchArgs &a) {
     a.stiles = h->d_stiles;
     a.stile_start = h->d_stile_start;
     a.nstiles = h->nstiles;
     a.LC_s = h->lc_s;
-    a.minb_s = h->minb_s;
     a.psym = h->d_psym;
     a.sgroups = h->d_sgroups;
     a.nsgroups = h->nsgroups;
@@ -434,7 +457,6 @@ LaunchArgs base_args(necg_handle *h, int K) {
     a.sg_ntail = h->sg_ntail;
     a.sg_parts = h->sg_parts;
     a.urange = h->d_urange;
-    return a;
 }
 
 // The gradient passes after E and norm are in scal: symmetric (unordered pairs)
@@ -443,13 +465,9 @@ LaunchArgs base_args(necg_handle *h, int K) {
 // symmetric pass alone is used.)
 int launch_gradient(necg_handle *h, LaunchArgs &a, cudaStream_t st) {
     if (h->grad_mode >= 1) {
-        int rc = ensure_sym_tiles(h, a.K, st, h->grad_mode == 2 ? 2 : 1);
+        int rc = ensure_sym_tiles(h, a.K, st, h->grad_mode == 2);
         if (rc) return rc;
-        a.stiles = h->d_stiles;
-        a.stile_start = h->d_stile_start;
-        a.nstiles = h->nstiles;
-        a.LC_s = h->lc_s;
-        a.psym = h->d_psym;
+        sym_args(h, a);
         mark(h, 3, st);
         necg::launch_gsym(a, st);
         mark(h, 4, st);
@@ -564,7 +582,7 @@ int necg_create(int n, int nst, int K_max, double efs, const double *mass_host,
     if (!rc) rc = dalloc(h, &h->d_scvv, (size_t)nst);
     if (!rc) rc = dalloc(h, &h->d_bra, (size_t)necg::bra_record_size(n) * K);
     if (!rc) rc = dalloc(h, &h->d_ket, (size_t)necg::ket_record_size(n) * K * nst);
-    if (!rc) rc = dalloc(h, &h->d_part, (size_t)necg::part_stride(n) * K * ((K + 3) / 4));
+    if (!rc) rc = dalloc(h, &h->d_part, necg::part_doubles(n, K_max));
     if (!rc) rc = dalloc(h, &h->d_H, K * K);
     if (!rc) rc = dalloc(h, &h->d_S, K * K);
     if (!rc) rc = dalloc(h, &h->d_rows, 2 * K);
@@ -688,25 +706,13 @@ int necg_outprod(necg_handle *h, int K, const double *x_dev, double *f_dev, doub
     a.H = H_dev ? H_dev : h->d_H;
     a.S = S_dev ? S_dev : h->d_S;
     a.g = g_dev;
-    if (h->grad_mode >= 1 && (rc = ensure_sym_tiles(h, K, st, h->grad_mode == 2 ? 2 : 1))) return rc;
+    if (h->grad_mode >= 1 && (rc = ensure_sym_tiles(h, K, st, h->grad_mode == 2))) return rc;
     if (fused) {
         // fused: one pass over unordered pairs writes H, S and the split gradients
-        a.stiles = h->d_stiles;
-        a.stile_start = h->d_stile_start;
-        a.nstiles = h->nstiles;
-        a.LC_s = h->lc_s;
-        a.psym = h->d_psym;
-        a.sgroups = h->d_sgroups;
-        a.nsgroups = h->nsgroups;
-        a.qcount = h->d_qcount;
+        sym_args(h, a);
         a.npc = necg::fused_splits(h);
         a.Hp = h->d_Hp;
         a.Sp = h->d_Sp;
-        a.xsym = h->d_xsym;
-        a.sg_tail0 = h->sg_tail0;
-        a.sg_ntail = h->sg_ntail;
-        a.sg_parts = h->sg_parts;
-        a.urange = h->d_urange;
         // A call that repeats the previous call's buffers, K and settings
         // replays the captured launch sequence (captured the second time the
         // same key is seen, so callers whose buffers change every call stay
@@ -743,7 +749,7 @@ int shard_args(necg_handle *h, int K, const double *x_dev, int t0, int t1, cudaS
     if (!x_dev) return NECG_ERR_ARG;
     if (!h->sym_ok) return NECG_ERR_UNSUPPORTED;
     CK(cudaSetDevice(h->device));
-    if ((rc = ensure_sym_tiles(h, K, st, 2))) return rc;
+    if ((rc = ensure_sym_tiles(h, K, st, true))) return rc;
     if (t0 < 0 || t1 < t0 || t1 > h->nstiles) return NECG_ERR_ARG;
     a = base_args(h, K);
     const size_t siv = (size_t)K * (h->n * (h->n + 1) / 2 + 3 * h->n);
@@ -751,11 +757,7 @@ int shard_args(necg_handle *h, int K, const double *x_dev, int t0, int t1, cudaS
     a.C = x_dev + siv;
     a.H = h->d_H;
     a.S = h->d_S;
-    a.stiles = h->d_stiles;
-    a.stile_start = h->d_stile_start;
-    a.nstiles = h->nstiles;
-    a.LC_s = h->lc_s;
-    a.psym = h->d_psym;
+    sym_args(h, a);
     a.st_begin = t0;
     a.st_end = t1;
     return NECG_OK;
@@ -768,7 +770,7 @@ int necg_shard_tiles(necg_handle *h, int K, int *ntiles) {
     if (rc) return rc;
     if (!h->sym_ok) return NECG_ERR_UNSUPPORTED;
     CK(cudaSetDevice(h->device));
-    if ((rc = ensure_sym_tiles(h, K, h->last_stream, 2))) return rc;
+    if ((rc = ensure_sym_tiles(h, K, h->last_stream, true))) return rc;
     *ntiles = h->nstiles;
     return NECG_OK;
 }
@@ -936,7 +938,7 @@ int necg_dipole(necg_handle *h, int K, const double *iv_dev, const double *C_dev
     LaunchArgs a = base_args(h, K);
     // the tile partials reuse the gradient-partial workspace
     const size_t need = (size_t)a.ntiles * (3 * h->n + 1);
-    const size_t cap = (size_t)necg::part_stride(h->n) * h->K_max * ((h->K_max + 3) / 4);
+    const size_t cap = necg::part_doubles(h->n, h->K_max);
     if (need > cap) return NECG_ERR_CAPACITY;
     a.iv = iv_dev;
     a.C = C_dev;

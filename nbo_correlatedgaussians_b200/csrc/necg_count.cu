@@ -1,12 +1,16 @@
-// necg_count.cu -- algorithmic FP64 operation count of one (k, l, P) term.
+// necg_count.cu -- FP64 operation counts of one (k, l, P) term.
 //
-// The term templates of necg_math.cuh are instantiated on the host with a
-// counting scalar: every add, subtract and multiply counts 1 (so a fused
-// multiply-add counts 2), every division, square root, reciprocal square root
-// and exponential counts 1 in a separate "special" tally.  Negation and
-// comparisons are free.  The count follows the Pade branch of F0 (the branch
-// all pairs of the synthetic workloads take) and excludes the per-basis and
-// per-(l, P) preparation, which is amortised over K terms.
+// Two measures.  `which` 0 .. 3 (energy, ordered gradient, symmetric, fused): the
+// direct formulation, in which every term forms its own complete bra and ket
+// gradients -- a fixed measure of a term's work, by which rates are quoted and
+// compared across versions of the kernels.  `which` 4 .. 7: what the kernels
+// execute per term, from the term templates of necg_math.cuh instantiated on the
+// host with a counting scalar (every add, subtract and multiply counts 1, so a
+// fused multiply-add counts 2; every division, square root, reciprocal,
+// reciprocal square root and exponential counts 1 in a separate "special"
+// tally; negation and comparisons are free).  They take fewer, because what
+// depends on one basis function alone multiplies its sums over all terms.
+// Both exclude the per-basis and per-(l, P) work, which is amortised over K terms.
 #include <math.h>
 #include <stdlib.h>
 
@@ -32,10 +36,10 @@ template <int N> void host_records(std::vector<double> &bra, std::vector<double>
         }
     for (int t = 0; t < tri(N); ++t) {
         bra[BL::A + t] = A[t];
-        bra[BL::Nk + t] = 0.5 * A[t];
+        bra[BL::N8 + t] = -4.0 * A[t];
         bra[BL::L + t] = A[t];
         ket[KL::Ap + t] = Ap[t];
-        ket[KL::Np + t] = 0.5 * Ap[t];
+        ket[KL::Np8 + t] = -4.0 * Ap[t];
     }
     for (int t = 0; t < 3 * N; ++t) {
         bra[BL::S + t] = 0.01 * (t + 1);
@@ -43,7 +47,6 @@ template <int N> void host_records(std::vector<double> &bra, std::vector<double>
         ket[KL::Sp + t] = -0.01 * (t + 2);
         ket[KL::ASp + t] = -0.015 * (t + 2);
     }
-    for (int t = 0; t < N * N; ++t) ket[KL::AMn4 + t] = -0.04 * t;
     bra[BL::i1] = 0.01;
     bra[BL::pre] = 1.0;
     bra[BL::tMA] = 2.0;
@@ -55,25 +58,32 @@ template <int N> void host_records(std::vector<double> &bra, std::vector<double>
     ket[KL::winv] = 1.0;
 }
 
-// Ket-side output of one term: put stores, add accumulates (one add counted).
-struct CountRow {
-    double r[64];
-    void put(int f, CD v) { r[f] = v.v; }
-    void add(int f, CD v) {
-        r[f] += v.v;
-        ++count_ctx().flops;
+// A term's output as the passes take it: the weighted raw values added to the
+// bra's sums and, with KET, scaled for the ket (S too, unless KE).  The ket's
+// sum over the warp is counted per (l, P), not per term.
+template <int N, bool KET, bool KE> struct CountOut {
+    CD acc[2][64], ket[2][64], wb = CD(1.0), wk = CD(1.0), wob, wok;
+    void begin(CD ov) {
+        wob = wb * ov;
+        if (KET) wok = wk * ov;
     }
-};
-// The fused pass's ket output: the H and S values of one field together.
-struct CountRow2 {
-    CountRow h, s;
-    void put(int f, CD vh, CD vs) {
-        h.put(f, vh);
-        s.put(f, vs);
+    void put(int m, int f, CD v) {
+        acc[m][f] += wob * v;
+        if (KET && !(KE && m)) ket[m][f] = wok * v;
     }
-    void add(int f, CD vh, CD vs) {
-        h.add(f, vh);
-        s.add(f, vs);
+    void s1(int f, CD v) { put(1, f, v); }
+    void h1(int f, CD v) { put(0, f, v); }
+    void s2(int, int fa, int fb, CD va, CD vb) {
+        put(1, fa, va);
+        put(1, fb, vb);
+    }
+    void h2(int, int fa, int fb, CD va, CD vb) {
+        put(0, fa, va);
+        put(0, fb, vb);
+    }
+    void scalar(CD e2) {
+        put(0, tri(N), e2);
+        acc[1][tri(N)] += wob;
     }
 };
 
@@ -98,28 +108,20 @@ template <int N> void count_term(int which, long long &flops, long long &special
         h += w * ov * (2.0 * tau + rho - sig);
         s += w * ov;
     } else if (which == 1) {
-        RegAcc<N, CD> acc;
-        acc.zero();
-        count_ctx() = CountCtx();  // zeroing the accumulators is not part of a term
-        term_grad<N>(b, kr, cs, CD(1.0), CD(0.5), CD(1.0), acc);
+        CountOut<N, false, false> out;
+        CD eta2, ov;
+        term_raw<N>(b, kr, cs, CD(0.0), out, eta2, ov);
     } else if (which == 2) {
-        RegAcc<N, CD> acc;
-        acc.zero();
-        CountRow ko;
-        count_ctx() = CountCtx();
-        // the ket row's warp column sum and frame map are counted per (l, P),
-        // not per term: they are amortised over the 32 bras of a tile
-        term_sym<N>(b, kr, cs, CD(0.5), CD(1.0), CD(1.0), acc, ko);
+        CountOut<N, true, true> out;
+        CD eta2, ov;
+        term_raw<N>(b, kr, cs, CD(0.5), out, eta2, ov);
     } else {
-        RegAcc<N, CD> aH, aS;
-        aH.zero();
-        aS.zero();
-        CountRow2 ko;
-        count_ctx() = CountCtx();
-        CD h, ov, hs(0.0), ss(0.0), w(1.0);
-        term_fused<N>(b, kr, cs, CD(1.0), CD(1.0), aH, aS, ko, h, ov);
-        hs += w * h;  // the pass's sums of w_P h and w_P ov over P
-        ss += w * ov;
+        CountOut<N, true, false> out;
+        CD eta2, ov, hs(0.0), ss(0.0), w(1.0);
+        term_raw<N>(b, kr, cs, CD(0.0), out, eta2, ov);
+        const CD wo = w * ov;  // the pass's sums of w_P h and w_P ov over P
+        hs += wo * eta2;
+        ss += wo;
     }
     flops = count_ctx().flops;
     special = count_ctx().special;
@@ -127,16 +129,27 @@ template <int N> void count_term(int which, long long &flops, long long &special
 
 }  // namespace necg
 
+namespace {
+// direct formulation: total operations (special ones included) by n and which;
+// the special ones are two per Coulomb pair, one per Cholesky pivot and the exponential
+const int kDirect[6][4] = {{93, 201, 253, 281},      {249, 585, 743, 795},     {496, 1206, 1547, 1626},
+                           {819, 2067, 2686, 2795}, {1254, 3222, 4232, 4374}, {1795, 4683, 6215, 6393}};
+}  // namespace
+
 extern "C" long long necg_term_flops(int n, int which, long long *special) {
     long long f = 0, s = 0;
+    if (n < 1 || n > 6 || which < 0 || which > 7) return -1;
+    if (which < 4) {
+        if (special) *special = n * (n + 1) + n + 1;
+        return kDirect[n - 1][which];
+    }
     switch (n) {
-    case 1: necg::count_term<1>(which, f, s); break;
-    case 2: necg::count_term<2>(which, f, s); break;
-    case 3: necg::count_term<3>(which, f, s); break;
-    case 4: necg::count_term<4>(which, f, s); break;
-    case 5: necg::count_term<5>(which, f, s); break;
-    case 6: necg::count_term<6>(which, f, s); break;
-    default: return -1;
+    case 1: necg::count_term<1>(which - 4, f, s); break;
+    case 2: necg::count_term<2>(which - 4, f, s); break;
+    case 3: necg::count_term<3>(which - 4, f, s); break;
+    case 4: necg::count_term<4>(which - 4, f, s); break;
+    case 5: necg::count_term<5>(which - 4, f, s); break;
+    default: necg::count_term<6>(which - 4, f, s); break;
     }
     if (special) *special = s;
     return f + s;

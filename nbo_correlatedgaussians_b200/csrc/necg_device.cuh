@@ -62,29 +62,118 @@ struct TileOut {
     int slot = -1;
 };
 
-// Shared memory of one warp's fused tile: bra accumulators for H and S
-// (2 * PS * 32 doubles), two ket tables of 16 rows (2 * 16 * 33) and two
-// reduction rows (64).  Sized by the caller for its largest n.
+// Doubles of a warp's ket tables (16 rows) in the fused pass (MATS = 2: H and S)
+// or the symmetric pass (MATS = 1: the combined gradient).
+template <int N> __host__ __device__ constexpr int ket_table(int mats) { return 16 * (mats * KetSlots<N>::SL + 1); }
+
+// Shared memory of one warp's tile: bra accumulators (2 * PS * 32 doubles), the
+// ket table (ket_table) and the reduced ket fields (64).  Sized by the caller
+// for its largest n.
 struct FusedSmem {
     double *sacc, *krow, *kred;
     double *sket;  // SKET: two ket-record buffers of this warp (16-byte aligned)
 };
 
-// One tile of the fused pass over unordered pairs (k >= l): the symmetric
-// gradient pass merged with the energy pass.  Each term gives the H element and
-// overlap (summed over P into H_kl = H_lk and S_kl = S_lk) and the bra and ket
-// gradients of h and of ov kept apart, since E is not known until finalize
-// has run on the H and S this pass writes; the partial sum combines them as
-// g_H - E g_S.  Tile t = (kb, lc): bras k = 32 kb + lane, kets l in
-// [lc LC, lc LC + LC).  Bra partials: part_b[((t * 2 + which) * PS + f) * 32 +
-// lane]; ket partials: part_k[((t * LC + l - l0) * 2 + which) * PS + f], which
-// = 0 for H and 1 for S.
+// term_raw's output in a tile: the weighted raw values are added to the lane's
+// bra accumulators and, for the ket, summed over lane pairs into the warp's
+// table.  Lanes 2i and 2i+1 exchange one value per pair of fields: lane 2i keeps
+// the first field, lane 2i+1 the second, each adds its partner's, and both store
+// to row i (one select-and-shuffle per two fields, and half the rows to sum).
+// KE (E known): the S fields go to the bra only, and H's are the combined ones.
+template <int N, bool KE> struct TileOutput {
+    using RP = RawPairs<N>;
+    static constexpr int PS = Part<N>::size, SL = KetSlots<N>::SL;
+    double *acc;  // this lane's accumulators: H fields, then S fields, 32 doubles apart
+    double *row;  // the lane pair's row, + 8 for the odd lane
+    bool odd;
+    double wb, wk, wob, wok;
+    __device__ __forceinline__ void begin(double ov) {
+        wob = wb * ov;
+        wok = wk * ov;
+    }
+    __device__ __forceinline__ void bra(int f, double v) { acc[f * 32] = fma(wob, v, acc[f * 32]); }
+    __device__ __forceinline__ void exchange(int slot, double va, double vb) {
+        const double send = wok * (odd ? va : vb);
+        row[slot] = fma(wok, odd ? vb : va, __shfl_xor_sync(0xffffffffu, send, 1));
+    }
+    __device__ __forceinline__ void s2(int i, int fa, int fb, double va, double vb) {
+        bra(PS + fa, va);
+        bra(PS + fb, vb);
+        if (!KE) exchange(SL + KetSlots<N>::of_pair(i), va, vb);
+    }
+    __device__ __forceinline__ void h2(int i, int fa, int fb, double va, double vb) {
+        bra(fa, va);
+        bra(fb, vb);
+        exchange(KetSlots<N>::of_pair(i), va, vb);
+    }
+    __device__ __forceinline__ void scalar(double e2) {
+        constexpr int p = KetSlots<N>::of_pair(RP::count - 1);
+        bra(RP::scalar, e2);
+        acc[(PS + RP::scalar) * 32] += wob;
+        if (KE) {
+            const double v = wok * e2;  // the odd lane's copy lands in an unused slot
+            row[p] = v + __shfl_xor_sync(0xffffffffu, v, 1);
+        } else {  // the even lane keeps H's scalar, the odd one S's
+            const double vh = wok * e2, send = odd ? vh : wok;
+            row[odd ? SL + p - 8 : p] = (odd ? wok : vh) + __shfl_xor_sync(0xffffffffu, send, 1);
+        }
+    }
+    __device__ __forceinline__ void s1(int, double) {}  // n = 6 has no symmetric passes
+    __device__ __forceinline__ void h1(int, double) {}
+};
+
+// One field of fold_raw at run time, from the reduced slots of one matrix (scale 1
+// for H and the combined gradient, 2 for S).
+template <int N>
+__device__ __noinline__ double fold_slot(const double *slots, double scale, int f, const double *kr) {
+    using KL = KetLayout<N>;
+    constexpr int TR = tri(N);
+    auto r = [&](int q) {
+        double v = 0.0;
+#pragma unroll
+        for (int u = 0; u < Part<N>::size; ++u)
+            if (u == q) v = slots[KetSlots<N>::slot(u)];
+        return scale * v;
+    };
+    const double F = 0.5 * r(TR);
+    if (f == TR) return 0.75 * F;
+    if (f < TR) {
+        int i = 0;
+        while ((i + 1) * (i + 2) / 2 <= f) ++i;
+        const int j = f - i * (i + 1) / 2;
+        double v = r(f);
+        for (int c = 0; c < 3; ++c) {
+            const double si = kr[KL::Sp + 3 * i + c], sj = kr[KL::Sp + 3 * j + c];
+            v += r(TR + 1 + 3 * i + c) * sj + si * r(TR + 1 + 3 * j + c) - 2.0 * F * si * sj;
+        }
+        return 0.5 * v;
+    }
+    const int i = (f - TR - 1) / 3, c = (f - TR - 1) - 3 * i;
+    double v = -2.0 * F * kr[KL::ASp + 3 * i + c];
+    for (int k = 0; k < N; ++k) v += kr[KL::Ap + (i >= k ? i * (i + 1) / 2 + k : k * (k + 1) / 2 + i)] * r(TR + 1 + 3 * k + c);
+    return v;
+}
+
+// One tile of the pair passes over unordered pairs (k >= l).  Each term gives
+// the raw values of term_raw (h, ov and their derivatives with respect to B and
+// e, the same for the bra and the ket); the bra's weighted sums stay in the
+// lane's accumulators, the ket's are summed over the warp per (l, P), mapped to
+// l's frame and summed over P.
+//   !KE, the fused pass: H_kl = H_lk and S_kl are the sums over P of h and ov;
+//        the H and S fields are kept apart, since E is not known until finalize
+//        has run on the H and S this pass writes.
+//   KE, the symmetric gradient pass (E = Egiven known): the combined gradient
+//        of h - E ov, and the S fields for the bra only (its explicit share).
+// Tile t = (kb, lc): bras k = 32 kb + lane, kets l in [lc LC, lc LC + LC).  Bra
+// partials: part_b[((t * 2 + which) * PS + f) * 32 + lane]; ket partials:
+// part_k[((t * LC + l - l0) * 2 + which) * PS + f], which = 0 for H (or the
+// combined gradient) and 1 for S (not written for the ket when KE).
 //
-// Shared memory per warp must stay under 228 KB / 8 for 8 resident warps: the
-// ket rows of two lanes are added with one shuffle before they are written,
-// so each of the two ket tables has 16 rows.  The shuffles need the whole warp,
-// so every lane evaluates a term: a lane without a pair (l > k, or k >= K)
-// evaluates the finite pair (l, l, P) with zero weights, which adds nothing.
+// Shared memory per warp must stay under 228 KB / 8 for 8 resident warps, so the
+// ket rows of two lanes are added before they are written (TileOutput) and the
+// table has 16 rows.  The shuffles need the whole warp, so every lane evaluates a
+// term: a lane without a pair (l > k, or k >= K) evaluates the finite pair
+// (l, l, P) with zero weights, which adds nothing.
 // VKET: ket records re-read at each use (fewer live registers).
 // BSYNC: the warps of a block step through their tiles' terms together (a
 // block barrier after every (l, P) term, so the warps sharing a scheduler
@@ -104,51 +193,51 @@ struct FusedSmem {
 // accumulators, left in sm.sacc, itself).
 // SYNC (with BSYNC): 0 -- every warp takes the block barrier at the end of
 // each term; 1, 2 -- warps 4-7 of the block take it inside the term instead
-// (at term_fused's mid(1): after B, Bi, T and ov; mid(2): after tau and sig),
+// (at term_raw's mid(1): after B, Bi, T and ov; mid(2): before the Coulomb sum),
 // so the two warps of each scheduler run different stretches of the body; 3 --
 // no barrier per term (the warps only meet at the tile group's barriers).
-template <int N, bool VKET, bool BSYNC = false, bool SBRA = false, bool SKET = false, int SYNC = 0, bool WB = true>
+template <int N, bool VKET, bool BSYNC = false, bool SBRA = false, bool SKET = false, int SYNC = 0, bool WB = true,
+          bool KE = false>
 __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst, const Consts<N> &cs,
                                           const double *__restrict__ bra, const double *__restrict__ ket,
-                                          const double *__restrict__ C, const KetMap &kmap,
+                                          const double *__restrict__ C, const RawMap &kmap,
                                           double *__restrict__ H, double *__restrict__ S,
                                           double *__restrict__ part_b, double *__restrict__ part_k,
                                           int *status, FusedSmem sm, bool idle = false,
                                           const double *sbra = nullptr, int p0 = 0, int p1 = -1,
-                                          TileOut xo = TileOut{}) {
+                                          TileOut xo = TileOut{}, double Egiven = 0.0) {
     using KL = KetLayout<N>;
-    constexpr int PS = Part<N>::size;
-    static_assert(PS <= 32, "the symmetric pass needs tri(n) + 1 + 3n <= 32");
+    constexpr int PS = Part<N>::size, SL = KetSlots<N>::SL;
+    constexpr int COLS = (KE ? 1 : 2) * SL;         // 16, 32 or 64 ket slots per row
+    constexpr int STRIDE = COLS + 1;
+    constexpr int NC = COLS > 32 ? 2 : 1;           // slots per lane
+    static_assert(PS <= 32 && SL <= 32, "the symmetric passes need tri(n) + 1 + 3n <= 32");
     // a barrier inside the term is taken only on the path that passes mid to
-    // term_fused; anywhere else the warps' barrier counts would not match
+    // term_raw; anywhere else the warps' barrier counts would not match
     static_assert(SYNC == 0 || SYNC == 3 || (BSYNC && SBRA && SKET), "mid-term barriers need BSYNC, SBRA, SKET");
     const int lane = threadIdx.x & 31;
-    double *krow0 = sm.krow, *krow1 = sm.krow + 16 * 33, *kred = sm.kred;
+    double *krow = sm.krow, *kred = sm.kred;
     const int k = tl.x * 32 + lane;
     const int l0 = tl.y * LC;
     const int l1 = BSYNC ? l0 + LC : min(l0 + LC, K);
     const bool kval = k < K && !idle;
     const double Ck = kval ? C[k] : 0.0;
-    SmemAcc<N> accH{sm.sacc + lane}, accS{sm.sacc + PS * 32 + lane};
-    accH.zero();
-    accS.zero();
-    // ket row output: lanes 2i and 2i+1 add their values of field f with one
-    // exchange, lane 2i the H values (into row i of the H table), lane 2i+1 the
-    // S values (row i of the S table)
-    struct PairOut {
-        double *r;
-        bool odd;
-        __device__ __forceinline__ double sum(double vh, double vs) const {
-            const double keep = odd ? vs : vh;
-            return keep + __shfl_xor_sync(0xffffffffu, odd ? vh : vs, 1);
-        }
-        __device__ __forceinline__ void put(int f, double vh, double vs) { r[f] = sum(vh, vs); }
-        __device__ __forceinline__ void add(int f, double vh, double vs) { r[f] += sum(vh, vs); }
-    } ko{((lane & 1) ? krow1 : krow0) + (lane >> 1) * 33, (lane & 1) != 0};
+#pragma unroll
+    for (int f = 0; f < 2 * PS; ++f) sm.sacc[f * 32 + lane] = 0.0;
+    TileOutput<N, KE> out{sm.sacc + lane, krow + (lane >> 1) * STRIDE + 8 * (lane & 1), (lane & 1) != 0,
+                          0.0, 0.0, 0.0, 0.0};
+    const double E2 = KE ? 2.0 * Egiven : 0.0;
+    // the slot this lane sums, maps and writes: js of matrix `which` (NC = 2: of both)
+    const int js = lane & (SL - 1), which = NC == 2 ? 0 : lane / SL;
+    int fld = -1;  // its field
+#pragma unroll
+    for (int f = 0; f < PS; ++f)
+        if (KetSlots<N>::slot(f) == js) fld = f;
+    const bool mine = fld >= 0 && lane < COLS;
     bool ok = true;
     int flags = 0, bad = 0x7fffffff;  // smallest failing pair (row-major k K + l)
     // where this warp takes its per-term block barrier (BSYNC): 0 at the end of
-    // the term, 1 / 2 at term_fused's mid(1) / mid(2), -1 nowhere.  Every warp
+    // the term, 1 / 2 at term_raw's mid(1) / mid(2), -1 nowhere.  Every warp
     // takes exactly one barrier per (l, P) term, or none (SYNC 3).
     const int sync_at = !BSYNC || SYNC == 3 ? -1 : SYNC == 0 || !((threadIdx.x >> 7) & 1) ? 0 : SYNC;
     struct MidSync {
@@ -164,11 +253,13 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
     int cur = 0;  // SKET: the buffer that holds the current term's record
     if constexpr (SKET) {
         if (l0 < l1 && p0 < pend && has_work(l0))
-            ket_fetch(sm.sket, ket + ((size_t)l0 * nst + p0) * KL::size, KL::size, lane);
+            ket_fetch(sm.sket, ket + ((size_t)l0 * nst + p0) * KL::size, KL::term, lane);
     }
     for (int l = l0; l < l1; ++l) {
         const bool lok = has_work(l);
-        double aH = 0.0, aS = 0.0, hsum = 0.0, ssum = 0.0;
+        double ak[NC], hsum = 0.0, ssum = 0.0;
+#pragma unroll
+        for (int q = 0; q < NC; ++q) ak[q] = 0.0;
         const bool active = kval && l <= k && lok;
         const BraRef b{bra + (active ? k : (lok ? l : 0)), (size_t)K};
         for (int P = p0; P < pend; ++P) {
@@ -185,68 +276,88 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
                     nP = p0;
                 }
                 if (nl < l1 && has_work(nl))
-                    ket_fetch(sm.sket + (cur ^ 1) * KL::size, ket + ((size_t)nl * nst + nP) * KL::size, KL::size,
+                    ket_fetch(sm.sket + (cur ^ 1) * KL::term, ket + ((size_t)nl * nst + nP) * KL::size, KL::term,
                               lane);
-                kr = sm.sket + cur * KL::size;
+                kr = sm.sket + cur * KL::term;
                 cur ^= 1;
             }
-            const double wb = active ? kr[KL::wC] : 0.0;
-            const double wk = active && l < k ? 2.0 * Ck * kr[KL::winv] : 0.0;
-            double h, ov;
+            out.wb = active ? kr[KL::wC] : 0.0;
+            out.wk = active && l < k ? 2.0 * Ck * kr[KL::winv] : 0.0;
+            double eta2, ov;
             bool tok;
             if constexpr (SBRA && SKET)
-                tok = term_fused<N, double>(BraSmem{sbra + lane}, KetSmem{kr}, cs, wb, wk, accH, accS, ko, h, ov,
-                                            mid);
+                tok = term_raw<N, double>(BraSmem{sbra + lane}, KetSmem{kr}, cs, E2, out, eta2, ov, mid);
             else if constexpr (SBRA)
-                tok = term_fused<N, double>(BraSmem{sbra + lane}, KetRefV{kr}, cs, wb, wk, accH, accS, ko, h, ov,
-                                            mid);
+                tok = term_raw<N, double>(BraSmem{sbra + lane}, KetRefV{kr}, cs, E2, out, eta2, ov, mid);
             else if constexpr (SKET)
-                tok = term_fused<N, double>(b, KetSmem{kr}, cs, wb, wk, accH, accS, ko, h, ov);
+                tok = term_raw<N, double>(b, KetSmem{kr}, cs, E2, out, eta2, ov);
             else if constexpr (VKET)
-                tok = term_fused<N, double>(b, KetRefV{kr}, cs, wb, wk, accH, accS, ko, h, ov);
+                tok = term_raw<N, double>(b, KetRefV{kr}, cs, E2, out, eta2, ov);
             else
-                tok = term_fused<N, double>(b, kr, cs, wb, wk, accH, accS, ko, h, ov);
+                tok = term_raw<N, double>(b, kr, cs, E2, out, eta2, ov);
             if (active) {
                 if (!tok && ok) {  // the first pair of this lane that is not positive definite
                     ok = false;
                     bad = min(bad, k * K + l);
                 }
-                const double w = kr[KL::w];
-                hsum += w * h;
-                ssum += w * ov;
+                if (!KE) {
+                    const double wo = kr[KL::w] * ov;
+                    hsum += wo * eta2;
+                    ssum += wo;
+                }
             }
             __syncwarp();
-            // the 16 rows of both ket tables, summed as trees (four dependent
-            // adds instead of sixteen), then mapped to l's frame together
-            if (lane < PS) {
-                double vh[16], vs[16];
+            // the 16 rows of the ket table, summed as trees (four dependent adds
+            // instead of sixteen), then mapped to l's frame
+            {
+                double v[NC][16];
 #pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    vh[r] = krow0[r * 33 + lane];
-                    vs[r] = krow1[r * 33 + lane];
-                }
+                for (int r = 0; r < 16; ++r)
+#pragma unroll
+                    for (int q = 0; q < NC; ++q) v[q][r] = krow[r * STRIDE + 32 * q + (COLS < 32 ? lane & (COLS - 1) : lane)];
 #pragma unroll
                 for (int w = 8; w >= 1; w >>= 1)
 #pragma unroll
-                    for (int r = 0; r < w; ++r) {
-                        vh[r] += vh[r + w];
-                        vs[r] += vs[r + w];
-                    }
-                kred[lane] = vh[0];
-                kred[32 + lane] = vs[0];
+                    for (int r = 0; r < w; ++r)
+#pragma unroll
+                        for (int q = 0; q < NC; ++q) v[q][r] += v[q][r + w];
+#pragma unroll
+                for (int q = 0; q < NC; ++q) kred[32 * q + lane] = v[q][0];
             }
             __syncwarp();
-            if (lane < PS) {
-                double mh, ms;
-                ket_map_apply2(kmap, P, lane, PS, kred, kred + 32, mh, ms);
-                aH += mh;
-                aS += ms;
+            if (kmap.fold) {  // gradients in P's frame instead of raw sums
+                const double *krg = ket + ((size_t)l * nst + P) * KL::size;
+                double v[NC];
+#pragma unroll
+                for (int q = 0; q < NC; ++q) {
+                    const int wq = which + q;
+                    v[q] = mine ? (wq ? 0.5 : 1.0) * fold_slot<N>(kred + wq * SL, wq ? 2.0 : 1.0, fld, krg) : 0.0;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < NC; ++q) kred[32 * q + lane] = v[q];
+                __syncwarp();
+            }
+            if (mine) {
+                const int e = P * SL + js, n = kmap.cnt[e];
+                double m[NC];
+#pragma unroll
+                for (int q = 0; q < NC; ++q) m[q] = 0.0;
+                for (int i = 0; i < n; ++i) {
+                    const double c = kmap.coef[(size_t)e * kmap.maxnz + i];
+                    const int s = kmap.src[(size_t)e * kmap.maxnz + i];
+#pragma unroll
+                    for (int q = 0; q < NC; ++q) m[q] += c * kred[(which + q) * SL + s];
+                }
+#pragma unroll
+                for (int q = 0; q < NC; ++q) ak[q] += m[q];
             }
             __syncwarp();
             if (BSYNC && sync_at == 0) cta_barrier();
         }
         if (BSYNC && !lok) continue;
-        if (active) {
+        if (!KE && active) {
+            hsum *= 0.5;
             if (!isfinite(hsum) || !isfinite(ssum)) {
                 bad = min(bad, k * K + l);
                 flags |= 2;
@@ -262,11 +373,11 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
                 S[(size_t)l * K + k] = ssum;
             }
         }
-        if (lane < PS) {
+        if (mine) {
             double *pk = xo.slot >= 0 ? xo.x + (size_t)xo.slot * fsym_tail_slot(PS, LC) + (size_t)(l - l0) * 2 * PS
                                       : part_k + ((size_t)t * LC + (l - l0)) * 2 * PS;
-            pk[lane] = aH;
-            pk[PS + lane] = aS;
+#pragma unroll
+            for (int q = 0; q < NC; ++q) pk[(which + q) * PS + fld] = ak[q];
         }
     }
     if (WB && kval) {
@@ -279,39 +390,37 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
     __syncwarp();
 }
 
-// Sum of the fused-pass partials of basis m for field f: its bra partials from
-// the tiles of block kb = m / 32 (lane m % 32) and its ket partials from the
-// tiles of chunk lc = m / LC in every block kb' >= that chunk; returns
-// sum_H - E sum_S.  Only tiles in [t0, t1) count (a shard of the pass).  With
-// the symmetry terms split npc ways, tile t's partials are slots t npc ..
-// t npc + npc - 1.
-template <int N>
-__device__ __forceinline__ double fsym_sum_one(const int *__restrict__ tstart, int LC, int K, int f, int m,
-                                               const double *__restrict__ part_b,
-                                               const double *__restrict__ part_k, double E, int t0 = 0,
-                                               int t1 = 0x7fffffff, int npc = 1) {
+// The ket partials of basis m for field f and matrix `which`: from the tiles of
+// chunk lc = m / LC in every row block q >= that chunk's, q = kb0 + seg, + nseg, ..
+// Only tiles in [t0, t1) count (a shard of the pass).  With the symmetry terms
+// split npc ways, tile t's partials are slots t npc .. t npc + npc - 1.
+template <int N, bool TWO>
+__device__ __forceinline__ void ket_partials(const int *__restrict__ tstart, int LC, int K, int f, int m,
+                                             const double *__restrict__ part_k, int t0, int t1, int npc, int seg,
+                                             int nseg, double &kH, double &kS) {
     constexpr int PS = Part<N>::size;
-    const int kb = m >> 5, lane = m & 31;
-    double sH = 0.0, sS = 0.0;
-    const int sa = max(tstart[kb], t0) * npc, sb = min(tstart[kb + 1], t1) * npc;
-    for (int t = sa; t < sb; ++t) {
-        sH += part_b[(((size_t)t * 2 + 0) * PS + f) * 32 + lane];
-        sS += part_b[(((size_t)t * 2 + 1) * PS + f) * 32 + lane];
-    }
     const int lc = m / LC, ll = m - lc * LC;
     const int nkb = (K + 31) >> 5;
     int kb0 = lc * LC - 31;
     kb0 = kb0 > 0 ? (kb0 + 31) >> 5 : 0;
-    for (int q = kb0; q < nkb; ++q) {
+    for (int q = kb0 + seg; q < nkb; q += nseg) {
         const int t = tstart[q] + lc;
         if (t < t0 || t >= t1) continue;
         for (int pc = 0; pc < npc; ++pc) {
             const size_t base = ((size_t)(t * npc + pc) * LC + ll) * 2;
-            sH += part_k[(base + 0) * PS + f];
-            sS += part_k[(base + 1) * PS + f];
+            kH += part_k[(base + 0) * PS + f];
+            if (TWO) kS += part_k[(base + 1) * PS + f];
         }
     }
-    return sH - E * sS;
+}
+
+// The per-basis sums (kSumSets sets of PS fields at out) of field f of basis m.
+__device__ __forceinline__ void put_sums(double *out, int PS, int K, int f, int m, double bH, double bS, double kH,
+                                         double kS, double E2, int folded) {
+    const double b = bH - E2 * bS, k = kH - E2 * kS;
+    out[(size_t)f * K + m] = folded ? b : b + k;
+    out[(size_t)(PS + f) * K + m] = bS;
+    if (folded) out[(size_t)(2 * PS + f) * K + m] = k;
 }
 
 }  // namespace necg

@@ -32,7 +32,7 @@ struct necg_handle {
     int *d_pinv = nullptr;
     int *d_kcnt = nullptr, *d_ksrc = nullptr;
     double *d_kcoef = nullptr;
-    int kmaxnz = 0;
+    int kmaxnz = 0, kfold = 0;  // the ket frame map (RawMap)
     int2 *d_stiles = nullptr;
     int *d_stile_start = nullptr;
     int stiles_cap = 0, stiles_K = -1, stiles_lc = -1, nstiles = 0;

@@ -169,10 +169,9 @@ __global__ void __launch_bounds__(1024) finalize_kernel(const double *__restrict
 
 // Gradient tiles over the full square of ordered pairs (the loop of
 // python/make_grad.py:37-55, contracted with C on the fly as lines 61-79 do).
-// Tile t = (kb, lc); lane k accumulates over l in the chunk and all P and
-// writes its partial to part[(lc * Part::size + f) * K + k].
-// SACC: accumulators in shared memory instead of registers.
-template <int N, int MINW, bool SACC>
+// Tile t = (kb, lc); lane k accumulates over l in the chunk and all P (raw H and
+// S sums in shared memory) and writes its gradient to part[(lc * Part::size + f) * K + k].
+template <int N, int MINW>
 __global__ void __launch_bounds__(32, MINW) grad_kernel(int nkb, int nlc, int LC, int K, int nst,
                                                    Consts<N> cs, const double *__restrict__ bra,
                                                    const double *__restrict__ ket,
@@ -184,91 +183,35 @@ __global__ void __launch_bounds__(32, MINW) grad_kernel(int nkb, int nlc, int LC
     int k, lc, l0, l1;
     if (!grad_lane_range(warp, lane, nkb, LC, K, k, lc, l0, l1)) return;
     double *out = part + (size_t)lc * Part<N>::size * K + k;
-    bool ok;
-    if (SACC) {
-        __shared__ double sacc[Part<N>::size * 32];
-        SmemAcc<N> acc{sacc + lane};
-        ok = grad_lane<N, double>(BraRef{bra + k, (size_t)K}, DevKet{ket}, l0, l1, nst, cs, lam, scal[0],
-                                  out, (size_t)K, acc);
-    } else {
-        ok = grad_lane<N, double>(BraRef{bra + k, (size_t)K}, DevKet{ket}, l0, l1, nst, cs, lam, scal[0],
-                                  out, (size_t)K);
-    }
+    __shared__ double sacc[2 * Part<N>::size * 32];
+    SmemAcc<N> accH{sacc + lane}, accS{sacc + Part<N>::size * 32 + lane};
+    const bool ok = grad_lane<N, double>(BraRef{bra + k, (size_t)K}, DevKet{ket}, l0, l1, nst, cs, lam, scal[0],
+                                         out, (size_t)K, accH, accS);
     if (!ok) flag_status(status, 1, k * K + l0);
 }
 
-
-// ---------------------------------------------------------------------------
-// Symmetric gradient tiles: each unordered pair (k >= l) once.  Tile (kb, lc)
-// of the lower-triangle tile list; lane = bra k.  For every ket (l, P) the
-// lane adds the bra gradient of its term to its shared-memory accumulator and
-// writes the term's ket gradient (in P's frame) to its row of a per-warp
-// table; the warp then sums the table column by column, each lane maps one
-// component back to l's frame (KetMap) and accumulates it over P.  Bra
-// partials: part_b[(t * PS + f) * 32 + lane]; ket partials:
-// part_k[(t * LC + l - l0) * PS + f].  Requires PS <= 32 (n <= 5).
-template <int N, int MINW>
+// Symmetric gradient pass (E = scal[0] known; python/make_grad.py's role when H
+// and S are given): each unordered pair (k >= l) once, bra and ket gradient from
+// one term.  One warp per tile; the body is fsym_tile with KE.
+template <int N, int MINW, bool SKET>
 __global__ void __launch_bounds__(32, MINW) gsym_kernel(const int2 *__restrict__ tiles, int ntiles,
                                                    int LC, int K, int nst, Consts<N> cs,
                                                    const double *__restrict__ bra,
                                                    const double *__restrict__ ket,
                                                    const double *__restrict__ C,
-                                                   const double *__restrict__ scal, KetMap kmap,
+                                                   const double *__restrict__ scal, RawMap kmap,
                                                    double *__restrict__ part_b,
                                                    double *__restrict__ part_k, int *status) {
-    using KL = KetLayout<N>;
-    constexpr int PS = Part<N>::size;
-    static_assert(PS <= 32, "the symmetric pass needs tri(n) + 1 + 3n <= 32");
-    __shared__ double sacc[PS * 32];
-    __shared__ double krow[32 * 33];
+    __shared__ double sacc[2 * Part<N>::size * 32];
+    __shared__ double krow[ket_table<N>(1)];
     __shared__ double kred[32];
+    __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::term : 2];
     const int t = blockIdx.x;
-    const int lane = threadIdx.x;
     if (t >= ntiles) return;
-    const int2 tl = tiles[t];
-    const int k = tl.x * 32 + lane;
-    const int l0 = tl.y * LC;
-    const int l1 = min(l0 + LC, K);
-    const bool kval = k < K;
-    const double E = scal[0];
-    const double Ck = kval ? C[k] : 0.0;
-    SmemAcc<N> acc{sacc + lane};
-    acc.zero();
-    const BraRef b{bra + (kval ? k : 0), (size_t)K};
-    struct RowOut {
-        double *r;
-        __device__ __forceinline__ void put(int f, double v) { r[f] = v; }
-        __device__ __forceinline__ void add(int f, double v) { r[f] += v; }
-    } ko{krow + lane * 33};
-    bool ok = true;
-    for (int l = l0; l < l1; ++l) {
-        double accl = 0.0;
-        for (int P = 0; P < nst; ++P) {
-            const double *kr = ket + ((size_t)l * nst + P) * KL::size;
-            if (kval && l <= k) {
-                const double wk = l < k ? 2.0 * Ck * kr[KL::winv] : 0.0;
-                ok = term_sym<N, double>(b, kr, cs, E, kr[KL::wC], wk, acc, ko) && ok;
-            } else {
-#pragma unroll
-                for (int f = 0; f < PS; ++f) ko.r[f] = 0.0;
-            }
-            __syncwarp();
-            double v = 0.0;
-            if (lane < PS)
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r) v += krow[r * 33 + lane];
-            kred[lane] = v;
-            __syncwarp();
-            if (lane < PS) accl += ket_map_apply(kmap, P, lane, PS, kred);
-            __syncwarp();
-        }
-        if (lane < PS) part_k[((size_t)t * LC + (l - l0)) * PS + lane] = accl;
-    }
-    if (kval) {
-#pragma unroll
-        for (int f = 0; f < PS; ++f) part_b[((size_t)t * PS + f) * 32 + lane] = sacc[f * 32 + lane];
-    }
-    if (!ok) flag_status(status, 1, k * K + l0);
+    fsym_tile<N, true, false, false, SKET, 0, true, true>(t, tiles[t], LC, K, nst, cs, bra, ket, C, kmap, nullptr,
+                                                          nullptr, part_b, part_k, status,
+                                                          FusedSmem{sacc, krow, kred, sket}, false, nullptr, 0, -1,
+                                                          TileOut{}, scal[0]);
 }
 
 // Fused pass over unordered pairs (k >= l): one warp per tile; the body is
@@ -282,14 +225,14 @@ __global__ void __launch_bounds__(32, MINW) fsym_kernel(const int2 *__restrict__
                                                    int LC, int K, int nst, int npc, Consts<N> cs,
                                                    const double *__restrict__ bra,
                                                    const double *__restrict__ ket,
-                                                   const double *__restrict__ C, KetMap kmap,
+                                                   const double *__restrict__ C, RawMap kmap,
                                                    double *__restrict__ H, double *__restrict__ S,
                                                    double *__restrict__ part_b,
                                                    double *__restrict__ part_k, int *status) {
     __shared__ double sacc[2 * Part<N>::size * 32];
-    __shared__ double krow[2 * 16 * 33];
+    __shared__ double krow[ket_table<N>(2)];
     __shared__ double kred[64];
-    __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::size : 2];
+    __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::term : 2];
     const int t = t_begin + blockIdx.x;
     if (t >= t_end) return;
     const int pc = blockIdx.y, PC = (nst + npc - 1) / npc;
@@ -323,37 +266,38 @@ __global__ void __launch_bounds__(256) hs_reduce_kernel(const double *__restrict
 // shared memory once for all warps; SKET: each warp stages its ket records in
 // two buffers (the next term's copied while the current one is evaluated).
 // SYNC: where the warps take their per-term barrier (fsym_tile).  Shared
-// memory (dynamic, 16-byte aligned): per warp 2 PS 32 + 2 16 33 + 64 (+ 2 ket
-// records) doubles, then the bras.
+// memory (dynamic, 16-byte aligned): per warp 2 PS 32 + ket table + 64 (+ 2 ket
+// records) doubles, then the bras.  KE: the symmetric pass with E known.
 template <int N> __host__ __device__ constexpr int fsym_warp_smem(bool sket) {
-    return 2 * Part<N>::size * 32 + 2 * 16 * 33 + 64 + (sket ? 2 * KetLayout<N>::size : 0);
+    return 2 * Part<N>::size * 32 + ket_table<N>(2) + 64 + (sket ? 2 * KetLayout<N>::term : 0);
 }
 template <int N> __host__ __device__ constexpr int fsym_block_smem_bytes(int warps, bool sbra, bool sket) {
-    return (warps * fsym_warp_smem<N>(sket) + (sbra ? BraLayout<N>::size * 32 : 0)) * 8;
+    return (warps * fsym_warp_smem<N>(sket) + (sbra ? BraLayout<N>::term * 32 : 0)) * 8;
 }
 
-template <int N, bool VKET, bool SBRA, bool SKET, int WARPS, int SYNC = 0>
+template <int N, bool VKET, bool SBRA, bool SKET, int WARPS, int SYNC = 0, bool KE = false>
 __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *__restrict__ groups, int ngroups,
                                                                 int *__restrict__ qcount,
                                                                 const int *__restrict__ tstart, int LC, int K,
                                                                 int nst, Consts<N> cs,
                                                                 const double *__restrict__ bra,
                                                                 const double *__restrict__ ket,
-                                                                const double *__restrict__ C, KetMap kmap,
+                                                                const double *__restrict__ C, RawMap kmap,
                                                                 double *__restrict__ H, double *__restrict__ S,
                                                                 double *__restrict__ part_b,
                                                                 double *__restrict__ part_k, int *status,
-                                                                double *__restrict__ xsym, int tail0) {
+                                                                double *__restrict__ xsym, int tail0,
+                                                                const double *__restrict__ scal) {
     extern __shared__ __align__(16) double smem[];
     __shared__ int gsh;
     constexpr int PS = Part<N>::size;
     constexpr int PER_WARP = fsym_warp_smem<N>(SKET);
-    constexpr int BS = BraLayout<N>::size;
+    constexpr int BS = BraLayout<N>::term;
+    constexpr int TBL = ket_table<N>(2);
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
     double *sbra = smem + WARPS * PER_WARP;  // SBRA: BS x 32 doubles after the warps' areas
-    const FusedSmem sm{base, base + 2 * PS * 32, base + 2 * PS * 32 + 2 * 16 * 33,
-                       base + 2 * PS * 32 + 2 * 16 * 33 + 64};
+    const FusedSmem sm{base, base + 2 * PS * 32, base + 2 * PS * 32 + TBL, base + 2 * PS * 32 + TBL + 64};
     for (;;) {
         if (threadIdx.x == 0) gsh = atomicAdd(qcount, 1);
         __syncthreads();
@@ -380,9 +324,9 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
             }
             __syncthreads();
         }
-        fsym_tile<N, VKET, true, SBRA, SKET, SYNC, false>(tstart[kb] + lc, make_int2(kb, lc), LC, K, nst, cs, bra,
-                                                          ket, C, kmap, H, S, part_b, part_k, status, sm, idle,
-                                                          sbra, p0, p1, xo);
+        fsym_tile<N, VKET, true, SBRA, SKET, SYNC, false, KE>(tstart[kb] + lc, make_int2(kb, lc), LC, K, nst, cs,
+                                                              bra, ket, C, kmap, H, S, part_b, part_k, status, sm,
+                                                              idle, sbra, p0, p1, xo, KE ? scal[0] : 0.0);
         // the group's bra partials: its warps share the 32 bras, so their
         // accumulators are summed (in warp order) and written once, to the
         // slot of queue unit g
@@ -403,7 +347,8 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
 // and H, S entries, which part 0 wrote (each part's bra partials have a queue
 // slot of their own).  Block = one tile (tail group j, warp w); entries that no
 // part wrote (kets past K or above the diagonal, tiles past the block's
-// triangle) are left alone.
+// triangle) are left alone.  H = nullptr: the symmetric pass, which has no H and
+// S sums and no S part of the ket partials.
 template <int N>
 __global__ void __launch_bounds__(256) fsym_tail_fix_kernel(const int2 *__restrict__ groups, int tail0, int W,
                                                             int LC, int K, const int *__restrict__ tstart,
@@ -422,12 +367,12 @@ __global__ void __launch_bounds__(256) fsym_tail_fix_kernel(const int2 *__restri
     const double *x0 = xsym + (size_t)(j * W + w) * (parts - 1) * XS;
     double *pk = part_k + (size_t)t * LC * 2 * PS;
     for (int i = threadIdx.x; i < LC * 2 * PS; i += blockDim.x) {
-        if (lc * LC + i / (2 * PS) >= K) continue;
+        if (lc * LC + i / (2 * PS) >= K || (!H && i % (2 * PS) >= PS)) continue;
         double v = pk[i];
         for (int q = 0; q < parts - 1; ++q) v += x0[q * XS + i];
         pk[i] = v;
     }
-    for (int i = threadIdx.x; i < LC * 64; i += blockDim.x) {
+    for (int i = threadIdx.x; H && i < LC * 64; i += blockDim.x) {
         const int l = lc * LC + i / 64, r = i & 63, k = kb * 32 + (r & 31);
         if (k >= K || l >= K || l > k) continue;
         double *M = r < 32 ? H : S;
@@ -438,20 +383,21 @@ __global__ void __launch_bounds__(256) fsym_tail_fix_kernel(const int2 *__restri
     }
 }
 
-// Sum the fused-pass partials and combine out[f * K + m] = sum_H - E sum_S with
-// E = scal[0] (written by finalize after the pass).  Block (kb, f): the 32
-// bases of row block kb, field f.  Their bra partials come from every tile of
-// block kb (up to K / LC of them) and their ket partials from one tile per
-// later row block, so the 8 warps of the block take every 8th of each and
-// their sums are combined in a fixed order.  Only tiles in [t0, t1) count (a
-// shard of the pass).
-template <int N>
+// Sum the partials of the fused (KE = false) or the symmetric pass into the
+// per-basis sums (put_sums), combined as H - 2 E S with E = scal[0] (written by
+// finalize after the fused pass; the symmetric pass has combined its own).
+// Block (kb, f): the 32 bases of row block kb, field f.  Their bra partials come
+// from every tile of block kb (up to K / LC of them) and their ket partials from
+// one tile per later row block, so the 8 warps of the block take every 8th of
+// each and their sums are combined in a fixed order.  Only tiles in [t0, t1)
+// count (a shard of the pass).
+template <int N, bool KE>
 __global__ void __launch_bounds__(256) fsym_sum_kernel(const int *__restrict__ tstart, int LC, int K,
                                                        const double *__restrict__ part_b,
                                                        const double *__restrict__ part_k,
                                                        const double *__restrict__ scal,
                                                        double *__restrict__ out, int t0, int t1, int npc,
-                                                       const int2 *__restrict__ urange) {
+                                                       const int2 *__restrict__ urange, int folded) {
     constexpr int PS = Part<N>::size;
     __shared__ double red[4][8][32];
     const int kb = blockIdx.x, f = blockIdx.y;
@@ -466,67 +412,47 @@ __global__ void __launch_bounds__(256) fsym_sum_kernel(const int *__restrict__ t
         sH += part_b[(((size_t)t * 2 + 0) * PS + f) * 32 + lane];
         sS += part_b[(((size_t)t * 2 + 1) * PS + f) * 32 + lane];
     }
-    // the ket partials of basis m: tile (q, lc) of every row block q from
-    // kb0 on, every 8th q per warp
     double kH = 0.0, kS = 0.0;
-    if (m < K) {
-        const int lc = m / LC, ll = m - lc * LC;
-        const int nkb = (K + 31) >> 5;
-        int kb0 = lc * LC - 31;
-        kb0 = kb0 > 0 ? (kb0 + 31) >> 5 : 0;
-        for (int q = kb0 + seg; q < nkb; q += 8) {
-            const int t = tstart[q] + lc;
-            if (t < t0 || t >= t1) continue;
-            for (int pc = 0; pc < npc; ++pc) {
-                const size_t base = ((size_t)(t * npc + pc) * LC + ll) * 2;
-                kH += part_k[(base + 0) * PS + f];
-                kS += part_k[(base + 1) * PS + f];
-            }
-        }
-    }
+    if (m < K) ket_partials<N, !KE>(tstart, LC, K, f, m, part_k, t0, t1, npc, seg, 8, kH, kS);
     red[0][seg][lane] = sH;
     red[1][seg][lane] = sS;
     red[2][seg][lane] = kH;
     red[3][seg][lane] = kS;
     __syncthreads();
     if (seg != 0 || m >= K) return;
-    // fixed order: the bra sums of the 8 warps, then their ket sums
-    sH = red[0][0][lane];
-    sS = red[1][0][lane];
-#pragma unroll
-    for (int q = 1; q < 8; ++q) {
-        sH += red[0][q][lane];
-        sS += red[1][q][lane];
-    }
+    // fixed order: the 8 warps' sums of each
+    sH = sS = kH = kS = 0.0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-        sH += red[2][q][lane];
-        sS += red[3][q][lane];
+        sH += red[0][q][lane];
+        sS += red[1][q][lane];
+        kH += red[2][q][lane];
+        kS += red[3][q][lane];
     }
-    out[(size_t)f * K + m] = sH - scal[0] * sS;
+    put_sums(out, PS, K, f, m, sH, sS, kH, kS, KE ? 0.0 : 2.0 * scal[0], folded);
 }
 
-// Sum the symmetric-pass partials of basis m into out[f * K + m]: its bra
-// partials from the tiles of block kb = m / 32 (lane m % 32) and its ket
-// partials from the tiles of chunk lc = m / LC in every block kb' >= that chunk.
+// The gradient of basis k from its sums (finish_one): written field-major to
+// `fields` (a shard's share, all-reduced before GRADA) or mapped to vech(L),
+// scaled by norm C_k and written to GRADA block k.
 template <int N>
-__global__ void __launch_bounds__(256) gsym_sum_kernel(const int *__restrict__ tstart, int LC, int K,
-                                                       const double *__restrict__ part_b,
-                                                       const double *__restrict__ part_k,
-                                                       double *__restrict__ out) {
+__global__ void __launch_bounds__(32) fsym_finish_kernel(const double *__restrict__ sums, int K, Consts<N> cs,
+                                                         const double *__restrict__ bra,
+                                                         const double *__restrict__ C,
+                                                         const double *__restrict__ scal, int folded,
+                                                         double *__restrict__ fields, double *__restrict__ g,
+                                                         int *status) {
     constexpr int PS = Part<N>::size;
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= PS * K) return;
-    const int f = id / K, m = id - f * K;
-    const int kb = m >> 5, lane = m & 31;
-    double s = 0.0;
-    for (int t = tstart[kb]; t < tstart[kb + 1]; ++t) s += part_b[((size_t)t * PS + f) * 32 + lane];
-    const int lc = m / LC, ll = m - lc * LC;
-    const int nkb = (K + 31) >> 5;
-    int kb0 = lc * LC - 31;
-    kb0 = kb0 > 0 ? (kb0 + 31) >> 5 : 0;
-    for (int q = kb0; q < nkb; ++q) s += part_k[((size_t)(tstart[q] + lc) * LC + ll) * PS + f];
-    out[(size_t)f * K + m] = s;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= K) return;
+    double o[PS];
+    finish_one<N>(sums, K, bra, cs, folded, k, o);
+    if (fields) {
+#pragma unroll
+        for (int f = 0; f < PS; ++f) fields[(size_t)f * K + k] = o[f];
+        return;
+    }
+    if (!fields_to_grad<N>(o, bra, K, scal[1] * C[k], g, k)) atomicOr(status, 2);
 }
 
 // Sum the gradient-tile partials over the ket chunks, in place into chunk 0:
@@ -738,10 +664,10 @@ __global__ void f0_kernel(const double *__restrict__ z, int count, double *__res
                           double *__restrict__ df) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    double fs, D, ia, zo;
-    boys<true>(1.0, z[i], fs, D, ia, zo);  // a = 1: fs = F0(z), D = F0'(z) / F0(z)
+    double fs, D2, ia, zo;
+    boys<true>(1.0, z[i], fs, D2, ia, zo);  // a = 1: fs = F0(z), D2 = 2 F0'(z) / F0(z)
     if (f) f[i] = fs;
-    if (df) df[i] = fs * D;
+    if (df) df[i] = 0.5 * fs * D2;
 }
 
 __global__ void reset_status_kernel(int *status) {
@@ -784,23 +710,20 @@ template <int N> struct Launch {
         default: energy_v<8>(a, st); break;
         }
     }
-    template <int MINW, bool SACC> static void grad_v(const LaunchArgs &a, cudaStream_t st) {
+    template <int MINW> static void grad_v(const LaunchArgs &a, cudaStream_t st) {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
         const int nkb = (a.K + 31) / 32, nlc = (a.K + a.LC_g - 1) / a.LC_g;
-        grad_kernel<N, MINW, SACC><<<nkb * nlc, 32, 0, st>>>(nkb, nlc, a.LC_g, a.K, a.nst, cs, a.bra,
-                                                             a.ket, a.scal, a.lam, a.part, a.status);
+        grad_kernel<N, MINW><<<nkb * nlc, 32, 0, st>>>(nkb, nlc, a.LC_g, a.K, a.nst, cs, a.bra, a.ket, a.scal, a.lam,
+                                                       a.part, a.status);
     }
-    // variant codes: 8, 12, 16, 20 = warps per SM with register accumulators;
-    // 112, 116 = 12, 16 warps per SM with shared-memory accumulators
+    // variant codes: warps per SM the kernel is compiled for (100 + w: the same
+    // as w); 128 registers spill the n > 3 term (LiH K = 700: 4.07 ms at 16 warps
+    // per SM, 3.32 at 12, 2.76 at 8), so 16 and 20 run 12 there
     static void grad_tiles(const LaunchArgs &a, cudaStream_t st) {
-        switch (a.minb_g) {
-        case 12: grad_v<12, false>(a, st); break;
-        case 16: grad_v<16, false>(a, st); break;
-        case 20: grad_v<20, false>(a, st); break;
-        case 112: grad_v<12, true>(a, st); break;
-        case 116: grad_v<16, true>(a, st); break;
-        default: grad_v<8, false>(a, st); break;
-        }
+        const int w = a.minb_g % 100;
+        if (w == 8) grad_v<8>(a, st);
+        else if (w == 12 || N > 3) grad_v<12>(a, st);
+        else grad_v<N <= 3 ? 16 : 12>(a, st);
     }
     static void grad_reduce(const LaunchArgs &a, cudaStream_t st) {
         const int nlc = (a.K + a.LC_g - 1) / a.LC_g;
@@ -810,30 +733,51 @@ template <int N> struct Launch {
         grad_reduce_kernel<N><<<(a.K + 127) / 128, 128, 0, st>>>(a.part, a.K, a.bra, a.C, a.scal, a.g,
                                                                   a.status);
     }
-    template <int MINW> static void gsym_v(const LaunchArgs &a, cudaStream_t st) {
+    template <int MINW, bool SKET> static void gsym_v(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
             Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
-            gsym_kernel<N, MINW><<<a.nstiles, 32, 0, st>>>(a.stiles, a.nstiles, a.LC_s, a.K, a.nst, cs, a.bra,
-                                                           a.ket, a.C, a.scal, a.kmap, a.psym,
-                                                           a.psym + (size_t)a.nstiles * Part<N>::size * 32,
-                                                           a.status);
+            gsym_kernel<N, MINW, SKET><<<a.nstiles, 32, 0, st>>>(a.stiles, a.nstiles, a.LC_s, a.K, a.nst, cs, a.bra,
+                                                                 a.ket, a.C, a.scal, a.kmap, a.psym,
+                                                                 a.psym + (size_t)a.nstiles * 2 * Part<N>::size * 32,
+                                                                 a.status);
         }
     }
+    // lockstep blocks when the handle's groups are 8 chunks wide
+    static bool gsym_block(const LaunchArgs &a) {
+        return a.minb_s >= 200 && fused_block_warps(a.minb_s) == 8 && a.sgroups && a.qcount && a.urange;
+    }
     static void gsym_tiles(const LaunchArgs &a, cudaStream_t st) {
+        if (gsym_block(a)) {
+            fsym_block<true, true, 8, 3, true>(a, st);
+            if (a.sg_ntail > 0 && a.sg_parts >= 2 && a.xsym) {  // the queue's split tail: no H and S sums to add
+                LaunchArgs b = a;
+                b.H = b.S = nullptr;
+                fsym_tail(b, st);
+            }
+            return;
+        }
         switch (a.minb_s) {
-        case 12: gsym_v<12>(a, st); break;
-        case 16: gsym_v<16>(a, st); break;
-        default: gsym_v<8>(a, st); break;
+        case 12:
+        case 112: gsym_v<12, false>(a, st); break;
+        case 16: gsym_v<16, false>(a, st); break;
+        case 118: gsym_v<8, true>(a, st); break;
+        case 122: gsym_v<12, true>(a, st); break;
+        default: gsym_v<8, false>(a, st); break;
         }
     }
     static void gsym_reduce(const LaunchArgs &a, cudaStream_t st) {
-        if constexpr (Part<N>::size <= 32) {
-            constexpr int PS = Part<N>::size;
-            gsym_sum_kernel<N><<<(PS * a.K + 255) / 256, 256, 0, st>>>(
-                a.stile_start, a.LC_s, a.K, a.psym, a.psym + (size_t)a.nstiles * PS * 32, a.part);
-            grad_reduce_kernel<N><<<(a.K + 127) / 128, 128, 0, st>>>(a.part, a.K, a.bra, a.C, a.scal, a.g,
-                                                                      a.status);
-        }
+        if constexpr (Part<N>::size <= 32) sum_finish<true>(a, gsym_block(a), 1, 0, a.nstiles, st);
+    }
+    // the per-basis sums and their gradients; lockstep: bra partials per queue unit
+    template <bool KE>
+    static void sum_finish(const LaunchArgs &a, bool lockstep, int npc, int t0, int t1, cudaStream_t st) {
+        constexpr int PS = Part<N>::size;
+        Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
+        fsym_sum_kernel<N, KE><<<dim3((a.K + 31) / 32, PS), 256, 0, st>>>(
+            a.stile_start, a.LC_s, a.K, a.psym, a.psym + (size_t)a.nstiles * npc * 2 * PS * 32, a.scal, a.part, t0, t1,
+            npc, lockstep ? a.urange : nullptr, a.kmap.fold);
+        fsym_finish_kernel<N><<<(a.K + 31) / 32, 32, 0, st>>>(a.part, a.K, cs, a.bra, a.C, a.scal, a.kmap.fold, a.sums,
+                                                              a.g, a.status);
     }
     template <int MINW, bool VKET, bool SKET = false> static void fsym_v(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
@@ -846,12 +790,12 @@ template <int N> struct Launch {
                 npc > 1 ? a.Sp : a.S, a.psym, a.psym + (size_t)a.nstiles * npc * 2 * Part<N>::size * 32, a.status);
         }
     }
-    template <bool SBRA, bool SKET, int WARPS, int SYNC = 0>
+    template <bool SBRA, bool SKET, int WARPS, int SYNC = 0, bool KE = false>
     static void fsym_block(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
             constexpr int smem = fsym_block_smem_bytes<N>(WARPS, SBRA, SKET);
             if constexpr (smem <= 232448) {
-                auto kern = fsym_block_kernel<N, true, SBRA, SKET, WARPS, SYNC>;
+                auto kern = fsym_block_kernel<N, true, SBRA, SKET, WARPS, SYNC, KE>;
                 int dev = 0, sms = 148;
                 cudaGetDevice(&dev);
                 // the shared-memory opt-in is per device: once per instantiation and device
@@ -868,7 +812,7 @@ template <int N> struct Launch {
                 kern<<<grid, 32 * WARPS, smem, st>>>(a.sgroups, a.nsgroups, a.qcount, a.stile_start, a.LC_s, a.K,
                                                      a.nst, cs, a.bra, a.ket, a.C, a.kmap, a.H, a.S, a.psym,
                                                      a.psym + (size_t)a.nstiles * 2 * Part<N>::size * 32, a.status,
-                                                     a.xsym, a.sg_tail0);
+                                                     a.xsym, a.sg_tail0, a.scal);
             }
         }
     }
@@ -906,18 +850,12 @@ template <int N> struct Launch {
     }
     static void fsym_reduce(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
-            constexpr int PS = Part<N>::size;
             const int t0 = a.st_end > 0 ? a.st_begin : 0, t1 = a.st_end > 0 ? a.st_end : a.nstiles;
             const int npc = a.npc > 1 && a.minb_s < 200 ? a.npc : 1;
             // the lockstep pass over the whole tile list writes its bra partials
             // per queue unit (the unit ranges of each row block in urange)
             const bool lockstep = a.minb_s >= 200 && a.st_end == 0 && a.sgroups && a.urange;
-            fsym_sum_kernel<N><<<dim3((a.K + 31) / 32, PS), 256, 0, st>>>(
-                a.stile_start, a.LC_s, a.K, a.psym, a.psym + (size_t)a.nstiles * npc * 2 * PS * 32, a.scal,
-                a.sums ? a.sums : a.part, t0, t1, npc, lockstep ? a.urange : nullptr);
-            if (!a.sums)
-                grad_reduce_kernel<N><<<(a.K + 127) / 128, 128, 0, st>>>(a.part, a.K, a.bra, a.C, a.scal, a.g,
-                                                                          a.status);
+            sum_finish<false>(a, lockstep, npc, t0, t1, st);
         }
     }
     static void rrms(const LaunchArgs &a, const int *terms, int nterms, double *out, cudaStream_t st) {
@@ -980,7 +918,7 @@ int launch_grad(const LaunchArgs &a, cudaStream_t st) {
     return launch_grad_reduce(a, st);
 }
 int launch_gsym(const LaunchArgs &a, cudaStream_t st) {
-    if (a.n > 5) return -1;
+    if (a.n > 5 || !a.psym || !a.stiles) return -1;
     NECG_DISPATCH(a.n, gsym_tiles(a, st));
     return 0;
 }
@@ -1022,7 +960,7 @@ int launch_fsym_tail(const LaunchArgs &a, cudaStream_t st) {
 }
 int launch_fsym_reduce(const LaunchArgs &a, cudaStream_t st) {
     if (a.n > 5) return -1;
-    if (!a.stile_start || !a.psym || !a.scal || (!a.sums && (!a.part || !a.bra || !a.C || !a.g))) return -1;
+    if (!a.stile_start || !a.psym || !a.scal || !a.part || !a.bra || (!a.sums && (!a.C || !a.g))) return -1;
     NECG_DISPATCH(a.n, fsym_reduce(a, st));
     return 0;
 }
@@ -1102,5 +1040,27 @@ int bra_record_size(int n) {
     }
 }
 int part_stride(int n) { return n >= 1 && n <= 6 ? tri(n) + 1 + 3 * n : 0; }
+size_t part_doubles(int n, int K) {
+    const size_t per = (size_t)part_stride(n) * K, nlc = (size_t)(K + 3) / 4;
+    return per * (nlc > kSumSets ? nlc : kSumSets);
+}
+int ket_slots(int n) {
+    switch (n) {
+    case 1: return KetSlots<1>::SL;
+    case 2: return KetSlots<2>::SL;
+    case 3: return KetSlots<3>::SL;
+    case 4: return KetSlots<4>::SL;
+    default: return KetSlots<5>::SL;
+    }
+}
+int ket_slot(int n, int f) {
+    switch (n) {
+    case 1: return KetSlots<1>::slot(f);
+    case 2: return KetSlots<2>::slot(f);
+    case 3: return KetSlots<3>::slot(f);
+    case 4: return KetSlots<4>::slot(f);
+    default: return KetSlots<5>::slot(f);
+    }
+}
 
 }  // namespace necg

@@ -22,7 +22,7 @@ struct LaunchArgs {
     int *status;
     // symmetric gradient pass
     const int *pinv;                       // index of P^-1 per symmetry term (null: none)
-    KetMap kmap;                           // ket frame map per (P, field)
+    RawMap kmap;                           // ket frame map per (P, slot)
     const int2 *stiles;                    // lower-triangle tiles of chunk LC_s
     const int *stile_start;                // first tile of each 32-row block (nkb + 1)
     int nstiles, LC_s, minb_s;
@@ -105,5 +105,11 @@ void launch_f0(const double *z, int count, double *f, double *df, cudaStream_t s
 int ket_record_size(int n);
 int bra_record_size(int n);
 int part_stride(int n);
+// the gradient-partial buffer of bases of up to K functions: tile partials of
+// the ordered pass (ket chunks of 4 or more) or the per-basis sums
+size_t part_doubles(int n, int K);
+// ket slots per (P, matrix) and the slot of a field (KetSlots, n <= 5)
+int ket_slots(int n);
+int ket_slot(int n, int f);
 
 }  // namespace necg

@@ -87,9 +87,9 @@ NECG_HD void prep_bra_one(const double *iv, int K, const Consts<N> &cs, double *
 #pragma unroll
     for (int t = 0; t < 3 * N; ++t) bra[(BL::AS + t) * KK + k] = AS[t];
 #pragma unroll
-    for (int t = 0; t < tri(N); ++t) bra[(BL::Nk + t) * KK + k] = AMA[t];
+    for (int t = 0; t < tri(N); ++t) bra[(BL::N8 + t) * KK + k] = -8.0 * AMA[t];
     bra[BL::i1 * KK + k] = i1;
-    bra[BL::pre * KK + k] = dl * ::sqrt(dl);
+    bra[BL::pre * KK + k] = cs.sqrt8n * (dl * ::sqrt(dl));
     bra[BL::tMA * KK + k] = tMA;
 #pragma unroll
     for (int t = 0; t < tri(N); ++t) bra[(BL::L + t) * KK + k] = L[t];
@@ -155,16 +155,15 @@ NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Cons
 #pragma unroll
     for (int t = 0; t < 3 * N; ++t) o[KL::ASp + t] = ASp[t];
 #pragma unroll
-    for (int t = 0; t < tri(N); ++t) o[KL::Np + t] = AMA[t];
-#pragma unroll
-    for (int t = 0; t < N * N; ++t) o[KL::AMn4 + t] = -4.0 * AM[t];
+    for (int t = 0; t < tri(N); ++t) o[KL::Np8 + t] = -8.0 * AMA[t];
     o[KL::i2] = i2;
     o[KL::pre] = dl * ::sqrt(dl);
     o[KL::tMA] = tMA;
     o[KL::w] = scvv[P];
     o[KL::wC] = C ? 2.0 * scvv[P] * C[l] : 0.0;
     o[KL::winv] = pinv ? scvv[pinv[P]] : 0.0;
-    if (KL::size > KL::winv + 1) o[KL::winv + 1] = 0.0;
+    if (KL::term > KL::winv + 1) o[KL::winv + 1] = 0.0;
+    if (KL::size > KL::tMA + 1) o[KL::tMA + 1] = 0.0;
 }
 
 // Energy tile lane: bra k against kets l in [l0, lend) (lend <= k + 1), all P.
@@ -220,33 +219,70 @@ template <int N> struct Part {
     static constexpr int size = S + 3 * N;
 };
 
+// Raw sums of one bra over its terms (term_raw's `out`): H and S fields into two
+// accumulators (g(t), d(), s(t)), weight w ov.
+template <int N, typename R, typename ACC> struct BraSums {
+    ACC &H, &S;
+    R w, wo;
+    NECG_HD static R &at(ACC &a, int f) { return f < tri(N) ? a.g(f) : f == tri(N) ? a.d() : a.s(f - tri(N) - 1); }
+    NECG_HD void begin(R ov) { wo = w * ov; }
+    NECG_HD void s1(int f, R v) { at(S, f) += wo * v; }
+    NECG_HD void h1(int f, R v) { at(H, f) += wo * v; }
+    NECG_HD void s2(int, int fa, int fb, R va, R vb) {
+        s1(fa, va);
+        s1(fb, vb);
+    }
+    NECG_HD void h2(int, int fa, int fb, R va, R vb) {
+        h1(fa, va);
+        h1(fb, vb);
+    }
+    NECG_HD void scalar(R e2) {
+        H.d() += wo * e2;
+        S.d() += wo;
+    }
+};
+
 // Gradient tile lane: bra k against kets l in [l0, l1), all P, weights
-// wC(l, P) = 2 scvv[P] C_l; writes the partial to part[f * stride] (f < Part::size).
+// wC(l, P) = 2 scvv[P] C_l: the raw sums in accH and accS, then the gradient of
+// lam H - E S folded from them into part[f * stride] (f < Part::size).
 template <int N, typename R, typename BA, typename KB, typename ACC>
 NECG_HD bool grad_lane(const BA &b, const KB &ket, int l0, int l1, int nst, const Consts<N> &cs,
-                       R lam, R E, double *part, size_t stride, ACC &acc) {
+                       R lam, R E, double *part, size_t stride, ACC &accH, ACC &accS) {
     using KL = KetLayout<N>;
-    using PL = Part<N>;
-    acc.zero();
+    using BL = BraLayout<N>;
+    constexpr int PS = Part<N>::size;
+    accH.zero();
+    accS.zero();
     bool ok = true;
+    BraSums<N, R, ACC> sums{accH, accS, R(0.0), R(0.0)};
     for (int l = l0; l < l1; ++l)
         for (int P = 0; P < nst; ++P) {
             const auto kr = ket.at(((size_t)l * nst + P) * KL::size);
-            ok = term_grad<N>(b, kr, cs, lam, E, R(kr[KL::wC]), acc) && ok;
+            sums.w = R(kr[KL::wC]);
+            R eta2, ov;
+            ok = term_raw<N>(b, kr, cs, R(0.0), sums, eta2, ov) && ok;
         }
+    R r[PS], o[PS];
+    const auto sr = [&](int f) { return BraSums<N, R, ACC>::at(accS, f); };
+    const auto A = [&](int t) { return b(BL::A + t); };
+    const auto s = [&](int t) { return b(BL::S + t); };
+    const auto e = [&](int t) { return b(BL::AS + t); };
 #pragma unroll
-    for (int t = 0; t < tri(N); ++t) part[(PL::G + t) * stride] = val(acc.g(t));
-    part[PL::D * stride] = val(acc.d());
+    for (int f = 0; f < PS; ++f) r[f] = BraSums<N, R, ACC>::at(accH, f);
+    explicit_tau<N>(sr, A, e, cs, r);
 #pragma unroll
-    for (int t = 0; t < 3 * N; ++t) part[(PL::S + t) * stride] = val(acc.s(t));
+    for (int f = 0; f < PS; ++f) r[f] = lam * r[f] - 2.0 * E * sr(f);
+    fold_raw<N>(FieldsOf<R>{r}, A, s, e, o);
+#pragma unroll
+    for (int f = 0; f < PS; ++f) part[f * stride] = val(o[f]);
     return ok;
 }
 
 template <int N, typename R, typename BA, typename KB>
 NECG_HD bool grad_lane(const BA &b, const KB &ket, int l0, int l1, int nst, const Consts<N> &cs,
                        R lam, R E, double *part, size_t stride) {
-    RegAcc<N, R> acc;
-    return grad_lane<N, R>(b, ket, l0, l1, nst, cs, lam, E, part, stride, acc);
+    RegAcc<N, R> accH, accS;
+    return grad_lane<N, R>(b, ket, l0, l1, nst, cs, lam, E, part, stride, accH, accS);
 }
 
 // Map an A-space gradient dF/dA = G + D A^-1 (G packed symmetric, D the
@@ -279,6 +315,21 @@ NECG_HD bool a_to_vech(const double (&G)[tri(N)], double D, const double (&gS)[3
         out[tri(N) + t] = v;
     }
     return fin;
+}
+
+// The GRADA block of basis k (scaled by sc) from its gradient fields.
+template <int N>
+NECG_HD bool fields_to_grad(const double (&o)[Part<N>::size], const double *bra, int K, double sc, double *g, int k) {
+    using BL = BraLayout<N>;
+    constexpr int blk = tri(N) + 3 * N;
+    double G[tri(N)], gS[3 * N], L[tri(N)];
+#pragma unroll
+    for (int t = 0; t < tri(N); ++t) G[t] = o[t];
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) gS[t] = o[tri(N) + 1 + t];
+#pragma unroll
+    for (int t = 0; t < tri(N); ++t) L[t] = bra[(BL::L + t) * (size_t)K + k];
+    return a_to_vech<N>(G, o[tri(N)], gS, L, sc, g + (size_t)k * blk);
 }
 
 // Sum the nlc partials of basis k and write its GRADA block scaled by sc.
@@ -323,19 +374,18 @@ NECG_HD bool matel_one(const BA &b, const KR &kr, const Consts<N> &cs, double *o
 template <int N, typename R, typename BA, typename KR>
 NECG_HD bool gradel_one(const BA &b, const KR &kr, const Consts<N> &cs, const double (&L)[tri(N)],
                         bool diag, double *tgvl, double *tgvls) {
-    bool ok = true;
+    constexpr int PS = Part<N>::size;
+    R bH[PS], bS[PS], h, ov;
+    const bool ok = term_gradients<N, false>(b, kr, cs, bH, bS, bH, bS, h, ov);
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
-        RegAcc<N, R> acc;
-        acc.zero();
-        // which 0: dH (lam 1, E 0); which 1: dS (lam 0, E -1)
-        ok = term_grad<N>(b, kr, cs, R(which == 0 ? 1.0 : 0.0), R(which == 0 ? 0.0 : -1.0), R(1.0), acc) && ok;
+        const R(&v)[PS] = which == 0 ? bH : bS;
         double G[tri(N)], gS[3 * N];
 #pragma unroll
-        for (int q = 0; q < tri(N); ++q) G[q] = val(acc.g(q));
+        for (int q = 0; q < tri(N); ++q) G[q] = val(v[q]);
 #pragma unroll
-        for (int q = 0; q < 3 * N; ++q) gS[q] = val(acc.s(q));
-        a_to_vech<N>(G, val(acc.d()), gS, L, diag ? 2.0 : 1.0, which == 0 ? tgvl : tgvls);
+        for (int q = 0; q < 3 * N; ++q) gS[q] = val(v[tri(N) + 1 + q]);
+        a_to_vech<N>(G, val(v[tri(N)]), gS, L, diag ? 2.0 : 1.0, which == 0 ? tgvl : tgvls);
     }
     return ok;
 }
@@ -386,6 +436,57 @@ NECG_HD void ket_map_apply2(const KetMap &m, int P, int f, int PS, const double 
     }
     out0 = v0;
     out1 = v1;
+}
+
+// Where the pair passes keep the ket's raw fields of a term: field f of matrix
+// `which` (0: H or the combined gradient, 1: S) in slot which * SL + slot(f) of a
+// table row.  The two fields of a pair (RawPairs) are 8 slots apart, so that the
+// even and the odd lanes of a warp, which store one side each, use different
+// shared-memory banks (rows are an odd number of doubles apart).
+template <int N> struct KetSlots {
+    static constexpr int SL = 16 * ((RawPairs<N>::count + 7) / 8);  // slots per matrix (16 or 32 for n <= 5)
+    __host__ __device__ static constexpr int of_pair(int i) { return 16 * (i >> 3) + (i & 7); }
+    __host__ __device__ static constexpr int slot(int f) {
+        return of_pair(RawPairs<N>::pair_of(f)) + 8 * RawPairs<N>::side_of(f);
+    }
+};
+
+// Sparse linear map of the ket's raw sums from P's transformed frame to the basis
+// function's own, by slot: entry (P, slot): cnt values at src/coef[(P * SL + slot)
+// * maxnz + i], src a slot of the same matrix.  fold: the set's shift maps are
+// not those of its coordinate maps (sms = kron(sml^-1, I3)), so that e' = A' s'
+// does not map as e does: the sums are folded into gradients in P's frame
+// (fold_raw) and those are mapped, with dF/ds' by sms^T.
+struct RawMap {
+    const int *cnt, *src;
+    const double *coef;
+    int maxnz, fold;
+};
+
+// Per-basis sums of the symmetric passes, field-major with stride K: the bra's
+// combined raw sums (H - 2 E S) plus, unless the kets were folded, the kets';
+// the bra's raw S sums; the kets' folded gradient when they were.
+constexpr int kSumSets = 3;
+
+// The gradient fields (Part<N>) of basis k from its sums.
+template <int N>
+NECG_HD void finish_one(const double *sums, int K, const double *bra, const Consts<N> &cs, int folded, int k,
+                        double (&o)[Part<N>::size]) {
+    using BL = BraLayout<N>;
+    constexpr int PS = Part<N>::size;
+    const size_t KK = (size_t)K;
+    double r[PS];
+#pragma unroll
+    for (int f = 0; f < PS; ++f) r[f] = sums[f * KK + k];
+    const auto sr = [&](int f) { return sums[(PS + f) * KK + k]; };
+    const auto A = [&](int t) { return bra[(BL::A + t) * KK + k]; };
+    const auto s = [&](int t) { return bra[(BL::S + t) * KK + k]; };
+    const auto e = [&](int t) { return bra[(BL::AS + t) * KK + k]; };
+    explicit_tau<N>(sr, A, e, cs, r);
+    fold_raw<N>(FieldsOf<double>{r}, A, s, e, o);
+    if (folded)
+#pragma unroll
+        for (int f = 0; f < PS; ++f) o[f] += sums[(2 * PS + f) * KK + k];
 }
 
 // Lane ranges of the two tile kinds (used by the kernels and the emulator).

@@ -12,23 +12,35 @@
 // Notation (n = N particles):
 //   A_k, A_l' = P^T A_l P    symmetric, packed lower (N(N+1)/2)
 //   S_k, S_l' = sms s_l      n x 3 (row = particle, column = x, y, z)
-//   B = A_k + A_l', Bi = B^-1, T = Bi (A_k S_k + A_l' S_l')   (st in the reference)
-//   Dk = S_k - T, Dl = T - S_l', Y = A_l' Dl (= A_k Dk)
-//   ov  = sqrt(8^n) (|L_k| |L_l|)^{3/2} / |B|^{3/2} exp(<E,T> - i1 - i2)
-//   tau = 3 tr(M X) - 2 <Y, M Y>, X = A_k Bi A_l',   tk = 2 ov tau
+//   B = A_k + A_l', Bi = B^-1, e = A_k S_k + A_l' S_l', T = Bi e   (st in the reference)
+//   D = T - S_k, N = A_k M A_k, U = 1.5 Bi + T T^T
+//   ov  = sqrt(8^n) (|L_k| |L_l|)^{3/2} / |B|^{3/2} exp(<e,T> - i1 - i2)
+//   tau = 3 tr(M A_k) - 3 <N, Bi> - 2 <D, N D>,   tk = 2 ov tau
 //   rho = sum_v c_v F0(|v^T T|^2 / v^T Bi v) (v^T Bi v)^{-1/2}, ert = ov rho
 //   sig = efs sum_i q_i T[i,z],  zht = ov sig
+//   eta = 2 tau + rho - sig,  h = tk + ert - zht = ov eta
 // Coulomb pairs v: e_q (nucleus-particle) or e_p - e_q (particle-particle),
 // c_v = 2 q_p q_q / sqrt(pi).
 //
-// Bra gradient of F = w (h - E ov) with h = tk + ert - zht:
-//   dF/dA_k = Fw (-Dk Dk^T - 1.5 Bi + 0.75 A_k^-1)
-//             + ovw (Bi (6 N_l' + W) Bi + Qk Dk^T + Dk Qk^T)
-//   dF/ds_k = -2 Fw Y + 2 ovw A_k Qk
-//   N_l' = A_l' M A_l',  Qk = Bi (Z' - 4 A_l' M Y),
+// Gradient.  h and ov depend on the pair through B and e alone, apart from
+// factors of one side only: |L_k|^{3/2} exp(-i1) of each side, and tau, which is
+// written with the bra's A_k and e_k = A_k S_k.  With F0's derivative pieces
 //   Z' = sum_v alpha_v v b_v^T - (efs/2) q e_z^T,  W = sum_v beta_v v v^T,
-//   alpha_v = c_v F0'(z) a^{-3/2},  beta_v = c_v a^{-3/2} (z F0'(z) + F0(z)/2).
-// The A_k^-1 term (coefficient D = 0.75 Fw) maps to vech(dF/dL) as 2 D / L_ii
+//   alpha_v = c_v F0'(z) a^{-3/2},  beta_v = c_v a^{-3/2} (z F0'(z) + F0(z)/2),
+//   Q = Bi (Z' - 4 N D)
+// the derivatives with respect to B and e are
+//   dh/dB = ov (Bi (6 N + W) Bi - Q T^T - T Q^T - eta U),  dh/de = 2 ov (Q + eta T)
+//   dS/dB = -ov U,                                         dS/de = 2 ov T
+// and serve the bra and the ket alike (term_raw).  A basis function sums them
+// over its terms as they are; what depends on its own A, s and e (the chain
+// from e = A s, its prefactors, and the bra's explicit share of tau) multiplies
+// only those sums, once per basis function (fold_raw, explicit_tau).  That
+// takes the products with A_k, A_l', S_k and S_l', the second sandwich and the
+// second outer products out of the term: 2816 instead of 4374 FLOP at n = 5 and
+// 1075 instead of 1626 at n = 3.  The FP64 pipe bounds the pair passes; whole
+// evaluations on a B200 went from 3.53 to 2.35 ms (LiH K = 1024), 1.06 to 0.76 ms
+// (H2 K = 2048) and 0.34 to 0.27 ms (He K = 2032).
+// The A^-1 term (coefficient D = 0.75 F) maps to vech(dF/dL) as 2 D / L_ii
 // on the diagonal only, so it is kept as one scalar per basis function.
 //
 // All term functions are templates over the scalar type R and over the bra and
@@ -72,23 +84,23 @@ __host__ __device__ constexpr int sx(int i, int j) {
 #define NECG_SQRT_PI 1.7724538509055159
 
 // Ket record: one per (l, P), read warp-uniformly by the tile kernels.
-// Layout (doubles): Ap[tri] Sp[3N] ASp[3N] Np[tri] AMn4[N*N] i2 pre tMA w wC winv pad
-// (AMn4 = -4 A_l' M, row-major: the factor of Z's update folded in, so that the
-// update is one FMA chain per output)
+// The pair passes read the first `term` doubles (staged in shared memory by the
+// lockstep blocks); Sp is for the fold of a symmetry term whose shift map is not
+// that of its coordinate map, Np8 = -8 A_l' M A_l' and tMA for the energy path.
 template <int N> struct KetLayout {
     static constexpr int T = tri(N);
     static constexpr int Ap = 0;
-    static constexpr int Sp = Ap + T;
-    static constexpr int ASp = Sp + 3 * N;
-    static constexpr int Np = ASp + 3 * N;
-    static constexpr int AMn4 = Np + T;
-    static constexpr int i2 = AMn4 + N * N;
+    static constexpr int ASp = Ap + T;
+    static constexpr int i2 = ASp + 3 * N;
     static constexpr int pre = i2 + 1;
-    static constexpr int tMA = pre + 1;  // tr(M A_l')
-    static constexpr int w = tMA + 1;    // symmetry weight scvv[P]
+    static constexpr int w = pre + 1;    // symmetry weight scvv[P]
     static constexpr int wC = w + 1;     // 2 scvv[P] C_l (gradient weight)
     static constexpr int winv = wC + 1;  // scvv[P^-1] (ket weight of the symmetric pass)
-    static constexpr int size = (winv + 1 + 1) & ~1;  // even, 16-byte records
+    static constexpr int term = (winv + 1 + 1) & ~1;  // even: 16-byte multiples
+    static constexpr int Sp = term;
+    static constexpr int Np8 = Sp + 3 * N;
+    static constexpr int tMA = Np8 + T;  // tr(M A_l')
+    static constexpr int size = (tMA + 1 + 1) & ~1;  // even, 16-byte records
 };
 
 // Bra record: structure of arrays over k, field f of basis k at f*K + k.
@@ -97,10 +109,11 @@ template <int N> struct BraLayout {
     static constexpr int A = 0;
     static constexpr int S = A + T;
     static constexpr int AS = S + 3 * N;
-    static constexpr int Nk = AS + 3 * N;  // A_k M A_k
-    static constexpr int i1 = Nk + T;
-    static constexpr int pre = i1 + 1;
+    static constexpr int N8 = AS + 3 * N;  // -8 A_k M A_k
+    static constexpr int i1 = N8 + T;
+    static constexpr int pre = i1 + 1;     // sqrt(8^n) |L_k|^{3/2}
     static constexpr int tMA = pre + 1;
+    static constexpr int term = tMA + 1;   // the fields above are all a term reads
     static constexpr int L = tMA + 1;      // L_k, packed lower
     static constexpr int size = L + T;
 };
@@ -108,15 +121,13 @@ template <int N> struct BraLayout {
 // Per-problem constants, passed to kernels by value (constant bank).
 template <int N> struct Consts {
     double M[N * N];    // inverse-mass tensor, row-major
-    double M4[N * N];   // 4 M (Q_l = Q_k + 4 M Y as one FMA chain per output)
     double Mq[tri(N)];  // packed lower: M_ii on the diagonal, M_ik + M_ki below (quadratic forms in M)
     double cv[tri(N)];  // c_v for the n(n+1)/2 Coulomb pairs (p<q, q-major order)
     double q[N];        // ncv[1..n]
     double efs;
     double sqrt8n;      // sqrt(8^n)
-    // M4 and Mq from M
+    // Mq from M
     NECG_HD void derive() {
-        for (int i = 0; i < N * N; ++i) M4[i] = 4.0 * M[i];
         for (int i = 0; i < N; ++i)
             for (int k = 0; k <= i; ++k) Mq[sx(i, k)] = i == k ? M[i * N + i] : M[i * N + k] + M[k * N + i];
     }
@@ -231,59 +242,47 @@ NECG_HD double rcp(double x) {
 #endif
 }
 
-// Cholesky of a packed SPD matrix B = R R^T; returns the inverse Bi (packed),
-// prod(1/R_ii) and a success flag.  Fully unrolled into registers.
+// Inverse Bi (packed) of a packed SPD matrix B by symmetric Gauss-Jordan
+// elimination: step k takes d = B_kk, t_i = B_ik / d, B_ij -= t_i B_jk, B_ik = t_i,
+// B_kk = -1 / d, and leaves -B^-1 after all of them.  The pivots d are those of
+// the LDL^T factorisation (all positive iff B is positive definite; det = prod d).
+// 70 products and 5 reciprocals at n = 5, against 95 and 5 inverse roots for
+// Cholesky and two triangular products; its errors measured the same or smaller.
+// det_m32 = det^{-3/2}.  Fully unrolled into registers.
 #pragma nv_exec_check_disable
 template <int N, typename R>
-NECG_HD bool chol_inverse(const R (&B)[tri(N)], R (&Bi)[tri(N)], R &prod_rinv) {
-    R Rm[tri(N)];
-    R rinv[N];
+NECG_HD bool spd_inverse(const R (&B)[tri(N)], R (&Bi)[tri(N)], R &det_m32) {
+    R a[tri(N)];
+#pragma unroll
+    for (int t = 0; t < tri(N); ++t) a[t] = B[t];
     bool ok = true;
+    R det = R(1.0);
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-        R d = B[sx(j, j)];
-#pragma unroll
-        for (int k = 0; k < j; ++k) d -= Rm[sx(j, k)] * Rm[sx(j, k)];
+    for (int k = 0; k < N; ++k) {
+        R d = a[sx(k, k)];
         const bool pos = d > 0.0;
         ok = ok && pos;
         if (!pos) d = R(1.0);
-        const R r = rsq(d);
-        rinv[j] = r;
-        Rm[sx(j, j)] = d * r;
+        det = (k == 0) ? d : det * d;
+        const R r = rcp(d);
+        R t[N];
 #pragma unroll
-        for (int i = j + 1; i < N; ++i) {
-            R s = B[sx(i, j)];
+        for (int i = 0; i < N; ++i)
+            if (i != k) t[i] = a[sx(i, k)] * r;
 #pragma unroll
-            for (int k = 0; k < j; ++k) s -= Rm[sx(i, k)] * Rm[sx(j, k)];
-            Rm[sx(i, j)] = s * r;
-        }
+        for (int i = 0; i < N; ++i)
+#pragma unroll
+            for (int j = 0; j <= i; ++j)
+                if (i != k && j != k) a[sx(i, j)] -= t[i] * a[sx(j, k)];
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i != k) a[sx(i, k)] = t[i];
+        a[sx(k, k)] = -r;
     }
-    // W = R^-1 (lower triangular), in place
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-        Rm[sx(j, j)] = rinv[j];
-#pragma unroll
-        for (int i = j + 1; i < N; ++i) {
-            R s = Rm[sx(i, j)] * rinv[j];
-#pragma unroll
-            for (int k = j + 1; k < i; ++k) s += Rm[sx(i, k)] * Rm[sx(k, j)];
-            Rm[sx(i, j)] = -(s * rinv[i]);
-        }
-    }
-    // Bi = W^T W : Bi_ij = sum_{k >= max(i,j)} W_ki W_kj
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int j = 0; j <= i; ++j) {
-            R s = Rm[sx(i, i)] * Rm[sx(i, j)];
-#pragma unroll
-            for (int k = i + 1; k < N; ++k) s += Rm[sx(k, i)] * Rm[sx(k, j)];
-            Bi[sx(i, j)] = s;
-        }
-    R p = rinv[0];
-#pragma unroll
-    for (int j = 1; j < N; ++j) p *= rinv[j];
-    prod_rinv = p;
+    for (int t = 0; t < tri(N); ++t) Bi[t] = -a[t];
+    const R y = rsq(det);
+    det_m32 = (y * y) * y;
     return ok;
 }
 
@@ -326,12 +325,12 @@ NECG_HD void symv3_acc(const Acc &S, int off, const R (&x)[3 * N], R (&y)[3 * N]
 
 // Boys-function pieces for one Coulomb pair.  Given a = v^T Bi v and
 // bb = |v^T T|^2 (z = bb / a) returns fs = F0(z) a^{-1/2} and, when GRAD,
-// D = F0'(z) / F0(z) (so F0'(z) a^{-1/2} = fs D) and ia = 1/a.  The Pade branch
+// D2 = 2 F0'(z) / F0(z) (so 2 F0'(z) a^{-1/2} = fs D2) and ia = 1/a.  The Pade branch
 // (z <= 16.3578) and the asymptotic branch sqrt(pi/(4z)) follow
 // python/utils.py:78-106; in the Pade branch F0 = sqrt(num / den), and from
 // F0^2 = num / den, F0' = F0 (num'/num - den'/den) / 2, so
-//   D = F0' / F0 = (num' den - den' num) / (2 num den)  (Pade),  -1 / (2 z)  (asymptotic),
-// with num'/2 den - den'/2 num evaluated as one polynomial.  Two
+//   D2 = 2 F0' / F0 = (num' den - den' num) / (num den)  (Pade),  -1 / z  (asymptotic),
+// with num' den - den' num evaluated as one polynomial.  Two
 // special functions give every quotient and root; RCP chooses between two ways:
 //   RCP:   ia = 1/a (rcp);  q = (num den a)^{-1/2} (Pade) or bb^{-1/2}:
 //          fs = num q or (sqrt(pi) / 2) q, and q^2 a = 1 / (num den) or 1 / z;
@@ -346,21 +345,20 @@ template <typename R> NECG_HD void boys_pade(R z, R &num, R &den) {
     num = ((((NECG_PC1 * z + NECG_PC2) * z + NECG_PC3) * z + NECG_PC4) * z + NECG_PC5) * z + 1.0;
     den = (((((NECG_PC6 * z + NECG_PC7) * z + NECG_PC8) * z + NECG_PC9) * z + NECG_PC10) * z + NECG_PC11) * z + 1.0;
 }
-// (num' den - den' num) / 2 as one polynomial of degree 10: its coefficients
-// are those of num'/2 den - den'/2 num, formed from the Pade coefficients when
-// the code is compiled
+// num' den - den' num as one polynomial of degree 10, its coefficients formed
+// from the Pade coefficients when the code is compiled
 struct BoysDP {
     double c[11];
     constexpr BoysDP() : c{} {
-        const double nh[5] = {0.5 * NECG_PC5, NECG_PC4, 1.5 * NECG_PC3, 2.0 * NECG_PC2, 2.5 * NECG_PC1};  // num'/2
+        const double nd[5] = {NECG_PC5, 2.0 * NECG_PC4, 3.0 * NECG_PC3, 4.0 * NECG_PC2, 5.0 * NECG_PC1};  // num'
         const double de[7] = {1.0, NECG_PC11, NECG_PC10, NECG_PC9, NECG_PC8, NECG_PC7, NECG_PC6};       // den
-        const double dh[6] = {0.5 * NECG_PC11, NECG_PC10, 1.5 * NECG_PC9, 2.0 * NECG_PC8, 2.5 * NECG_PC7,
-                              3.0 * NECG_PC6};                                                         // den'/2
+        const double dd[6] = {NECG_PC11, 2.0 * NECG_PC10, 3.0 * NECG_PC9, 4.0 * NECG_PC8, 5.0 * NECG_PC7,
+                              6.0 * NECG_PC6};                                                         // den'
         const double nu[6] = {1.0, NECG_PC5, NECG_PC4, NECG_PC3, NECG_PC2, NECG_PC1};                  // num
         for (int i = 0; i < 5; ++i)
-            for (int j = 0; j < 7; ++j) c[i + j] += nh[i] * de[j];
+            for (int j = 0; j < 7; ++j) c[i + j] += nd[i] * de[j];
         for (int i = 0; i < 6; ++i)
-            for (int j = 0; j < 6; ++j) c[i + j] -= dh[i] * nu[j];
+            for (int j = 0; j < 6; ++j) c[i + j] -= dd[i] * nu[j];
     }
 };
 template <typename R> NECG_HD R boys_pade_dp(R z) {
@@ -372,7 +370,7 @@ template <typename R> NECG_HD R boys_pade_dp(R z) {
 }
 #pragma nv_exec_check_disable
 template <bool GRAD, bool RCP = true, typename R>
-NECG_HD void boys(R a, R bb, R &fs, R &D, R &ia, R &z) {
+NECG_HD void boys(R a, R bb, R &fs, R &D2, R &ia, R &z) {
     R ra = R(1.0);
     if constexpr (RCP) {
         ia = rcp(a);
@@ -400,30 +398,26 @@ NECG_HD void boys(R a, R bb, R &fs, R &D, R &ia, R &z) {
         if constexpr (RCP) {
             const R qa = (q * q) * a;
             dp = qa * P;
-            da = -0.5 * qa;
+            da = -qa;
         } else {
             const R qq = q * q;
             dp = qq * P;
-            da = -0.5 * a * qq;
+            da = -(a * qq);
         }
-        D = pade ? dp : da;
+        D2 = pade ? dp : da;
     } else {
-        D = R(0.0);
+        D2 = R(0.0);
     }
 }
 
 // Coulomb sum with the pieces of its derivative (python/gradel.py:266-337):
-// rho = sum_v c_v F0(z_v) a_v^-1/2, Z' = sum_v alpha_v v b_v^T - (efs/2) q e_z^T
-// (the Stark part folded in), W = sum_v beta_v v v^T (packed).
+// returns rho = sum_v c_v F0(z_v) a_v^-1/2 and adds 2 sum_v alpha_v v b_v^T to Z
+// and 2 sum_v beta_v v v^T to W (packed).
 #pragma nv_exec_check_disable
 template <int N, typename R>
-NECG_HD void coulomb_grad(const R (&Bi)[tri(N)], const R (&T)[3 * N], const Consts<N> &cs, R &rho,
-                          R (&Z)[3 * N], R (&W)[tri(N)]) {
-#pragma unroll
-    for (int t = 0; t < 3 * N; ++t) Z[t] = R(0.0);
-#pragma unroll
-    for (int t = 0; t < tri(N); ++t) W[t] = R(0.0);
-    rho = R(0.0);
+NECG_HD R coulomb_grad(const R (&Bi)[tri(N)], const R (&T)[3 * N], const Consts<N> &cs, R (&Z)[3 * N],
+                       R (&W)[tri(N)]) {
+    R rho = R(0.0);
 #pragma unroll
     for (int q = 1; q <= N; ++q)
 #pragma unroll
@@ -438,14 +432,15 @@ NECG_HD void coulomb_grad(const R (&Bi)[tri(N)], const R (&T)[3 * N], const Cons
                 for (int c = 0; c < 3; ++c) bv[c] -= T[3 * (p - 1) + c];
             }
             const R bb = bv[0] * bv[0] + bv[1] * bv[1] + bv[2] * bv[2];
-            R fs, D, ia, z;
-            boys<true, (N > 3)>(a, bb, fs, D, ia, z);
-            // alpha = c F0' a^{-3/2} = c fs D / a, beta = c a^{-3/2} (z F0' + F0 / 2) = (c fs / a)(z D + 1/2)
+            R fs, D2, ia, z;
+            boys<true, (N > 3)>(a, bb, fs, D2, ia, z);
+            // 2 alpha = 2 c F0' a^{-3/2} = c fs D2 / a,
+            // 2 beta = 2 c a^{-3/2} (z F0' + F0 / 2) = (c fs / a)(z D2 + 1)
             const R cf = cs.cv[vidx(p, q)] * fs;
             rho += cf;
             const R cfi = cf * ia;
-            const R al = cfi * D;
-            const R be = cfi * (D * z + 0.5);
+            const R al = cfi * D2;
+            const R be = al * z + cfi;
 #pragma unroll
             for (int cc = 0; cc < 3; ++cc) Z[3 * (q - 1) + cc] += al * bv[cc];
             W[sx(q - 1, q - 1)] += be;
@@ -456,73 +451,22 @@ NECG_HD void coulomb_grad(const R (&Bi)[tri(N)], const R (&T)[3 * N], const Cons
                 W[sx(q - 1, p - 1)] -= be;
             }
         }
-#pragma unroll
-    for (int i = 0; i < N; ++i) Z[3 * i + 2] -= 0.5 * cs.efs * cs.q[i];
-}
-
-// acc += Bi Mt Bi (Mt packed symmetric), column by column of Mt Bi.
-#pragma nv_exec_check_disable
-template <int N, typename R, typename OUT>
-NECG_HD void sandwich(const R (&Bi)[tri(N)], const R (&Mt)[tri(N)], OUT &&add) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-        R col[N];
-#pragma unroll
-        for (int a = 0; a < N; ++a) {
-            R s = Mt[sx(a, 0)] * Bi[sx(0, j)];
-#pragma unroll
-            for (int k = 1; k < N; ++k) s += Mt[sx(a, k)] * Bi[sx(k, j)];
-            col[a] = s;
-        }
-#pragma unroll
-        for (int i = j; i < N; ++i) {
-            R s = Bi[sx(i, 0)] * col[0];
-#pragma unroll
-            for (int a = 1; a < N; ++a) s += Bi[sx(i, a)] * col[a];
-            add(sx(i, j), s);
-        }
-    }
-}
-
-// The same with each output's sum started from seed(t) (an accumulator's value,
-// so the products fuse into it): put(t, seed(t) + (Bi Mt Bi)_t).
-#pragma nv_exec_check_disable
-template <int N, typename R, typename SEED, typename OUT>
-NECG_HD void sandwich_seeded(const R (&Bi)[tri(N)], const R (&Mt)[tri(N)], SEED &&seed, OUT &&put) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-        R col[N];
-#pragma unroll
-        for (int a = 0; a < N; ++a) {
-            R s = Mt[sx(a, 0)] * Bi[sx(0, j)];
-#pragma unroll
-            for (int k = 1; k < N; ++k) s += Mt[sx(a, k)] * Bi[sx(k, j)];
-            col[a] = s;
-        }
-#pragma unroll
-        for (int i = j; i < N; ++i) {
-            R s = seed(sx(i, j));
-#pragma unroll
-            for (int a = 0; a < N; ++a) s += Bi[sx(i, a)] * col[a];
-            put(sx(i, j), s);
-        }
-    }
+    return rho;
 }
 
 // B = A_k + A_l', its inverse, T = Bi (A_k S_k + A_l' S_l') and the overlap.
 #pragma nv_exec_check_disable
 template <int N, typename R, typename BA, typename KA>
-NECG_HD bool term_core(const BA &b, const KA &kr, const Consts<N> &cs, R (&Bi)[tri(N)],
-                       R (&T)[3 * N], R &ov) {
+NECG_HD bool term_core(const BA &b, const KA &kr, R (&Bi)[tri(N)], R (&T)[3 * N], R &ov) {
     using KL = KetLayout<N>;
     using BL = BraLayout<N>;
-    R prinv;
+    R m32;
     bool ok;
     {
         R B[tri(N)];
 #pragma unroll
         for (int t = 0; t < tri(N); ++t) B[t] = b(BL::A + t) + kr[KL::Ap + t];
-        ok = chol_inverse<N>(B, Bi, prinv);
+        ok = spd_inverse<N>(B, Bi, m32);
     }
     R Ev[3 * N];
 #pragma unroll
@@ -539,43 +483,42 @@ NECG_HD bool term_core(const BA &b, const KA &kr, const Consts<N> &cs, R (&Bi)[t
     R i3 = Ev[0] * T[0];
 #pragma unroll
     for (int t = 1; t < 3 * N; ++t) i3 += Ev[t] * T[t];
-    const R p3 = prinv * prinv * prinv;
-    ov = cs.sqrt8n * b(BL::pre) * kr[KL::pre] * p3 * exp(i3 - b(BL::i1) - kr[KL::i2]);
+    ov = b(BL::pre) * kr[KL::pre] * m32 * exp(i3 - b(BL::i1) - kr[KL::i2]);
     return ok;
 }
 
 // tau = 3 tr(M X) - 2 <Y, M Y>.  tr(M X) with X = A_k Bi A_l' is written through
 // the matrix with the smaller tr(M A): X = A_s - A_s Bi A_s, which keeps the
 // subtraction free of cancellation.  The choice differs from lane to lane, so
-// both N_s are read and one is selected (no divergent branch).  Y = A_l' (T - S_l')
-// is returned for the gradient formulas.
+// both N_s are read and one is selected (no divergent branch).  Y = A_l' (T - S_l').
 #pragma nv_exec_check_disable
 template <int N, typename R, typename BA, typename KA>
 NECG_HD R term_tau(const BA &b, const KA &kr, const Consts<N> &cs, const R (&Bi)[tri(N)],
-                   const R (&T)[3 * N], R (&Y)[3 * N]) {
+                   const R (&T)[3 * N]) {
     using KL = KetLayout<N>;
     using BL = BraLayout<N>;
     R tMX;
     {
         const R tl = kr[KL::tMA], tk = b(BL::tMA);
         const bool use_l = tl <= tk;
-        // tr(Bi N_s): the diagonal and the off-diagonal products summed apart
+        // -8 tr(Bi N_s): the diagonal and the off-diagonal products summed apart
         R dg = R(0.0), od = R(0.0);
 #pragma unroll
         for (int i = 0; i < N; ++i)
 #pragma unroll
             for (int j = 0; j <= i; ++j) {
-                const R nl = kr[KL::Np + sx(i, j)], nk = b(BL::Nk + sx(i, j));
+                const R nl = kr[KL::Np8 + sx(i, j)], nk = b(BL::N8 + sx(i, j));
                 const R v = Bi[sx(i, j)] * (use_l ? nl : nk);
                 if (i == j)
                     dg = (i == 0) ? v : dg + v;
                 else
                     od = (i == 1) ? v : od + v;
             }
-        tMX = (use_l ? tl : tk) - (dg + 2.0 * od);
+        tMX = (use_l ? tl : tk) + 0.125 * (dg + 2.0 * od);
     }
     R yMy = R(0.0);
     {
+        R Y[3 * N];
         // Y = A_l' (T - S_l') = A_l' T - A_l' S_l', the second product from the ket record
 #pragma unroll
         for (int t = 0; t < 3 * N; ++t) Y[t] = -kr[KL::ASp + t];
@@ -594,14 +537,6 @@ NECG_HD R term_tau(const BA &b, const KA &kr, const Consts<N> &cs, const R (&Bi)
     return 3.0 * tMX - 2.0 * yMy;
 }
 #pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA>
-NECG_HD R term_tau(const BA &b, const KA &kr, const Consts<N> &cs, const R (&Bi)[tri(N)],
-                   const R (&T)[3 * N]) {
-    R Y[3 * N];
-    return term_tau<N>(b, kr, cs, Bi, T, Y);
-}
-
-#pragma nv_exec_check_disable
 template <int N, typename R>
 NECG_HD R term_sig(const Consts<N> &cs, const R (&T)[3 * N]) {
     R sg = cs.q[0] * T[2];
@@ -616,7 +551,7 @@ template <int N, typename R, typename BA, typename KA>
 NECG_HD bool term_energy(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R &tau, R &rho,
                          R &sig) {
     R Bi[tri(N)], T[3 * N];
-    const bool ok = term_core<N>(b, kr, cs, Bi, T, ov);
+    const bool ok = term_core<N>(b, kr, Bi, T, ov);
     tau = term_tau<N>(b, kr, cs, Bi, T);
     sig = term_sig<N>(cs, T);
     // Coulomb sum (python/matel.py:162-197)
@@ -643,395 +578,375 @@ NECG_HD bool term_energy(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, 
     return ok;
 }
 
-// Full term with bra gradient.  Fw = wgt (lam h - E ov), ovw = wgt lam ov:
-// lam = 1, E = current energy gives the gradient of H - E S (the optimiser's
-// combination); lam = 1, E = 0 gives dH alone; lam = 0, E = -1 gives dS alone.
-// acc: accumulator with g(t) (packed dF/dA_k), d() (coefficient of A_k^-1 in
-// dF/dA_k) and s(t) (dF/ds_k, n x 3), each returning a reference -- registers
-// (RegAcc) or, on the device, lane-interleaved shared memory.
-#pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA, typename ACC>
-NECG_HD bool term_grad(const BA &b, const KA &kr, const Consts<N> &cs, R lam, R E, R wgt, ACC &acc) {
-    using KL = KetLayout<N>;
-    using BL = BraLayout<N>;
-    R Bi[tri(N)], T[3 * N], ov;
-    const bool ok = term_core<N>(b, kr, cs, Bi, T, ov);
-    const R tau = term_tau<N>(b, kr, cs, Bi, T);
-    const R sig = term_sig<N>(cs, T);
-    R Z[3 * N], W[tri(N)], rho;
-    coulomb_grad<N>(Bi, T, cs, rho, Z, W);
-    const R h = ov * (2.0 * tau + rho - sig);
-    const R Fw = wgt * (lam * h - E * ov);
-    const R ovw = wgt * lam * ov;
-    acc.d() += 0.75 * Fw;
-    // accG += Bi (ovw (6 N_l' + W) - 1.5 Fw B) Bi,  B = A_k + A_l'
-    {
-        const R f15 = 1.5 * Fw;
-#pragma unroll
-        for (int t = 0; t < tri(N); ++t)
-            W[t] = ovw * (6.0 * kr[KL::Np + t] + W[t]) - f15 * (b(BL::A + t) + kr[KL::Ap + t]);
-#pragma unroll
-        for (int j = 0; j < N; ++j) {
-            R col[N];  // column j of W Bi
-#pragma unroll
-            for (int a = 0; a < N; ++a) {
-                R s = W[sx(a, 0)] * Bi[sx(0, j)];
-#pragma unroll
-                for (int k = 1; k < N; ++k) s += W[sx(a, k)] * Bi[sx(k, j)];
-                col[a] = s;
-            }
-#pragma unroll
-            for (int i = j; i < N; ++i) {
-                R s = Bi[sx(i, 0)] * col[0];
-#pragma unroll
-                for (int a = 1; a < N; ++a) s += Bi[sx(i, a)] * col[a];
-                acc.g(sx(i, j)) += s;
-            }
-        }
+// Fields of the raw sums of one basis function (Part<N>::size of them, the same
+// count and order as the partial buffers): G[tri] (derivative with respect to
+// B), one scalar, g[3N] (derivative with respect to e).  Raw values of one term,
+// before the weight w ov:
+//   H:  X = 2 (Bi (6 N + W) Bi - Q T^T - T Q^T - eta U),  2 eta,  2 (Q + eta T)
+//   S:  -U,                                               1,      T
+// so that H - 2 E S holds twice the G, twice the scalar and once the g of the
+// gradient of h - E ov.  term_raw hands the fields out in pairs, for outputs
+// that combine two values at a time: pair i < tri holds G_i and g_i, the
+// remaining g follow two by two, and the scalar comes with the last g when
+// their number is odd, alone otherwise (n <= 5, where tri <= 3 n).
+template <int N> struct RawPairs {
+    static constexpr int T = tri(N), V = 3 * N;
+    static constexpr int lead = T < V ? T : V;
+    static constexpr int left = V - lead;
+    static constexpr bool odd = left & 1;               // the scalar's pair also holds g[V - 1]
+    static constexpr int count = lead + left / 2 + 1;   // the last one holds the scalar
+    static constexpr int scalar = T;                    // its field index
+    // pair and side (0, 1) of field f
+    __host__ __device__ static constexpr int pair_of(int f) {
+        return f < T ? f : f == T ? count - 1 : f - T - 1 < lead ? f - T - 1 : lead + (f - T - 1 - lead) / 2;
     }
-    // Y = A_l' (T - S_l') ; Zk = Z' - 4 (A_l' M) Y ; Qk = Bi Zk
-    R Y[3 * N];
-    {
-        R Dl[3 * N];
-#pragma unroll
-        for (int t = 0; t < 3 * N; ++t) Dl[t] = T[t] - kr[KL::Sp + t];
-        symv3<N>(kr, KL::Ap, Dl, Y);
+    __host__ __device__ static constexpr int side_of(int f) {
+        return f < T ? 0 : f == T ? (odd ? 1 : 0) : f - T - 1 < lead ? 1 : (f - T - 1 - lead) & 1;
     }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R s = Z[3 * i + c];
-#pragma unroll
-            for (int k = 0; k < N; ++k) s += kr[KL::AMn4 + i * N + k] * Y[3 * k + c];
-            Z[3 * i + c] = s;
-        }
-    R Q[3 * N];
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R s = Bi[sx(i, 0)] * Z[c];
-#pragma unroll
-            for (int k = 1; k < N; ++k) s += Bi[sx(i, k)] * Z[3 * k + c];
-            Q[3 * i + c] = s;
-        }
-    // accS += 2 ovw A_k Q - 2 Fw Y
-    {
-        const R o2 = 2.0 * ovw, f2 = 2.0 * Fw;
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                R s = b(BL::A + sx(i, 0)) * Q[c];
-#pragma unroll
-                for (int k = 1; k < N; ++k) s += b(BL::A + sx(i, k)) * Q[3 * k + c];
-                acc.s(3 * i + c) += o2 * s - f2 * Y[3 * i + c];
-            }
-    }
-    // Rk = ovw Qk - Fw/2 Dk ; accG += Rk Dk^T + Dk Rk^T,  Dk = S_k - T
-    {
-        const R fh = 0.5 * Fw;
-#pragma unroll
-        for (int t = 0; t < 3 * N; ++t) {
-            const R dk = b(BL::S + t) - T[t];
-            T[t] = dk;
-            Q[t] = ovw * Q[t] - fh * dk;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int j = 0; j <= i; ++j) {
-            R s = Q[3 * i] * T[3 * j] + T[3 * i] * Q[3 * j];
-#pragma unroll
-            for (int c = 1; c < 3; ++c) s += Q[3 * i + c] * T[3 * j + c] + T[3 * i + c] * Q[3 * j + c];
-            acc.g(sx(i, j)) += s;
-        }
-    return ok;
-}
+};
 
-// Both gradients of one (k, l, P) term: the bra gradient (with respect to A_k,
-// s_k; weight wb) into acc, and the ket gradient with respect to the
-// transformed ket (A_l' = sml^T A_l sml, s_l' = sms s_l; weight wk) through
-// kout.put(f, value) / kout.add(f, value) for f in [0, tri(N) + 1 + 3N):
-// packed dF/dA_l', the coefficient of A_l'^-1, dF/ds_l'.  The element is symmetric under exchanging
-// bra and (transformed) ket, so the ket formulas are the bra formulas with the
-// roles swapped:
-//   dF/dA_l' = Fk (-Dl Dl^T - 1.5 Bi) + 0.75 Fk A_l'^-1
-//              + ovk (Bi (6 A_k M A_k + W) Bi - Ql Dl^T - Dl Ql^T)
-//   dF/ds_l' = 2 Fk Y + 2 ovk A_l' Ql,   Ql = Bi (Z' + 4 A_k M Y),  Dl = T - S_l'
-// with Fk = wk (h - E ov), ovk = wk ov.
-#pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA, typename ACC, typename KOUT>
-NECG_HD bool term_sym(const BA &b, const KA &kr, const Consts<N> &cs, R E, R wb, R wk, ACC &acc,
-                      KOUT &kout) {
-    using KL = KetLayout<N>;
-    using BL = BraLayout<N>;
-    R Bi[tri(N)], T[3 * N], ov;
-    const bool ok = term_core<N>(b, kr, cs, Bi, T, ov);
-    const R tau = term_tau<N>(b, kr, cs, Bi, T);
-    const R sig = term_sig<N>(cs, T);
-    R Z[3 * N], W[tri(N)], rho;
-    coulomb_grad<N>(Bi, T, cs, rho, Z, W);
-    const R phi = ov * (2.0 * tau + rho - sig) - E * ov;
-    const R Fb = wb * phi, ovb = wb * ov;
-    const R Fk = wk * phi, ovk = wk * ov;
-    acc.d() += 0.75 * Fb;
-    kout.put(tri(N), 0.75 * Fk);
-    // bra: acc += Bi (ovb (6 N_l' + W) - 1.5 Fb B) Bi ; ket: Bi (ovk (6 N_k + W) - 1.5 Fk B) Bi
-    {
-        R Mt[tri(N)];
-        const R fb = 1.5 * Fb, fk = 1.5 * Fk;
-#pragma unroll
-        for (int t = 0; t < tri(N); ++t)
-            Mt[t] = ovb * (6.0 * kr[KL::Np + t] + W[t]) - fb * (b(BL::A + t) + kr[KL::Ap + t]);
-        sandwich<N>(Bi, Mt, [&](int t, R v) { acc.g(t) += v; });
-#pragma unroll
-        for (int t = 0; t < tri(N); ++t)
-            W[t] = ovk * (6.0 * b(BL::Nk + t) + W[t]) - fk * (b(BL::A + t) + kr[KL::Ap + t]);
-        sandwich<N>(Bi, W, [&](int t, R v) { kout.put(t, v); });
-    }
-    // Y = A_l' (T - S_l'); Qk = Bi (Z' - 4 A_l' M Y); Ql = Bi (Z' + 4 A_k M Y) = Qk + 4 M Y
-    // (the difference of the two right-hand sides is 4 B M Y and Bi B = I)
-    R Dl[3 * N], Y[3 * N];
-#pragma unroll
-    for (int t = 0; t < 3 * N; ++t) Dl[t] = T[t] - kr[KL::Sp + t];
-    symv3<N>(kr, KL::Ap, Dl, Y);
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R s = Z[3 * i + c];
-#pragma unroll
-            for (int k = 0; k < N; ++k) s += kr[KL::AMn4 + i * N + k] * Y[3 * k + c];
-            Z[3 * i + c] = s;
-        }
-    R Qk[3 * N], Ql[3 * N];
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R s = Bi[sx(i, 0)] * Z[c];
-#pragma unroll
-            for (int k = 1; k < N; ++k) s += Bi[sx(i, k)] * Z[3 * k + c];
-            Qk[3 * i + c] = s;
-        }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R s = Qk[3 * i + c];
-#pragma unroll
-            for (int k = 0; k < N; ++k) s += cs.M4[i * N + k] * Y[3 * k + c];
-            Ql[3 * i + c] = s;
-        }
-    // bra: acc.s += 2 ovb A_k Qk - 2 Fb Y ; ket: put 2 ovk A_l' Ql + 2 Fk Y
-    {
-        const R ob2 = 2.0 * ovb, fb2 = 2.0 * Fb, ok2 = 2.0 * ovk, fk2 = 2.0 * Fk;
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                R s = b(BL::A + sx(i, 0)) * Qk[c];
-                R t = kr[KL::Ap + sx(i, 0)] * Ql[c];
-#pragma unroll
-                for (int k = 1; k < N; ++k) {
-                    s += b(BL::A + sx(i, k)) * Qk[3 * k + c];
-                    t += kr[KL::Ap + sx(i, k)] * Ql[3 * k + c];
-                }
-                acc.s(3 * i + c) += ob2 * s - fb2 * Y[3 * i + c];
-                kout.put(tri(N) + 1 + 3 * i + c, ok2 * t + fk2 * Y[3 * i + c]);
-            }
-    }
-    // bra: Rk = ovb Qk - Fb/2 Dk, acc.g += Rk Dk^T + Dk Rk^T   (Dk = S_k - T)
-    // ket: Rl = ovk Ql + Fk/2 Dl, dF/dA_l' -= Rl Dl^T + Dl Rl^T
-    {
-        const R fbh = 0.5 * Fb, fkh = 0.5 * Fk;
-#pragma unroll
-        for (int t = 0; t < 3 * N; ++t) {
-            const R dk = b(BL::S + t) - T[t];
-            T[t] = dk;
-            Qk[t] = ovb * Qk[t] - fbh * dk;
-            Ql[t] = ovk * Ql[t] + fkh * Dl[t];
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int j = 0; j <= i; ++j) {
-            R s = Qk[3 * i] * T[3 * j] + T[3 * i] * Qk[3 * j];
-            R t = Ql[3 * i] * Dl[3 * j] + Dl[3 * i] * Ql[3 * j];
-#pragma unroll
-            for (int c = 1; c < 3; ++c) {
-                s += Qk[3 * i + c] * T[3 * j + c] + T[3 * i + c] * Qk[3 * j + c];
-                t += Ql[3 * i + c] * Dl[3 * j + c] + Dl[3 * i + c] * Ql[3 * j + c];
-            }
-            acc.g(sx(i, j)) += s;
-            kout.add(sx(i, j), -t);
-        }
-    return ok;
-}
-
-// One (k, l, P) term of the fused pass: the H element h and overlap ov (for H
-// and S), and the bra and ket gradients of h and of ov kept apart -- the pass
-// runs before E is known, and g = g_H - E g_S is formed once E is.  With
-// Fb = wb h, ovb = wb ov (Fk, ovk with wk):
-//   bra, H: the formulas of term_grad with Fw = Fb, ovw = ovb
-//   bra, S: d(ov)/dA_k = ov (-Dk Dk^T - 1.5 Bi + 0.75 A_k^-1), d(ov)/ds_k = -2 ov Y
-// and the ket formulas of term_sym with the same split.  The ket values of H
-// and of S for field f go out together: ko.put(f, vH, vS) / ko.add(f, vH, vS).
-// mid(i) is called at two points of the body (i = 1 after B, Bi, T and ov;
-// i = 2 after tau and sig), for callers that synchronise warps there.  tau's
-// Y = A_l' (T - S_l') goes on to the gradient formulas (it is not formed
-// twice).  For n <= 3 the Coulomb sum comes before tau (and before mid(2)),
-// otherwise after: the order that measured faster on a B200 for each n, since
-// the values live across the Coulomb sum (Y, or Z and W) set the register
-// pressure; the results are the same either way, bit for bit.
+// One (k, l, P) term: the overlap and the raw values above, handed to `out`:
+//   out.begin(ov)              once, first
+//   out.s2(i, fa, fb, va, vb)  pair i of the S values (fields fa, fb)
+//   out.h2(i, fa, fb, va, vb)  pair i of the H values, with eta - E2 / 2 in the
+//                              place of eta (E2 = 2 E gives the gradient of h - E ov)
+//   out.scalar(eta2)           the scalar pair when it holds nothing else
+//   out.s1 / out.h1(f, v)      single fields (n = 6 only)
+// eta2_out = 2 eta (so h = ov eta2_out / 2).  The S values leave before the
+// Coulomb sum, so that U is not live across it; mid(i) is called at two points
+// (i = 1 after B, Bi, T and ov; i = 2 before the Coulomb sum) for callers that
+// synchronise warps there.
 struct NoMid {
     NECG_HD void operator()(int) const {}
 };
 #pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA, typename ACC, typename KOUT, typename MID = NoMid>
-NECG_HD bool term_fused(const BA &b, const KA &kr, const Consts<N> &cs, R wb, R wk, ACC &accH, ACC &accS,
-                        KOUT &ko, R &h_out, R &ov_out, const MID &mid = MID{}) {
-    using KL = KetLayout<N>;
+template <int N, typename R, typename BA, typename KA, typename OUT, typename MID = NoMid>
+NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT &out, R &eta2_out, R &ov_out,
+                      const MID &mid = MID{}) {
     using BL = BraLayout<N>;
-    R Bi[tri(N)], T[3 * N], ov;
-    const bool ok = term_core<N>(b, kr, cs, Bi, T, ov);
-    mid(1);
-    constexpr bool coulomb_first = N <= 3;
-    R Z[3 * N], W[tri(N)], rho, Y[3 * N];
-    if constexpr (coulomb_first) coulomb_grad<N>(Bi, T, cs, rho, Z, W);
-    const R tau = term_tau<N>(b, kr, cs, Bi, T, Y);
-    const R sig = term_sig<N>(cs, T);
-    mid(2);
-    if constexpr (!coulomb_first) coulomb_grad<N>(Bi, T, cs, rho, Z, W);
-    const R h = ov * (2.0 * tau + rho - sig);
-    h_out = h;
+    using RP = RawPairs<N>;
+    constexpr int TR = tri(N), V = 3 * N;
+    R Bi[TR], T[V], ov;
+    const bool ok = term_core<N>(b, kr, Bi, T, ov);
     ov_out = ov;
-    const R Fb = wb * h, ovb = wb * ov;
-    const R Fk = wk * h, ovk = wk * ov;
-    accH.d() += 0.75 * Fb;
-    accS.d() += 0.75 * ovb;
-    ko.put(tri(N), 0.75 * Fk, 0.75 * ovk);
-    // Bi (ovb (6 N_l' + W) - 1.5 Fb B) Bi = Bi ovb (6 N_l' + W) Bi - 1.5 Fb Bi, since
-    // Bi B Bi = Bi (and the same for the ket)
+    mid(1);
+    out.begin(ov);
+    // S: -U = -(1.5 Bi + T T^T), T, 1
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+            R u = 1.5 * Bi[sx(i, j)];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) u += T[3 * i + c] * T[3 * j + c];
+            if (sx(i, j) < RP::lead)
+                out.s2(sx(i, j), sx(i, j), TR + 1 + sx(i, j), -u, T[sx(i, j) < V ? sx(i, j) : 0]);
+            else
+                out.s1(sx(i, j), -u);
+        }
+#pragma unroll
+    for (int q = 0; q < RP::left / 2; ++q)
+        out.s2(RP::lead + q, TR + 1 + RP::lead + 2 * q, TR + 2 + RP::lead + 2 * q, T[RP::lead + 2 * q],
+               T[RP::lead + 2 * q + 1]);
+    if (RP::odd) out.s2(RP::count - 1, TR + V, RP::scalar, T[V - 1], R(1.0));
+    // tau and the bra's part of Q's right-hand side: V8 = -8 N D, D = T - S_k;
+    // 4 tau = 12 tr(M A_k) + 1.5 <-8 N, Bi> + <D, V8>
+    R Z[V], W[TR], eta2;
     {
-        R Mt[tri(N)];
-        const R fb = 1.5 * Fb, fk = 1.5 * Fk, sb = 1.5 * ovb, sk = 1.5 * ovk;
+        R D[V];
 #pragma unroll
-        for (int t = 0; t < tri(N); ++t) Mt[t] = ovb * (6.0 * kr[KL::Np + t] + W[t]);
-        sandwich_seeded<N>(Bi, Mt, [&](int t) { return accH.g(t) - fb * Bi[t]; },
-                           [&](int t, R v) { accH.g(t) = v; });
+        for (int t = 0; t < V; ++t) D[t] = T[t] - b(BL::S + t);
+        R dg = R(0.0), od = R(0.0);
 #pragma unroll
-        for (int t = 0; t < tri(N); ++t) W[t] = ovk * (6.0 * b(BL::Nk + t) + W[t]);
-        // S parts: Bi (-1.5 ov B) Bi = -1.5 ov Bi
-        sandwich_seeded<N>(Bi, W, [&](int t) { return -(fk * Bi[t]); },
-                           [&](int t, R v) { ko.put(t, v, -(sk * Bi[t])); });
+        for (int i = 0; i < N; ++i)
 #pragma unroll
-        for (int t = 0; t < tri(N); ++t) accS.g(t) = accS.g(t) - sb * Bi[t];
+            for (int k = 0; k <= i; ++k) {
+                // each element of N is read once and used for the three columns
+                const R a = b(BL::N8 + sx(i, k));
+                W[sx(i, k)] = -1.5 * a;
+                if (i == k)
+                    dg = (i == 0) ? a * Bi[0] : dg + a * Bi[sx(i, k)];
+                else
+                    od = (i == 1) ? a * Bi[sx(1, 0)] : od + a * Bi[sx(i, k)];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    // element (i, k) is the first of row i when k = 0, and the first of row k when i = k = 0
+                    if (k == 0)
+                        Z[3 * i + c] = a * D[c];
+                    else
+                        Z[3 * i + c] += a * D[3 * k + c];
+                    if (k < i) Z[3 * k + c] += a * D[3 * i + c];
+                }
+            }
+        R e0 = D[0] * Z[0], e1 = D[1] * Z[1], e2 = D[2] * Z[2];
+#pragma unroll
+        for (int i = 1; i < N; ++i) {
+            e0 += D[3 * i] * Z[3 * i];
+            e1 += D[3 * i + 1] * Z[3 * i + 1];
+            e2 += D[3 * i + 2] * Z[3 * i + 2];
+        }
+        eta2 = 12.0 * b(BL::tMA) + (1.5 * (dg + 2.0 * od) + (e0 + e1 + e2));
     }
-    // Qk = Bi (Z' - 4 A_l' M Y); Ql = Bi (Z' + 4 A_k M Y) = Qk + 4 M Y (the
-    // difference of the two right-hand sides is 4 B M Y and Bi B = I)
-    R Dl[3 * N];
-#pragma unroll
-    for (int t = 0; t < 3 * N; ++t) Dl[t] = T[t] - kr[KL::Sp + t];
-    // the ket and bra matrices below are read once per element and used for
-    // the three columns; each output's products are summed in the same order
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            const R a = kr[KL::AMn4 + i * N + k];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) Z[3 * i + c] += a * Y[3 * k + c];
-        }
-    R Qk[3 * N], Ql[3 * N];
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R s = Bi[sx(i, 0)] * Z[c];
-#pragma unroll
-            for (int k = 1; k < N; ++k) s += Bi[sx(i, k)] * Z[3 * k + c];
-            Qk[3 * i + c] = s;
-        }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R s = Qk[3 * i + c];
-#pragma unroll
-            for (int k = 0; k < N; ++k) s += cs.M4[i * N + k] * Y[3 * k + c];
-            Ql[3 * i + c] = s;
-        }
-    // H: bra s += 2 ovb A_k Qk - 2 Fb Y, ket 2 ovk A_l' Ql + 2 Fk Y ; S: -2 ovb Y, +2 ovk Y
     {
-        const R ob2 = 2.0 * ovb, fb2 = 2.0 * Fb, ok2 = 2.0 * ovk, fk2 = 2.0 * Fk;
+        R sg = R(0.0);
 #pragma unroll
         for (int i = 0; i < N; ++i) {
-            R s[3], t[3];
-            {
-                const R a = b(BL::A + sx(i, 0)), ap = kr[KL::Ap + sx(i, 0)];
+            const R eq = cs.efs * cs.q[i];
+            sg = (i == 0) ? eq * T[2] : sg + eq * T[3 * i + 2];
+            Z[3 * i + 2] -= eq;
+        }
+        eta2 -= 2.0 * sg;
+    }
+    mid(2);
+    const R rho = coulomb_grad<N>(Bi, T, cs, Z, W);
+    eta2 += 2.0 * rho;
+    eta2_out = eta2;
+    const R et = eta2 - E2;
+    if (!RP::odd) out.scalar(et);
+    // X = Bi W Bi - 1.5 et Bi - Q' T^T - T Q'^T with Q' = Q + et T / 2 (the T T^T
+    // part of et U folded into the outer products); g = Q' + et T / 2
+    R Q[V];
+    const R eh = 0.5 * et;
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    s[c] = a * Qk[c];
-                    t[c] = ap * Ql[c];
-                }
-            }
+    for (int i = 0; i < N; ++i)
 #pragma unroll
-            for (int k = 1; k < N; ++k) {
-                const R a = b(BL::A + sx(i, k)), ap = kr[KL::Ap + sx(i, k)];
+        for (int c = 0; c < 3; ++c) {
+            R s = eh * T[3 * i + c];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    s[c] += a * Qk[3 * k + c];
-                    t[c] += ap * Ql[3 * k + c];
-                }
-            }
+            for (int k = 0; k < N; ++k) s += Bi[sx(i, k)] * Z[3 * k + c];
+            Q[3 * i + c] = s;
+        }
+    const R e15 = 1.5 * et;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        R col[N];  // column j of W Bi
+#pragma unroll
+        for (int a = 0; a < N; ++a) {
+            R s = W[sx(a, 0)] * Bi[sx(0, j)];
+#pragma unroll
+            for (int k = 1; k < N; ++k) s += W[sx(a, k)] * Bi[sx(k, j)];
+            col[a] = s;
+        }
+#pragma unroll
+        for (int i = j; i < N; ++i) {
+            R s = -(e15 * Bi[sx(i, j)]);
+#pragma unroll
+            for (int a = 0; a < N; ++a) s += Bi[sx(i, a)] * col[a];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const R y = Y[3 * i + c];
-                accH.s(3 * i + c) = (accH.s(3 * i + c) - fb2 * y) + ob2 * s[c];
-                accS.s(3 * i + c) = accS.s(3 * i + c) - ob2 * y;
-                ko.put(tri(N) + 1 + 3 * i + c, ok2 * t[c] + fk2 * y, ok2 * y);
+                s -= Q[3 * i + c] * T[3 * j + c];
+                s -= T[3 * i + c] * Q[3 * j + c];
             }
+            const int t = sx(i, j), u = t < V ? t : 0;
+            if (t < RP::lead)
+                out.h2(t, t, TR + 1 + t, s, Q[u] + eh * T[u]);
+            else
+                out.h1(t, s);
         }
     }
-    // H: Rk = ovb Qk - Fb/2 Dk, acc += Rk Dk^T + Dk Rk^T ; Rl = ovk Ql + Fk/2 Dl, ket -= Rl Dl^T + Dl Rl^T
-    // S: bra -= ovb Dk Dk^T, ket -= ovk Dl Dl^T
-    {
-        const R fbh = 0.5 * Fb, fkh = 0.5 * Fk;
 #pragma unroll
-        for (int t = 0; t < 3 * N; ++t) {
-            const R dk = b(BL::S + t) - T[t];
-            T[t] = dk;
-            Qk[t] = ovb * Qk[t] - fbh * dk;
-            Ql[t] = ovk * Ql[t] + fkh * Dl[t];
+    for (int q = 0; q < RP::left / 2; ++q) {
+        const int u = RP::lead + 2 * q;
+        out.h2(RP::lead + q, TR + 1 + u, TR + 2 + u, Q[u] + eh * T[u], Q[u + 1] + eh * T[u + 1]);
+    }
+    if (RP::odd) out.h2(RP::count - 1, TR + V, RP::scalar, Q[V - 1] + eh * T[V - 1], et);
+    return ok;
+}
+
+// The gradient of one side from its raw sums.  r: raw fields (H, 2 S, or their
+// combination H - 2 E S), A, s, e = A s of the function in the frame of the sums:
+//   dF/dA = G + (g s^T + s g^T) / 2 - F s s^T + 0.75 F A^-1,   dF/ds = A g - 2 F e
+// with G = r_G / 2, F = r_scalar / 2 and g = r_g.  o: Part<N> fields.
+#pragma nv_exec_check_disable
+template <int N, typename R, typename RAW, typename FA, typename FS, typename FE>
+NECG_HD void fold_raw(const RAW &r, const FA &A, const FS &s, const FE &e, R (&o)[tri(N) + 1 + 3 * N]) {
+    constexpr int TR = tri(N);
+    const R F = 0.5 * r(TR);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+            R v = R(0.0);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const R si = s(3 * i + c), sj = s(3 * j + c);
+                v += r(TR + 1 + 3 * i + c) * sj + si * r(TR + 1 + 3 * j + c) - 2.0 * F * si * sj;
+            }
+            o[sx(i, j)] = 0.5 * (r(sx(i, j)) + v);
+        }
+    o[TR] = 0.75 * F;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = -2.0 * F * e(3 * i + c);
+#pragma unroll
+            for (int k = 0; k < N; ++k) v += A(sx(i, k)) * r(TR + 1 + 3 * k + c);
+            o[TR + 1 + 3 * i + c] = v;
+        }
+}
+
+// The bra's explicit share of dh through tau, added to its combined raw sums r:
+// tau depends on A_k and e_k = A_k S_k directly (not through B and e), so that
+// with the bra's raw S sums s = (-U, 1, T) and p = M e_k
+//   dh/dA_k |_{e_k} += 2 (3 M s_1 + 2 (M A s_U + s_U A M) + 2 (s_T p^T + p s_T^T))
+//   dh/de_k         += -8 M (e_k s_1 - A s_T)
+// (r's G is held twice).
+#pragma nv_exec_check_disable
+template <int N, typename R, typename SRAW, typename FA, typename FE>
+NECG_HD void explicit_tau(const SRAW &sr, const FA &A, const FE &e, const Consts<N> &cs,
+                          R (&r)[tri(N) + 1 + 3 * N]) {
+    constexpr int TR = tri(N);
+    const R s1 = sr(TR);
+    R y[3 * N];  // e s_1 - A s_T
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = e(3 * i + c) * s1;
+#pragma unroll
+            for (int k = 0; k < N; ++k) v -= A(sx(i, k)) * sr(TR + 1 + 3 * k + c);
+            y[3 * i + c] = v;
+        }
+    R MA[N * N], p[3 * N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            R v = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) v += cs.M[i * N + k] * A(sx(k, j));
+            MA[i * N + j] = v;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = R(0.0), g = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                v += cs.M[i * N + k] * e(3 * k + c);
+                g += cs.M[i * N + k] * y[3 * k + c];
+            }
+            p[3 * i + c] = v;
+            r[TR + 1 + 3 * i + c] -= 8.0 * g;
         }
     }
 #pragma unroll
     for (int i = 0; i < N; ++i)
 #pragma unroll
         for (int j = 0; j <= i; ++j) {
-            R s = accH.g(sx(i, j));  // the products fuse into the accumulator
-            R t = Ql[3 * i] * Dl[3 * j] + Dl[3 * i] * Ql[3 * j];
-            R dd = T[3 * i] * T[3 * j], ee = Dl[3 * i] * Dl[3 * j];
+            R v = 3.0 * cs.M[i * N + j] * s1;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                s += Qk[3 * i + c] * T[3 * j + c];
-                s += T[3 * i + c] * Qk[3 * j + c];
-            }
+            for (int k = 0; k < N; ++k)
+                v += 2.0 * (MA[i * N + k] * sr(sx(k, j)) + sr(sx(i, k)) * MA[j * N + k]);
 #pragma unroll
-            for (int c = 1; c < 3; ++c) {
-                t += Ql[3 * i + c] * Dl[3 * j + c] + Dl[3 * i + c] * Ql[3 * j + c];
-                dd += T[3 * i + c] * T[3 * j + c];
-                ee += Dl[3 * i + c] * Dl[3 * j + c];
-            }
-            accH.g(sx(i, j)) = s;
-            accS.g(sx(i, j)) = accS.g(sx(i, j)) - ovb * dd;
-            ko.add(sx(i, j), -t, -(ovk * ee));
+            for (int c = 0; c < 3; ++c)
+                v += 2.0 * (sr(TR + 1 + 3 * i + c) * p[3 * j + c] + p[3 * i + c] * sr(TR + 1 + 3 * j + c));
+            r[sx(i, j)] += 4.0 * v;
         }
+}
+
+// One side's fields in an array, read as a functor.
+template <typename R> struct FieldsOf {
+    const R *p;
+    NECG_HD const R &operator()(int f) const { return p[f]; }
+};
+
+// Raw values of one term kept in arrays (unit weight: ov included).
+template <int N, typename R> struct RawValues {
+    static constexpr int PS = tri(N) + 1 + 3 * N;
+    R h[PS], s[PS], ov;
+    NECG_HD void begin(R o) { ov = o; }
+    NECG_HD void s2(int, int fa, int fb, R va, R vb) {
+        s[fa] = ov * va;
+        s[fb] = ov * vb;
+    }
+    NECG_HD void h2(int, int fa, int fb, R va, R vb) {
+        h[fa] = ov * va;
+        h[fb] = ov * vb;
+    }
+    NECG_HD void s1(int f, R v) { s[f] = ov * v; }
+    NECG_HD void h1(int f, R v) { h[f] = ov * v; }
+    NECG_HD void scalar(R e2) {
+        h[tri(N)] = ov * e2;
+        s[tri(N)] = ov;
+    }
+};
+
+// Gradients of h and of ov of one term, with respect to the bra (oH, oS; Part<N>
+// fields) and, when KET, to the transformed ket (A_l', s_l').
+#pragma nv_exec_check_disable
+template <int N, bool KET, typename R, typename BA, typename KA>
+NECG_HD bool term_gradients(const BA &b, const KA &kr, const Consts<N> &cs, R (&bH)[tri(N) + 1 + 3 * N],
+                            R (&bS)[tri(N) + 1 + 3 * N], R (&kH)[tri(N) + 1 + 3 * N],
+                            R (&kS)[tri(N) + 1 + 3 * N], R &h, R &ov) {
+    using BL = BraLayout<N>;
+    using KL = KetLayout<N>;
+    constexpr int PS = tri(N) + 1 + 3 * N;
+    RawValues<N, R> v;
+    R eta2;
+    const bool ok = term_raw<N>(b, kr, cs, R(0.0), v, eta2, ov);
+    h = 0.5 * ov * eta2;
+    const auto A = [&](int t) { return b(BL::A + t); };
+    const auto s = [&](int t) { return b(BL::S + t); };
+    const auto e = [&](int t) { return b(BL::AS + t); };
+    R s2[PS];  // the raw fields of ov alone in the scale of H's (twice G and scalar, once g): 2 S
+#pragma unroll
+    for (int f = 0; f < PS; ++f) s2[f] = 2.0 * v.s[f];
+    if (KET) {
+        const auto Ak = [&](int t) { return kr[KL::Ap + t]; };
+        const auto sk = [&](int t) { return kr[KL::Sp + t]; };
+        const auto ek = [&](int t) { return kr[KL::ASp + t]; };
+        fold_raw<N>(FieldsOf<R>{v.h}, Ak, sk, ek, kH);
+        fold_raw<N>(FieldsOf<R>{s2}, Ak, sk, ek, kS);
+    }
+    explicit_tau<N>(FieldsOf<R>{v.s}, A, e, cs, v.h);
+    fold_raw<N>(FieldsOf<R>{v.h}, A, s, e, bH);
+    fold_raw<N>(FieldsOf<R>{s2}, A, s, e, bS);
+    return ok;
+}
+
+// One unordered term of the fused pass with both gradients folded per term: the
+// bra's into the accumulators (weight wb), the ket's out through ko.put(f, vH,
+// vS) (weight wk), for callers that keep gradients and not raw sums (the
+// host emulation of the passes).
+#pragma nv_exec_check_disable
+template <int N, typename R, typename BA, typename KA, typename ACC, typename KOUT>
+NECG_HD bool term_fused(const BA &b, const KA &kr, const Consts<N> &cs, R wb, R wk, ACC &accH, ACC &accS,
+                        KOUT &ko, R &h, R &ov) {
+    constexpr int TR = tri(N), PS = TR + 1 + 3 * N;
+    R bH[PS], bS[PS], kH[PS], kS[PS];
+    const bool ok = term_gradients<N, true>(b, kr, cs, bH, bS, kH, kS, h, ov);
+#pragma unroll
+    for (int t = 0; t < TR; ++t) {
+        accH.g(t) += wb * bH[t];
+        accS.g(t) += wb * bS[t];
+    }
+    accH.d() += wb * bH[TR];
+    accS.d() += wb * bS[TR];
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) {
+        accH.s(t) += wb * bH[TR + 1 + t];
+        accS.s(t) += wb * bS[TR + 1 + t];
+    }
+#pragma unroll
+    for (int f = 0; f < PS; ++f) ko.put(f, wk * kH[f], wk * kS[f]);
+    return ok;
+}
+
+// The same for the gradient of h - E ov.
+#pragma nv_exec_check_disable
+template <int N, typename R, typename BA, typename KA, typename ACC, typename KOUT>
+NECG_HD bool term_sym(const BA &b, const KA &kr, const Consts<N> &cs, R E, R wb, R wk, ACC &acc, KOUT &ko) {
+    constexpr int TR = tri(N), PS = TR + 1 + 3 * N;
+    R bH[PS], bS[PS], kH[PS], kS[PS], h, ov;
+    const bool ok = term_gradients<N, true>(b, kr, cs, bH, bS, kH, kS, h, ov);
+#pragma unroll
+    for (int t = 0; t < TR; ++t) acc.g(t) += wb * (bH[t] - E * bS[t]);
+    acc.d() += wb * (bH[TR] - E * bS[TR]);
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) acc.s(t) += wb * (bH[TR + 1 + t] - E * bS[TR + 1 + t]);
+#pragma unroll
+    for (int f = 0; f < PS; ++f) ko.put(f, wk * (kH[f] - E * kS[f]));
     return ok;
 }
 
@@ -1044,13 +959,13 @@ NECG_HD bool term_fused(const BA &b, const KA &kr, const Consts<N> &cs, R wb, R 
 template <int N, typename R, typename KA, typename KB>
 NECG_HD bool term_dipole(const KA &kb, const KB &kr, const Consts<N> &cs, R (&T)[3 * N], R &ov) {
     using KL = KetLayout<N>;
-    R Bi[tri(N)], prinv;
+    R Bi[tri(N)], m32;
     bool ok;
     {
         R B[tri(N)];
 #pragma unroll
         for (int t = 0; t < tri(N); ++t) B[t] = kb[KL::Ap + t] + kr[KL::Ap + t];
-        ok = chol_inverse<N>(B, Bi, prinv);
+        ok = spd_inverse<N>(B, Bi, m32);
     }
     R e[3 * N];
 #pragma unroll
@@ -1067,8 +982,7 @@ NECG_HD bool term_dipole(const KA &kb, const KB &kr, const Consts<N> &cs, R (&T)
     R i3 = e[0] * T[0];
 #pragma unroll
     for (int t = 1; t < 3 * N; ++t) i3 += e[t] * T[t];
-    const R p3 = prinv * prinv * prinv;
-    ov = cs.sqrt8n * kb[KL::pre] * kr[KL::pre] * p3 * exp(i3 - kb[KL::i2] - kr[KL::i2]);
+    ov = cs.sqrt8n * kb[KL::pre] * kr[KL::pre] * m32 * exp(i3 - kb[KL::i2] - kr[KL::i2]);
     return ok;
 }
 

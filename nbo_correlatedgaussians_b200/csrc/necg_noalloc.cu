@@ -61,6 +61,14 @@ int scratch_address(double **out) {
 
 size_t up32(size_t v) { return (v + 31) / 32 * 32; }  // 256-byte alignment in doubles
 
+// Doubles set aside per (l, P) in the scratch layout, which fixes the largest
+// accepted K (include/necg.h states it): at least the ket record's size.
+int ket_room(int n) {
+    const int t = n * (n + 1) / 2;
+    const int room = (2 * t + 6 * n + n * n + 6 + 1) & ~1;
+    return room > necg::ket_record_size(n) ? room : necg::ket_record_size(n);
+}
+
 struct Carve {
     size_t bra, ket, part, H, S, rows, scal, status, tiles, sml, sms, scvv, total;
 };
@@ -73,7 +81,7 @@ Carve carve(int n, int nst, int K) {
     const int ntiles = necg::energy_tile_count(K, kLcEnergy);
     size_t off = 0;
     c.bra = off;    off = up32(off + (size_t)necg::bra_record_size(n) * k);
-    c.ket = off;    off = up32(off + (size_t)necg::ket_record_size(n) * k * nst);
+    c.ket = off;    off = up32(off + (size_t)ket_room(n) * k * nst);
     c.part = off;   off = up32(off + (size_t)necg::part_stride(n) * k * nlc);
     c.H = off;      off = up32(off + k * k);
     c.S = off;      off = up32(off + k * k);

@@ -262,8 +262,10 @@ def boys_f0(z) -> tuple[np.ndarray, np.ndarray]:
 
 
 def term_flops(n: int) -> dict:
-    """Algorithmic FLOPs per (k, l, P) term: energy, ordered gradient, and one
-    unordered term of the symmetric ("sym") and fused ("fused") passes."""
+    """FP64 operations per (k, l, P) term: energy, ordered gradient, and one
+    unordered term of the symmetric ("sym") and fused ("fused") passes -- in the
+    direct formulation (the fixed measure rates are quoted by) and, under
+    "<name>_executed", what the kernels execute."""
     L = _lib.lib()
     out = {}
     for which, name in ((0, "energy"), (1, "grad"), (2, "sym"), (3, "fused")):
@@ -271,4 +273,5 @@ def term_flops(n: int) -> dict:
         tot = L.necg_term_flops(int(n), which, ctypes.byref(s))
         out[name] = int(tot)
         out[name + "_special"] = int(s.value)
+        out[name + "_executed"] = int(L.necg_term_flops(int(n), which + 4, None))
     return out
