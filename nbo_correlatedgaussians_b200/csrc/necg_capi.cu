@@ -138,7 +138,7 @@ void free_all(necg_handle *h) {
                     h->d_S, h->d_rows, h->d_scal, h->d_x, h->d_g, h->d_f, h->d_status,
                     h->d_tiles, h->d_pinv, h->d_kcnt, h->d_ksrc, h->d_kcoef, h->d_stiles,
                     h->d_stile_start, h->d_psym, h->d_sgroups, h->d_qcount, h->d_bgroups,
-                    h->d_Hp, h->d_Sp, h->d_xsym, h->d_urange};
+                    h->d_Hp, h->d_Sp, h->d_xsym, h->d_urange, h->d_dipcls};
     for (void *p : ptrs) pool_free(h, p);
 }
 
@@ -411,6 +411,58 @@ int setup_symmetric(necg_handle *h) {
     return NECG_OK;
 }
 
+// Classes of the dipole's nst^2 terms (Pe, P) of a pair (dipole_group_kernel):
+// Q = P Pe^-1, when every Q is in the set and the shift maps follow the
+// coordinate maps (sms = kron(sml^-1, I3), which also gives Pe^-1).  Larger sets
+// than 128 terms keep the general path (the search for Q grows as nst^3).
+int setup_dipole(necg_handle *h) {
+    const int n = h->n, nst = h->nst, m = 3 * n, nn = n * n;
+    if (nst < 2 || nst > 128) return NECG_OK;
+    std::vector<double> inv((size_t)nst * nn);
+    for (int p = 0; p < nst; ++p) {
+        const double *S = &h->sms[(size_t)p * m * m], *P = &h->sml[(size_t)p * nn];
+        double *I = &inv[(size_t)p * nn];
+        for (int i = 0; i < n; ++i)
+            for (int j = 0; j < n; ++j) I[i * n + j] = S[(3 * i) * m + 3 * j];
+        for (int r = 0; r < m; ++r)  // sms = kron(I, I3) ...
+            for (int c = 0; c < m; ++c)
+                if (fabs(S[r * m + c] - (r % 3 == c % 3 ? I[(r / 3) * n + c / 3] : 0.0)) > 1e-12) return NECG_OK;
+        for (int i = 0; i < n; ++i)  // ... and I = P^-1
+            for (int j = 0; j < n; ++j) {
+                double v = 0.0;
+                for (int k = 0; k < n; ++k) v += I[i * n + k] * P[k * n + j];
+                if (fabs(v - (i == j ? 1.0 : 0.0)) > 1e-12) return NECG_OK;
+            }
+    }
+    std::vector<double> cls((size_t)nst * (nn + 1), 0.0), Q(nn);
+    for (int pe = 0; pe < nst; ++pe)
+        for (int p = 0; p < nst; ++p) {
+            for (int i = 0; i < n; ++i)
+                for (int j = 0; j < n; ++j) {
+                    double v = 0.0;
+                    for (int k = 0; k < n; ++k) v += h->sml[(size_t)p * nn + i * n + k] * inv[(size_t)pe * nn + k * n + j];
+                    Q[i * n + j] = v;
+                }
+            int q = 0;
+            for (; q < nst; ++q) {
+                bool same = true;
+                for (int x = 0; x < nn && same; ++x) same = fabs(Q[x] - h->sml[(size_t)q * nn + x]) < 1e-12;
+                if (same) break;
+            }
+            if (q == nst) return NECG_OK;  // not closed under products
+            double *c = &cls[(size_t)q * (nn + 1)];
+            const double w = h->scvv[pe] * h->scvv[p];
+            c[0] += w;
+            for (int x = 0; x < nn; ++x) c[1 + x] += w * inv[(size_t)pe * nn + x];
+        }
+    int rc = dalloc(h, &h->d_dipcls, cls.size());
+    if (rc) return rc;
+    cudaStream_t ls = lib_stream(h);
+    CK(cudaMemcpyAsync(h->d_dipcls, cls.data(), cls.size() * sizeof(double), cudaMemcpyHostToDevice, ls));
+    CK(cudaStreamSynchronize(ls));  // cls ends with this scope
+    return NECG_OK;
+}
+
 LaunchArgs base_args(necg_handle *h, int K) {
     LaunchArgs a;
     memset(&a, 0, sizeof(a));
@@ -439,6 +491,7 @@ LaunchArgs base_args(necg_handle *h, int K) {
     a.pinv = h->d_pinv;
     a.kmap = necg::RawMap{h->d_kcnt, h->d_ksrc, h->d_kcoef, h->kmaxnz, h->kfold};
     a.minb_s = h->minb_s;
+    a.dip_cls = h->d_dipcls;
     return a;
 }
 
@@ -597,6 +650,7 @@ int necg_create(int n, int nst, int K_max, double efs, const double *mass_host,
     if (!rc) rc = cuda_fail(cudaMemcpyAsync(h->d_scvv, h->scvv.data(), h->scvv.size() * 8, cudaMemcpyHostToDevice, ls));
     if (!rc) rc = cuda_fail(cudaMemsetAsync(h->d_status, 0, 16, ls));
     if (!rc) rc = setup_symmetric(h);
+    if (!rc) rc = setup_dipole(h);
     // the workspace is allocated in the library stream's order: make it usable on every stream
     if (!rc) rc = cuda_fail(cudaStreamSynchronize(ls));
     if (rc) {
@@ -943,7 +997,7 @@ int necg_dipole(necg_handle *h, int K, const double *iv_dev, const double *C_dev
     a.iv = iv_dev;
     a.C = C_dev;
     if (necg::launch_prep(a, st)) return NECG_ERR_UNSUPPORTED;
-    necg::launch_dipole(a, h->d_part, comps_dev, dipole_dev, st);
+    necg::launch_dipole(a, h->d_part, cap, comps_dev, dipole_dev, st);
     return finish_launch();
 }
 

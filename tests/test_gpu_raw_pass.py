@@ -126,3 +126,35 @@ def test_executed_counts_below_the_direct_formulation(n):
     from nbo_correlatedgaussians_b200.engine import term_flops
     t = term_flops(n)
     assert t["energy_executed"] < t["grad_executed"] < t["sym_executed"] < t["fused_executed"] < t["fused"]
+
+
+def _subset(system, K, keep, shift=None):
+    from nbo_correlatedgaussians_b200 import synth
+    p = synth.make_problem(system, K, 31 * K)
+    p.C = np.random.default_rng(K).normal(size=K)
+    p.sml, p.sms, p.scvv = p.sml[keep], p.sms[keep], np.random.default_rng(1).uniform(0.5, 1.5, len(keep))
+    if shift:
+        p.sms = np.stack([np.kron(m.T, np.eye(3)) for m in p.sml])
+    return p
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("system,K,keep,shift", [
+    ("LiH", 1, range(24), None), ("LiH", 33, range(24), None), ("LiH", 40, [0, 1, 2, 3, 4, 5], None),  # groups
+    ("LiH", 20, [0, 3, 4], None),              # three-cycles: a group without involutions
+    ("LiH", 20, [0, 1, 2], None),              # not closed under products: every (Pe, P)
+    ("H2", 45, [0, 1, 2, 3], None), ("H2", 45, [0, 3], None), ("H2", 30, [2], None),
+    ("H2", 30, [0, 1, 2, 3], "sml^T"),         # shift maps of their own: every (Pe, P)
+    ("He", 70, [0, 1], None)])
+def test_dipole_classes(system, K, keep, shift):
+    """The dipole by classes of a group and by every pair of terms otherwise, unequal
+    weights, against the oracle (the tolerance of the emulation's dipole test)."""
+    p = _subset(system, K, list(keep), shift)
+    comps_o, dip_o = Oracle.from_problem(p).dipole(p.iv, p.C, nthreads=8)
+    eng = engine(p)
+    for lc in (1, 2, 7):
+        eng.set_tiles(lc, 4)
+        comps, dip = eng.dipole(p.iv, p.C)
+        scale = max(np.max(np.abs(comps_o)), 1e-300)
+        assert np.max(np.abs(comps - comps_o)) <= 1e-11 * scale
+        assert np.max(np.abs(dip - dip_o)) <= 1e-11 * max(np.max(np.abs(dip_o)), scale)
