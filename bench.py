@@ -78,9 +78,9 @@ def parse():
     return ap.parse_args()
 
 
-DEFAULT_TILES = {"lc_e": 2, "minb_e": 16, "lc_g": 4, "minb_g": 8, "sym": 2, "lc_s": 2, "minw_s": 268}
-# the fused-pass variant measured fastest for other n (n = 3: one-warp blocks, 12 per SM)
-DEFAULT_FUSED = {3: {"lc_s": 2, "minw_s": 122}}
+DEFAULT_TILES = {"lc_e": 2, "minb_e": 16, "lc_g": 4, "minb_g": 8, "sym": 2, "lc_s": 2, "minw_s": 248}
+# the fused-pass variant measured fastest for other n (n = 3: one-warp blocks, 16 per SM)
+DEFAULT_FUSED = {3: {"lc_s": 4, "minw_s": 16}}
 PASS_MODE = {"ordered": 0, "symmetric": 1, "fused": 2}
 # FP64 FLOPs per (k, l, P) term (FMA = 2; each div/sqrt/rsqrt/exp = 1), frozen at
 # the counts the kernels' own templates gave when the fused pass was first

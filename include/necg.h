@@ -87,18 +87,11 @@ int necg_set_variant(necg_handle *h, int minw_energy, int minw_grad);
  * n <= 5; otherwise NECG_ERR_UNSUPPORTED.  lc: kets per tile (1..64); minw: 8,
  * 12 or 16 warps per SM, and for mode 2 also 108 and 112 (8 and 12 warps with
  * the ket records re-read at each use instead of held in registers), 118 and
- * 122 (the same with each warp's ket record staged in shared memory), 208
- * (as 108, with the 8 warps of an SM in one block stepping through their terms
- * together), 218 (as 208, with the block's bra records staged in shared
- * memory), 228 (as 218, each warp's ket records staged too, the next one
- * copied while the current term runs), 248 (as 228 without the barrier after
- * every term), 258 and 268 (as 228, with warps 4-7 taking their per-term
- * barrier inside the term -- after the pair's Cholesky factor, inverse and
- * overlap for 258, after the kinetic and field terms (and, for n <= 3, the
- * Coulomb sum) for 268 -- so the two
- * warps of each scheduler run different parts of the term), 222 and 232 (218
- * and 228 with 12 warps per block; NECG_ERR_UNSUPPORTED where their shared
- * memory does not fit, n = 5).  Set by the autotuner. */
+ * 122 (the same with each warp's ket record staged in shared memory), and
+ * 248 and 232 (blocks of 8 and 12 warps, one block per SM, with bra and ket
+ * records in shared memory; 232 is NECG_ERR_UNSUPPORTED where its shared memory
+ * does not fit, n = 5).  208, 218, 228, 258 and 268 are accepted and run as 248,
+ * 222 as 232.  Set by the autotuner. */
 int necg_set_symmetric(necg_handle *h, int mode, int lc, int minw);
 
 /* Fused pass (mode 2) with one-warp tiles (variants below 200): split the nst

@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(128) batch_prep_kernel(PlanPtrs p) {
             const int q = find_inst(p.pref_bra, ninst, i);
             const InstDesc &d = p.inst[q];
             const int k = i - p.pref_bra[q];
-            BATCH_SWITCH(d.n, prep_bra_one<N>(d.iv, d.K, consts_of<N>(d), d.bra, k));
+            BATCH_SWITCH(d.n, prep_bra_at<N>(d.iv + (size_t)k * (tri(N) + 3 * N), consts_of<N>(d), bra_at<N>(d.bra, k), 32));
         } else {
             const int j = i - nb;
             const int q = find_inst(p.pref_ket, ninst, j);
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(32) batch_energy_kernel(PlanPtrs p) {
         int k, l0, lend;
         if (energy_lane_range(e.y, e.z, lane, d.lc_e, d.K, k, l0, lend)) {
             int bad = 0, fl = 0;
-            BATCH_SWITCH(d.n, fl = (energy_lane<N, double>(BraRef{d.bra + k, (size_t)d.K}, DevKetB{d.ket}, k,
+            BATCH_SWITCH(d.n, fl = (energy_lane<N, double>(BraRef{bra_at<N>(d.bra, k)}, DevKetB{d.ket}, k,
                                                            l0, lend, d.K, d.nst, consts_of<N>(d), d.H,
                                                            d.S, nullptr, nullptr, bad)));
             flag_inst(d.status, fl, bad);
@@ -199,9 +199,8 @@ __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
 // tiles first) and over each instance's groups (one 32-row block, 8 consecutive
 // ket chunks, one per warp).  The warps of a block work on the same instance and
 // bras; the group's bras are staged in shared memory once, each warp's ket
-// records too, in two buffers (fsym_tile with BSYNC, SBRA, SKET), and the warps
-// meet only at the group's barriers (no barrier per term, as the single-
-// instance variant 248).  Shared memory is sized for n = kMaxN.
+// records too, in two buffers (fsym_tile with SBRA, SKET), and the warps meet only
+// at the group's ends.  Shared memory is sized for n = kMaxN.
 template <int N> __host__ __device__ constexpr int bfused_warp_smem() {
     return 2 * Part<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
 }
@@ -220,15 +219,12 @@ __device__ __forceinline__ void batch_fused_group(const InstDesc &d, int2 gr, do
     const int K = d.K, kb = gr.x, lc = gr.y + w;
     const int last = min(kb * 32 + 31, K - 1);
     const bool idle = lc * d.lc_s > last;
-    for (int i = threadIdx.x; i < BS * 32; i += 256) {
-        const int f = i >> 5, kk = min(kb * 32 + (i & 31), K - 1);
-        sbra[i] = d.bra[(size_t)f * K + kk];
-    }
+    const double *bk = bra_at<N>(d.bra, kb * 32);
+    for (int i = threadIdx.x; i < BS * 32; i += 256) sbra[i] = bk[(i & ~31) + min(i & 31, K - 1 - kb * 32)];
     __syncthreads();
     double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * 2 * PS * 32;
-    fsym_tile<N, true, true, true, true, 3>(d.stile_start[kb] + lc, make_int2(kb, lc), d.lc_s, K, d.nst,
-                                            consts_of<N>(d), d.bra, d.ket, d.C, d.kmap, d.H, d.S, part_b, part_k,
-                                            d.status, sm, idle, sbra);
+    fsym_tile<N, true, true, true>(d.stile_start[kb] + lc, make_int2(kb, lc), d.lc_s, K, d.nst, consts_of<N>(d),
+                                   d.bra, d.ket, d.C, d.kmap, d.H, d.S, part_b, part_k, d.status, sm, idle, sbra);
     __syncthreads();  // sbra and the warps' areas are reused by the next group
 }
 
@@ -396,7 +392,7 @@ __global__ void __launch_bounds__(32) batch_grad_kernel(PlanPtrs p) {
             bool ok = true;
             BATCH_SWITCH(d.n, {
                 SmemAcc<N> accH{sacc + lane}, accS{sacc + Part<N>::size * 32 + lane};
-                ok = grad_lane<N, double>(BraRef{d.bra + k, (size_t)d.K}, DevKetB{d.ket}, l0, l1, d.nst,
+                ok = grad_lane<N, double>(BraRef{bra_at<N>(d.bra, k)}, DevKetB{d.ket}, l0, l1, d.nst,
                                           consts_of<N>(d), 1.0, d.scal[0],
                                           d.part + (size_t)lc * Part<N>::size * d.K + k, (size_t)d.K, accH, accS);
             });
@@ -432,11 +428,11 @@ template <bool FUSED> __global__ void __launch_bounds__(128) batch_reduce_kernel
         if (FUSED) {
             BATCH_SWITCH(d.n, {
                 double o[Part<N>::size];
-                finish_one<N>(d.part, d.K, d.bra, consts_of<N>(d), d.kmap.fold, k, o);
-                fin = fields_to_grad<N>(o, d.bra, d.K, sc, d.g, k);
+                finish_one<N>(d.part, d.K, bra_at<N>(d.bra, k), consts_of<N>(d), d.kmap.fold, k, o);
+                fin = fields_to_grad<N>(o, bra_at<N>(d.bra, k), 32, sc, d.g, k);
             });
         } else {
-            BATCH_SWITCH(d.n, fin = grad_reduce_one<N>(d.part, 1, d.K, d.bra, sc, d.g, k));
+            BATCH_SWITCH(d.n, fin = grad_reduce_at<N>(d.part, 1, d.K, bra_at<N>(d.bra, k), 32, sc, d.g, k));
         }
         if (!fin) atomicOr(d.status, 2);
     }

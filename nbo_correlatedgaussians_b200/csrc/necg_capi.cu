@@ -3,7 +3,7 @@
 // A handle owns one particle system's constants (mass, charges, symmetry set)
 // on the device plus the workspace one evaluation needs for bases of up to
 // K_max functions:
-//   bra   BraLayout<n>::size * K_max       per-basis data (structure of arrays)
+//   bra   BraLayout<n>::size * K_max       per-basis data (K_max rounded up to 32)
 //   ket   KetLayout<n>::size * K_max * nst per-(l, P) ket records
 //   part  part_stride(n) * K_max * ceil(K_max / lc_grad)   gradient tile partials
 //   H, S  K_max^2 each (used when the caller passes no H/S)
@@ -415,8 +415,15 @@ int setup_symmetric(necg_handle *h) {
 // Q = P Pe^-1, when every Q is in the set and the shift maps follow the
 // coordinate maps (sms = kron(sml^-1, I3), which also gives Pe^-1).  Larger sets
 // than 128 terms keep the general path (the search for Q grows as nst^3).
-int setup_dipole(necg_handle *h) {
+// Set up by the handle's first dipole outside a stream capture (it allocates and
+// waits; until then the general path runs).
+int setup_dipole(necg_handle *h, cudaStream_t st) {
     const int n = h->n, nst = h->nst, m = 3 * n, nn = n * n;
+    if (h->dip_ready) return NECG_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return NECG_OK;
+    h->dip_ready = true;
     if (nst < 2 || nst > 128) return NECG_OK;
     std::vector<double> inv((size_t)nst * nn);
     for (int p = 0; p < nst; ++p) {
@@ -633,7 +640,7 @@ int necg_create(int n, int nst, int K_max, double efs, const double *mass_host,
     if (!rc) rc = dalloc(h, &h->d_sml, h->sml.size());
     if (!rc) rc = dalloc(h, &h->d_sms, h->sms.size());
     if (!rc) rc = dalloc(h, &h->d_scvv, (size_t)nst);
-    if (!rc) rc = dalloc(h, &h->d_bra, (size_t)necg::bra_record_size(n) * K);
+    if (!rc) rc = dalloc(h, &h->d_bra, (size_t)necg::bra_record_size(n) * ((K + 31) / 32 * 32));
     if (!rc) rc = dalloc(h, &h->d_ket, (size_t)necg::ket_record_size(n) * K * nst);
     if (!rc) rc = dalloc(h, &h->d_part, necg::part_doubles(n, K_max));
     if (!rc) rc = dalloc(h, &h->d_H, K * K);
@@ -650,7 +657,6 @@ int necg_create(int n, int nst, int K_max, double efs, const double *mass_host,
     if (!rc) rc = cuda_fail(cudaMemcpyAsync(h->d_scvv, h->scvv.data(), h->scvv.size() * 8, cudaMemcpyHostToDevice, ls));
     if (!rc) rc = cuda_fail(cudaMemsetAsync(h->d_status, 0, 16, ls));
     if (!rc) rc = setup_symmetric(h);
-    if (!rc) rc = setup_dipole(h);
     // the workspace is allocated in the library stream's order: make it usable on every stream
     if (!rc) rc = cuda_fail(cudaStreamSynchronize(ls));
     if (rc) {
@@ -989,6 +995,7 @@ int necg_dipole(necg_handle *h, int K, const double *iv_dev, const double *C_dev
     cudaStream_t st = (cudaStream_t)stream;
     if ((rc = begin(h, st))) return rc;
     if ((rc = ensure_tiles(h, K, st))) return rc;
+    if ((rc = setup_dipole(h, st))) return rc;
     LaunchArgs a = base_args(h, K);
     // the tile partials reuse the gradient-partial workspace
     const size_t need = (size_t)a.ntiles * (3 * h->n + 1);

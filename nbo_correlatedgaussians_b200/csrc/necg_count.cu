@@ -73,13 +73,13 @@ template <int N, bool KET, bool KE> struct CountOut {
     }
     void s1(int f, CD v) { put(1, f, v); }
     void h1(int f, CD v) { put(0, f, v); }
-    void s2(int, int fa, int fb, CD va, CD vb) {
-        put(1, fa, va);
-        put(1, fb, vb);
+    template <int I> void s2(CD va, CD vb) {
+        put(1, RawPairs<N>::fa(I), va);
+        put(1, RawPairs<N>::fb(I), vb);
     }
-    void h2(int, int fa, int fb, CD va, CD vb) {
-        put(0, fa, va);
-        put(0, fb, vb);
+    template <int I> void h2(CD va, CD vb) {
+        put(0, RawPairs<N>::fa(I), va);
+        put(0, RawPairs<N>::fb(I), vb);
     }
     void scalar(CD e2) {
         put(0, tri(N), e2);

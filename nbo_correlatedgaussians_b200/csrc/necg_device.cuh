@@ -23,12 +23,6 @@ template <int N> struct SmemAcc {
     __device__ __forceinline__ double &s(int t) { return p[(tri(N) + 1 + t) * 32]; }
 };
 
-// Block barrier that warps may reach from different places in the code (the
-// non-aligned form of bar.sync: __syncthreads requires every thread of the
-// block to execute the same barrier instruction).  Every warp of the block
-// must still call it the same number of times.
-__device__ __forceinline__ void cta_barrier() { asm volatile("barrier.sync 0;" ::: "memory"); }
-
 // Copy a ket record of nd doubles (nd even: records are 16-byte multiples, at
 // 16-byte aligned addresses) from global to shared memory without waiting:
 // 16-byte cp.async per lane, one commit group per record.
@@ -91,21 +85,52 @@ template <int N, bool KE> struct TileOutput {
         wob = wb * ov;
         wok = wk * ov;
     }
+    // The accumulators and the table row are read and written BATCH pairs at a
+    // time: the loads of a batch are issued together, ahead of its arithmetic,
+    // and do not wait for the stores of the pair before (the compiler cannot tell
+    // that a row and an accumulator never alias).
     __device__ __forceinline__ void bra(int f, double v) { acc[f * 32] = fma(wob, v, acc[f * 32]); }
-    __device__ __forceinline__ void exchange(int slot, double va, double vb) {
+    __device__ __forceinline__ double exchange(double va, double vb) {
         const double send = wok * (odd ? va : vb);
-        row[slot] = fma(wok, odd ? vb : va, __shfl_xor_sync(0xffffffffu, send, 1));
+        return fma(wok, odd ? vb : va, __shfl_xor_sync(0xffffffffu, send, 1));
     }
-    __device__ __forceinline__ void s2(int i, int fa, int fb, double va, double vb) {
-        bra(PS + fa, va);
-        bra(PS + fb, vb);
-        if (!KE) exchange(SL + KetSlots<N>::of_pair(i), va, vb);
+    // n <= 3: the accumulators and the table row are read and written BATCH pairs at
+    // a time, so that the loads of a batch are issued together, ahead of its
+    // arithmetic, and do not wait for the stores of the pair before (the compiler
+    // cannot tell that rows and accumulators never alias).  H2 K = 2048 on a B200,
+    // 16 warps per SM: 761 us pair by pair, 740 in batches of 5; at n = 5 the
+    // registers a batch holds cost more (2336 us pair by pair, 2364 to 2450).
+    static constexpr int BATCH = N > 3 ? 1 : 5;
+    double av[2 * BATCH], rv[BATCH];
+    template <bool H, int E> __device__ __forceinline__ void put(double va, double vb) {
+        constexpr int off = H ? 0 : PS, b = E % BATCH, e0 = E - b, base = H ? 0 : SL;
+        constexpr bool ket = H || !KE;
+        if constexpr (BATCH == 1) {
+            constexpr int i = H ? RP::h_pair(E) : E;
+            if constexpr (ket) row[base + KetSlots<N>::of_pair(i)] = exchange(va, vb);
+            bra(off + RP::fa(i), va);
+            bra(off + RP::fb(i), vb);
+        } else {
+            if constexpr (b == 0)
+                unrolled<e0, (e0 + BATCH < RP::paired ? e0 + BATCH : RP::paired)>([&](auto q) {
+                    constexpr int e = decltype(q)::value, i = H ? RP::h_pair(e) : e;
+                    av[2 * (e - e0)] = acc[(off + RP::fa(i)) * 32];
+                    av[2 * (e - e0) + 1] = acc[(off + RP::fb(i)) * 32];
+                });
+            av[2 * b] = fma(wob, va, av[2 * b]);
+            av[2 * b + 1] = fma(wob, vb, av[2 * b + 1]);
+            if constexpr (ket) rv[b] = exchange(va, vb);
+            if constexpr (b == BATCH - 1 || E == RP::paired - 1)
+                unrolled<e0, E + 1>([&](auto q) {
+                    constexpr int e = decltype(q)::value, i = H ? RP::h_pair(e) : e;
+                    acc[(off + RP::fa(i)) * 32] = av[2 * (e - e0)];
+                    acc[(off + RP::fb(i)) * 32] = av[2 * (e - e0) + 1];
+                    if constexpr (ket) row[base + KetSlots<N>::of_pair(i)] = rv[e - e0];
+                });
+        }
     }
-    __device__ __forceinline__ void h2(int i, int fa, int fb, double va, double vb) {
-        bra(fa, va);
-        bra(fb, vb);
-        exchange(KetSlots<N>::of_pair(i), va, vb);
-    }
+    template <int I> __device__ __forceinline__ void s2(double va, double vb) { put<false, I>(va, vb); }
+    template <int I> __device__ __forceinline__ void h2(double va, double vb) { put<true, RP::h_seq(I)>(va, vb); }
     __device__ __forceinline__ void scalar(double e2) {
         constexpr int p = KetSlots<N>::of_pair(RP::count - 1);
         bra(RP::scalar, e2);
@@ -175,10 +200,7 @@ __device__ __noinline__ double fold_slot(const double *slots, double scale, int 
 // term: a lane without a pair (l > k, or k >= K) evaluates the finite pair
 // (l, l, P) with zero weights, which adds nothing.
 // VKET: ket records re-read at each use (fewer live registers).
-// BSYNC: the warps of a block step through their tiles' terms together (a
-// block barrier after every (l, P) term, so the warps sharing a scheduler
-// execute the same stretch of code); every warp then runs LC x nst iterations,
-// and an idle warp (no tile: idle = true, or l >= K) only takes the barriers.
+// idle: the warp has no tile (its accumulators are set to zero all the same).
 // SBRA: the block's 32 bras of row block tl.x are staged in shared memory at
 // sbra (field f of lane j at sbra[f * 32 + j]; rows past K hold row K - 1) and
 // read there instead of from global memory.
@@ -191,13 +213,7 @@ __device__ __noinline__ double fold_slot(const double *slots, double scale, int 
 // to the compact buffers of one part of a split tile.
 // WB: write the bra partials to part_b (false: the caller reduces the warps'
 // accumulators, left in sm.sacc, itself).
-// SYNC (with BSYNC): 0 -- every warp takes the block barrier at the end of
-// each term; 1, 2 -- warps 4-7 of the block take it inside the term instead
-// (at term_raw's mid(1): after B, Bi, T and ov; mid(2): before the Coulomb sum),
-// so the two warps of each scheduler run different stretches of the body; 3 --
-// no barrier per term (the warps only meet at the tile group's barriers).
-template <int N, bool VKET, bool BSYNC = false, bool SBRA = false, bool SKET = false, int SYNC = 0, bool WB = true,
-          bool KE = false>
+template <int N, bool VKET, bool SBRA = false, bool SKET = false, bool WB = true, bool KE = false>
 __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst, const Consts<N> &cs,
                                           const double *__restrict__ bra, const double *__restrict__ ket,
                                           const double *__restrict__ C, const RawMap &kmap,
@@ -212,20 +228,19 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
     constexpr int STRIDE = COLS + 1;
     constexpr int NC = COLS > 32 ? 2 : 1;           // slots per lane
     static_assert(PS <= 32 && SL <= 32, "the symmetric passes need tri(n) + 1 + 3n <= 32");
-    // a barrier inside the term is taken only on the path that passes mid to
-    // term_raw; anywhere else the warps' barrier counts would not match
-    static_assert(SYNC == 0 || SYNC == 3 || (BSYNC && SBRA && SKET), "mid-term barriers need BSYNC, SBRA, SKET");
     const int lane = threadIdx.x & 31;
     double *krow = sm.krow, *kred = sm.kred;
     const int k = tl.x * 32 + lane;
     const int l0 = tl.y * LC;
-    const int l1 = BSYNC ? l0 + LC : min(l0 + LC, K);
+    const int l1 = idle ? l0 : min(l0 + LC, K);
     const bool kval = k < K && !idle;
     const double Ck = kval ? C[k] : 0.0;
 #pragma unroll
     for (int f = 0; f < 2 * PS; ++f) sm.sacc[f * 32 + lane] = 0.0;
-    TileOutput<N, KE> out{sm.sacc + lane, krow + (lane >> 1) * STRIDE + 8 * (lane & 1), (lane & 1) != 0,
-                          0.0, 0.0, 0.0, 0.0};
+    TileOutput<N, KE> out;
+    out.acc = sm.sacc + lane;
+    out.row = krow + (lane >> 1) * STRIDE + 8 * (lane & 1);
+    out.odd = (lane & 1) != 0;
     const double E2 = KE ? 2.0 * Egiven : 0.0;
     // the slot this lane sums, maps and writes: js of matrix `which` (NC = 2: of both)
     const int js = lane & (SL - 1), which = NC == 2 ? 0 : lane / SL;
@@ -236,37 +251,19 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
     const bool mine = fld >= 0 && lane < COLS;
     bool ok = true;
     int flags = 0, bad = 0x7fffffff;  // smallest failing pair (row-major k K + l)
-    // where this warp takes its per-term block barrier (BSYNC): 0 at the end of
-    // the term, 1 / 2 at term_raw's mid(1) / mid(2), -1 nowhere.  Every warp
-    // takes exactly one barrier per (l, P) term, or none (SYNC 3).
-    const int sync_at = !BSYNC || SYNC == 3 ? -1 : SYNC == 0 || !((threadIdx.x >> 7) & 1) ? 0 : SYNC;
-    struct MidSync {
-        int at;
-        __device__ __forceinline__ void operator()(int i) const {
-            if (i == at) cta_barrier();
-        }
-    } mid{sync_at};
     const int pend = p1 < 0 ? nst : p1;
-    // warp-uniform: ket l has work (always, without BSYNC); false from the
-    // first l without work to the end of the tile
-    auto has_work = [&](int l) { return !BSYNC || (!idle && l < K); };
     int cur = 0;  // SKET: the buffer that holds the current term's record
     if constexpr (SKET) {
-        if (l0 < l1 && p0 < pend && has_work(l0))
+        if (l0 < l1 && p0 < pend)
             ket_fetch(sm.sket, ket + ((size_t)l0 * nst + p0) * KL::size, KL::term, lane);
     }
     for (int l = l0; l < l1; ++l) {
-        const bool lok = has_work(l);
         double ak[NC], hsum = 0.0, ssum = 0.0;
 #pragma unroll
         for (int q = 0; q < NC; ++q) ak[q] = 0.0;
-        const bool active = kval && l <= k && lok;
-        const BraRef b{bra + (active ? k : (lok ? l : 0)), (size_t)K};
+        const bool active = kval && l <= k;
+        const BraRef b{bra_at<N>(bra, active ? k : l)};
         for (int P = p0; P < pend; ++P) {
-            if (BSYNC && !lok) {
-                if (sync_at >= 0) cta_barrier();
-                continue;
-            }
             const double *kr = ket + ((size_t)l * nst + P) * KL::size;
             if constexpr (SKET) {
                 ket_wait();  // this term's record is in buffer cur
@@ -275,7 +272,7 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
                     nl = l + 1;
                     nP = p0;
                 }
-                if (nl < l1 && has_work(nl))
+                if (nl < l1)
                     ket_fetch(sm.sket + (cur ^ 1) * KL::term, ket + ((size_t)nl * nst + nP) * KL::size, KL::term,
                               lane);
                 kr = sm.sket + cur * KL::term;
@@ -286,9 +283,9 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
             double eta2, ov;
             bool tok;
             if constexpr (SBRA && SKET)
-                tok = term_raw<N, double>(BraSmem{sbra + lane}, KetSmem{kr}, cs, E2, out, eta2, ov, mid);
+                tok = term_raw<N, double>(BraSmem{sbra + lane}, KetSmem{kr}, cs, E2, out, eta2, ov);
             else if constexpr (SBRA)
-                tok = term_raw<N, double>(BraSmem{sbra + lane}, KetRefV{kr}, cs, E2, out, eta2, ov, mid);
+                tok = term_raw<N, double>(BraSmem{sbra + lane}, KetRefV{kr}, cs, E2, out, eta2, ov);
             else if constexpr (SKET)
                 tok = term_raw<N, double>(b, KetSmem{kr}, cs, E2, out, eta2, ov);
             else if constexpr (VKET)
@@ -353,9 +350,7 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
                 for (int q = 0; q < NC; ++q) ak[q] += m[q];
             }
             __syncwarp();
-            if (BSYNC && sync_at == 0) cta_barrier();
         }
-        if (BSYNC && !lok) continue;
         if (!KE && active) {
             hsum *= 0.5;
             if (!isfinite(hsum) || !isfinite(ssum)) {

@@ -26,6 +26,7 @@ struct necg_handle {
     bool profile = false;
     cudaEvent_t ev[6] = {};
     double *d_dipcls = nullptr;  // classes of the dipole's terms (set when the symmetry set is a group)
+    bool dip_ready = false;      // ... looked for
     // symmetric gradient pass (when the symmetry set is closed under inverse)
     bool sym_ok = false;
     int grad_mode = 0;  // 0 ordered pairs, 1 symmetric, 2 fused energy + symmetric

@@ -34,7 +34,7 @@ template <int N>
 __global__ void __launch_bounds__(128) prep_bra_kernel(const double *__restrict__ iv, int K,
                                                        Consts<N> cs, double *__restrict__ bra) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < K) prep_bra_one<N>(iv, K, cs, bra, k);
+    if (k < K) prep_bra_at<N>(iv + (size_t)k * (tri(N) + 3 * N), cs, bra_at<N>(bra, k), 32);
 }
 
 template <int N>
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(32, MINW) energy_kernel(const int2 *__restrict
     int k, l0, lend;
     if (!energy_lane_range(tl.x, tl.y, lane, LC, K, k, l0, lend)) return;
     int bad = 0;
-    const int fl = energy_lane<N, double>(BraRef{bra + k, (size_t)K}, DevKet{ket}, k, l0, lend, K, nst,
+    const int fl = energy_lane<N, double>(BraRef{bra_at<N>(bra, k)}, DevKet{ket}, k, l0, lend, K, nst,
                                           cs, H, S, Kin, Pot, bad);
     flag_status(status, fl, bad);
 }
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(32, MINW) grad_kernel(int nkb, int nlc, int LC
     double *out = part + (size_t)lc * Part<N>::size * K + k;
     __shared__ double sacc[2 * Part<N>::size * 32];
     SmemAcc<N> accH{sacc + lane}, accS{sacc + Part<N>::size * 32 + lane};
-    const bool ok = grad_lane<N, double>(BraRef{bra + k, (size_t)K}, DevKet{ket}, l0, l1, nst, cs, lam, scal[0],
+    const bool ok = grad_lane<N, double>(BraRef{bra_at<N>(bra, k)}, DevKet{ket}, l0, l1, nst, cs, lam, scal[0],
                                          out, (size_t)K, accH, accS);
     if (!ok) flag_status(status, 1, k * K + l0);
 }
@@ -208,10 +208,9 @@ __global__ void __launch_bounds__(32, MINW) gsym_kernel(const int2 *__restrict__
     __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::term : 2];
     const int t = blockIdx.x;
     if (t >= ntiles) return;
-    fsym_tile<N, true, false, false, SKET, 0, true, true>(t, tiles[t], LC, K, nst, cs, bra, ket, C, kmap, nullptr,
-                                                          nullptr, part_b, part_k, status,
-                                                          FusedSmem{sacc, krow, kred, sket}, false, nullptr, 0, -1,
-                                                          TileOut{}, scal[0]);
+    fsym_tile<N, true, false, SKET, true, true>(t, tiles[t], LC, K, nst, cs, bra, ket, C, kmap, nullptr, nullptr,
+                                                part_b, part_k, status, FusedSmem{sacc, krow, kred, sket}, false,
+                                                nullptr, 0, -1, TileOut{}, scal[0]);
 }
 
 // Fused pass over unordered pairs (k >= l): one warp per tile; the body is
@@ -238,7 +237,7 @@ __global__ void __launch_bounds__(32, MINW) fsym_kernel(const int2 *__restrict__
     const int pc = blockIdx.y, PC = (nst + npc - 1) / npc;
     const int p0 = min(pc * PC, nst), p1 = min(p0 + PC, nst);
     const size_t off = (size_t)pc * K * K;
-    fsym_tile<N, VKET, false, false, SKET>(t * npc + pc, tiles[t], LC, K, nst, cs, bra, ket, C, kmap, H + off,
+    fsym_tile<N, VKET, false, SKET>(t * npc + pc, tiles[t], LC, K, nst, cs, bra, ket, C, kmap, H + off,
                                            S + off, part_b, part_k, status, FusedSmem{sacc, krow, kred, sket},
                                            false, nullptr, p0, p1);
 }
@@ -260,22 +259,22 @@ __global__ void __launch_bounds__(256) hs_reduce_kernel(const double *__restrict
 
 // The fused pass with W-warp blocks (W = 8 or 12), one per SM, persistent over
 // a queue of tile groups: group g = row block kb and ket chunks lc0 .. lc0 + W
-// - 1, one per warp.  The warps read the same 32 bras and step through their
-// terms together (fsym_tile with BSYNC), so the warps sharing a scheduler run
-// the same stretch of the long term body.  SBRA: the group's bras are staged in
-// shared memory once for all warps; SKET: each warp stages its ket records in
-// two buffers (the next term's copied while the current one is evaluated).
-// SYNC: where the warps take their per-term barrier (fsym_tile).  Shared
-// memory (dynamic, 16-byte aligned): per warp 2 PS 32 + ket table + 64 (+ 2 ket
-// records) doubles, then the bras.  KE: the symmetric pass with E known.
-template <int N> __host__ __device__ constexpr int fsym_warp_smem(bool sket) {
-    return 2 * Part<N>::size * 32 + ket_table<N>(2) + 64 + (sket ? 2 * KetLayout<N>::term : 0);
+// - 1, one per warp.  The group's bras are staged in shared memory once for all
+// warps, each warp stages its ket records in two buffers (the next term's copied
+// while the current one is evaluated), and the warps meet only at the group's
+// ends: a block barrier per term, which once kept the warps of a scheduler in
+// step, now only costs (LiH K = 1024 on a B200: 2.54 ms with it, 2.76 ms and more
+// with half of the warps taking it in mid-term, 2.34 ms without).  Shared
+// memory (dynamic, 16-byte aligned): per warp 2 PS 32 + ket table + 64 + 2 ket
+// records doubles, then the bras.  KE: the symmetric pass with E known.
+template <int N> __host__ __device__ constexpr int fsym_warp_smem() {
+    return 2 * Part<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
 }
-template <int N> __host__ __device__ constexpr int fsym_block_smem_bytes(int warps, bool sbra, bool sket) {
-    return (warps * fsym_warp_smem<N>(sket) + (sbra ? BraLayout<N>::term * 32 : 0)) * 8;
+template <int N> __host__ __device__ constexpr int fsym_block_smem_bytes(int warps) {
+    return (warps * fsym_warp_smem<N>() + BraLayout<N>::term * 32) * 8;
 }
 
-template <int N, bool VKET, bool SBRA, bool SKET, int WARPS, int SYNC = 0, bool KE = false>
+template <int N, int WARPS, bool KE = false>
 __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *__restrict__ groups, int ngroups,
                                                                 int *__restrict__ qcount,
                                                                 const int *__restrict__ tstart, int LC, int K,
@@ -291,12 +290,12 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
     extern __shared__ __align__(16) double smem[];
     __shared__ int gsh;
     constexpr int PS = Part<N>::size;
-    constexpr int PER_WARP = fsym_warp_smem<N>(SKET);
+    constexpr int PER_WARP = fsym_warp_smem<N>();
     constexpr int BS = BraLayout<N>::term;
     constexpr int TBL = ket_table<N>(2);
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
-    double *sbra = smem + WARPS * PER_WARP;  // SBRA: BS x 32 doubles after the warps' areas
+    double *sbra = smem + WARPS * PER_WARP;  // BS x 32 doubles after the warps' areas
     const FusedSmem sm{base, base + 2 * PS * 32, base + 2 * PS * 32 + TBL, base + 2 * PS * 32 + TBL + 64};
     for (;;) {
         if (threadIdx.x == 0) gsh = atomicAdd(qcount, 1);
@@ -307,7 +306,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
         const int2 gr = groups[g];
         const int kb = gr.x, lc = sgroup_lc0(gr) + w;
         const int last = min(kb * 32 + 31, K - 1);
-        const bool idle = lc * LC > last;  // past this block's triangle: barriers only
+        const bool idle = lc * LC > last;  // past this block's triangle
         // a split group of the queue's tail: this unit takes symmetry terms
         // [p0, p1); parts after the first write to their own slots in xsym
         const int part = sgroup_part(gr), parts = sgroup_parts(gr);
@@ -317,16 +316,14 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
             xo.x = xsym;
             xo.slot = (((g - tail0) / parts) * WARPS + w) * (parts - 1) + (part - 1);
         }
-        if constexpr (SBRA) {  // the group's 32 bras, once for all warps
-            for (int i = threadIdx.x; i < BS * 32; i += 32 * WARPS) {
-                const int f = i >> 5, kk = min(kb * 32 + (i & 31), K - 1);
-                sbra[i] = bra[(size_t)f * K + kk];
-            }
-            __syncthreads();
-        }
-        fsym_tile<N, VKET, true, SBRA, SKET, SYNC, false, KE>(tstart[kb] + lc, make_int2(kb, lc), LC, K, nst, cs,
-                                                              bra, ket, C, kmap, H, S, part_b, part_k, status, sm,
-                                                              idle, sbra, p0, p1, xo, KE ? scal[0] : 0.0);
+        // the group's 32 bras, once for all warps (rows past K hold row K - 1)
+        const double *bk = bra_at<N>(bra, kb * 32);
+        for (int i = threadIdx.x; i < BS * 32; i += 32 * WARPS)
+            sbra[i] = bk[(i & ~31) + min(i & 31, K - 1 - kb * 32)];
+        __syncthreads();
+        fsym_tile<N, true, true, true, false, KE>(tstart[kb] + lc, make_int2(kb, lc), LC, K, nst, cs, bra, ket, C,
+                                                  kmap, H, S, part_b, part_k, status, sm, idle, sbra, p0, p1, xo,
+                                                  KE ? scal[0] : 0.0);
         // the group's bra partials: its warps share the 32 bras, so their
         // accumulators are summed (in warp order) and written once, to the
         // slot of queue unit g
@@ -338,7 +335,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
             for (int q = 1; q < WARPS; ++q) v += smem[q * PER_WARP + i];
             part_b[(size_t)g * 2 * PS * 32 + i] = v;
         }
-        if constexpr (SBRA) __syncthreads();  // sbra is rewritten for the next group
+        __syncthreads();  // sbra and the warps' areas are rewritten for the next group
     }
 }
 
@@ -446,13 +443,14 @@ __global__ void __launch_bounds__(32) fsym_finish_kernel(const double *__restric
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= K) return;
     double o[PS];
-    finish_one<N>(sums, K, bra, cs, folded, k, o);
+    const double *brak = bra_at<N>(bra, k);
+    finish_one<N>(sums, K, brak, cs, folded, k, o);
     if (fields) {
 #pragma unroll
         for (int f = 0; f < PS; ++f) fields[(size_t)f * K + k] = o[f];
         return;
     }
-    if (!fields_to_grad<N>(o, bra, K, scal[1] * C[k], g, k)) atomicOr(status, 2);
+    if (!fields_to_grad<N>(o, brak, 32, scal[1] * C[k], g, k)) atomicOr(status, 2);
 }
 
 // Sum the gradient-tile partials over the ket chunks, in place into chunk 0:
@@ -478,7 +476,7 @@ __global__ void __launch_bounds__(128) grad_reduce_kernel(const double *__restri
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= K) return;
     const double sc = scal[1] * (C ? C[k] : 1.0);
-    if (!grad_reduce_one<N>(part, 1, K, bra, sc, g, k)) atomicOr(status, 2);
+    if (!grad_reduce_at<N>(part, 1, K, bra_at<N>(bra, k), 32, sc, g, k)) atomicOr(status, 2);
 }
 
 // python/rrms.py:21-120 rrms(stfe, stf, ii, jj, n1) per term: terms[5 t ..] =
@@ -592,7 +590,7 @@ __global__ void __launch_bounds__(32) dipole_group_kernel(const int2 *__restrict
     bool ok = true;
     if (energy_lane_range(tl.x, tl.y, lane, LC, K, k, l0, lend)) {
         const double Ck = C[k];
-        const BraRef b{bra + k, (size_t)K};
+        const BraRef b{bra_at<N>(bra, k)};
         for (int q = q0; q < q1; ++q) {
             double a[3 * N], a0 = 0.0;
 #pragma unroll
@@ -680,7 +678,7 @@ __global__ void __launch_bounds__(128) matel_kernel(const int *__restrict__ term
         return;
     }
     const double *kr = ket + ((size_t)jj * nst + stf) * KetLayout<N>::size;
-    if (!matel_one<N, double>(BraRef{bra + ii, (size_t)K}, kr, cs, out + 4 * t))
+    if (!matel_one<N, double>(BraRef{bra_at<N>(bra, ii)}, kr, cs, out + 4 * t))
         flag_status(status, 1, ii * K + jj);
 }
 
@@ -703,8 +701,8 @@ __global__ void __launch_bounds__(128) gradel_kernel(const int *__restrict__ ter
     const double *kr = ket + ((size_t)jj * nst + stf) * KetLayout<N>::size;
     double L[tri(N)];
 #pragma unroll
-    for (int q = 0; q < tri(N); ++q) L[q] = bra[(BraLayout<N>::L + q) * (size_t)K + ii];
-    if (!gradel_one<N, double>(BraRef{bra + ii, (size_t)K}, kr, cs, L, ii == jj,
+    for (int q = 0; q < tri(N); ++q) L[q] = bra_at<N>(bra, ii)[(BraLayout<N>::L + q) * 32];
+    if (!gradel_one<N, double>(BraRef{bra_at<N>(bra, ii)}, kr, cs, L, ii == jj,
                                tgvl + (size_t)t * blk, tgvls + (size_t)t * blk))
         flag_status(status, 1, ii * K + jj);
 }
@@ -814,7 +812,7 @@ template <int N> struct Launch {
     }
     static void gsym_tiles(const LaunchArgs &a, cudaStream_t st) {
         if (gsym_block(a)) {
-            fsym_block<true, true, 8, 3, true>(a, st);
+            fsym_block<8, true>(a, st);
             if (a.sg_ntail > 0 && a.sg_parts >= 2 && a.xsym) {  // the queue's split tail: no H and S sums to add
                 LaunchArgs b = a;
                 b.H = b.S = nullptr;
@@ -856,12 +854,11 @@ template <int N> struct Launch {
                 npc > 1 ? a.Sp : a.S, a.psym, a.psym + (size_t)a.nstiles * npc * 2 * Part<N>::size * 32, a.status);
         }
     }
-    template <bool SBRA, bool SKET, int WARPS, int SYNC = 0, bool KE = false>
-    static void fsym_block(const LaunchArgs &a, cudaStream_t st) {
+    template <int WARPS, bool KE = false> static void fsym_block(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
-            constexpr int smem = fsym_block_smem_bytes<N>(WARPS, SBRA, SKET);
+            constexpr int smem = fsym_block_smem_bytes<N>(WARPS);
             if constexpr (smem <= 232448) {
-                auto kern = fsym_block_kernel<N, true, SBRA, SKET, WARPS, SYNC, KE>;
+                auto kern = fsym_block_kernel<N, WARPS, KE>;
                 int dev = 0, sms = 148;
                 cudaGetDevice(&dev);
                 // the shared-memory opt-in is per device: once per instantiation and device
@@ -884,16 +881,8 @@ template <int N> struct Launch {
     }
     static void fsym_tiles(const LaunchArgs &a, cudaStream_t st) {
         if (a.minb_s >= 200 && a.st_end == 0 && a.sgroups && a.qcount) {
-            switch (a.minb_s) {  // 2xy: lockstep blocks; see fused_variant_ok
-            case 218: fsym_block<true, false, 8>(a, st); break;
-            case 228: fsym_block<true, true, 8>(a, st); break;
-            case 248: fsym_block<true, true, 8, 3>(a, st); break;
-            case 258: fsym_block<true, true, 8, 1>(a, st); break;
-            case 268: fsym_block<true, true, 8, 2>(a, st); break;
-            case 222: fsym_block<true, false, 12>(a, st); break;
-            case 232: fsym_block<true, true, 12>(a, st); break;
-            default: fsym_block<false, false, 8>(a, st); break;
-            }
+            if (fused_block_warps(a.minb_s) == 12) fsym_block<12>(a, st);  // 2xy: block variants
+            else fsym_block<8>(a, st);
             return;
         }
         switch (a.minb_s) {  // 100 + w: ket records read at the point of use
@@ -1014,16 +1003,14 @@ int fused_block_warps(int variant) { return variant == 222 || variant == 232 ? 1
 bool fused_variant_ok(int n, int variant) {
     if (variant < 200) return true;
     if (n < 1 || n > 5) return false;
-    const bool sbra = variant != 208,
-               sket = variant == 228 || variant == 232 || variant == 248 || variant == 258 || variant == 268;
     const int warps = fused_block_warps(variant);
     int bytes = 0;
     switch (n) {
-    case 1: bytes = fsym_block_smem_bytes<1>(warps, sbra, sket); break;
-    case 2: bytes = fsym_block_smem_bytes<2>(warps, sbra, sket); break;
-    case 3: bytes = fsym_block_smem_bytes<3>(warps, sbra, sket); break;
-    case 4: bytes = fsym_block_smem_bytes<4>(warps, sbra, sket); break;
-    default: bytes = fsym_block_smem_bytes<5>(warps, sbra, sket); break;
+    case 1: bytes = fsym_block_smem_bytes<1>(warps); break;
+    case 2: bytes = fsym_block_smem_bytes<2>(warps); break;
+    case 3: bytes = fsym_block_smem_bytes<3>(warps); break;
+    case 4: bytes = fsym_block_smem_bytes<4>(warps); break;
+    default: bytes = fsym_block_smem_bytes<5>(warps); break;
     }
     return bytes <= 232448;
 }

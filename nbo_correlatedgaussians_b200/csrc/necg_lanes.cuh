@@ -60,12 +60,10 @@ NECG_HD void mass_products(const double (&A)[tri(N)], const double *M, double (&
     tMA = t;
 }
 
-// Bra record of basis k (structure of arrays, field f at f*K + k).
+// Bra record of the basis function with parameters b: field f at bra[f * stride].
 template <int N>
-NECG_HD void prep_bra_one(const double *iv, int K, const Consts<N> &cs, double *bra, int k) {
+NECG_HD void prep_bra_at(const double *b, const Consts<N> &cs, double *bra, size_t stride) {
     using BL = BraLayout<N>;
-    constexpr int blk = tri(N) + 3 * N;
-    const double *b = iv + (size_t)k * blk;
     double L[tri(N)], A[tri(N)], S[3 * N], AS[3 * N], AM[N * N], AMA[tri(N)], tMA;
     unpack_L<N>(b, L);
 #pragma unroll
@@ -79,20 +77,24 @@ NECG_HD void prep_bra_one(const double *iv, int K, const Consts<N> &cs, double *
 #pragma unroll
     for (int i = 0; i < N; ++i) dl *= L[sx(i, i)];
     dl = ::fabs(dl);
-    const size_t KK = (size_t)K;
 #pragma unroll
-    for (int t = 0; t < tri(N); ++t) bra[(BL::A + t) * KK + k] = A[t];
+    for (int t = 0; t < tri(N); ++t) bra[(BL::A + t) * stride] = A[t];
 #pragma unroll
-    for (int t = 0; t < 3 * N; ++t) bra[(BL::S + t) * KK + k] = S[t];
+    for (int t = 0; t < 3 * N; ++t) bra[(BL::S + t) * stride] = S[t];
 #pragma unroll
-    for (int t = 0; t < 3 * N; ++t) bra[(BL::AS + t) * KK + k] = AS[t];
+    for (int t = 0; t < 3 * N; ++t) bra[(BL::AS + t) * stride] = AS[t];
 #pragma unroll
-    for (int t = 0; t < tri(N); ++t) bra[(BL::N8 + t) * KK + k] = -8.0 * AMA[t];
-    bra[BL::i1 * KK + k] = i1;
-    bra[BL::pre * KK + k] = cs.sqrt8n * (dl * ::sqrt(dl));
-    bra[BL::tMA * KK + k] = tMA;
+    for (int t = 0; t < tri(N); ++t) bra[(BL::N8 + t) * stride] = -8.0 * AMA[t];
+    bra[BL::i1 * stride] = i1;
+    bra[BL::pre * stride] = cs.sqrt8n * (dl * ::sqrt(dl));
+    bra[BL::tMA * stride] = tMA;
 #pragma unroll
-    for (int t = 0; t < tri(N); ++t) bra[(BL::L + t) * KK + k] = L[t];
+    for (int t = 0; t < tri(N); ++t) bra[(BL::L + t) * stride] = L[t];
+}
+
+// The same for basis k of a buffer with field f at f * K + k (the host emulation).
+template <int N> NECG_HD void prep_bra_one(const double *iv, int K, const Consts<N> &cs, double *bra, int k) {
+    prep_bra_at<N>(iv + (size_t)k * (tri(N) + 3 * N), cs, bra + k, (size_t)K);
 }
 
 // Ket record of (l, P) = id / nst, id % nst: python/matel.py:76-87
@@ -228,13 +230,13 @@ template <int N, typename R, typename ACC> struct BraSums {
     NECG_HD void begin(R ov) { wo = w * ov; }
     NECG_HD void s1(int f, R v) { at(S, f) += wo * v; }
     NECG_HD void h1(int f, R v) { at(H, f) += wo * v; }
-    NECG_HD void s2(int, int fa, int fb, R va, R vb) {
-        s1(fa, va);
-        s1(fb, vb);
+    template <int I> NECG_HD void s2(R va, R vb) {
+        s1(RawPairs<N>::fa(I), va);
+        s1(RawPairs<N>::fb(I), vb);
     }
-    NECG_HD void h2(int, int fa, int fb, R va, R vb) {
-        h1(fa, va);
-        h1(fb, vb);
+    template <int I> NECG_HD void h2(R va, R vb) {
+        h1(RawPairs<N>::fa(I), va);
+        h1(RawPairs<N>::fb(I), vb);
     }
     NECG_HD void scalar(R e2) {
         H.d() += wo * e2;
@@ -317,9 +319,11 @@ NECG_HD bool a_to_vech(const double (&G)[tri(N)], double D, const double (&gS)[3
     return fin;
 }
 
-// The GRADA block of basis k (scaled by sc) from its gradient fields.
+// The GRADA block of basis k (scaled by sc) from its gradient fields; brak:
+// field f of its bra record at brak[f * stride].
 template <int N>
-NECG_HD bool fields_to_grad(const double (&o)[Part<N>::size], const double *bra, int K, double sc, double *g, int k) {
+NECG_HD bool fields_to_grad(const double (&o)[Part<N>::size], const double *brak, size_t stride, double sc, double *g,
+                            int k) {
     using BL = BraLayout<N>;
     constexpr int blk = tri(N) + 3 * N;
     double G[tri(N)], gS[3 * N], L[tri(N)];
@@ -328,33 +332,28 @@ NECG_HD bool fields_to_grad(const double (&o)[Part<N>::size], const double *bra,
 #pragma unroll
     for (int t = 0; t < 3 * N; ++t) gS[t] = o[tri(N) + 1 + t];
 #pragma unroll
-    for (int t = 0; t < tri(N); ++t) L[t] = bra[(BL::L + t) * (size_t)K + k];
+    for (int t = 0; t < tri(N); ++t) L[t] = brak[(BL::L + t) * stride];
     return a_to_vech<N>(G, o[tri(N)], gS, L, sc, g + (size_t)k * blk);
 }
 
 // Sum the nlc partials of basis k and write its GRADA block scaled by sc.
 template <int N>
-NECG_HD bool grad_reduce_one(const double *part, int nlc, int K, const double *bra, double sc,
-                             double *g, int k) {
-    using BL = BraLayout<N>;
-    using PL = Part<N>;
-    constexpr int blk = tri(N) + 3 * N;
-    double G[tri(N)], gS[3 * N], D = 0.0, L[tri(N)];
+NECG_HD bool grad_reduce_at(const double *part, int nlc, int K, const double *brak, size_t stride, double sc, double *g,
+                            int k) {
+    constexpr int PS = Part<N>::size;
+    double o[PS];
 #pragma unroll
-    for (int t = 0; t < tri(N); ++t) G[t] = 0.0;
-#pragma unroll
-    for (int t = 0; t < 3 * N; ++t) gS[t] = 0.0;
+    for (int f = 0; f < PS; ++f) o[f] = 0.0;
     for (int lc = 0; lc < nlc; ++lc) {
-        const double *p = part + (size_t)lc * PL::size * K + k;
+        const double *p = part + (size_t)lc * PS * K + k;
 #pragma unroll
-        for (int t = 0; t < tri(N); ++t) G[t] += p[(size_t)(PL::G + t) * K];
-        D += p[(size_t)PL::D * K];
-#pragma unroll
-        for (int t = 0; t < 3 * N; ++t) gS[t] += p[(size_t)(PL::S + t) * K];
+        for (int f = 0; f < PS; ++f) o[f] += p[(size_t)f * K];
     }
-#pragma unroll
-    for (int t = 0; t < tri(N); ++t) L[t] = bra[(BL::L + t) * (size_t)K + k];
-    return a_to_vech<N>(G, D, gS, L, sc, g + (size_t)k * blk);
+    return fields_to_grad<N>(o, brak, stride, sc, g, k);
+}
+template <int N>
+NECG_HD bool grad_reduce_one(const double *part, int nlc, int K, const double *bra, double sc, double *g, int k) {
+    return grad_reduce_at<N>(part, nlc, K, bra + k, (size_t)K, sc, g, k);
 }
 
 // One matel term (python/matel.py:28-210): out = (ov, tk, ert, zht).
@@ -468,9 +467,9 @@ struct RawMap {
 // the bra's raw S sums; the kets' folded gradient when they were.
 constexpr int kSumSets = 3;
 
-// The gradient fields (Part<N>) of basis k from its sums.
+// The gradient fields (Part<N>) of basis k from its sums (brak = bra_at(bra, k)).
 template <int N>
-NECG_HD void finish_one(const double *sums, int K, const double *bra, const Consts<N> &cs, int folded, int k,
+NECG_HD void finish_one(const double *sums, int K, const double *brak, const Consts<N> &cs, int folded, int k,
                         double (&o)[Part<N>::size]) {
     using BL = BraLayout<N>;
     constexpr int PS = Part<N>::size;
@@ -479,9 +478,9 @@ NECG_HD void finish_one(const double *sums, int K, const double *bra, const Cons
 #pragma unroll
     for (int f = 0; f < PS; ++f) r[f] = sums[f * KK + k];
     const auto sr = [&](int f) { return sums[(PS + f) * KK + k]; };
-    const auto A = [&](int t) { return bra[(BL::A + t) * KK + k]; };
-    const auto s = [&](int t) { return bra[(BL::S + t) * KK + k]; };
-    const auto e = [&](int t) { return bra[(BL::AS + t) * KK + k]; };
+    const auto A = [&](int t) { return brak[(BL::A + t) * 32]; };
+    const auto s = [&](int t) { return brak[(BL::S + t) * 32]; };
+    const auto e = [&](int t) { return brak[(BL::AS + t) * 32]; };
     explicit_tau<N>(sr, A, e, cs, r);
     fold_raw<N>(FieldsOf<double>{r}, A, s, e, o);
     if (folded)

@@ -103,7 +103,11 @@ template <int N> struct KetLayout {
     static constexpr int size = (tMA + 1 + 1) & ~1;  // even, 16-byte records
 };
 
-// Bra record: structure of arrays over k, field f of basis k at f*K + k.
+// Bra record: structure of arrays in blocks of 32 basis functions, field f of
+// basis k at ((k / 32) size + f) 32 + k % 32 (bra_at): a warp's lanes read 256
+// contiguous bytes, and the fields of a lane are a constant distance apart, so a
+// load needs no address arithmetic of its own (with a stride of K doubles the
+// n = 3 term spent about 60 of its 1480 instructions on addresses).
 template <int N> struct BraLayout {
     static constexpr int T = tri(N);
     static constexpr int A = 0;
@@ -117,6 +121,11 @@ template <int N> struct BraLayout {
     static constexpr int L = tMA + 1;      // L_k, packed lower
     static constexpr int size = L + T;
 };
+
+// Field 0 of basis k in the blocked layout; further fields are 32 doubles apart.
+template <int N, typename P> __host__ __device__ __forceinline__ P *bra_at(P *bra, int k) {
+    return bra + (size_t)(k >> 5) * (BraLayout<N>::size * 32) + (k & 31);
+}
 
 // Per-problem constants, passed to kernels by value (constant bank).
 template <int N> struct Consts {
@@ -156,9 +165,8 @@ __device__ __forceinline__ double ldv(const double *p) {
     return v;
 }
 struct BraRef {
-    const double *p;  // bra + k
-    size_t K;
-    __device__ __forceinline__ double operator()(int f) const { return ldv(p + (size_t)f * K); }
+    const double *p;  // bra_at(bra, k)
+    __device__ __forceinline__ double operator()(int f) const { return ldv(p + f * 32); }
 };
 // Bra record staged in shared memory (field f of this lane at p[f * 32]), read
 // at the point of use through a volatile shared load (not hoisted into registers).
@@ -578,6 +586,17 @@ NECG_HD bool term_energy(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, 
     return ok;
 }
 
+// f(integral_constant<int, I>) for I = A .. END - 1, unrolled
+template <int I> struct IntC {
+    static constexpr int value = I;
+};
+template <int A, int END, typename F> NECG_HD void unrolled(F &&f) {
+    if constexpr (A < END) {
+        f(IntC<A>{});
+        unrolled<A + 1, END>(f);
+    }
+}
+
 // Fields of the raw sums of one basis function (Part<N>::size of them, the same
 // count and order as the partial buffers): G[tri] (derivative with respect to
 // B), one scalar, g[3N] (derivative with respect to e).  Raw values of one term,
@@ -600,6 +619,28 @@ template <int N> struct RawPairs {
     __host__ __device__ static constexpr int pair_of(int f) {
         return f < T ? f : f == T ? count - 1 : f - T - 1 < lead ? f - T - 1 : lead + (f - T - 1 - lead) / 2;
     }
+    // the pairs in the order in which the H values are formed (X by columns)
+    __host__ __device__ static constexpr int h_pair(int e) {
+        if (e >= lead) return e;
+        int j = 0, n = N;
+        while (e >= n) {
+            e -= n;
+            --n;
+            ++j;
+        }
+        return sx(j + e, j);
+    }
+    __host__ __device__ static constexpr int h_seq(int i) {
+        int e = 0;
+        while (h_pair(e) != i) ++e;
+        return e;
+    }
+    // fields of pair i
+    __host__ __device__ static constexpr int fa(int i) { return i < lead ? i : T + 1 + lead + 2 * (i - lead); }
+    __host__ __device__ static constexpr int fb(int i) {
+        return i < lead ? T + 1 + i : odd && i == count - 1 ? scalar : fa(i) + 1;
+    }
+    static constexpr int paired = odd ? count : count - 1;  // pairs with two fields
     __host__ __device__ static constexpr int side_of(int f) {
         return f < T ? 0 : f == T ? (odd ? 1 : 0) : f - T - 1 < lead ? 1 : (f - T - 1 - lead) & 1;
     }
@@ -607,48 +648,42 @@ template <int N> struct RawPairs {
 
 // One (k, l, P) term: the overlap and the raw values above, handed to `out`:
 //   out.begin(ov)              once, first
-//   out.s2(i, fa, fb, va, vb)  pair i of the S values (fields fa, fb)
-//   out.h2(i, fa, fb, va, vb)  pair i of the H values, with eta - E2 / 2 in the
-//                              place of eta (E2 = 2 E gives the gradient of h - E ov)
+//   out.s2<i>(va, vb)          pair i of the S values, i = 0, 1, ...
+//   out.h2<i>(va, vb)          pair i of the H values (in the order h_pair), with
+//                              eta - E2 / 2 in the place of eta (E2 = 2 E gives the
+//                              gradient of h - E ov)
 //   out.scalar(eta2)           the scalar pair when it holds nothing else
 //   out.s1 / out.h1(f, v)      single fields (n = 6 only)
 // eta2_out = 2 eta (so h = ov eta2_out / 2).  The S values leave before the
-// Coulomb sum, so that U is not live across it; mid(i) is called at two points
-// (i = 1 after B, Bi, T and ov; i = 2 before the Coulomb sum) for callers that
-// synchronise warps there.
-struct NoMid {
-    NECG_HD void operator()(int) const {}
-};
+// Coulomb sum, so that U is not live across it (n = 5, 255 registers: 15 FP64
+// operations fewer with U kept, but 64 bytes of spill, 2.37 against 2.34 ms).
 #pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA, typename OUT, typename MID = NoMid>
-NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT &out, R &eta2_out, R &ov_out,
-                      const MID &mid = MID{}) {
+template <int N, typename R, typename BA, typename KA, typename OUT>
+NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT &out, R &eta2_out, R &ov_out) {
     using BL = BraLayout<N>;
     using RP = RawPairs<N>;
     constexpr int TR = tri(N), V = 3 * N;
     R Bi[TR], T[V], ov;
     const bool ok = term_core<N>(b, kr, Bi, T, ov);
     ov_out = ov;
-    mid(1);
     out.begin(ov);
     // S: -U = -(1.5 Bi + T T^T), T, 1
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int j = 0; j <= i; ++j) {
-            R u = 1.5 * Bi[sx(i, j)];
+    unrolled<0, N>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        unrolled<0, i + 1>([&](auto jc) {
+            constexpr int j = decltype(jc)::value, t = sx(i, j);
+            R u = 1.5 * Bi[t];
 #pragma unroll
             for (int c = 0; c < 3; ++c) u += T[3 * i + c] * T[3 * j + c];
-            if (sx(i, j) < RP::lead)
-                out.s2(sx(i, j), sx(i, j), TR + 1 + sx(i, j), -u, T[sx(i, j) < V ? sx(i, j) : 0]);
-            else
-                out.s1(sx(i, j), -u);
-        }
-#pragma unroll
-    for (int q = 0; q < RP::left / 2; ++q)
-        out.s2(RP::lead + q, TR + 1 + RP::lead + 2 * q, TR + 2 + RP::lead + 2 * q, T[RP::lead + 2 * q],
-               T[RP::lead + 2 * q + 1]);
-    if (RP::odd) out.s2(RP::count - 1, TR + V, RP::scalar, T[V - 1], R(1.0));
+            if constexpr (t < RP::lead) out.template s2<t>(-u, T[t]);
+            else out.s1(t, -u);
+        });
+    });
+    unrolled<0, RP::left / 2>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        out.template s2<RP::lead + q>(T[RP::lead + 2 * q], T[RP::lead + 2 * q + 1]);
+    });
+    if constexpr (RP::odd) out.template s2<RP::count - 1>(T[V - 1], R(1.0));
     // tau and the bra's part of Q's right-hand side: V8 = -8 N D, D = T - S_k;
     // 4 tau = 12 tr(M A_k) + 1.5 <-8 N, Bi> + <D, V8>
     R Z[V], W[TR], eta2;
@@ -697,7 +732,6 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
         }
         eta2 -= 2.0 * sg;
     }
-    mid(2);
     const R rho = coulomb_grad<N>(Bi, T, cs, Z, W);
     eta2 += 2.0 * rho;
     eta2_out = eta2;
@@ -717,8 +751,8 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
             Q[3 * i + c] = s;
         }
     const R e15 = 1.5 * et;
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
+    unrolled<0, N>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
         R col[N];  // column j of W Bi
 #pragma unroll
         for (int a = 0; a < N; ++a) {
@@ -727,9 +761,9 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
             for (int k = 1; k < N; ++k) s += W[sx(a, k)] * Bi[sx(k, j)];
             col[a] = s;
         }
-#pragma unroll
-        for (int i = j; i < N; ++i) {
-            R s = -(e15 * Bi[sx(i, j)]);
+        unrolled<j, N>([&](auto ic) {
+            constexpr int i = decltype(ic)::value, t = sx(i, j);
+            R s = -(e15 * Bi[t]);
 #pragma unroll
             for (int a = 0; a < N; ++a) s += Bi[sx(i, a)] * col[a];
 #pragma unroll
@@ -737,19 +771,15 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
                 s -= Q[3 * i + c] * T[3 * j + c];
                 s -= T[3 * i + c] * Q[3 * j + c];
             }
-            const int t = sx(i, j), u = t < V ? t : 0;
-            if (t < RP::lead)
-                out.h2(t, t, TR + 1 + t, s, Q[u] + eh * T[u]);
-            else
-                out.h1(t, s);
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < RP::left / 2; ++q) {
-        const int u = RP::lead + 2 * q;
-        out.h2(RP::lead + q, TR + 1 + u, TR + 2 + u, Q[u] + eh * T[u], Q[u + 1] + eh * T[u + 1]);
-    }
-    if (RP::odd) out.h2(RP::count - 1, TR + V, RP::scalar, Q[V - 1] + eh * T[V - 1], et);
+            if constexpr (t < RP::lead) out.template h2<t>(s, Q[t] + eh * T[t]);
+            else out.h1(t, s);
+        });
+    });
+    unrolled<0, RP::left / 2>([&](auto qc) {
+        constexpr int q = decltype(qc)::value, u = RP::lead + 2 * q;
+        out.template h2<RP::lead + q>(Q[u] + eh * T[u], Q[u + 1] + eh * T[u + 1]);
+    });
+    if constexpr (RP::odd) out.template h2<RP::count - 1>(Q[V - 1] + eh * T[V - 1], et);
     return ok;
 }
 
@@ -856,13 +886,13 @@ template <int N, typename R> struct RawValues {
     static constexpr int PS = tri(N) + 1 + 3 * N;
     R h[PS], s[PS], ov;
     NECG_HD void begin(R o) { ov = o; }
-    NECG_HD void s2(int, int fa, int fb, R va, R vb) {
-        s[fa] = ov * va;
-        s[fb] = ov * vb;
+    template <int I> NECG_HD void s2(R va, R vb) {
+        s[RawPairs<N>::fa(I)] = ov * va;
+        s[RawPairs<N>::fb(I)] = ov * vb;
     }
-    NECG_HD void h2(int, int fa, int fb, R va, R vb) {
-        h[fa] = ov * va;
-        h[fb] = ov * vb;
+    template <int I> NECG_HD void h2(R va, R vb) {
+        h[RawPairs<N>::fa(I)] = ov * va;
+        h[RawPairs<N>::fb(I)] = ov * vb;
     }
     NECG_HD void s1(int f, R v) { s[f] = ov * v; }
     NECG_HD void h1(int f, R v) { h[f] = ov * v; }

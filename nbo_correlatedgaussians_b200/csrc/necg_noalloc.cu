@@ -61,12 +61,16 @@ int scratch_address(double **out) {
 
 size_t up32(size_t v) { return (v + 31) / 32 * 32; }  // 256-byte alignment in doubles
 
-// Doubles set aside per (l, P) in the scratch layout, which fixes the largest
-// accepted K (include/necg.h states it): at least the ket record's size.
-int ket_room(int n) {
-    const int t = n * (n + 1) / 2;
-    const int room = (2 * t + 6 * n + n * n + 6 + 1) & ~1;
-    return room > necg::ket_record_size(n) ? room : necg::ket_record_size(n);
+// Doubles set aside for the bra and ket records in the scratch layout.  The part
+// of the rule that grows with K nst fixes the largest accepted K (include/necg.h
+// states it) and leaves room for the records' actual layout; the smallest
+// problems take what that needs.
+size_t records_room(int n, int nst, int K) {
+    const size_t t = n * (n + 1) / 2, k = (size_t)K;
+    const size_t bra = (size_t)necg::bra_record_size(n), ket = (2 * t + 6 * n + n * n + 6 + 1) / 2 * 2;
+    const size_t rule = up32(bra * k) + up32(ket * k * nst);
+    const size_t need = up32(bra * ((k + 31) / 32 * 32)) + up32((size_t)necg::ket_record_size(n) * k * nst);
+    return rule > need ? rule : need;
 }
 
 struct Carve {
@@ -80,8 +84,9 @@ Carve carve(int n, int nst, int K) {
     const int nlc = (K + kLcGrad - 1) / kLcGrad;
     const int ntiles = necg::energy_tile_count(K, kLcEnergy);
     size_t off = 0;
-    c.bra = off;    off = up32(off + (size_t)necg::bra_record_size(n) * k);
-    c.ket = off;    off = up32(off + (size_t)ket_room(n) * k * nst);
+    c.bra = off;
+    c.ket = up32((size_t)necg::bra_record_size(n) * ((k + 31) / 32 * 32));
+    off = up32(off + records_room(n, nst, K));
     c.part = off;   off = up32(off + (size_t)necg::part_stride(n) * k * nlc);
     c.H = off;      off = up32(off + k * k);
     c.S = off;      off = up32(off + k * k);

@@ -48,15 +48,16 @@ def workspace_estimate(p: Problem, K_max: int | None = None) -> int:
     """Device bytes a run's Engine allocates (mirror of necg_create's sizes)."""
     K, n, nst = int(K_max or p.K), p.n, p.nst
     tri = n * (n + 1) // 2
-    ket = (2 * tri + 6 * n + n * n + 5 + 2) & ~1
+    ket = (((tri + 3 * n + 6) & ~1) + 3 * n + tri + 2) & ~1
     bra = tri + 6 * n + tri + 3 + tri
+    Kb = (K + 31) // 32 * 32
     ps = tri + 1 + 3 * n
     blk = tri + 3 * n
     # symmetric-pass partials at the tuner's narrowest ket chunk (2), doubled
     # for the fused pass (H and S partials kept apart)
     ntiles = sum(min(kb * 32 + 31, K - 1) // 2 + 1 for kb in range((K + 31) // 32))
     sym = 2 * ntiles * ps * (32 + 2) if n <= 5 else 0
-    doubles = (bra * K + ket * K * nst + ps * K * ((K + 3) // 4) + 2 * K * K + 2 * K + 4
+    doubles = (bra * Kb + ket * K * nst + ps * K * max((K + 3) // 4, 3) + 2 * K * K + 2 * K + 4
                + 2 * (K * blk + K) + 2 + nst * (n * n + 9 * n * n + 1) + sym)
     return 8 * doubles + 3 * 8 * (K * blk + K) + 4096
 
