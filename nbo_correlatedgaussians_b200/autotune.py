@@ -36,7 +36,7 @@ from .engine import Engine
 
 CACHE = os.environ.get("NECG_TUNE_CACHE", os.path.join(os.path.dirname(os.path.abspath(__file__)), "tune_cache.json"))
 
-LC_E = (2, 4, 8, 16, 32)
+LC_E = (1, 2, 4, 8, 16)
 LC_G = (4, 8, 16, 32, 64)
 MINB = (8, 12, 16, 20)
 MINB_GRAD_EXTRA = (112, 116)  # gradient kernel with shared-memory accumulators

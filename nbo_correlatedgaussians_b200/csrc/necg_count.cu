@@ -101,12 +101,13 @@ template <int N> void count_term(int which, long long &flops, long long &special
     HostKet kr{ket.data()};
     count_ctx() = CountCtx();
     if (which == 0) {
-        CD ov, tau, rho, sig;
-        term_energy<N>(b, kr, cs, ov, tau, rho, sig);
-        // the energy kernel's per-term accumulation: h, s, kinetic, potential
+        CD ov, t2, rho, sig;
+        term_value<N>(b, kr, cs, ov, t2, rho, sig);
+        // the energy kernel's per-term accumulation: h and s
         CD w(1.0), h(0.0), s(0.0);
-        h += w * ov * (2.0 * tau + rho - sig);
-        s += w * ov;
+        const CD wov = w * ov;
+        h += wov * (t2 + rho - sig);
+        s += wov;
     } else if (which == 1) {
         CountOut<N, false, false> out;
         CD eta2, ov;

@@ -73,6 +73,55 @@ __global__ void __launch_bounds__(32, MINW) energy_kernel(const int2 *__restrict
     flag_status(status, fl, bad);
 }
 
+// The same with W warps per tile, each over its share of the symmetry terms, for
+// bases with too few tiles to fill the GPU (a tile is a chain of LC nst terms):
+// the warps' sums of a pair meet in shared memory and are added in warp order.
+// FP64 latency bounds it.  LiH K = 301 with H, S, Kinetic and Potential on a
+// B200: 222 us one warp per tile, 145 us with 2 and the shorter term.
+template <int N, int W>
+__global__ void __launch_bounds__(32 * W) energy_split_kernel(const int2 *__restrict__ tiles, int LC, int K, int nst,
+                                                              Consts<N> cs, const double *__restrict__ bra,
+                                                              const double *__restrict__ ket,
+                                                              double *__restrict__ H, double *__restrict__ S,
+                                                              double *__restrict__ Kin, double *__restrict__ Pot,
+                                                              int *status) {
+    __shared__ double red[W][4][32];
+    __shared__ int bad[W][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int2 tl = tiles[blockIdx.x];
+    int k, l0, lend;
+    const bool mine = energy_lane_range(tl.x, tl.y, lane, LC, K, k, l0, lend);
+    const BraRef b{bra_at<N>(bra, mine ? k : 0)};
+    const int p0 = w * nst / W, p1 = (w + 1) * nst / W;
+    int flags = 0, pair = 0x7fffffff;
+    for (int l = tl.y * LC; l < min(tl.y * LC + LC, K); ++l) {
+        const bool has = mine && l < lend;
+        if (has) {
+            double sum[4];
+            bad[w][lane] = !energy_sums<N, double>(b, DevKet{ket}, l, nst, p0, p1, cs, sum);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) red[w][i][lane] = sum[i];
+        }
+        __syncthreads();
+        if (w == 0 && has) {
+            double v[4];
+            bool ok = !bad[0][lane];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = red[0][i][lane];
+            for (int q = 1; q < W; ++q) {
+                ok = ok && !bad[q][lane];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] += red[q][i][lane];
+            }
+            const int fl = energy_store(v, ok, k, l, K, H, S, Kin, Pot);
+            if (fl && !flags) pair = k * K + l;
+            flags |= fl;
+        }
+        __syncthreads();
+    }
+    flag_status(status, flags, pair);
+}
+
 // rows[i] = (H C)_i, rows[K + i] = (S C)_i ; one warp per row
 __global__ void __launch_bounds__(256) rows_kernel(const double *__restrict__ H,
                                                    const double *__restrict__ S,
@@ -766,7 +815,21 @@ template <int N> struct Launch {
         energy_kernel<N, MINW><<<a.ntiles, 32, 0, st>>>(a.tiles, a.ntiles, a.LC_e, a.K, a.nst, cs, a.bra,
                                                         a.ket, a.H, a.S, a.Kin, a.Pot, a.status);
     }
+    template <int W> static void energy_split(const LaunchArgs &a, cudaStream_t st) {
+        Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
+        energy_split_kernel<N, W><<<a.ntiles, 32 * W, 0, st>>>(a.tiles, a.LC_e, a.K, a.nst, cs, a.bra, a.ket, a.H, a.S,
+                                                               a.Kin, a.Pot, a.status);
+    }
     static void energy(const LaunchArgs &a, cudaStream_t st) {
+        // warps per tile: enough for about 12 warps per SM of a 148-SM GPU, at
+        // most one per symmetry term
+        int w = 1;
+        while (2 * w <= a.nst && w < 8 && a.ntiles * w < 148 * 12) w *= 2;
+        switch (w) {
+        case 2: energy_split<2>(a, st); return;
+        case 4: energy_split<4>(a, st); return;
+        case 8: energy_split<8>(a, st); return;
+        }
         switch (a.minb_e) {
         case 12: energy_v<12>(a, st); break;
         case 16: energy_v<16>(a, st); break;

@@ -168,6 +168,42 @@ NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Cons
     if (KL::size > KL::tMA + 1) o[KL::tMA + 1] = 0.0;
 }
 
+// Sums over the symmetry terms [p0, p1) of one pair: sum[0] = H, [1] = S, [2] =
+// kinetic, [3] = Coulomb; false if some B is not positive definite.
+template <int N, typename R, typename BA, typename KB>
+NECG_HD bool energy_sums(const BA &b, const KB &ket, int l, int nst, int p0, int p1, const Consts<N> &cs,
+                         R (&sum)[4]) {
+    using KL = KetLayout<N>;
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum[i] = R(0.0);
+    for (int P = p0; P < p1; ++P) {
+        const auto kr = ket.at(((size_t)l * nst + P) * KL::size);
+        R ov, t2, rho, sig;
+        ok = term_value<N>(b, kr, cs, ov, t2, rho, sig) && ok;
+        const R wov = kr[KL::w] * ov;
+        sum[0] += wov * (t2 + rho - sig);
+        sum[1] += wov;
+        sum[2] += wov * t2;
+        sum[3] += wov * rho;
+    }
+    return ok;
+}
+
+// Write one pair's sums to H, S (and Kin, Pot when non-null) symmetrically; returns
+// the status flags (1: not positive definite, 2: non-finite).
+NECG_HD int energy_store(const double (&v)[4], bool ok, int k, int l, int K, double *H, double *S, double *Kin,
+                         double *Pot) {
+    double *M[4] = {H, S, Kin, Pot};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (M[i]) {
+            M[i][(size_t)k * K + l] = v[i];
+            M[i][(size_t)l * K + k] = v[i];
+        }
+    return (ok ? 0 : 1) | (isfinite(v[0]) && isfinite(v[1]) ? 0 : 2);
+}
+
 // Energy tile lane: bra k against kets l in [l0, lend) (lend <= k + 1), all P.
 // Writes H, S (and Kin, Pot when non-null) symmetrically.  Returns status
 // flags (1: a pair not positive definite, 2: non-finite) and the first pair.
@@ -175,39 +211,14 @@ template <int N, typename R, typename BA, typename KB>
 NECG_HD int energy_lane(const BA &b, const KB &ket, int k, int l0, int lend, int K, int nst,
                         const Consts<N> &cs, double *H, double *S, double *Kin, double *Pot,
                         int &bad_pair) {
-    using KL = KetLayout<N>;
     int flags = 0;
     for (int l = l0; l < lend; ++l) {
-        R h = R(0.0), s = R(0.0), tkin = R(0.0), tpot = R(0.0);
-        bool ok = true;
-        for (int P = 0; P < nst; ++P) {
-            const auto kr = ket.at(((size_t)l * nst + P) * KL::size);
-            R ov, tau, rho, sig;
-            ok = term_energy<N>(b, kr, cs, ov, tau, rho, sig) && ok;
-            const R wov = kr[KL::w] * ov;
-            const R t2 = 2.0 * tau;
-            h += wov * (t2 + rho - sig);
-            s += wov;
-            tkin += wov * t2;
-            tpot += wov * rho;
-        }
-        const double hv = val(h), sv = val(s);
-        int fl = ok ? 0 : 1;
-        if (!isfinite(hv) || !isfinite(sv)) fl |= 2;
+        R sum[4];
+        const bool ok = energy_sums<N, R>(b, ket, l, nst, 0, nst, cs, sum);
+        const double v[4] = {val(sum[0]), val(sum[1]), val(sum[2]), val(sum[3])};
+        const int fl = energy_store(v, ok, k, l, K, H, S, Kin, Pot);
         if (fl && !flags) bad_pair = k * K + l;
         flags |= fl;
-        H[(size_t)k * K + l] = hv;
-        H[(size_t)l * K + k] = hv;
-        S[(size_t)k * K + l] = sv;
-        S[(size_t)l * K + k] = sv;
-        if (Kin) {
-            Kin[(size_t)k * K + l] = val(tkin);
-            Kin[(size_t)l * K + k] = val(tkin);
-        }
-        if (Pot) {
-            Pot[(size_t)k * K + l] = val(tpot);
-            Pot[(size_t)l * K + k] = val(tpot);
-        }
     }
     return flags;
 }

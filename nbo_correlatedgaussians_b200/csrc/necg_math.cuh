@@ -553,16 +553,10 @@ NECG_HD R term_sig(const Consts<N> &cs, const R (&T)[3 * N]) {
     return cs.efs * sg;
 }
 
-// Energy part: returns false if B is not positive definite.
+// Coulomb sum (python/matel.py:162-197)
 #pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA>
-NECG_HD bool term_energy(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R &tau, R &rho,
-                         R &sig) {
-    R Bi[tri(N)], T[3 * N];
-    const bool ok = term_core<N>(b, kr, Bi, T, ov);
-    tau = term_tau<N>(b, kr, cs, Bi, T);
-    sig = term_sig<N>(cs, T);
-    // Coulomb sum (python/matel.py:162-197)
+template <int N, typename R>
+NECG_HD R coulomb_sum(const R (&Bi)[tri(N)], const R (&T)[3 * N], const Consts<N> &cs) {
     R r = R(0.0);
 #pragma unroll
     for (int q = 1; q <= N; ++q)
@@ -582,7 +576,52 @@ NECG_HD bool term_energy(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, 
             boys<false, (N > 3)>(a, bb, fs, D, ia, z);
             r += cs.cv[vidx(p, q)] * fs;
         }
-    rho = r;
+    return r;
+}
+
+// The matrix passes' value of one term: ov, 2 tau, rho and sig, with tau written
+// with the bra's N and D = T - S_k (as in term_raw: 4 tau = 12 tr(M A_k) +
+// <-8 N, 1.5 Bi + D D^T>), which needs neither the ket's N and S nor a choice
+// between the two.  Returns false if B is not positive definite.
+#pragma nv_exec_check_disable
+template <int N, typename R, typename BA, typename KA>
+NECG_HD bool term_value(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R &tau2, R &rho, R &sig) {
+    using BL = BraLayout<N>;
+    R Bi[tri(N)], T[3 * N];
+    const bool ok = term_core<N>(b, kr, Bi, T, ov);
+    sig = term_sig<N>(cs, T);
+    rho = coulomb_sum<N>(Bi, T, cs);
+    R dg = R(0.0), od = R(0.0);
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) T[t] -= b(BL::S + t);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+            R u = 1.5 * Bi[sx(i, j)];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) u += T[3 * i + c] * T[3 * j + c];
+            const R a = b(BL::N8 + sx(i, j));
+            if (i == j)
+                dg = (i == 0) ? a * u : dg + a * u;
+            else
+                od = (i == 1) ? a * u : od + a * u;
+        }
+    tau2 = 6.0 * b(BL::tMA) + (0.5 * dg + od);
+    return ok;
+}
+
+// Energy part of a single element (the matel API): returns false if B is not
+// positive definite.  tau through the smaller of the two traces (term_tau).
+#pragma nv_exec_check_disable
+template <int N, typename R, typename BA, typename KA>
+NECG_HD bool term_energy(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R &tau, R &rho,
+                         R &sig) {
+    R Bi[tri(N)], T[3 * N];
+    const bool ok = term_core<N>(b, kr, Bi, T, ov);
+    tau = term_tau<N>(b, kr, cs, Bi, T);
+    sig = term_sig<N>(cs, T);
+    rho = coulomb_sum<N>(Bi, T, cs);
     return ok;
 }
 
