@@ -7,14 +7,13 @@
 // plan).  Fused mode (every instance's symmetry set closed under inverse):
 //   reset        queue heads and per-instance status words
 //   prep         grid-stride over all (instance, k) bra and (instance, l, P) ket records
-//   fused        persistent warps over the fused tile queue (all instances): H, S
-//                and the H and S gradient partials in one pass over unordered pairs
-//   rows         grid-stride warps over all (instance, row): (H C)_i, (S C)_i
-//   finalize     block per instance: E, norm, GRADC
-//   fsum         grid-stride over all (instance, field, k): g_H - E g_S
+//   fused        persistent warps over the fused tile queue (all instances): the row
+//                and gradient partials of H and S in one pass over unordered pairs
+//   fsum         blocks over all (instance, 32-row block, field): per-basis sums
+//   finalize     block per instance: E, norm, GRADC from the row sums
 //   reduce       grid-stride over all (instance, k): GRADA blocks
-// Ordered mode (any other set): energy tiles over the triangle and gradient
-// tiles over ordered pairs in place of fused, and a plain partial sum.
+// Ordered mode (any other set): energy tiles over the triangle, rows (H C, S C),
+// finalize, gradient tiles over ordered pairs and a plain partial sum.
 // The plan (instance table, prefix sums, tile queues ordered by decreasing
 // cost) is built on the host and copied to device buffers before the step.
 #include <cuda_runtime.h>
@@ -48,8 +47,10 @@ struct InstDesc {
     const int2 *bgroups; // groups of 8 consecutive chunks of one row block (kb, first lc)
     int nbgroups;
     int npc;             // one-warp fused kernel: symmetry terms split npc ways per tile
+    const int2 *burange; // groups of each row block (their bra partial slots)
+    int groups;          // 1: the bra partials are per group (lockstep kernel)
+    int general;         // prep: general shift maps
     double *psym;
-    double *Hp, *Sp;     // npc > 1: the splits' H, S sums (npc K x K each)
     RawMap kmap;
     double cs[kConstsDoubles];
 };
@@ -67,7 +68,7 @@ struct PlanPtrs {
     InstDesc *inst;
     int *pref_bra;  // cumulative K            (ninst + 1)
     int *pref_ket;  // cumulative K * nst      (ninst + 1)
-    int *pref_sum;  // cumulative PS * K       (ninst + 1)
+    int *pref_sum;  // cumulative PS * K, or, fused, 32-row blocks times fields (ninst + 1)
     int *pref_ft;   // cumulative fused tile groups, or tiles when fine (ninst + 1), over `order`
     int *order;     // instances by decreasing tile cost (fused queue order)
     int4 *etiles;   // (inst, kb, lc, 0); fused mode: (inst, kb, lc, tile index in the instance)
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(128) batch_prep_kernel(PlanPtrs p) {
             const InstDesc &d = p.inst[q];
             const int id = j - p.pref_ket[q];
             BATCH_SWITCH(d.n, prep_ket_one<N>(d.iv, d.C, d.nst, consts_of<N>(d), d.sml, d.sms, d.scvv,
-                                             d.ket, id, d.pinv));
+                                             d.ket, id, d.pinv, d.general, d.kmap.fold));
         }
     }
 }
@@ -169,7 +170,7 @@ __global__ void __launch_bounds__(32) batch_energy_kernel(PlanPtrs p) {
 // that runs over the instances in plan order and over each instance's own
 // device tile list.  Shared memory is sized for n = kMaxN.
 __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
-    __shared__ double sacc[2 * Part<kMaxN>::size * 32];
+    __shared__ double sacc[2 * SumFields<kMaxN>::size * 32];
     __shared__ double krow[ket_table<kMaxN>(2)];
     __shared__ double kred[64];
     const int lane = threadIdx.x & 31;
@@ -184,12 +185,10 @@ __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
         const int slot = t - p.pref_ft[j];  // tile ti, split pc of the instance
         const int npc = d.npc, ti = slot / npc, pc = slot - ti * npc;
         const int PC = (d.nst + npc - 1) / npc, p0 = min(pc * PC, d.nst), p1 = min(p0 + PC, d.nst);
-        const size_t PSd = (size_t)(tri(d.n) + 1 + 3 * d.n);
-        double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * npc * 2 * PSd * 32;
-        double *H = npc > 1 ? d.Hp + (size_t)pc * d.K * d.K : d.H;
-        double *S = npc > 1 ? d.Sp + (size_t)pc * d.K * d.K : d.S;
+        const size_t PBd = (size_t)(tri(d.n) + 2 + 3 * d.n);
+        double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * npc * 2 * PBd * 32;
         BATCH_SWITCH(d.n, (fsym_tile<N, true>(slot, d.stiles[ti], d.lc_s, d.K, d.nst, consts_of<N>(d), d.bra,
-                                              d.ket, d.C, d.kmap, H, S, part_b, part_k, d.status,
+                                              d.ket, d.C, d.kmap, nullptr, nullptr, part_b, part_k, d.status,
                                               FusedSmem{sacc, krow, kred, nullptr}, false, nullptr, p0, p1)));
     }
 }
@@ -202,29 +201,41 @@ __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
 // records too, in two buffers (fsym_tile with SBRA, SKET), and the warps meet only
 // at the group's ends.  Shared memory is sized for n = kMaxN.
 template <int N> __host__ __device__ constexpr int bfused_warp_smem() {
-    return 2 * Part<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
+    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
 }
 constexpr int kBatchFusedSmem = (8 * bfused_warp_smem<kMaxN>() + BraLayout<kMaxN>::term * 32) * 8;
 
 template <int N>
-__device__ __forceinline__ void batch_fused_group(const InstDesc &d, int2 gr, double *smem) {
-    constexpr int PS = Part<N>::size;
+__device__ __forceinline__ void batch_fused_group(const InstDesc &d, int g, double *smem) {
+    constexpr int PB = SumFields<N>::size;
     constexpr int PER_WARP = bfused_warp_smem<N>();
     constexpr int BS = BraLayout<N>::term;
     constexpr int TBL = ket_table<N>(2);
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
     double *sbra = smem + 8 * PER_WARP;
-    const FusedSmem sm{base, base + 2 * PS * 32, base + 2 * PS * 32 + TBL, base + 2 * PS * 32 + TBL + 64};
+    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + 64};
+    const int2 gr = d.bgroups[g];
     const int K = d.K, kb = gr.x, lc = gr.y + w;
     const int last = min(kb * 32 + 31, K - 1);
     const bool idle = lc * d.lc_s > last;
     const double *bk = bra_at<N>(d.bra, kb * 32);
     for (int i = threadIdx.x; i < BS * 32; i += 256) sbra[i] = bk[(i & ~31) + min(i & 31, K - 1 - kb * 32)];
     __syncthreads();
-    double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * 2 * PS * 32;
-    fsym_tile<N, true, true, true>(d.stile_start[kb] + lc, make_int2(kb, lc), d.lc_s, K, d.nst, consts_of<N>(d),
-                                   d.bra, d.ket, d.C, d.kmap, d.H, d.S, part_b, part_k, d.status, sm, idle, sbra);
+    double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * 2 * PB * 32;
+    fsym_tile<N, true, true, true, false>(d.stile_start[kb] + lc, make_int2(kb, lc), d.lc_s, K, d.nst,
+                                          consts_of<N>(d), d.bra, d.ket, d.C, d.kmap, nullptr, nullptr, part_b,
+                                          part_k, d.status, sm, idle, sbra);
+    // the warps share the group's bras: their accumulators are summed in warp
+    // order and written once, to the group's slot
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * PB * 32; i += 256) {
+        if (kb * 32 + (i & 31) >= K) continue;
+        double v = smem[i];
+#pragma unroll
+        for (int q = 1; q < 8; ++q) v += smem[q * PER_WARP + i];
+        part_b[(size_t)g * 2 * PB * 32 + i] = v;
+    }
     __syncthreads();  // sbra and the warps' areas are reused by the next group
 }
 
@@ -240,53 +251,46 @@ __global__ void __launch_bounds__(256, 1) batch_fused_kernel(PlanPtrs p) {
         if (t >= nf) break;
         const int j = find_inst(p.pref_ft, ninst, t);
         const InstDesc &d = p.inst[p.order[j]];
-        const int2 gr = d.bgroups[t - p.pref_ft[j]];
-        BATCH_SWITCH(d.n, batch_fused_group<N>(d, gr, smem));
+        BATCH_SWITCH(d.n, batch_fused_group<N>(d, t - p.pref_ft[j], smem));
     }
 }
 
-// H, S of every instance whose symmetry terms were split: the sum over its
-// splits, in a fixed order (before rows / finalize read them).
-__global__ void __launch_bounds__(256) batch_hs_reduce_kernel(PlanPtrs p) {
-    const int ninst = p.hdr->ninst;
-    for (int q = 0; q < ninst; ++q) {
-        const InstDesc &d = p.inst[q];
-        if (d.npc <= 1) continue;
-        const size_t KK = (size_t)d.K * d.K;
-        for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < KK; i += (size_t)gridDim.x * blockDim.x) {
-            double h = d.Hp[i], s = d.Sp[i];
-            for (int pc = 1; pc < d.npc; ++pc) {
-                h += d.Hp[pc * KK + i];
-                s += d.Sp[pc * KK + i];
-            }
-            d.H[i] = h;
-            d.S[i] = s;
-        }
-    }
-}
-
-// The per-basis sums of every instance (put_sums) into its part.
+// The per-basis sums of every instance into its part: one block of 256 threads per
+// (instance, 32-row block, field) at a time.
 __global__ void __launch_bounds__(256) batch_fsum_kernel(PlanPtrs p) {
+    __shared__ double red[4][8][32];
     const int ninst = p.hdr->ninst;
     const int total = p.pref_sum[ninst];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    for (int i = blockIdx.x; i < total; i += gridDim.x) {
         const int q = find_inst(p.pref_sum, ninst, i);
         const InstDesc &d = p.inst[q];
-        const int id = i - p.pref_sum[q];
-        const int f = id / d.K, m = id - f * d.K;
-        const int PS = tri(d.n) + 1 + 3 * d.n;
-        const int npc = d.npc > 1 ? d.npc : 1;
-        const double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * npc * 2 * PS * 32;
-        const int kb = m >> 5, lane = m & 31;
-        double bH = 0.0, bS = 0.0, kH = 0.0, kS = 0.0;
-        const int sa = d.stile_start[kb] * npc, sb = d.stile_start[kb + 1] * npc;
-        for (int t = sa; t < sb; ++t) {
-            bH += part_b[(((size_t)t * 2 + 0) * PS + f) * 32 + lane];
-            bS += part_b[(((size_t)t * 2 + 1) * PS + f) * 32 + lane];
+        const int id = i - p.pref_sum[q], nkb = (d.K + 31) >> 5;
+        const int f = id / nkb, kb = id - f * nkb;
+        const size_t PBd = (size_t)(tri(d.n) + 2 + 3 * d.n);
+        const PassParts pp{d.stile_start, d.groups ? d.burange : nullptr, nullptr, d.psym,
+                           d.psym + (size_t)d.nstiles * d.npc * 2 * PBd * 32, nullptr, d.lc_s, d.K, 0, 0x7fffffff,
+                           d.npc, 1};
+        BATCH_SWITCH(d.n, (sum_partials<N, true>(pp, kb, f, d.part, red)));
+    }
+}
+
+// E, norm and GRADC of every instance from its row sums.
+__global__ void __launch_bounds__(256) batch_ffinalize_kernel(PlanPtrs p) {
+    __shared__ double sh[2][32], en[4];
+    const int ninst = p.hdr->ninst;
+    for (int q = blockIdx.x; q < ninst; q += gridDim.x) {
+        const InstDesc &d = p.inst[q];
+        const size_t siv = (size_t)d.K * (d.n * (d.n + 1) / 2 + 3 * d.n);
+        BATCH_SWITCH(d.n, {
+            energy_from_rows<N>(d.part, d.C, d.K, sh, en);
+            for (int i = threadIdx.x; i < d.K; i += blockDim.x) d.g[siv + i] = gradc_from_rows<N>(d.part, d.K, i, en);
+        });
+        if (threadIdx.x == 0) {
+            for (int i = 0; i < 4; ++i) d.scal[i] = en[i];
+            if (d.f) d.f[0] = en[0];
+            if (!isfinite(en[0])) atomicOr(d.status, 2);
         }
-        BATCH_SWITCH(d.n, (ket_partials<N, true>(d.stile_start, d.lc_s, d.K, f, m, part_k, 0, 0x7fffffff, npc, 0, 1,
-                                                 kH, kS)));
-        put_sums(d.part, PS, d.K, f, m, bH, bS, kH, kS, 2.0 * d.scal[0], d.kmap.fold);
+        __syncthreads();
     }
 }
 
@@ -428,7 +432,7 @@ template <bool FUSED> __global__ void __launch_bounds__(128) batch_reduce_kernel
         if (FUSED) {
             BATCH_SWITCH(d.n, {
                 double o[Part<N>::size];
-                finish_one<N>(d.part, d.K, bra_at<N>(d.bra, k), consts_of<N>(d), d.kmap.fold, k, o);
+                finish_one<N>(d.part, d.K, bra_at<N>(d.bra, k), consts_of<N>(d), d.kmap.fold, 2.0 * d.scal[0], k, o);
                 fin = fields_to_grad<N>(o, bra_at<N>(d.bra, k), 32, sc, d.g, k);
             });
         } else {
@@ -519,13 +523,11 @@ void launch_step(necg_batch *b, cudaStream_t st, int mode) {
     if (mode) {
         if (mode == 2) {
             batch_fused_warp_kernel<<<g * b->occ_fwarp, 32, 0, st>>>(p);
-            batch_hs_reduce_kernel<<<g * 2, 256, 0, st>>>(p);
         } else {
             batch_fused_kernel<<<g, 256, kBatchFusedSmem, st>>>(p);
         }
-        batch_rows_kernel<<<g * 4, 256, 0, st>>>(p);
-        batch_finalize_kernel<<<g, 256, 0, st>>>(p);
-        batch_fsum_kernel<<<g * 4, 256, 0, st>>>(p);
+        batch_fsum_kernel<<<g * 8, 256, 0, st>>>(p);
+        batch_ffinalize_kernel<<<g, 256, 0, st>>>(p);
         batch_reduce_kernel<true><<<g * 2, 128, 0, st>>>(p);
     } else {
         batch_energy_kernel<<<g * b->occ_energy, 32, 0, st>>>(p);
@@ -681,14 +683,14 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
             d.bgroups = h->d_bgroups;
             d.nbgroups = h->nbgroups;
             d.npc = 1;  // set below for the one-warp kernel
-            d.Hp = h->d_Hp;
-            d.Sp = h->d_Sp;
+            d.burange = h->d_burange;
         }
+        d.general = h->sms_general ? 1 : 0;
         const int ps = tri(n) + 1 + 3 * n;
         hp.pref_bra[q + 1] = hp.pref_bra[q] + K;
         hp.pref_ket[q + 1] = hp.pref_ket[q] + K * h->nst;
-        hp.pref_sum[q + 1] = hp.pref_sum[q] + ps * K;
         const int nkb = (K + 31) / 32;
+        hp.pref_sum[q + 1] = hp.pref_sum[q] + (fused ? (ps + 1) * nkb : ps * K);
         if (fused) {  // tiles come from the instance's device list; only its cost is needed here
             fcost[q] = (double)flops_fused[n] * h->nst * d.lc_s;
             continue;
@@ -710,9 +712,10 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
         for (int q = 0; q < count; ++q) ng += hp.inst[q].nbgroups;
         fine = ng < 4LL * b->sms;  // too few groups to fill the SMs with 8-warp blocks
         // the one-warp kernel splits each instance's symmetry terms as its handle does
-        // (its partial buffers and H, S split buffers are sized for that)
+        // (its partial buffers are sized for that)
         if (fine)
             for (int q = 0; q < count; ++q) hp.inst[q].npc = fused_splits(hs[q]);
+        for (int q = 0; q < count; ++q) hp.inst[q].groups = fine ? 0 : 1;
         hp.pref_ft[0] = 0;
         for (int j = 0; j < count; ++j) {
             const InstDesc &dj = hp.inst[hp.order[j]];

@@ -36,6 +36,9 @@ using necg::LaunchArgs;
 
 namespace {
 
+// Doubles before g in a handle's output block: f, the two status words, padding.
+constexpr size_t kOutHead = 4;
+
 // Status code of the two device status words (flags, first failing pair).
 int status_code(const int st[2], long long *bad_pair) {
     if (bad_pair) *bad_pair = st[1] == 0x7fffffff ? -1 : (long long)st[1];
@@ -135,10 +138,10 @@ void free_all(necg_handle *h) {
     for (cudaEvent_t &e : h->ev)
         if (e) cudaEventDestroy(e);
     void *ptrs[] = {h->d_sml, h->d_sms, h->d_scvv, h->d_bra, h->d_ket, h->d_part, h->d_H,
-                    h->d_S, h->d_rows, h->d_scal, h->d_x, h->d_g, h->d_f, h->d_status,
+                    h->d_S, h->d_rows, h->d_scal, h->d_x, h->d_out,
                     h->d_tiles, h->d_pinv, h->d_kcnt, h->d_ksrc, h->d_kcoef, h->d_stiles,
                     h->d_stile_start, h->d_psym, h->d_sgroups, h->d_qcount, h->d_bgroups,
-                    h->d_Hp, h->d_Sp, h->d_xsym, h->d_urange, h->d_dipcls};
+                    h->d_Hp, h->d_Sp, h->d_xsym, h->d_urange, h->d_dipcls, h->d_tslot, h->d_burange};
     for (void *p : ptrs) pool_free(h, p);
 }
 
@@ -171,7 +174,7 @@ int ensure_tiles(necg_handle *h, int K, cudaStream_t st) {
 // The fused pass with npc splits needs npc partial slots per tile and npc K x K
 // buffers for H and S.
 int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
-    const int PS = necg::part_stride(h->n);
+    const int PB = necg::part_stride(h->n) + 1;
     const int gw = necg::fused_block_warps(h->minb_s);  // tiles per group of the lockstep-block pass
     const int npc = fused ? necg::fused_splits(h) : 1;
     const size_t hp_need = npc > 1 ? (size_t)npc * K * K : 0;
@@ -187,7 +190,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
         h->hp_cap = hp_need;
     }
     if (h->stiles_K == K && h->stiles_lc == h->lc_s && h->sgroups_w == gw &&
-        (size_t)h->nstiles * PS * (32 + h->lc_s) * 2 * npc <= h->psym_cap)
+        (size_t)h->nstiles * PB * (32 + h->lc_s) * 2 * npc <= h->psym_cap)
         return NECG_OK;
     std::vector<int2> t;
     std::vector<int> start;
@@ -205,7 +208,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
         h->stiles_cap = (int)t.size();
     }
     if (!h->d_stile_start) CK(pool_alloc(h, &h->d_stile_start, ((h->K_max + 31) / 32 + 2) * sizeof(int), st));
-    const size_t need = t.size() * (size_t)PS * (32 + LC) * 2 * npc;
+    const size_t need = t.size() * (size_t)PB * (32 + LC) * 2 * npc;
     if (need > h->psym_cap) {
         pool_free(h, h->d_psym, st);
         h->d_psym = nullptr;
@@ -247,7 +250,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
             h->sg_tail0 = G - T;
             h->sg_ntail = T;
             h->sg_parts = parts;
-            const size_t xneed = (size_t)T * gw * (parts - 1) * necg::fsym_tail_slot(PS, LC);
+            const size_t xneed = (size_t)T * gw * (parts - 1) * necg::fsym_tail_slot(PB, LC);
             if (xneed > h->xsym_cap) {
                 pool_free(h, h->d_xsym, st);
                 h->d_xsym = nullptr;
@@ -279,15 +282,42 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
         CK(pool_alloc(h, &h->d_urange, nkb * sizeof(int2), st));
         h->urange_cap = nkb;
     }
+    // the tiles of the split tail groups: warp w of tail group j has slots
+    // (j gw + w)(parts - 1) .. of xsym
+    std::vector<int> tslot(t.size(), -1);
+    for (int j = 0; j < h->sg_ntail; ++j) {
+        const int2 g = groups[h->sg_tail0 + j * h->sg_parts];
+        for (int w = 0; w < gw; ++w) {
+            const int lc = necg::sgroup_lc0(g) + w;
+            if (start[g.x] + lc < start[g.x + 1]) tslot[start[g.x] + lc] = (j * gw + w) * (h->sg_parts - 1);
+        }
+    }
+    if ((int)t.size() > h->tslot_cap) {
+        pool_free(h, h->d_tslot, st);
+        h->d_tslot = nullptr;
+        CK(pool_alloc(h, &h->d_tslot, t.size() * sizeof(int), st));
+        h->tslot_cap = (int)t.size();
+    }
+    CK(cudaMemcpyAsync(h->d_tslot, tslot.data(), tslot.size() * sizeof(int), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(h->d_urange, urange.data(), nkb * sizeof(int2), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(h->d_sgroups, groups.data(), groups.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
     h->nsgroups = (int)groups.size();
     h->sgroups_w = gw;
     std::vector<int2> bgroups;  // width 8, for the batched step
+    std::vector<int2> burange(nkb);
     for (int kb = nkb - 1; kb >= 0; --kb) {
         const int ntk = start[kb + 1] - start[kb];
+        burange[kb].x = (int)bgroups.size();
         for (int lc0 = 0; lc0 < ntk; lc0 += 8) bgroups.push_back(make_int2(kb, lc0));
+        burange[kb].y = (int)bgroups.size();
     }
+    if (nkb > h->burange_cap) {
+        pool_free(h, h->d_burange, st);
+        h->d_burange = nullptr;
+        CK(pool_alloc(h, &h->d_burange, nkb * sizeof(int2), st));
+        h->burange_cap = nkb;
+    }
+    CK(cudaMemcpyAsync(h->d_burange, burange.data(), nkb * sizeof(int2), cudaMemcpyHostToDevice, st));
     if ((int)bgroups.size() > h->bgroups_cap) {
         pool_free(h, h->d_bgroups, st);
         h->d_bgroups = nullptr;
@@ -499,6 +529,7 @@ LaunchArgs base_args(necg_handle *h, int K) {
     a.kmap = necg::RawMap{h->d_kcnt, h->d_ksrc, h->d_kcoef, h->kmaxnz, h->kfold};
     a.minb_s = h->minb_s;
     a.dip_cls = h->d_dipcls;
+    a.sms_general = h->sms_general ? 1 : 0;
     return a;
 }
 
@@ -517,6 +548,7 @@ void sym_args(const necg_handle *h, LaunchArgs &a) {
     a.sg_ntail = h->sg_ntail;
     a.sg_parts = h->sg_parts;
     a.urange = h->d_urange;
+    a.tslot = h->d_tslot;
 }
 
 // The gradient passes after E and norm are in scal: symmetric (unordered pairs)
@@ -552,8 +584,7 @@ int check_K(necg_handle *h, int K) {
 
 int begin(necg_handle *h, cudaStream_t st) {
     CK(cudaSetDevice(h->device));
-    h->last_stream = st;
-    necg::launch_reset_status(h->d_status, st);  // status = {0, INT_MAX}
+    h->last_stream = st;  // the entry point's prep resets the status words
     return NECG_OK;
 }
 
@@ -562,10 +593,9 @@ int finish_launch() {
     return cuda_fail(e);
 }
 
-// The fused evaluation's launch sequence, from the status reset to the
-// partial sums, enqueued on st (no host synchronisation, so it can be captured).
+// The fused evaluation's launch sequence, from the records to the gradient,
+// enqueued on st (no host synchronisation, so it can be captured).
 int enqueue_fused(necg_handle *h, LaunchArgs &a, double *f_dev, double *g_dev, size_t siv, cudaStream_t st) {
-    necg::launch_reset_status(h->d_status, st);
     mark(h, 0, st);
     if (necg::launch_prep(a, st)) return NECG_ERR_UNSUPPORTED;
     mark(h, 1, st);
@@ -573,10 +603,10 @@ int enqueue_fused(necg_handle *h, LaunchArgs &a, double *f_dev, double *g_dev, s
     if (necg::launch_fsym_tail(a, st)) return NECG_ERR_ARG;
     if (necg::launch_hs_reduce(a, st)) return NECG_ERR_ARG;
     mark(h, 2, st);
-    necg::launch_rows_finalize(a, f_dev, g_dev + siv, 0, 0.0, 0.0, st);
     mark(h, 3, st);
+    if (necg::launch_fsym_sum(a, st)) return NECG_ERR_ARG;
     mark(h, 4, st);
-    if (necg::launch_fsym_reduce(a, st)) return NECG_ERR_ARG;
+    if (necg::launch_fsym_finish(a, f_dev, g_dev + siv, true, st)) return NECG_ERR_ARG;
     mark(h, 5, st);
     return NECG_OK;
 }
@@ -630,6 +660,13 @@ int necg_create(int n, int nst, int K_max, double efs, const double *mass_host,
     h->scvv.assign(scvv_host, scvv_host + nst);
     h->sml.assign(sml_host, sml_host + (size_t)nst * n * n);
     h->sms.assign(sms_host, sms_host + (size_t)nst * 9 * n * n);
+    h->sms_general = false;
+    for (int p = 0; p < nst && !h->sms_general; ++p)
+        for (int r = 0; r < 3 * n && !h->sms_general; ++r)
+            for (int c = 0; c < 3 * n && !h->sms_general; ++c) {
+                const double *S = &h->sms[(size_t)p * 9 * n * n];
+                h->sms_general = S[r * 3 * n + c] != (r % 3 == c % 3 ? S[(r / 3 * 3) * 3 * n + c / 3 * 3] : 0.0);
+            }
     // default tile widths per particle count
     h->lc_e = n >= 5 ? 4 : 8;
     h->lc_g = n >= 5 ? 4 : 8;
@@ -648,9 +685,13 @@ int necg_create(int n, int nst, int K_max, double efs, const double *mass_host,
     if (!rc) rc = dalloc(h, &h->d_rows, 2 * K);
     if (!rc) rc = dalloc(h, &h->d_scal, (size_t)4);
     if (!rc) rc = dalloc(h, &h->d_x, K * blk + K);
-    if (!rc) rc = dalloc(h, &h->d_g, K * blk + K);
-    if (!rc) rc = dalloc(h, &h->d_f, (size_t)2);
-    if (!rc) rc = dalloc(h, &h->d_status, (size_t)4);
+    // f, the status words and g side by side, for one copy to the host
+    if (!rc) rc = dalloc(h, &h->d_out, kOutHead + K * blk + K);
+    if (!rc) {
+        h->d_f = h->d_out;
+        h->d_status = (int *)(h->d_out + 1);
+        h->d_g = h->d_out + kOutHead;
+    }
     cudaStream_t ls = rc ? nullptr : lib_stream(h);
     if (!rc) rc = cuda_fail(cudaMemcpyAsync(h->d_sml, h->sml.data(), h->sml.size() * 8, cudaMemcpyHostToDevice, ls));
     if (!rc) rc = cuda_fail(cudaMemcpyAsync(h->d_sms, h->sms.data(), h->sms.size() * 8, cudaMemcpyHostToDevice, ls));
@@ -672,7 +713,7 @@ int necg_destroy(necg_handle *h) {
     if (!h) return NECG_ERR_ARG;
     cudaSetDevice(h->device);
     free_all(h);
-    if (h->h_tail) cudaFreeHost(h->h_tail);
+    if (h->h_out) cudaFreeHost(h->h_out);
     if (h->gexec) cudaGraphExecDestroy(h->gexec);
     if (h->gstream) cudaStreamDestroy(h->gstream);
     delete h;
@@ -770,6 +811,8 @@ int necg_outprod(necg_handle *h, int K, const double *x_dev, double *f_dev, doub
     if (fused) {
         // fused: one pass over unordered pairs writes H, S and the split gradients
         sym_args(h, a);
+        // H and S are written only for a caller that wants one of them
+        if (!H_dev && !S_dev) a.H = a.S = nullptr;
         a.npc = necg::fused_splits(h);
         a.Hp = h->d_Hp;
         a.Sp = h->d_Sp;
@@ -815,12 +858,16 @@ int shard_args(necg_handle *h, int K, const double *x_dev, int t0, int t1, cudaS
     const size_t siv = (size_t)K * (h->n * (h->n + 1) / 2 + 3 * h->n);
     a.iv = x_dev;
     a.C = x_dev + siv;
-    a.H = h->d_H;
-    a.S = h->d_S;
     sym_args(h, a);
     a.st_begin = t0;
     a.st_end = t1;
     return NECG_OK;
+}
+// The per-basis sums of this shard's tiles (all 0 for an empty range, which
+// st_end = 0 cannot say).
+int shard_sums(const LaunchArgs &a, cudaStream_t st) {
+    if (a.st_end > a.st_begin) return necg::launch_fsym_sum(a, st);
+    return cudaMemsetAsync(a.part, 0, sizeof(double) * necg::sums_doubles(a.n, a.K), st) == cudaSuccess ? 0 : -1;
 }
 }  // namespace
 
@@ -844,12 +891,10 @@ int necg_shard_pairs(necg_handle *h, int K, const double *x_dev, int tile_begin,
     if (rc) return rc;
     if (!rows_dev) return NECG_ERR_ARG;
     if ((rc = begin(h, st))) return rc;
-    // this shard writes only its tiles' entries of H and S: the rest must be 0
-    CK(cudaMemsetAsync(h->d_H, 0, sizeof(double) * (size_t)K * K, st));
-    CK(cudaMemsetAsync(h->d_S, 0, sizeof(double) * (size_t)K * K, st));
     if (necg::launch_prep(a, st)) return NECG_ERR_UNSUPPORTED;
     if (tile_end > tile_begin && necg::launch_fsym(a, st)) return NECG_ERR_ARG;
-    if (necg::launch_rows(a, rows_dev, st)) return NECG_ERR_ARG;
+    if (shard_sums(a, st)) return NECG_ERR_ARG;
+    if (necg::launch_rows_from_sums(a, rows_dev, st)) return NECG_ERR_ARG;
     return finish_launch();
 }
 
@@ -866,7 +911,8 @@ int necg_shard_grad(necg_handle *h, int K, const double *x_dev, const double *ro
     a.g = g_dev;
     a.sums = sums_dev;
     necg::launch_finalize(a, rows_dev, f_dev, g_dev + siv, st);
-    if (necg::launch_fsym_reduce(a, st)) return NECG_ERR_ARG;  // per-basis sums of this shard's tiles only
+    if (shard_sums(a, st)) return NECG_ERR_ARG;  // per-basis sums of this shard's tiles only
+    if (necg::launch_fsym_finish(a, nullptr, nullptr, false, st)) return NECG_ERR_ARG;
     return finish_launch();
 }
 
@@ -900,15 +946,20 @@ int necg_outprod_host(necg_handle *h, int K, const double *x_host, double *f_hos
     CK(cudaMemcpyAsync(h->d_x, x_host, len * sizeof(double), cudaMemcpyHostToDevice, st));
     rc = necg_outprod(h, K, h->d_x, h->d_f, h->d_g, nullptr, nullptr, stream);
     if (rc) return rc;
-    // f and the status words land in a pinned buffer, so the stream is waited for once
-    if (!h->h_tail) CK(cudaMallocHost((void **)&h->h_tail, 4 * sizeof(double)));
-    CK(cudaMemcpyAsync(g_host, h->d_g, len * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(h->h_tail, h->d_f, sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(h->h_tail + 1, h->d_status, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    // f, the status words and g come back in one copy into a pinned buffer of the
+    // handle, and the stream is waited for once; a pinned g_host gets its copy
+    // straight (a copy into pageable memory would go through the driver's own
+    // staging, one more wait)
+    if (!h->h_out) CK(cudaMallocHost((void **)&h->h_out, (kOutHead + (size_t)h->K_max * (len / K)) * sizeof(double)));
+    cudaPointerAttributes at;
+    const bool pinned = cudaPointerGetAttributes(&at, g_host) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    CK(cudaMemcpyAsync(h->h_out, h->d_out, (kOutHead + (pinned ? 0 : len)) * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (pinned) CK(cudaMemcpyAsync(g_host, h->d_g, len * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (f_host) *f_host = h->h_tail[0];
+    if (!pinned) memcpy(g_host, h->h_out + kOutHead, len * sizeof(double));
+    if (f_host) *f_host = h->h_out[0];
     int sw[2];
-    memcpy(sw, h->h_tail + 1, sizeof(sw));
+    memcpy(sw, h->h_out + 1, sizeof(sw));
     return status_code(sw, nullptr);
 }
 
@@ -967,6 +1018,7 @@ int necg_matel(necg_handle *h, int K, const double *iv_dev, int nterms, const in
     LaunchArgs a = base_args(h, K);
     a.iv = iv_dev;
     a.C = nullptr;
+    a.full = 1;  // matel chooses between the bra's and the ket's A M A
     if (necg::launch_prep(a, st)) return NECG_ERR_UNSUPPORTED;
     if (nterms > 0) necg::launch_matel(a, terms_dev, nterms, out_dev, st);
     return finish_launch();

@@ -48,8 +48,8 @@ __device__ __forceinline__ void flag_status(int *status, int flags, int pair) {
 
 // Where a part of a split tile of the lockstep pass writes instead of the
 // main buffers (slot < 0: the main buffers): slot `slot` of x, fsym_tail_slot
-// doubles holding its LC x 2 PS ket partials, then its LC x 64 H and S sums (H
-// for the 32 bras, then S).  The address is formed where it is used, so that
+// doubles holding its ket partials, then its LC x 64 H and S sums (H for the 32
+// bras, then S).  The address is formed where it is used, so that
 // it does not hold registers through the term loop.
 struct TileOut {
     double *x = nullptr;
@@ -60,7 +60,7 @@ struct TileOut {
 // or the symmetric pass (MATS = 1: the combined gradient).
 template <int N> __host__ __device__ constexpr int ket_table(int mats) { return 16 * (mats * KetSlots<N>::SL + 1); }
 
-// Shared memory of one warp's tile: bra accumulators (2 * PS * 32 doubles), the
+// Shared memory of one warp's tile: bra accumulators (2 * PB * 32 doubles), the
 // ket table (ket_table) and the reduced ket fields (64).  Sized by the caller
 // for its largest n.
 struct FusedSmem {
@@ -76,7 +76,7 @@ struct FusedSmem {
 // KE (E known): the S fields go to the bra only, and H's are the combined ones.
 template <int N, bool KE> struct TileOutput {
     using RP = RawPairs<N>;
-    static constexpr int PS = Part<N>::size, SL = KetSlots<N>::SL;
+    static constexpr int PB = SumFields<N>::size, SL = KetSlots<N>::SL;
     double *acc;  // this lane's accumulators: H fields, then S fields, 32 doubles apart
     double *row;  // the lane pair's row, + 8 for the odd lane
     bool odd;
@@ -103,7 +103,7 @@ template <int N, bool KE> struct TileOutput {
     static constexpr int BATCH = N > 3 ? 1 : 5;
     double av[2 * BATCH], rv[BATCH];
     template <bool H, int E> __device__ __forceinline__ void put(double va, double vb) {
-        constexpr int off = H ? 0 : PS, b = E % BATCH, e0 = E - b, base = H ? 0 : SL;
+        constexpr int off = H ? 0 : PB, b = E % BATCH, e0 = E - b, base = H ? 0 : SL;
         constexpr bool ket = H || !KE;
         if constexpr (BATCH == 1) {
             constexpr int i = H ? RP::h_pair(E) : E;
@@ -134,7 +134,7 @@ template <int N, bool KE> struct TileOutput {
     __device__ __forceinline__ void scalar(double e2) {
         constexpr int p = KetSlots<N>::of_pair(RP::count - 1);
         bra(RP::scalar, e2);
-        acc[(PS + RP::scalar) * 32] += wob;
+        acc[(PB + RP::scalar) * 32] += wob;
         if (KE) {
             const double v = wok * e2;  // the odd lane's copy lands in an unused slot
             row[p] = v + __shfl_xor_sync(0xffffffffu, v, 1);
@@ -184,15 +184,16 @@ __device__ __noinline__ double fold_slot(const double *slots, double scale, int 
 // e, the same for the bra and the ket); the bra's weighted sums stay in the
 // lane's accumulators, the ket's are summed over the warp per (l, P), mapped to
 // l's frame and summed over P.
-//   !KE, the fused pass: H_kl = H_lk and S_kl are the sums over P of h and ov;
-//        the H and S fields are kept apart, since E is not known until finalize
-//        has run on the H and S this pass writes.
+//   !KE, the fused pass: H_kl = H_lk and S_kl are the sums over P of h and ov,
+//        written when H is not null and always summed into the rows of H C and
+//        S C (SumFields::row); the H and S fields are kept apart, since E is not
+//        known until those rows are.
 //   KE, the symmetric gradient pass (E = Egiven known): the combined gradient
 //        of h - E ov, and the S fields for the bra only (its explicit share).
 // Tile t = (kb, lc): bras k = 32 kb + lane, kets l in [lc LC, lc LC + LC).  Bra
-// partials: part_b[((t * 2 + which) * PS + f) * 32 + lane]; ket partials:
-// part_k[((t * LC + l - l0) * 2 + which) * PS + f], which = 0 for H (or the
-// combined gradient) and 1 for S (not written for the ket when KE).
+// partials (PB = SumFields::size): part_b[((t * 2 + which) * PB + f) * 32 + lane];
+// ket partials: part_k[((t * LC + l - l0) * 2 + which) * PB + f], which = 0 for H
+// (or the combined gradient) and 1 for S (not written for the ket when KE).
 //
 // Shared memory per warp must stay under 228 KB / 8 for 8 resident warps, so the
 // ket rows of two lanes are added before they are written (TileOutput) and the
@@ -223,7 +224,7 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
                                           const double *sbra = nullptr, int p0 = 0, int p1 = -1,
                                           TileOut xo = TileOut{}, double Egiven = 0.0) {
     using KL = KetLayout<N>;
-    constexpr int PS = Part<N>::size, SL = KetSlots<N>::SL;
+    constexpr int PS = Part<N>::size, PB = SumFields<N>::size, SL = KetSlots<N>::SL;
     constexpr int COLS = (KE ? 1 : 2) * SL;         // 16, 32 or 64 ket slots per row
     constexpr int STRIDE = COLS + 1;
     constexpr int NC = COLS > 32 ? 2 : 1;           // slots per lane
@@ -236,7 +237,7 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
     const bool kval = k < K && !idle;
     const double Ck = kval ? C[k] : 0.0;
 #pragma unroll
-    for (int f = 0; f < 2 * PS; ++f) sm.sacc[f * 32 + lane] = 0.0;
+    for (int f = 0; f < 2 * PB; ++f) sm.sacc[f * 32 + lane] = 0.0;
     TileOutput<N, KE> out;
     out.acc = sm.sacc + lane;
     out.row = krow + (lane >> 1) * STRIDE + 8 * (lane & 1);
@@ -351,71 +352,161 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
             }
             __syncwarp();
         }
-        if (!KE && active) {
+        double *pk = xo.slot >= 0 ? xo.x + (size_t)xo.slot * fsym_tail_slot(PB, LC) + (size_t)(l - l0) * 2 * PB
+                                  : part_k + ((size_t)t * LC + (l - l0)) * 2 * PB;
+        if (!KE) {
             hsum *= 0.5;
-            if (!isfinite(hsum) || !isfinite(ssum)) {
-                bad = min(bad, k * K + l);
-                flags |= 2;
+            if (active) {
+                if (!isfinite(hsum) || !isfinite(ssum)) {
+                    bad = min(bad, k * K + l);
+                    flags |= 2;
+                }
+                if (H) {
+                    if (xo.slot >= 0) {
+                        double *hs = xo.x + (size_t)xo.slot * fsym_tail_slot(PB, LC) + (size_t)LC * 2 * PB;
+                        hs[(l - l0) * 64 + lane] = hsum;
+                        hs[(l - l0) * 64 + 32 + lane] = ssum;
+                    } else {
+                        H[(size_t)k * K + l] = hsum;
+                        H[(size_t)l * K + k] = hsum;
+                        S[(size_t)k * K + l] = ssum;
+                        S[(size_t)l * K + k] = ssum;
+                    }
+                }
+                const double Cl = C[l];
+                out.acc[PS * 32] += hsum * Cl;
+                out.acc[(PB + PS) * 32] += ssum * Cl;
             }
-            if (xo.slot >= 0) {
-                double *hs = xo.x + (size_t)xo.slot * fsym_tail_slot(PS, LC) + (size_t)LC * 2 * PS;
-                hs[(l - l0) * 64 + lane] = hsum;
-                hs[(l - l0) * 64 + 32 + lane] = ssum;
-            } else {
-                H[(size_t)k * K + l] = hsum;
-                H[(size_t)l * K + k] = hsum;
-                S[(size_t)k * K + l] = ssum;
-                S[(size_t)l * K + k] = ssum;
-            }
-        }
-        if (mine) {
-            double *pk = xo.slot >= 0 ? xo.x + (size_t)xo.slot * fsym_tail_slot(PS, LC) + (size_t)(l - l0) * 2 * PS
-                                      : part_k + ((size_t)t * LC + (l - l0)) * 2 * PS;
+            // the ket's row: sum over the bras k > l (lane 0 ends with H's, lane 1 with S's)
+            const double ch = active && l < k ? hsum * Ck : 0.0, cs_ = active && l < k ? ssum * Ck : 0.0;
+            double r = (lane & 1 ? cs_ : ch) + __shfl_xor_sync(0xffffffffu, lane & 1 ? ch : cs_, 1);
 #pragma unroll
-            for (int q = 0; q < NC; ++q) pk[(which + q) * PS + fld] = ak[q];
+            for (int o = 2; o < 32; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+            if (lane < 2) pk[lane * PB + PS] = r;
         }
+        if (mine)
+#pragma unroll
+            for (int q = 0; q < NC; ++q) pk[(which + q) * PB + fld] = ak[q];
     }
     if (WB && kval) {
-        double *pb = part_b + (size_t)t * 2 * PS * 32;
+        double *pb = part_b + (size_t)t * 2 * PB * 32;
 #pragma unroll
-        for (int f = 0; f < 2 * PS; ++f) pb[f * 32 + lane] = sm.sacc[f * 32 + lane];
+        for (int f = 0; f < 2 * PB; ++f) pb[f * 32 + lane] = sm.sacc[f * 32 + lane];
     }
     if (!ok) flags |= 1;
     flag_status(status, flags, bad);
     __syncwarp();
 }
 
-// The ket partials of basis m for field f and matrix `which`: from the tiles of
-// chunk lc = m / LC in every row block q >= that chunk's, q = kb0 + seg, + nseg, ..
-// Only tiles in [t0, t1) count (a shard of the pass).  With the symmetry terms
-// split npc ways, tile t's partials are slots t npc .. t npc + npc - 1.
+// Where the partials of a symmetric pass are and which of them count: tiles
+// [t0, t1) (a shard of the pass) of the tile list whose row blocks start at
+// tstart.  Bra partials: tile t's splits are slots t npc .. t npc + npc - 1, or
+// (urange: the block variants) row block kb's are the queue units urange[kb].
+// Ket partials: the tile's splits likewise and, for a tile of a split group
+// (tslot[t] >= 0), slots tslot[t] .. + parts - 2 of xsym.
+struct PassParts {
+    const int *tstart;
+    const int2 *urange;
+    const int *tslot;
+    const double *part_b, *part_k, *xsym;
+    int LC, K, t0, t1, npc, parts;
+};
+
+// One block of 256 threads sums field f of the 32 bases of row block kb: their
+// bra partials come from every tile of the block (up to K / LC of them), their
+// ket partials from one tile per later row block, so the 8 warps take every 8th
+// of each and their sums are combined in a fixed order.  Into sums (kSumSets
+// sets); TWO: the ket has S partials too.
 template <int N, bool TWO>
-__device__ __forceinline__ void ket_partials(const int *__restrict__ tstart, int LC, int K, int f, int m,
-                                             const double *__restrict__ part_k, int t0, int t1, int npc, int seg,
-                                             int nseg, double &kH, double &kS) {
-    constexpr int PS = Part<N>::size;
-    const int lc = m / LC, ll = m - lc * LC;
-    const int nkb = (K + 31) >> 5;
-    int kb0 = lc * LC - 31;
-    kb0 = kb0 > 0 ? (kb0 + 31) >> 5 : 0;
-    for (int q = kb0 + seg; q < nkb; q += nseg) {
-        const int t = tstart[q] + lc;
-        if (t < t0 || t >= t1) continue;
-        for (int pc = 0; pc < npc; ++pc) {
-            const size_t base = ((size_t)(t * npc + pc) * LC + ll) * 2;
-            kH += part_k[(base + 0) * PS + f];
-            if (TWO) kS += part_k[(base + 1) * PS + f];
+__device__ __forceinline__ void sum_partials(const PassParts &p, int kb, int f, double *__restrict__ sums,
+                                             double (*red)[8][32]) {
+    constexpr int PB = SumFields<N>::size;
+    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+    const int K = p.K, LC = p.LC, m = kb * 32 + lane;
+    const int ta = p.urange ? p.urange[kb].x : max(p.tstart[kb], p.t0) * p.npc;
+    const int tb = p.urange ? p.urange[kb].y : min(p.tstart[kb + 1], p.t1) * p.npc;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int t = ta + seg; t < tb; t += 8) {
+        v[0] += p.part_b[(((size_t)t * 2 + 0) * PB + f) * 32 + lane];
+        v[1] += p.part_b[(((size_t)t * 2 + 1) * PB + f) * 32 + lane];
+    }
+    if (m < K) {
+        const int lc = m / LC, ll = m - lc * LC;
+        const int nkb = (K + 31) >> 5;
+        int kb0 = lc * LC - 31;
+        kb0 = kb0 > 0 ? (kb0 + 31) >> 5 : 0;
+        for (int q = kb0 + seg; q < nkb; q += 8) {
+            const int t = p.tstart[q] + lc;
+            if (t < p.t0 || t >= p.t1) continue;
+            for (int pc = 0; pc < p.npc; ++pc) {
+                const double *pk = p.part_k + ((size_t)(t * p.npc + pc) * LC + ll) * 2 * PB + f;
+                v[2] += pk[0];
+                if (TWO) v[3] += pk[PB];
+            }
+            if (p.tslot && p.tslot[t] >= 0)
+                for (int pc = 0; pc < p.parts - 1; ++pc) {
+                    const double *pk = p.xsym + (size_t)(p.tslot[t] + pc) * fsym_tail_slot(PB, LC) + (size_t)ll * 2 * PB + f;
+                    v[2] += pk[0];
+                    if (TWO) v[3] += pk[PB];
+                }
         }
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) red[i][seg][lane] = v[i];
+    __syncthreads();
+    if (seg < 4 && m < K) {  // warp i: set i
+        double s = red[seg][0][lane];
+#pragma unroll
+        for (int q = 1; q < 8; ++q) s += red[seg][q][lane];
+        sums[((size_t)seg * PB + f) * K + m] = s;
+    }
+    __syncthreads();
 }
 
-// The per-basis sums (kSumSets sets of PS fields at out) of field f of basis m.
-__device__ __forceinline__ void put_sums(double *out, int PS, int K, int f, int m, double bH, double bS, double kH,
-                                         double kS, double E2, int folded) {
-    const double b = bH - E2 * bS, k = kH - E2 * kS;
-    out[(size_t)f * K + m] = folded ? b : b + k;
-    out[(size_t)(PS + f) * K + m] = bS;
-    if (folded) out[(size_t)(2 * PS + f) * K + m] = k;
+// E = C^T H C / C^T S C and norm = 1 / C^T S C (python/outprod.py:65-68) from the
+// row sums, by every thread of the block in the same fixed order; en = {E, norm,
+// cHc, cSc} in shared memory, sh: 2 x 32 doubles.
+template <int N>
+__device__ __forceinline__ void energy_from_rows(const double *__restrict__ sums, const double *__restrict__ C, int K,
+                                                 double (*sh)[32], double *en) {
+    constexpr int PB = SumFields<N>::size, R = SumFields<N>::row;
+    double ah = 0.0, as = 0.0;
+    for (int i = threadIdx.x; i < K; i += blockDim.x) {
+        const double c = C[i];
+        ah += c * (sums[(size_t)R * K + i] + sums[(size_t)(2 * PB + R) * K + i]);
+        as += c * (sums[(size_t)(PB + R) * K + i] + sums[(size_t)(3 * PB + R) * K + i]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        ah += __shfl_xor_sync(0xffffffffu, ah, o);
+        as += __shfl_xor_sync(0xffffffffu, as, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = ah;
+        sh[1][threadIdx.x >> 5] = as;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double th = 0.0, ts = 0.0;
+        for (int j = 0; j < (int)(blockDim.x >> 5); ++j) {
+            th += sh[0][j];
+            ts += sh[1][j];
+        }
+        en[0] = th / ts;
+        en[1] = 1.0 / ts;
+        en[2] = th;
+        en[3] = ts;
+    }
+    __syncthreads();
+}
+
+// GRADC of basis i: 2 norm (H C - E S C)_i (python/make_grad.py:85).
+template <int N>
+__device__ __forceinline__ double gradc_from_rows(const double *__restrict__ sums, int K, int i, const double *en) {
+    constexpr int PB = SumFields<N>::size, R = SumFields<N>::row;
+    return 2.0 * en[1] * ((sums[(size_t)R * K + i] + sums[(size_t)(2 * PB + R) * K + i]) -
+                          en[0] * (sums[(size_t)(PB + R) * K + i] + sums[(size_t)(3 * PB + R) * K + i]));
 }
 
 }  // namespace necg

@@ -49,15 +49,20 @@ struct necg_handle {
     size_t xsym_cap = 0;  // doubles
     int2 *d_urange = nullptr;  // queue units of each row block (bra partial slots)
     int urange_cap = 0;
+    int *d_tslot = nullptr;    // per tile: its slots in d_xsym, or -1
+    int tslot_cap = 0;
+    bool sms_general = true;   // some shift map is not kron(m, I3)
     int *d_qcount = nullptr;    // queue head of the block-synchronised fused pass
     int2 *d_bgroups = nullptr;  // the same groups with 8 chunks each (the batched step's blocks)
     int bgroups_cap = 0, nbgroups = 0;
+    int2 *d_burange = nullptr;  // groups of each row block in d_bgroups
+    int burange_cap = 0;
     // fused pass with one-warp tiles: symmetry terms split over npc warps per tile
     int npc = 1;
     double *d_Hp = nullptr, *d_Sp = nullptr;  // npc K x K sums each
     size_t hp_cap = 0;                        // doubles per buffer
-    // pinned host landing area of the host entry point: f, then the two status words
-    double *h_tail = nullptr;
+    double *d_out = nullptr;  // f, the status words and g (d_f, d_status and d_g point into it)
+    double *h_out = nullptr;  // its pinned copy, of the host entry point
     // the fused evaluation's launch sequence as a CUDA graph: captured (on the
     // handle's own stream) the second time a call repeats the same key, then
     // replayed on the caller's stream while the key stays the same

@@ -1,15 +1,19 @@
 // necg_kernels.cu -- sm_100a FP64 kernels of the ECG energy+gradient path.
 //
 // One outprod evaluation (python/outprod.py:20-76 + python/make_grad.py:18-90)
-// is the launch sequence
-//   prep_bra    per basis k:     A_k, S_k, A_k S_k, A_k M A_k, i1, |L_k|^{3/2}
-//   prep_ket    per (l, P):      A_l' = P^T A_l P, S_l' = sms s_l and derived data
+// is, with separate passes for the matrices and the gradient, the launch sequence
+//   prep        per basis k:     A_k, S_k, A_k S_k, A_k M A_k, i1, |L_k|^{3/2}
+//               per (l, P):      A_l' = P^T A_l P, S_l' = sms s_l and derived data
 //   energy      triangle tiles:  H_kl, S_kl for k >= l  (the matel loop)
 //   rows        per row:         (H C)_i, (S C)_i
 //   finalize    one block:       E = C^T H C / C^T S C, norm, GRADC
 //   grad        square tiles:    sum over (l, P) of the bra gradient of
 //                                2 C_l w_P (h - E ov)    (the gradel loop)
 //   grad_reduce per basis k:     sum the tile partials, map A-space to vech(L)
+// and with the fused pass (unordered pairs)
+//   prep, fsym  triangle tiles:  H and S sums and both gradients as raw sums
+//   fsym_sum    per (32 bases, field): the tile partials
+//   fsym_finish per basis k:     E, norm, GRADC from the row sums; gradient, vech(L)
 // Tiles are one warp wide: lane = bra basis function k, while the ket (l, P)
 // loops are warp-uniform, so ket records are read once per warp as broadcasts.
 // The per-thread bodies live in necg_lanes.cuh.
@@ -30,23 +34,27 @@ struct DevKet {
     __device__ __forceinline__ const double *at(size_t off) const { return p + off; }
 };
 
+// Bra records (the first nbb blocks) and ket records (the others), in one launch
+// with the reset of the status words and of the block variants' queue head.
 template <int N>
-__global__ void __launch_bounds__(128) prep_bra_kernel(const double *__restrict__ iv, int K,
-                                                       Consts<N> cs, double *__restrict__ bra) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < K) prep_bra_at<N>(iv + (size_t)k * (tri(N) + 3 * N), cs, bra_at<N>(bra, k), 32);
-}
-
-template <int N>
-__global__ void __launch_bounds__(128) prep_ket_kernel(const double *__restrict__ iv,
-                                                       const double *__restrict__ C, int K, int nst,
-                                                       Consts<N> cs, const double *__restrict__ sml,
-                                                       const double *__restrict__ sms,
-                                                       const double *__restrict__ scvv,
-                                                       double *__restrict__ ket,
-                                                       const int *__restrict__ pinv) {
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id < K * nst) prep_ket_one<N>(iv, C, nst, cs, sml, sms, scvv, ket, id, pinv);
+__global__ void __launch_bounds__(64) prep_kernel(const double *__restrict__ iv, const double *__restrict__ C, int K,
+                                                  int nst, int nbb, Consts<N> cs, const double *__restrict__ sml,
+                                                  const double *__restrict__ sms, const double *__restrict__ scvv,
+                                                  const int *__restrict__ pinv, int general, int full,
+                                                  double *__restrict__ bra, double *__restrict__ ket, int *status,
+                                                  int *qcount) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        status[0] = 0;
+        status[1] = 0x7fffffff;
+        if (qcount) *qcount = 0;
+    }
+    if ((int)blockIdx.x < nbb) {
+        const int k = blockIdx.x * blockDim.x + threadIdx.x;
+        if (k < K) prep_bra_at<N>(iv + (size_t)k * (tri(N) + 3 * N), cs, bra_at<N>(bra, k), 32);
+        return;
+    }
+    const int id = (blockIdx.x - nbb) * blockDim.x + threadIdx.x;
+    if (id < K * nst) prep_ket_one<N>(iv, C, nst, cs, sml, sms, scvv, ket, id, pinv, general, full);
 }
 
 // Energy tiles over the lower triangle (the loop of python/outprod.py:49-54 and
@@ -251,7 +259,7 @@ __global__ void __launch_bounds__(32, MINW) gsym_kernel(const int2 *__restrict__
                                                    const double *__restrict__ scal, RawMap kmap,
                                                    double *__restrict__ part_b,
                                                    double *__restrict__ part_k, int *status) {
-    __shared__ double sacc[2 * Part<N>::size * 32];
+    __shared__ double sacc[2 * SumFields<N>::size * 32];
     __shared__ double krow[ket_table<N>(1)];
     __shared__ double kred[32];
     __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::term : 2];
@@ -277,7 +285,7 @@ __global__ void __launch_bounds__(32, MINW) fsym_kernel(const int2 *__restrict__
                                                    double *__restrict__ H, double *__restrict__ S,
                                                    double *__restrict__ part_b,
                                                    double *__restrict__ part_k, int *status) {
-    __shared__ double sacc[2 * Part<N>::size * 32];
+    __shared__ double sacc[2 * SumFields<N>::size * 32];
     __shared__ double krow[ket_table<N>(2)];
     __shared__ double kred[64];
     __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::term : 2];
@@ -286,9 +294,9 @@ __global__ void __launch_bounds__(32, MINW) fsym_kernel(const int2 *__restrict__
     const int pc = blockIdx.y, PC = (nst + npc - 1) / npc;
     const int p0 = min(pc * PC, nst), p1 = min(p0 + PC, nst);
     const size_t off = (size_t)pc * K * K;
-    fsym_tile<N, VKET, false, SKET>(t * npc + pc, tiles[t], LC, K, nst, cs, bra, ket, C, kmap, H + off,
-                                           S + off, part_b, part_k, status, FusedSmem{sacc, krow, kred, sket},
-                                           false, nullptr, p0, p1);
+    fsym_tile<N, VKET, false, SKET>(t * npc + pc, tiles[t], LC, K, nst, cs, bra, ket, C, kmap, H ? H + off : nullptr,
+                                    H ? S + off : nullptr, part_b, part_k, status,
+                                    FusedSmem{sacc, krow, kred, sket}, false, nullptr, p0, p1);
 }
 
 // H, S = sum over the npc splits of the fused pass (fixed order: deterministic).
@@ -314,10 +322,10 @@ __global__ void __launch_bounds__(256) hs_reduce_kernel(const double *__restrict
 // ends: a block barrier per term, which once kept the warps of a scheduler in
 // step, now only costs (LiH K = 1024 on a B200: 2.54 ms with it, 2.76 ms and more
 // with half of the warps taking it in mid-term, 2.34 ms without).  Shared
-// memory (dynamic, 16-byte aligned): per warp 2 PS 32 + ket table + 64 + 2 ket
+// memory (dynamic, 16-byte aligned): per warp 2 PB 32 + ket table + 64 + 2 ket
 // records doubles, then the bras.  KE: the symmetric pass with E known.
 template <int N> __host__ __device__ constexpr int fsym_warp_smem() {
-    return 2 * Part<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
+    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
 }
 template <int N> __host__ __device__ constexpr int fsym_block_smem_bytes(int warps) {
     return (warps * fsym_warp_smem<N>() + BraLayout<N>::term * 32) * 8;
@@ -338,14 +346,14 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
                                                                 const double *__restrict__ scal) {
     extern __shared__ __align__(16) double smem[];
     __shared__ int gsh;
-    constexpr int PS = Part<N>::size;
+    constexpr int PB = SumFields<N>::size;
     constexpr int PER_WARP = fsym_warp_smem<N>();
     constexpr int BS = BraLayout<N>::term;
     constexpr int TBL = ket_table<N>(2);
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
     double *sbra = smem + WARPS * PER_WARP;  // BS x 32 doubles after the warps' areas
-    const FusedSmem sm{base, base + 2 * PS * 32, base + 2 * PS * 32 + TBL, base + 2 * PS * 32 + TBL + 64};
+    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + 64};
     for (;;) {
         if (threadIdx.x == 0) gsh = atomicAdd(qcount, 1);
         __syncthreads();
@@ -377,129 +385,102 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
         // accumulators are summed (in warp order) and written once, to the
         // slot of queue unit g
         __syncthreads();
-        for (int i = threadIdx.x; i < 2 * PS * 32; i += 32 * WARPS) {
+        for (int i = threadIdx.x; i < 2 * PB * 32; i += 32 * WARPS) {
             if (kb * 32 + (i & 31) >= K) continue;
             double v = smem[i];
 #pragma unroll
             for (int q = 1; q < WARPS; ++q) v += smem[q * PER_WARP + i];
-            part_b[(size_t)g * 2 * PS * 32 + i] = v;
+            part_b[(size_t)g * 2 * PB * 32 + i] = v;
         }
         __syncthreads();  // sbra and the warps' areas are rewritten for the next group
     }
 }
 
-// The split tail of the lockstep pass: add parts 1 .. parts - 1 of each tile
-// (their compact slots in xsym, in part order) into the tile's ket partials
-// and H, S entries, which part 0 wrote (each part's bra partials have a queue
-// slot of their own).  Block = one tile (tail group j, warp w); entries that no
-// part wrote (kets past K or above the diagonal, tiles past the block's
-// triangle) are left alone.  H = nullptr: the symmetric pass, which has no H and
-// S sums and no S part of the ket partials.
+// H and S of the tiles of the block variants' split tail, when the caller wants
+// them: add parts 1 .. parts - 1 of each tile (their compact slots in xsym, in
+// part order) to what part 0 wrote.  Block = one tile (tail group j, warp w);
+// entries that no part wrote (kets past K or above the diagonal, tiles past the
+// block's triangle) are left alone.
 template <int N>
 __global__ void __launch_bounds__(256) fsym_tail_fix_kernel(const int2 *__restrict__ groups, int tail0, int W,
-                                                            int LC, int K, const int *__restrict__ tstart,
-                                                            const double *__restrict__ xsym,
-                                                            double *__restrict__ part_k, double *__restrict__ H,
-                                                            double *__restrict__ S) {
-    constexpr int PS = Part<N>::size;
+                                                            int LC, int K, const double *__restrict__ xsym,
+                                                            double *__restrict__ H, double *__restrict__ S) {
+    constexpr int PB = SumFields<N>::size;
     const int j = blockIdx.x / W, w = blockIdx.x - j * W;
     const int2 gr = groups[tail0 + j * sgroup_parts(groups[tail0])];
     const int parts = sgroup_parts(gr);
     const int kb = gr.x, lc = sgroup_lc0(gr) + w;
-    const int last = min(kb * 32 + 31, K - 1);
-    if (lc * LC > last) return;
-    const int t = tstart[kb] + lc;
-    const size_t XS = fsym_tail_slot(PS, LC);
-    const double *x0 = xsym + (size_t)(j * W + w) * (parts - 1) * XS;
-    double *pk = part_k + (size_t)t * LC * 2 * PS;
-    for (int i = threadIdx.x; i < LC * 2 * PS; i += blockDim.x) {
-        if (lc * LC + i / (2 * PS) >= K || (!H && i % (2 * PS) >= PS)) continue;
-        double v = pk[i];
-        for (int q = 0; q < parts - 1; ++q) v += x0[q * XS + i];
-        pk[i] = v;
-    }
-    for (int i = threadIdx.x; H && i < LC * 64; i += blockDim.x) {
+    if (lc * LC > min(kb * 32 + 31, K - 1)) return;
+    const size_t XS = fsym_tail_slot(PB, LC);
+    const double *x0 = xsym + (size_t)(j * W + w) * (parts - 1) * XS + (size_t)LC * 2 * PB;
+    for (int i = threadIdx.x; i < LC * 64; i += blockDim.x) {
         const int l = lc * LC + i / 64, r = i & 63, k = kb * 32 + (r & 31);
         if (k >= K || l >= K || l > k) continue;
         double *M = r < 32 ? H : S;
         double v = M[(size_t)k * K + l];
-        for (int q = 0; q < parts - 1; ++q) v += x0[q * XS + (size_t)LC * 2 * PS + i];
+        for (int q = 0; q < parts - 1; ++q) v += x0[q * XS + i];
         M[(size_t)k * K + l] = v;
         M[(size_t)l * K + k] = v;
     }
 }
 
-// Sum the partials of the fused (KE = false) or the symmetric pass into the
-// per-basis sums (put_sums), combined as H - 2 E S with E = scal[0] (written by
-// finalize after the fused pass; the symmetric pass has combined its own).
-// Block (kb, f): the 32 bases of row block kb, field f.  Their bra partials come
-// from every tile of block kb (up to K / LC of them) and their ket partials from
-// one tile per later row block, so the 8 warps of the block take every 8th of
-// each and their sums are combined in a fixed order.  Only tiles in [t0, t1)
-// count (a shard of the pass).
+// Partials of the fused (KE = false) or the symmetric pass into the per-basis
+// sums: block (kb, f) (sum_partials).  The symmetric pass has no row field.
 template <int N, bool KE>
-__global__ void __launch_bounds__(256) fsym_sum_kernel(const int *__restrict__ tstart, int LC, int K,
-                                                       const double *__restrict__ part_b,
-                                                       const double *__restrict__ part_k,
-                                                       const double *__restrict__ scal,
-                                                       double *__restrict__ out, int t0, int t1, int npc,
-                                                       const int2 *__restrict__ urange, int folded) {
-    constexpr int PS = Part<N>::size;
+__global__ void __launch_bounds__(256) fsym_sum_kernel(PassParts p, double *__restrict__ sums) {
     __shared__ double red[4][8][32];
-    const int kb = blockIdx.x, f = blockIdx.y;
-    const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
-    const int m = kb * 32 + lane;
-    // bra partial slots: tile t's splits are slots t npc .. t npc + npc - 1, or
-    // (urange, the lockstep pass) the queue units [urange[kb].x, urange[kb].y)
-    const int ta = urange ? urange[kb].x : max(tstart[kb], t0) * npc;
-    const int tb = urange ? urange[kb].y : min(tstart[kb + 1], t1) * npc;
-    double sH = 0.0, sS = 0.0;
-    for (int t = ta + seg; t < tb; t += 8) {
-        sH += part_b[(((size_t)t * 2 + 0) * PS + f) * 32 + lane];
-        sS += part_b[(((size_t)t * 2 + 1) * PS + f) * 32 + lane];
-    }
-    double kH = 0.0, kS = 0.0;
-    if (m < K) ket_partials<N, !KE>(tstart, LC, K, f, m, part_k, t0, t1, npc, seg, 8, kH, kS);
-    red[0][seg][lane] = sH;
-    red[1][seg][lane] = sS;
-    red[2][seg][lane] = kH;
-    red[3][seg][lane] = kS;
-    __syncthreads();
-    if (seg != 0 || m >= K) return;
-    // fixed order: the 8 warps' sums of each
-    sH = sS = kH = kS = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        sH += red[0][q][lane];
-        sS += red[1][q][lane];
-        kH += red[2][q][lane];
-        kS += red[3][q][lane];
-    }
-    put_sums(out, PS, K, f, m, sH, sS, kH, kS, KE ? 0.0 : 2.0 * scal[0], folded);
+    sum_partials<N, !KE>(p, blockIdx.x, blockIdx.y, sums, red);
 }
 
-// The gradient of basis k from its sums (finish_one): written field-major to
-// `fields` (a shard's share, all-reduced before GRADA) or mapped to vech(L),
-// scaled by norm C_k and written to GRADA block k.
+// rows[i] = (H C)_i, rows[K + i] = (S C)_i from the per-basis sums (a shard's share).
 template <int N>
-__global__ void __launch_bounds__(32) fsym_finish_kernel(const double *__restrict__ sums, int K, Consts<N> cs,
-                                                         const double *__restrict__ bra,
-                                                         const double *__restrict__ C,
-                                                         const double *__restrict__ scal, int folded,
-                                                         double *__restrict__ fields, double *__restrict__ g,
-                                                         int *status) {
+__global__ void __launch_bounds__(128) rows_from_sums_kernel(const double *__restrict__ sums, int K,
+                                                             double *__restrict__ rows) {
+    constexpr int PB = SumFields<N>::size, R = SumFields<N>::row;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2 * K) return;
+    const int which = i >= K, m = i - which * K;
+    rows[i] = sums[(size_t)(which * PB + R) * K + m] + sums[(size_t)((2 + which) * PB + R) * K + m];
+}
+
+// From the per-basis sums to the gradient, 32 bases per block.  OWN_E: every block
+// forms E and norm from the row sums (the same order in each, 5 K reads that cost
+// less than a kernel of their own), block 0 writes them and f, and GRADC of the
+// block's bases goes to gradc; else E and norm are scal's (KE: the sums are
+// combined already).  Then the gradient of basis k (finish_one): written
+// field-major to `fields` (a shard's share, all-reduced before GRADA) or mapped to
+// vech(L), scaled by norm C_k and written to GRADA block k.
+template <int N, bool KE, bool OWN_E>
+__global__ void __launch_bounds__(128) fsym_finish_kernel(const double *__restrict__ sums, int K, Consts<N> cs,
+                                                          const double *__restrict__ bra,
+                                                          const double *__restrict__ C, double *__restrict__ scal,
+                                                          int folded, double *__restrict__ fields,
+                                                          double *__restrict__ g, double *__restrict__ gradc,
+                                                          double *__restrict__ f_out, int *status) {
     constexpr int PS = Part<N>::size;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
+    __shared__ double sh[2][32], en[4];
+    const int k = blockIdx.x * 32 + threadIdx.x;
+    if (OWN_E) {
+        energy_from_rows<N>(sums, C, K, sh, en);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) scal[i] = en[i];
+            if (f_out) *f_out = en[0];
+            if (!isfinite(en[0])) atomicOr(status, 2);
+        }
+    }
+    if (threadIdx.x >= 32 || k >= K) return;
+    const double E = OWN_E ? en[0] : scal[0], norm = OWN_E ? en[1] : scal[1];
+    if (OWN_E) gradc[k] = gradc_from_rows<N>(sums, K, k, en);
     double o[PS];
     const double *brak = bra_at<N>(bra, k);
-    finish_one<N>(sums, K, brak, cs, folded, k, o);
+    finish_one<N>(sums, K, brak, cs, folded, KE ? 0.0 : 2.0 * E, k, o);
     if (fields) {
 #pragma unroll
         for (int f = 0; f < PS; ++f) fields[(size_t)f * K + k] = o[f];
         return;
     }
-    if (!fields_to_grad<N>(o, brak, 32, scal[1] * C[k], g, k)) atomicOr(status, 2);
+    if (!fields_to_grad<N>(o, brak, 32, norm * C[k], g, k)) atomicOr(status, 2);
 }
 
 // Sum the gradient-tile partials over the ket chunks, in place into chunk 0:
@@ -783,11 +764,6 @@ __global__ void f0_kernel(const double *__restrict__ z, int count, double *__res
     if (df) df[i] = 0.5 * fs * D2;
 }
 
-__global__ void reset_status_kernel(int *status) {
-    status[0] = 0;
-    status[1] = 0x7fffffff;
-}
-
 // ---------------------------------------------------------------------------
 // Host-side launchers (one instantiation per supported particle count)
 template <int N> Consts<N> make_consts(const double *mass, const double *ncv, double efs) {
@@ -805,10 +781,9 @@ template <int N> Consts<N> make_consts(const double *mass, const double *ncv, do
 template <int N> struct Launch {
     static void prep(const LaunchArgs &a, cudaStream_t st) {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
-        prep_bra_kernel<N><<<(a.K + 127) / 128, 128, 0, st>>>(a.iv, a.K, cs, a.bra);
-        const int nk = a.K * a.nst;
-        prep_ket_kernel<N><<<(nk + 127) / 128, 128, 0, st>>>(a.iv, a.C, a.K, a.nst, cs, a.sml, a.sms,
-                                                             a.scvv, a.ket, a.pinv);
+        const int nbb = (a.K + 63) / 64, nbk = (a.K * a.nst + 63) / 64;
+        prep_kernel<N><<<nbb + nbk, 64, 0, st>>>(a.iv, a.C, a.K, a.nst, nbb, cs, a.sml, a.sms, a.scvv, a.pinv,
+                                                 a.sms_general, a.full || a.kmap.fold, a.bra, a.ket, a.status, a.qcount);
     }
     template <int MINW> static void energy_v(const LaunchArgs &a, cudaStream_t st) {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
@@ -865,7 +840,7 @@ template <int N> struct Launch {
             Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
             gsym_kernel<N, MINW, SKET><<<a.nstiles, 32, 0, st>>>(a.stiles, a.nstiles, a.LC_s, a.K, a.nst, cs, a.bra,
                                                                  a.ket, a.C, a.scal, a.kmap, a.psym,
-                                                                 a.psym + (size_t)a.nstiles * 2 * Part<N>::size * 32,
+                                                                 a.psym + (size_t)a.nstiles * 2 * SumFields<N>::size * 32,
                                                                  a.status);
         }
     }
@@ -876,11 +851,6 @@ template <int N> struct Launch {
     static void gsym_tiles(const LaunchArgs &a, cudaStream_t st) {
         if (gsym_block(a)) {
             fsym_block<8, true>(a, st);
-            if (a.sg_ntail > 0 && a.sg_parts >= 2 && a.xsym) {  // the queue's split tail: no H and S sums to add
-                LaunchArgs b = a;
-                b.H = b.S = nullptr;
-                fsym_tail(b, st);
-            }
             return;
         }
         switch (a.minb_s) {
@@ -893,18 +863,26 @@ template <int N> struct Launch {
         }
     }
     static void gsym_reduce(const LaunchArgs &a, cudaStream_t st) {
-        if constexpr (Part<N>::size <= 32) sum_finish<true>(a, gsym_block(a), 1, 0, a.nstiles, st);
+        if constexpr (Part<N>::size <= 32) {
+            sum<true>(a, gsym_block(a), 1, 0, a.nstiles, st);
+            finish<true, false>(a, nullptr, nullptr, st);
+        }
     }
-    // the per-basis sums and their gradients; lockstep: bra partials per queue unit
+    // the per-basis sums; blocks: the pass ran as a block variant over the whole tile list
     template <bool KE>
-    static void sum_finish(const LaunchArgs &a, bool lockstep, int npc, int t0, int t1, cudaStream_t st) {
-        constexpr int PS = Part<N>::size;
+    static void sum(const LaunchArgs &a, bool blocks, int npc, int t0, int t1, cudaStream_t st) {
+        constexpr int PB = SumFields<N>::size;
+        const bool tail = blocks && a.sg_ntail > 0 && a.sg_parts >= 2;
+        const PassParts p{a.stile_start, blocks ? a.urange : nullptr, tail ? a.tslot : nullptr, a.psym,
+                          a.psym + (size_t)a.nstiles * npc * 2 * PB * 32, a.xsym, a.LC_s, a.K, t0, t1, npc, a.sg_parts};
+        fsym_sum_kernel<N, KE><<<dim3((a.K + 31) / 32, KE ? PB - 1 : PB), 256, 0, st>>>(p, a.part);
+    }
+    template <bool KE, bool OWN_E>
+    static void finish(const LaunchArgs &a, double *f_out, double *gradc, cudaStream_t st) {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
-        fsym_sum_kernel<N, KE><<<dim3((a.K + 31) / 32, PS), 256, 0, st>>>(
-            a.stile_start, a.LC_s, a.K, a.psym, a.psym + (size_t)a.nstiles * npc * 2 * PS * 32, a.scal, a.part, t0, t1,
-            npc, lockstep ? a.urange : nullptr, a.kmap.fold);
-        fsym_finish_kernel<N><<<(a.K + 31) / 32, 32, 0, st>>>(a.part, a.K, cs, a.bra, a.C, a.scal, a.kmap.fold, a.sums,
-                                                              a.g, a.status);
+        fsym_finish_kernel<N, KE, OWN_E><<<(a.K + 31) / 32, 128, 0, st>>>(a.part, a.K, cs, a.bra, a.C, a.scal,
+                                                                         a.kmap.fold, a.sums, a.g, gradc, f_out,
+                                                                         a.status);
     }
     template <int MINW, bool VKET, bool SKET = false> static void fsym_v(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
@@ -913,8 +891,8 @@ template <int N> struct Launch {
             if (t1 <= t0) return;
             const int npc = a.npc > 1 ? a.npc : 1;
             fsym_kernel<N, MINW, VKET, SKET><<<dim3(t1 - t0, npc), 32, 0, st>>>(
-                a.stiles, t0, t1, a.LC_s, a.K, a.nst, npc, cs, a.bra, a.ket, a.C, a.kmap, npc > 1 ? a.Hp : a.H,
-                npc > 1 ? a.Sp : a.S, a.psym, a.psym + (size_t)a.nstiles * npc * 2 * Part<N>::size * 32, a.status);
+                a.stiles, t0, t1, a.LC_s, a.K, a.nst, npc, cs, a.bra, a.ket, a.C, a.kmap, npc > 1 && a.H ? a.Hp : a.H,
+                npc > 1 && a.H ? a.Sp : a.S, a.psym, a.psym + (size_t)a.nstiles * npc * 2 * SumFields<N>::size * 32, a.status);
         }
     }
     template <int WARPS, bool KE = false> static void fsym_block(const LaunchArgs &a, cudaStream_t st) {
@@ -932,12 +910,13 @@ template <int N> struct Launch {
                 }
                 cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
                 Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
-                cudaMemsetAsync(a.qcount, 0, sizeof(int), st);
+                // the fused sequence's prep has reset the queue; the gradient alone comes later
+                if (KE) cudaMemsetAsync(a.qcount, 0, sizeof(int), st);
                 const int grid = a.nsgroups < sms ? a.nsgroups : sms;
                 if (grid < 1) return;
                 kern<<<grid, 32 * WARPS, smem, st>>>(a.sgroups, a.nsgroups, a.qcount, a.stile_start, a.LC_s, a.K,
                                                      a.nst, cs, a.bra, a.ket, a.C, a.kmap, a.H, a.S, a.psym,
-                                                     a.psym + (size_t)a.nstiles * 2 * Part<N>::size * 32, a.status,
+                                                     a.psym + (size_t)a.nstiles * 2 * SumFields<N>::size * 32, a.status,
                                                      a.xsym, a.sg_tail0, a.scal);
             }
         }
@@ -961,20 +940,27 @@ template <int N> struct Launch {
     static void fsym_tail(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
             const int W = fused_block_warps(a.minb_s);
-            fsym_tail_fix_kernel<N><<<a.sg_ntail * W, 256, 0, st>>>(
-                a.sgroups, a.sg_tail0, W, a.LC_s, a.K, a.stile_start, a.xsym,
-                a.psym + (size_t)a.nstiles * 2 * Part<N>::size * 32, a.H, a.S);
+            fsym_tail_fix_kernel<N><<<a.sg_ntail * W, 256, 0, st>>>(a.sgroups, a.sg_tail0, W, a.LC_s, a.K, a.xsym, a.H,
+                                                                    a.S);
         }
     }
-    static void fsym_reduce(const LaunchArgs &a, cudaStream_t st) {
+    static void fsym_sum(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
             const int t0 = a.st_end > 0 ? a.st_begin : 0, t1 = a.st_end > 0 ? a.st_end : a.nstiles;
             const int npc = a.npc > 1 && a.minb_s < 200 ? a.npc : 1;
-            // the lockstep pass over the whole tile list writes its bra partials
-            // per queue unit (the unit ranges of each row block in urange)
-            const bool lockstep = a.minb_s >= 200 && a.st_end == 0 && a.sgroups && a.urange;
-            sum_finish<false>(a, lockstep, npc, t0, t1, st);
+            const bool blocks = a.minb_s >= 200 && a.st_end == 0 && a.sgroups && a.urange;
+            sum<false>(a, blocks, npc, t0, t1, st);
         }
+    }
+    static void fsym_finish(const LaunchArgs &a, double *f_out, double *gradc, bool own_e, cudaStream_t st) {
+        if constexpr (Part<N>::size <= 32) {
+            if (own_e) finish<false, true>(a, f_out, gradc, st);
+            else finish<false, false>(a, f_out, gradc, st);
+        }
+    }
+    static void rows_from_sums(const LaunchArgs &a, double *rows, cudaStream_t st) {
+        if constexpr (Part<N>::size <= 32)
+            rows_from_sums_kernel<N><<<(2 * a.K + 127) / 128, 128, 0, st>>>(a.part, a.K, rows);
     }
     static void rrms(const LaunchArgs &a, const int *terms, int nterms, double *out, cudaStream_t st) {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
@@ -1079,27 +1065,39 @@ bool fused_variant_ok(int n, int variant) {
 }
 int launch_fsym(const LaunchArgs &a, cudaStream_t st) {
     if (a.n > 5) return -1;
-    // every buffer the pass writes must be set (no launch on a null pointer)
-    if (!a.H || !a.S || !a.psym || !a.stiles || !a.bra || !a.ket || !a.C || !a.status) return -1;
+    // every buffer the pass writes must be set (no launch on a null pointer); H
+    // and S are written when both are
+    if (!a.H != !a.S || !a.psym || !a.stiles || !a.bra || !a.ket || !a.C || !a.status) return -1;
+    if (a.npc > 1 && a.minb_s < 200 && a.H && (!a.Hp || !a.Sp)) return -1;
     NECG_DISPATCH(a.n, fsym_tiles(a, st));
     return 0;
 }
 int launch_fsym_tail(const LaunchArgs &a, cudaStream_t st) {
-    // only the lockstep pass over the whole tile list splits its tail
-    if (a.minb_s < 200 || a.st_end > 0 || a.sg_ntail <= 0 || a.sg_parts < 2) return 0;
-    if (a.n > 5 || !a.sgroups || !a.xsym || !a.psym || !a.H || !a.S || !a.stile_start) return -1;
+    // only a block variant over the whole tile list splits its tail; the sums read
+    // the parts themselves, so this is for H and S alone
+    if (!a.H || a.minb_s < 200 || a.st_end > 0 || a.sg_ntail <= 0 || a.sg_parts < 2) return 0;
+    if (a.n > 5 || !a.sgroups || !a.xsym || !a.S) return -1;
     NECG_DISPATCH(a.n, fsym_tail(a, st));
     return 0;
 }
-int launch_fsym_reduce(const LaunchArgs &a, cudaStream_t st) {
-    if (a.n > 5) return -1;
-    if (!a.stile_start || !a.psym || !a.scal || !a.part || !a.bra || (!a.sums && (!a.C || !a.g))) return -1;
-    NECG_DISPATCH(a.n, fsym_reduce(a, st));
+int launch_fsym_sum(const LaunchArgs &a, cudaStream_t st) {
+    if (a.n > 5 || !a.stile_start || !a.psym || !a.part) return -1;
+    NECG_DISPATCH(a.n, fsym_sum(a, st));
+    return 0;
+}
+int launch_fsym_finish(const LaunchArgs &a, double *f_out, double *gradc, bool own_e, cudaStream_t st) {
+    if (a.n > 5 || !a.part || !a.bra || !a.C || !a.scal || !a.status || (!a.sums && !a.g) || (own_e && !gradc)) return -1;
+    NECG_DISPATCH(a.n, fsym_finish(a, f_out, gradc, own_e, st));
+    return 0;
+}
+int launch_rows_from_sums(const LaunchArgs &a, double *rows, cudaStream_t st) {
+    if (a.n > 5 || !a.part || !rows) return -1;
+    NECG_DISPATCH(a.n, rows_from_sums(a, rows, st));
     return 0;
 }
 int launch_hs_reduce(const LaunchArgs &a, cudaStream_t st) {
-    if (a.npc <= 1) return 0;
-    if (!a.Hp || !a.Sp || !a.H || !a.S) return -1;
+    if (a.npc <= 1 || !a.H) return 0;  // H and S not wanted: nothing to sum
+    if (!a.Hp || !a.Sp || !a.S) return -1;
     const size_t KK = (size_t)a.K * a.K;
     const size_t blocks = (KK + 255) / 256 < 4096 ? (KK + 255) / 256 : 4096;
     hs_reduce_kernel<<<(int)blocks, 256, 0, st>>>(a.Hp, a.Sp, a.npc, KK, a.H, a.S);
@@ -1133,16 +1131,10 @@ void launch_rows_finalize(const LaunchArgs &a, double *f_out, double *gradc, int
     finalize_kernel<<<1, 1024, 0, st>>>(a.rows, a.C, a.K, a.scal, f_out, gradc, a.status, given, eng,
                                         norm, given_dev, en_out);
 }
-int launch_rows(const LaunchArgs &a, double *rows, cudaStream_t st) {
-    if (!a.H || !a.S || !a.C || !rows) return -1;
-    rows_kernel<<<(a.K * 32 + 255) / 256, 256, 0, st>>>(a.H, a.S, a.C, a.K, rows);
-    return 0;
-}
 void launch_finalize(const LaunchArgs &a, const double *rows, double *f_out, double *gradc, cudaStream_t st) {
     finalize_kernel<<<1, 1024, 0, st>>>(rows, a.C, a.K, a.scal, f_out, gradc, a.status, 0, 0.0, 0.0, nullptr,
                                         nullptr);
 }
-void launch_reset_status(int *status, cudaStream_t st) { reset_status_kernel<<<1, 1, 0, st>>>(status); }
 void launch_fp64_probe(int blocks, int iters, double *sink, cudaStream_t st) {
     fp64_probe_kernel<<<blocks, 256, 0, st>>>(iters, 1.0, sink);
 }
@@ -1173,9 +1165,11 @@ int bra_record_size(int n) {
     }
 }
 int part_stride(int n) { return n >= 1 && n <= 6 ? tri(n) + 1 + 3 * n : 0; }
+size_t sums_doubles(int n, int K) { return (size_t)kSumSets * (part_stride(n) + 1) * K; }
 size_t part_doubles(int n, int K) {
-    const size_t per = (size_t)part_stride(n) * K, nlc = (size_t)(K + 3) / 4;
-    return per * (nlc > kSumSets ? nlc : kSumSets);
+    const size_t ordered = (size_t)part_stride(n) * K * ((K + 3) / 4);
+    const size_t sums = sums_doubles(n, K);
+    return ordered > sums ? ordered : sums;
 }
 int ket_slots(int n) {
     switch (n) {

@@ -48,6 +48,8 @@ struct LaunchArgs {
     // lockstep pass: bra partials are written per queue unit; row block kb's
     // units are [urange[kb].x, urange[kb].y)
     const int2 *urange;
+    const int *tslot;                      // first xsym slot of each tile of a split tail group, else -1
+    int sms_general, full;                 // prep: general shift maps; whole ket records (else the terms' part)
 };
 
 // A tile group of the lockstep pass: row block kb, first ket chunk lc0 and, for
@@ -66,18 +68,22 @@ int launch_energy(const LaunchArgs &a, cudaStream_t st);
 int launch_grad(const LaunchArgs &a, cudaStream_t st);
 int launch_gsym(const LaunchArgs &a, cudaStream_t st);
 int launch_gsym_reduce(const LaunchArgs &a, cudaStream_t st);
-// fused energy + symmetric gradient pass (writes H, S and split partials) and
-// its reduction (needs E in scal, i.e. after launch_rows_finalize)
+// fused energy + symmetric gradient pass (writes split partials, and H and S when
+// a.H is set), the per-basis sums of its partials (a.part), and the gradient from
+// them: own_e: E, norm and GRADC (gradc) too, from the row sums; else E and norm
+// are in a.scal, and with a.sums the fields go there instead of GRADA
+int launch_fsym_sum(const LaunchArgs &a, cudaStream_t st);
+int launch_fsym_finish(const LaunchArgs &a, double *f_out, double *gradc, bool own_e, cudaStream_t st);
+int launch_rows_from_sums(const LaunchArgs &a, double *rows, cudaStream_t st);
 int launch_fsym(const LaunchArgs &a, cudaStream_t st);
 // lockstep-block variants of the fused pass (2xy): warps per block, and
 // whether the variant's shared memory fits for n particles
 int fused_block_warps(int variant);
 bool fused_variant_ok(int n, int variant);
-int launch_fsym_reduce(const LaunchArgs &a, cudaStream_t st);
 // H, S = sum over the splits of Hp, Sp (fused pass with npc > 1), before rows/finalize
 int launch_hs_reduce(const LaunchArgs &a, cudaStream_t st);
-// add the split parts of the lockstep pass's tail tiles into the main buffers
-// (after launch_fsym, before H and S are read)
+// add the split parts of the block variants' tail tiles into H and S (after
+// launch_fsym, before H and S are read)
 int launch_fsym_tail(const LaunchArgs &a, cudaStream_t st);
 int launch_grad_tiles(const LaunchArgs &a, cudaStream_t st);
 int launch_grad_reduce(const LaunchArgs &a, cudaStream_t st);
@@ -93,10 +99,8 @@ int launch_gradel(const LaunchArgs &a, const int *terms, int nterms, double *tg,
 void launch_rows_finalize(const LaunchArgs &a, double *f_out, double *gradc, int given,
                           double eng, double norm, cudaStream_t st,
                           const double *given_dev = nullptr, double *en_out = nullptr);
-void launch_reset_status(int *status, cudaStream_t st);
-// pieces of a sharded evaluation: rows (H C, S C) of this shard's H and S;
-// E, norm and GRADC from given rows; GRADA from given per-basis sums
-int launch_rows(const LaunchArgs &a, double *rows, cudaStream_t st);
+// pieces of a sharded evaluation: E, norm and GRADC from given rows; GRADA from
+// given per-basis sums
 void launch_finalize(const LaunchArgs &a, const double *rows, double *f_out, double *gradc, cudaStream_t st);
 int launch_reduce_sums(const LaunchArgs &a, const double *sums, cudaStream_t st);
 void launch_fp64_probe(int blocks, int iters, double *sink, cudaStream_t st);
@@ -109,6 +113,7 @@ int part_stride(int n);
 // the gradient-partial buffer of bases of up to K functions: tile partials of
 // the ordered pass (ket chunks of 4 or more) or the per-basis sums
 size_t part_doubles(int n, int K);
+size_t sums_doubles(int n, int K);
 // ket slots per (P, matrix) and the slot of a field (KetSlots, n <= 5)
 int ket_slots(int n);
 int ket_slot(int n, int f);

@@ -98,11 +98,13 @@ template <int N> NECG_HD void prep_bra_one(const double *iv, int K, const Consts
 }
 
 // Ket record of (l, P) = id / nst, id % nst: python/matel.py:76-87
-// (al <- sml^T al sml, st2 <- sms st2) plus the data the tiles reuse.
+// (al <- sml^T al sml, st2 <- sms st2) plus the data the tiles reuse.  general =
+// false: the shift map is kron(m, I3), so that m alone is read (25 instead of 225
+// entries at n = 5).  full = false: only the `term` part of the record.
 template <int N>
 NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Consts<N> &cs,
                           const double *sml, const double *sms, const double *scvv, double *ket,
-                          int id, const int *pinv = nullptr) {
+                          int id, const int *pinv = nullptr, bool general = true, bool full = true) {
     using KL = KetLayout<N>;
     constexpr int blk = tri(N) + 3 * N;
     const int l = id / nst, P = id - l * nst;
@@ -131,18 +133,32 @@ NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Cons
             for (int k = 0; k < N; ++k) s += pm[k * N + i] * Apm[k * N + j];
             Ap[sx(i, j)] = s;
         }
-    const double *sm = sms + (size_t)P * 9 * N * N;  // general 3n x 3n shift map
+    const double *sm = sms + (size_t)P * 9 * N * N;  // 3n x 3n shift map
     double Sp[3 * N];
+    if (general) {
 #pragma unroll
-    for (int r = 0; r < 3 * N; ++r) {
-        double s = 0.0;
+        for (int r = 0; r < 3 * N; ++r) {
+            double s = 0.0;
 #pragma unroll
-        for (int c = 0; c < 3 * N; ++c) s += sm[r * 3 * N + c] * b[tri(N) + c];
-        Sp[r] = s;
+            for (int c = 0; c < 3 * N; ++c) s += sm[r * 3 * N + c] * b[tri(N) + c];
+            Sp[r] = s;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            double s[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const double m = sm[(3 * i) * 3 * N + 3 * j];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) s[c] += m * b[tri(N) + 3 * j + c];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) Sp[3 * i + c] = s[c];
+        }
     }
-    double ASp[3 * N], AM[N * N], AMA[tri(N)], tMA;
+    double ASp[3 * N];
     symv3<N>(Ap, 0, Sp, ASp);
-    mass_products<N>(Ap, cs.M, AM, AMA, tMA);
     double i2 = 0.0, dl = 1.0;
 #pragma unroll
     for (int t = 0; t < 3 * N; ++t) i2 += Sp[t] * ASp[t];
@@ -153,18 +169,21 @@ NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Cons
 #pragma unroll
     for (int t = 0; t < tri(N); ++t) o[KL::Ap + t] = Ap[t];
 #pragma unroll
-    for (int t = 0; t < 3 * N; ++t) o[KL::Sp + t] = Sp[t];
-#pragma unroll
     for (int t = 0; t < 3 * N; ++t) o[KL::ASp + t] = ASp[t];
-#pragma unroll
-    for (int t = 0; t < tri(N); ++t) o[KL::Np8 + t] = -8.0 * AMA[t];
     o[KL::i2] = i2;
     o[KL::pre] = dl * ::sqrt(dl);
-    o[KL::tMA] = tMA;
     o[KL::w] = scvv[P];
     o[KL::wC] = C ? 2.0 * scvv[P] * C[l] : 0.0;
     o[KL::winv] = pinv ? scvv[pinv[P]] : 0.0;
     if (KL::term > KL::winv + 1) o[KL::winv + 1] = 0.0;
+    if (!full) return;
+    double AM[N * N], AMA[tri(N)], tMA;
+    mass_products<N>(Ap, cs.M, AM, AMA, tMA);
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) o[KL::Sp + t] = Sp[t];
+#pragma unroll
+    for (int t = 0; t < tri(N); ++t) o[KL::Np8 + t] = -8.0 * AMA[t];
+    o[KL::tMA] = tMA;
     if (KL::size > KL::tMA + 1) o[KL::tMA + 1] = 0.0;
 }
 
@@ -473,22 +492,40 @@ struct RawMap {
     int maxnz, fold;
 };
 
-// Per-basis sums of the symmetric passes, field-major with stride K: the bra's
-// combined raw sums (H - 2 E S) plus, unless the kets were folded, the kets';
-// the bra's raw S sums; the kets' folded gradient when they were.
-constexpr int kSumSets = 3;
+// Fields the symmetric passes sum per basis function and matrix: the raw fields
+// and, last, its row of H C or S C.
+template <int N> struct SumFields {
+    static constexpr int row = Part<N>::size;
+    static constexpr int size = row + 1;
+};
 
-// The gradient fields (Part<N>) of basis k from its sums (brak = bra_at(bra, k)).
+// Per-basis sums of the symmetric passes: kSumSets sets of SumFields, field f of
+// set i of basis k at (i SumFields::size + f) K + k: the bra's H (or, with E
+// known, combined) and S sums, then the ket's.
+constexpr int kSumSets = 4;
+
+// The gradient fields (Part<N>) of basis k from its sums (brak = bra_at(bra, k)),
+// for the gradient of h - E ov; E2 = 2 E, or 0 where the sums are combined already
+// (then there is no S set of the ket).
 template <int N>
-NECG_HD void finish_one(const double *sums, int K, const double *brak, const Consts<N> &cs, int folded, int k,
-                        double (&o)[Part<N>::size]) {
+NECG_HD void finish_one(const double *sums, int K, const double *brak, const Consts<N> &cs, int folded, double E2,
+                        int k, double (&o)[Part<N>::size]) {
     using BL = BraLayout<N>;
-    constexpr int PS = Part<N>::size;
+    constexpr int PS = Part<N>::size, PB = SumFields<N>::size;
     const size_t KK = (size_t)K;
-    double r[PS];
+    const auto sum = [&](int set, int f) { return sums[(set * PB + f) * KK + k]; };
+    double r[PS], kt[PS];
 #pragma unroll
-    for (int f = 0; f < PS; ++f) r[f] = sums[f * KK + k];
-    const auto sr = [&](int f) { return sums[(PS + f) * KK + k]; };
+    for (int f = 0; f < PS; ++f) {
+        r[f] = sum(0, f);
+        kt[f] = sum(2, f);
+        if (E2 != 0.0) {
+            r[f] -= E2 * sum(1, f);
+            kt[f] -= E2 * sum(3, f);
+        }
+        if (!folded) r[f] += kt[f];
+    }
+    const auto sr = [&](int f) { return sum(1, f); };
     const auto A = [&](int t) { return brak[(BL::A + t) * 32]; };
     const auto s = [&](int t) { return brak[(BL::S + t) * 32]; };
     const auto e = [&](int t) { return brak[(BL::AS + t) * 32]; };
@@ -496,7 +533,7 @@ NECG_HD void finish_one(const double *sums, int K, const double *brak, const Con
     fold_raw<N>(FieldsOf<double>{r}, A, s, e, o);
     if (folded)
 #pragma unroll
-        for (int f = 0; f < PS; ++f) o[f] += sums[(2 * PS + f) * KK + k];
+        for (int f = 0; f < PS; ++f) o[f] += kt[f];
 }
 
 // Lane ranges of the two tile kinds (used by the kernels and the emulator).

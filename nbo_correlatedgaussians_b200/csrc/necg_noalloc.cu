@@ -138,7 +138,6 @@ extern "C" int necg_outprod_noalloc(int n, int nst, int K, double efs, const dou
         cudaMemcpyAsync(base + c.sms, sms_host, sizeof(double) * nst * 9 * n * n, cudaMemcpyHostToDevice, st) ||
         cudaMemcpyAsync(base + c.scvv, scvv_host, sizeof(double) * nst, cudaMemcpyHostToDevice, st))
         return NECG_ERR_CUDA;
-    necg::launch_reset_status(status, st);
     const int nkb = (K + 31) / 32;
     noalloc_tiles_kernel<<<(nkb + 127) / 128, 128, 0, st>>>(tiles, K, kLcEnergy);
 
@@ -172,6 +171,7 @@ extern "C" int necg_outprod_noalloc(int n, int nst, int K, double efs, const dou
     a.g = g_dev;
     a.status = status;
     a.lam = 1.0;
+    a.sms_general = 1;
     if (necg::launch_prep(a, st) || necg::launch_energy(a, st)) return NECG_ERR_UNSUPPORTED;
     necg::launch_rows_finalize(a, f_dev, g_dev + siv, 0, 0.0, 0.0, st);
     if (necg::launch_grad(a, st)) return NECG_ERR_UNSUPPORTED;
