@@ -88,9 +88,9 @@ int necg_set_variant(necg_handle *h, int minw_energy, int minw_grad);
  * 12 or 16 warps per SM, and for mode 2 also 108 and 112 (8 and 12 warps with
  * the ket records re-read at each use instead of held in registers), 118 and
  * 122 (the same with each warp's ket record staged in shared memory), and
- * 248 and 232 (blocks of 8 and 12 warps, one block per SM, with bra and ket
- * records in shared memory; 232 is NECG_ERR_UNSUPPORTED where its shared memory
- * does not fit, n = 5).  208, 218, 228, 258 and 268 are accepted and run as 248,
+ * 248, 232 and 216 (blocks of 8, 12 and 16 warps, one block per SM, with bra and
+ * ket records in shared memory; NECG_ERR_UNSUPPORTED where that does not fit:
+ * 232 for n = 5, 216 for n > 3).  208, 218, 228, 258 and 268 are accepted and run as 248,
  * 222 as 232.  Set by the autotuner. */
 int necg_set_symmetric(necg_handle *h, int mode, int lc, int minw);
 

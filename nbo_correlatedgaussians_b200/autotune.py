@@ -42,12 +42,12 @@ MINB = (8, 12, 16, 20)
 MINB_GRAD_EXTRA = (112, 116)  # gradient kernel with shared-memory accumulators
 LC_S = (1, 2, 4, 8, 16)       # kets per tile of the symmetric gradient pass
 MINW_SYM = (8, 12)
-MINW_FUSED = (8, 12, 16, 108, 112, 118, 122, 248, 232)
+MINW_FUSED = (8, 12, 16, 108, 112, 118, 122, 248, 232, 216)
 SPLITS = (1, 2, 3, 4, 6, 8, 12, 24)
 SPLIT_TILES = 2048  # try splits below this many fused tiles
 # 100 + w: ket records re-read at each use (118 / 122: staged in shared memory,
-# 8 / 12 warps); 248 / 232: blocks of 8 / 12 warps with bras and ket records in
-# shared memory (the library also takes the codes 208 .. 268 of earlier block
+# 8 / 12 warps); 248 / 232 / 216: blocks of 8 / 12 / 16 warps with bras and ket
+# records in shared memory (the library also takes the codes 208 .. 268 of earlier block
 # variants and runs the one with the same number of warps); a variant whose
 # shared memory does not fit for n is refused by necg_set_symmetric and skipped
 

@@ -11,9 +11,9 @@
 //                and gradient partials of H and S in one pass over unordered pairs
 //   fsum         blocks over all (instance, 32-row block, field): per-basis sums
 //   finalize     block per instance: E, norm, GRADC from the row sums
-//   reduce       grid-stride over all (instance, k): GRADA blocks
+//   finish       blocks over all (instance, 32-row block): GRADA
 // Ordered mode (any other set): energy tiles over the triangle, rows (H C, S C),
-// finalize, gradient tiles over ordered pairs and a plain partial sum.
+// finalize, gradient tiles over ordered pairs, a plain partial sum and GRADA.
 // The plan (instance table, prefix sums, tile queues ordered by decreasing
 // cost) is built on the host and copied to device buffers before the step.
 #include <cuda_runtime.h>
@@ -69,6 +69,7 @@ struct PlanPtrs {
     int *pref_bra;  // cumulative K            (ninst + 1)
     int *pref_ket;  // cumulative K * nst      (ninst + 1)
     int *pref_sum;  // cumulative PS * K, or, fused, 32-row blocks times fields (ninst + 1)
+    int *pref_kb;   // cumulative 32-row blocks (ninst + 1)
     int *pref_ft;   // cumulative fused tile groups, or tiles when fine (ninst + 1), over `order`
     int *order;     // instances by decreasing tile cost (fused queue order)
     int4 *etiles;   // (inst, kb, lc, 0); fused mode: (inst, kb, lc, tile index in the instance)
@@ -419,8 +420,7 @@ __global__ void __launch_bounds__(256) batch_sum_kernel(PlanPtrs p) {
     }
 }
 
-// GRADA of every instance: from its per-basis sums (FUSED) or from its gradient fields.
-template <bool FUSED> __global__ void __launch_bounds__(128) batch_reduce_kernel(PlanPtrs p) {
+__global__ void __launch_bounds__(128) batch_reduce_kernel(PlanPtrs p) {
     const int ninst = p.hdr->ninst;
     const int total = p.pref_bra[ninst];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -429,15 +429,23 @@ template <bool FUSED> __global__ void __launch_bounds__(128) batch_reduce_kernel
         const int k = i - p.pref_bra[q];
         const double sc = d.scal[1] * d.C[k];
         bool fin = true;
-        if (FUSED) {
-            BATCH_SWITCH(d.n, {
-                double o[Part<N>::size];
-                finish_one<N>(d.part, d.K, bra_at<N>(d.bra, k), consts_of<N>(d), d.kmap.fold, 2.0 * d.scal[0], k, o);
-                fin = fields_to_grad<N>(o, bra_at<N>(d.bra, k), 32, sc, d.g, k);
-            });
-        } else {
-            BATCH_SWITCH(d.n, fin = grad_reduce_at<N>(d.part, 1, d.K, bra_at<N>(d.bra, k), 32, sc, d.g, k));
-        }
+        BATCH_SWITCH(d.n, fin = grad_reduce_at<N>(d.part, 1, d.K, bra_at<N>(d.bra, k), 32, sc, d.g, k));
+        if (!fin) atomicOr(d.status, 2);
+    }
+}
+
+// GRADA of every instance of a fused step from its per-basis sums: one block of 256
+// threads per (instance, 32-row block) at a time (finish_block).
+__global__ void __launch_bounds__(256) batch_finish_kernel(PlanPtrs p) {
+    extern __shared__ __align__(16) double smem[];
+    const int ninst = p.hdr->ninst;
+    const int total = p.pref_kb[ninst];
+    for (int i = blockIdx.x; i < total; i += gridDim.x) {
+        const int q = find_inst(p.pref_kb, ninst, i);
+        const InstDesc &d = p.inst[q];
+        bool fin = true;
+        BATCH_SWITCH(d.n, fin = finish_block<N>(d.part, d.K, d.bra, d.C, consts_of<N>(d), d.kmap.fold,
+                                                2.0 * d.scal[0], d.scal[1], i - p.pref_kb[q], nullptr, d.g, smem));
         if (!fin) atomicOr(d.status, 2);
     }
 }
@@ -501,6 +509,8 @@ void layout(necg_batch *b, char *base, PlanPtrs &p, size_t *total) {
     off = align_up(off + sizeof(int) * (b->cap_inst + 1), 256);
     p.pref_sum = (int *)(base + off);
     off = align_up(off + sizeof(int) * (b->cap_inst + 1), 256);
+    p.pref_kb = (int *)(base + off);
+    off = align_up(off + sizeof(int) * (b->cap_inst + 1), 256);
     p.pref_ft = (int *)(base + off);
     off = align_up(off + sizeof(int) * (b->cap_inst + 1), 256);
     p.order = (int *)(base + off);
@@ -528,14 +538,14 @@ void launch_step(necg_batch *b, cudaStream_t st, int mode) {
         }
         batch_fsum_kernel<<<g * 8, 256, 0, st>>>(p);
         batch_ffinalize_kernel<<<g, 256, 0, st>>>(p);
-        batch_reduce_kernel<true><<<g * 2, 128, 0, st>>>(p);
+        batch_finish_kernel<<<g * 3, 256, FinishSmem<kMaxN>::size * 8, st>>>(p);
     } else {
         batch_energy_kernel<<<g * b->occ_energy, 32, 0, st>>>(p);
         batch_rows_kernel<<<g * 4, 256, 0, st>>>(p);
         batch_finalize_kernel<<<g, 256, 0, st>>>(p);
         batch_grad_kernel<<<g * b->occ_grad, 32, 0, st>>>(p);
         batch_sum_kernel<<<g * 4, 256, 0, st>>>(p);
-        batch_reduce_kernel<false><<<g * 2, 128, 0, st>>>(p);
+        batch_reduce_kernel<<<g * 2, 128, 0, st>>>(p);
     }
     batch_status_kernel<<<1, 256, 0, st>>>(p);
 }
@@ -634,7 +644,7 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
         for (int n = 1; n <= kMaxN; ++n) v[n] = necg_term_flops(n, 7, nullptr);
         return v;
     }();
-    hp.pref_bra[0] = hp.pref_ket[0] = hp.pref_sum[0] = 0;
+    hp.pref_bra[0] = hp.pref_ket[0] = hp.pref_sum[0] = hp.pref_kb[0] = 0;
     bool fused = count > 0;
     for (int q = 0; q < count; ++q) {
         if (!hs[q] || !hs[q]->sym_ok || hs[q]->n > kMaxN) fused = false;
@@ -690,6 +700,7 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
         hp.pref_bra[q + 1] = hp.pref_bra[q] + K;
         hp.pref_ket[q + 1] = hp.pref_ket[q] + K * h->nst;
         const int nkb = (K + 31) / 32;
+        hp.pref_kb[q + 1] = hp.pref_kb[q] + nkb;
         hp.pref_sum[q + 1] = hp.pref_sum[q] + (fused ? (ps + 1) * nkb : ps * K);
         if (fused) {  // tiles come from the instance's device list; only its cost is needed here
             fcost[q] = (double)flops_fused[n] * h->nst * d.lc_s;

@@ -501,6 +501,176 @@ __device__ __forceinline__ void energy_from_rows(const double *__restrict__ sums
     __syncthreads();
 }
 
+// Shared memory of finish_block (doubles).
+template <int N> struct FinishSmem {
+    static constexpr int PS = Part<N>::size, blk = tri(N) + 3 * N;
+    static constexpr int r = 0;                    // combined raw sums, then the gradient fields
+    static constexpr int s = r + PS * 32;          // the bra's S sums, then the output
+    static constexpr int out = s;                  // blk x 32, basis-major with an odd stride (<= PS)
+    static constexpr int rec = s + PS * 32;        // A, S, AS and L of the 32 bases
+    static constexpr int y = rec + (tri(N) + 6 * N + tri(N)) * 32;
+    static constexpr int p = y + 3 * N * 32;
+    static constexpr int MA = p + 3 * N * 32;
+    static constexpr int size = MA + N * N * 32;
+    static_assert((blk | 1) <= PS, "the output fits where the S sums were");
+    // more than 48 KB would need the opt-in and another split of the SM's L1 (n = 5
+    // took 61 KB with areas of their own: 10 us more per evaluation at any K)
+    static_assert(N > 5 || size * 8 <= 48 * 1024, "shared memory");
+};
+
+// The gradients of the 32 bases of row block kb from their per-basis sums, by one
+// block of 256 threads: every step is split over the warps by matrix row, lane =
+// basis, so that the loads of all fields are in flight at once and no thread
+// walks the whole chain (one thread per basis took 11 us at n = 5 for any K).  E2 =
+// 2 E, or 0 where the sums are combined already (no S set of the ket then).  The
+// bra's explicit share of tau (explicit_tau), the fold (fold_raw) and the map to
+// vech(L) (a_to_vech) as there, row by row.  GRADA (scaled by norm C_k) goes to g,
+// or the gradient fields, field-major, to `fields`.  Returns whether this
+// thread's outputs are finite.
+template <int N>
+__device__ __forceinline__ bool finish_block(const double *__restrict__ sums, int K, const double *__restrict__ bra,
+                                             const double *__restrict__ C, const Consts<N> &cs, int folded, double E2,
+                                             double norm, int kb, double *__restrict__ fields,
+                                             double *__restrict__ g, double *sm) {
+    using BL = BraLayout<N>;
+    using FS = FinishSmem<N>;
+    constexpr int TR = tri(N), PS = Part<N>::size, PB = SumFields<N>::size, blk = FS::blk;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k = min(kb * 32 + lane, K - 1);
+    const int nk = min(32, K - kb * 32);
+    constexpr int A = FS::rec, S = A + TR * 32, AS = S + 3 * N * 32, L = AS + 3 * N * 32;
+    const double *bk = bra_at<N>(bra, kb * 32) + min(lane, nk - 1);
+    auto ket = [&](int f) {  // the kets' combined sum (folded: their gradient)
+        const double *q = sums + (size_t)(2 * PB + f) * K + k;
+        return E2 != 0.0 ? q[0] - E2 * q[(size_t)PB * K] : q[0];
+    };
+#pragma unroll
+    for (int f = w; f < PS; f += 8) {
+        const double *q = sums + (size_t)f * K + k;
+        const size_t set = (size_t)PB * K;
+        double r = q[0];
+        const double bs = q[set];
+        if (E2 != 0.0) r -= E2 * bs;
+        sm[FS::r + f * 32 + lane] = folded ? r : r + ket(f);
+        sm[FS::s + f * 32 + lane] = bs;
+    }
+#pragma unroll
+    for (int f = w; f < TR + 6 * N; f += 8) {  // A, S, AS are fields 0 .. of the record
+        static_assert(BL::A == 0 && BL::S == TR && BL::AS == TR + 3 * N, "record order");
+        sm[A + f * 32 + lane] = bk[f * 32];
+    }
+#pragma unroll
+    for (int f = w; f < TR; f += 8) sm[L + f * 32 + lane] = bk[(BL::L + f) * 32];
+    __syncthreads();
+    auto at = [&](int base, int f) -> double & { return sm[base + f * 32 + lane]; };
+    const int i = w;  // this warp's matrix row
+    if (i < N) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double v = at(AS, 3 * i + c) * at(FS::s, TR), p = 0.0;
+#pragma unroll
+            for (int q = 0; q < N; ++q) {
+                v -= at(A, sx(i, q)) * at(FS::s, TR + 1 + 3 * q + c);
+                p += cs.M[i * N + q] * at(AS, 3 * q + c);
+            }
+            at(FS::y, 3 * i + c) = v;
+            at(FS::p, 3 * i + c) = p;
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            double v = 0.0;
+#pragma unroll
+            for (int q = 0; q < N; ++q) v += cs.M[i * N + q] * at(A, sx(q, j));
+            at(FS::MA, i * N + j) = v;
+        }
+    }
+    __syncthreads();
+    if (i < N) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double v = 0.0;
+#pragma unroll
+            for (int q = 0; q < N; ++q) v += cs.M[i * N + q] * at(FS::y, 3 * q + c);
+            at(FS::r, TR + 1 + 3 * i + c) -= 8.0 * v;
+        }
+        for (int j = 0; j <= i; ++j) {
+            double v = 3.0 * cs.M[i * N + j] * at(FS::s, TR);
+#pragma unroll
+            for (int q = 0; q < N; ++q)
+                v += 2.0 * (at(FS::MA, i * N + q) * at(FS::s, sx(q, j)) + at(FS::s, sx(i, q)) * at(FS::MA, j * N + q));
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                v += 2.0 * (at(FS::s, TR + 1 + 3 * i + c) * at(FS::p, 3 * j + c) +
+                            at(FS::p, 3 * i + c) * at(FS::s, TR + 1 + 3 * j + c));
+            at(FS::r, sx(i, j)) += 4.0 * v;
+        }
+    }
+    __syncthreads();
+    // the fold: matrix row i (in place: entry (i, j) reads only itself) and dF/ds row i
+    const double F = 0.5 * at(FS::r, TR);
+    double gs[3];
+    if (i < N) {
+        for (int j = 0; j <= i; ++j) {
+            double v = 0.0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double si = at(S, 3 * i + c), sj = at(S, 3 * j + c);
+                v += at(FS::r, TR + 1 + 3 * i + c) * sj + si * at(FS::r, TR + 1 + 3 * j + c) - 2.0 * F * si * sj;
+            }
+            v = 0.5 * (at(FS::r, sx(i, j)) + v);
+            at(FS::r, sx(i, j)) = folded ? v + ket(sx(i, j)) : v;
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double v = -2.0 * F * at(AS, 3 * i + c);
+#pragma unroll
+            for (int q = 0; q < N; ++q) v += at(A, sx(i, q)) * at(FS::r, TR + 1 + 3 * q + c);
+            gs[c] = folded ? v + ket(TR + 1 + 3 * i + c) : v;
+        }
+    }
+    const double D = folded ? 0.75 * F + ket(TR) : 0.75 * F;
+    __syncthreads();
+    bool fin = true;
+    if (fields) {
+        if (i < N) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) at(FS::r, TR + 1 + 3 * i + c) = gs[c];
+        }
+        if (w == 0) at(FS::r, TR) = D;
+        __syncthreads();
+        if (lane < nk)
+            for (int f = w; f < PS; f += 8) fields[(size_t)f * K + k] = at(FS::r, f);
+    } else {
+        const double sc = norm * C[k];
+        double *o = sm + FS::out + lane * (blk | 1);
+        if (i < N) {  // column i of vech(dF/dL): rows a = i .. N - 1
+            const int j = i;
+            int idx = j * N - j * (j - 1) / 2;
+            for (int a = j; a < N; ++a) {
+                double v = 0.0;
+                for (int q = j; q < N; ++q) v += at(FS::r, sx(a, q)) * at(L, sx(q, j));
+                v *= 2.0;
+                if (a == j) v += 2.0 * D / at(L, sx(j, j));
+                v *= sc;
+                fin = fin && isfinite(v);
+                o[idx++] = v;
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double v = sc * gs[c];
+                fin = fin && isfinite(v);
+                o[TR + 3 * i + c] = v;
+            }
+        }
+        __syncthreads();
+        // the 32 blocks of g are contiguous
+        for (int q = threadIdx.x; q < nk * blk; q += 256)
+            g[(size_t)kb * 32 * blk + q] = sm[FS::out + (q / blk) * (blk | 1) + q % blk];
+    }
+    __syncthreads();
+    return fin || lane >= nk;
+}
+
 // GRADC of basis i: 2 norm (H C - E S C)_i (python/make_grad.py:85).
 template <int N>
 __device__ __forceinline__ double gradc_from_rows(const double *__restrict__ sums, int K, int i, const double *en) {

@@ -130,7 +130,9 @@ __global__ void __launch_bounds__(32 * W) energy_split_kernel(const int2 *__rest
     flag_status(status, flags, pair);
 }
 
-// rows[i] = (H C)_i, rows[K + i] = (S C)_i ; one warp per row
+// rows[i] = (H C)_i, rows[K + i] = (S C)_i ; one warp per row.  Memory bound (16
+// K^2 bytes); eight loads of each matrix in flight per lane (K = 2048 on a B200:
+// 26 us with one, 22 us with eight).
 __global__ void __launch_bounds__(256) rows_kernel(const double *__restrict__ H,
                                                    const double *__restrict__ S,
                                                    const double *__restrict__ C, int K,
@@ -141,7 +143,22 @@ __global__ void __launch_bounds__(256) rows_kernel(const double *__restrict__ H,
     const double *h = H + (size_t)warp * K;
     const double *s = S + (size_t)warp * K;
     double ah = 0.0, as = 0.0;
-    for (int j = lane; j < K; j += 32) {
+    int j = lane;
+    for (; j + 7 * 32 < K; j += 8 * 32) {
+        double a[8], b[8], c[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            a[q] = h[j + 32 * q];
+            b[q] = s[j + 32 * q];
+            c[q] = C[j + 32 * q];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            ah += a[q] * c[q];
+            as += b[q] * c[q];
+        }
+    }
+    for (; j < K; j += 32) {
         const double c = C[j];
         ah += h[j] * c;
         as += s[j] * c;
@@ -314,7 +331,7 @@ __global__ void __launch_bounds__(256) hs_reduce_kernel(const double *__restrict
     }
 }
 
-// The fused pass with W-warp blocks (W = 8 or 12), one per SM, persistent over
+// The fused pass with W-warp blocks (W = 8, 12 or 16), one per SM, persistent over
 // a queue of tile groups: group g = row block kb and ket chunks lc0 .. lc0 + W
 // - 1, one per warp.  The group's bras are staged in shared memory once for all
 // warps, each warp stages its ket records in two buffers (the next term's copied
@@ -443,23 +460,20 @@ __global__ void __launch_bounds__(128) rows_from_sums_kernel(const double *__res
     rows[i] = sums[(size_t)(which * PB + R) * K + m] + sums[(size_t)((2 + which) * PB + R) * K + m];
 }
 
-// From the per-basis sums to the gradient, 32 bases per block.  OWN_E: every block
-// forms E and norm from the row sums (the same order in each, 5 K reads that cost
-// less than a kernel of their own), block 0 writes them and f, and GRADC of the
-// block's bases goes to gradc; else E and norm are scal's (KE: the sums are
-// combined already).  Then the gradient of basis k (finish_one): written
-// field-major to `fields` (a shard's share, all-reduced before GRADA) or mapped to
-// vech(L), scaled by norm C_k and written to GRADA block k.
+// From the per-basis sums to the gradient, 32 bases per block (finish_block).
+// OWN_E: every block forms E and norm from the row sums (the same order in each,
+// 5 K reads that cost less than a kernel of their own), block 0 writes them and f,
+// and GRADC of the block's bases goes to gradc; else E and norm are scal's (KE:
+// the sums are combined already).
 template <int N, bool KE, bool OWN_E>
-__global__ void __launch_bounds__(128) fsym_finish_kernel(const double *__restrict__ sums, int K, Consts<N> cs,
+__global__ void __launch_bounds__(256) fsym_finish_kernel(const double *__restrict__ sums, int K, Consts<N> cs,
                                                           const double *__restrict__ bra,
                                                           const double *__restrict__ C, double *__restrict__ scal,
                                                           int folded, double *__restrict__ fields,
                                                           double *__restrict__ g, double *__restrict__ gradc,
                                                           double *__restrict__ f_out, int *status) {
-    constexpr int PS = Part<N>::size;
+    extern __shared__ __align__(16) double smem[];
     __shared__ double sh[2][32], en[4];
-    const int k = blockIdx.x * 32 + threadIdx.x;
     if (OWN_E) {
         energy_from_rows<N>(sums, C, K, sh, en);
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -468,19 +482,12 @@ __global__ void __launch_bounds__(128) fsym_finish_kernel(const double *__restri
             if (f_out) *f_out = en[0];
             if (!isfinite(en[0])) atomicOr(status, 2);
         }
+        const int k = blockIdx.x * 32 + threadIdx.x;
+        if (threadIdx.x < 32 && k < K) gradc[k] = gradc_from_rows<N>(sums, K, k, en);
     }
-    if (threadIdx.x >= 32 || k >= K) return;
     const double E = OWN_E ? en[0] : scal[0], norm = OWN_E ? en[1] : scal[1];
-    if (OWN_E) gradc[k] = gradc_from_rows<N>(sums, K, k, en);
-    double o[PS];
-    const double *brak = bra_at<N>(bra, k);
-    finish_one<N>(sums, K, brak, cs, folded, KE ? 0.0 : 2.0 * E, k, o);
-    if (fields) {
-#pragma unroll
-        for (int f = 0; f < PS; ++f) fields[(size_t)f * K + k] = o[f];
-        return;
-    }
-    if (!fields_to_grad<N>(o, brak, 32, norm * C[k], g, k)) atomicOr(status, 2);
+    if (!finish_block<N>(sums, K, bra, C, cs, folded, KE ? 0.0 : 2.0 * E, norm, blockIdx.x, fields, g, smem))
+        atomicOr(status, 2);
 }
 
 // Sum the gradient-tile partials over the ket chunks, in place into chunk 0:
@@ -660,27 +667,26 @@ __global__ void __launch_bounds__(32) dipole_group_kernel(const int2 *__restrict
 // comps[m] = num[m] / den (0 when den = 0, as python/necg.py:228) and the
 // dipole d_c = sum_i ncv[i + 1] comps[3 i + c].
 template <int N>
-__global__ void __launch_bounds__(256) dipole_sum_kernel(const double *__restrict__ part, int ntiles,
-                                                         Consts<N> cs, double *__restrict__ comps,
-                                                         double *__restrict__ dip) {
+__global__ void __launch_bounds__(1024) dipole_sum_kernel(const double *__restrict__ part, int nslots, Consts<N> cs,
+                                                          double *__restrict__ comps, double *__restrict__ dip) {
     constexpr int NM = 3 * N + 1;
-    __shared__ double red[NM][256];
+    constexpr int F = NM <= 16 ? 16 : 32, ROWS = 1024 / F;  // F fields side by side, every ROWS-th slot per thread
+    __shared__ double red[ROWS][F + 1];
     __shared__ double tot[NM];
-    const int j = threadIdx.x;
-#pragma unroll
-    for (int m = 0; m < NM; ++m) {
-        double s = 0.0;
-        for (int t = j; t < ntiles; t += 256) s += part[(size_t)t * NM + m];
-        red[m][j] = s;
+    const int m = threadIdx.x % F, r = threadIdx.x / F;
+    double s = 0.0;
+    if (m < NM) {
+#pragma unroll 8
+        for (int t = r; t < nslots; t += ROWS) s += part[(size_t)t * NM + m];
     }
+    red[r][m] = s;
     __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (j < w)
-#pragma unroll
-            for (int m = 0; m < NM; ++m) red[m][j] += red[m][j + w];
+    for (int w = ROWS / 2; w > 0; w >>= 1) {
+        if (r < w) red[r][m] += red[r + w][m];
         __syncthreads();
     }
-    if (j < NM) tot[j] = red[j][0];
+    const int j = threadIdx.x;
+    if (j < NM) tot[j] = red[0][j];
     __syncthreads();
     if (j < 3 * N) comps[j] = tot[0] != 0.0 ? tot[1 + j] / tot[0] : 0.0;
     __syncthreads();
@@ -880,9 +886,10 @@ template <int N> struct Launch {
     template <bool KE, bool OWN_E>
     static void finish(const LaunchArgs &a, double *f_out, double *gradc, cudaStream_t st) {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
-        fsym_finish_kernel<N, KE, OWN_E><<<(a.K + 31) / 32, 128, 0, st>>>(a.part, a.K, cs, a.bra, a.C, a.scal,
-                                                                         a.kmap.fold, a.sums, a.g, gradc, f_out,
-                                                                         a.status);
+        constexpr int smem = FinishSmem<N>::size * 8;
+        fsym_finish_kernel<N, KE, OWN_E><<<(a.K + 31) / 32, 256, smem, st>>>(a.part, a.K, cs, a.bra, a.C, a.scal,
+                                                                            a.kmap.fold, a.sums, a.g, gradc, f_out,
+                                                                            a.status);
     }
     template <int MINW, bool VKET, bool SKET = false> static void fsym_v(const LaunchArgs &a, cudaStream_t st) {
         if constexpr (Part<N>::size <= 32) {
@@ -923,7 +930,9 @@ template <int N> struct Launch {
     }
     static void fsym_tiles(const LaunchArgs &a, cudaStream_t st) {
         if (a.minb_s >= 200 && a.st_end == 0 && a.sgroups && a.qcount) {
-            if (fused_block_warps(a.minb_s) == 12) fsym_block<12>(a, st);  // 2xy: block variants
+            const int w = fused_block_warps(a.minb_s);  // 2xy: block variants
+            if (w == 16) fsym_block<16>(a, st);
+            else if (w == 12) fsym_block<12>(a, st);
             else fsym_block<8>(a, st);
             return;
         }
@@ -988,7 +997,7 @@ template <int N> struct Launch {
             dipole_kernel<N><<<a.ntiles, 32, 0, st>>>(a.tiles, a.ntiles, a.LC_e, a.K, a.nst, cs, a.ket, a.C, part,
                                                       a.status);
         }
-        dipole_sum_kernel<N><<<1, 256, 0, st>>>(part, slots, cs, comps, dip);
+        dipole_sum_kernel<N><<<1, 1024, 0, st>>>(part, slots, cs, comps, dip);
     }
     static void reduce_sums(const LaunchArgs &a, const double *sums, cudaStream_t st) {
         grad_reduce_kernel<N><<<(a.K + 127) / 128, 128, 0, st>>>(sums, a.K, a.bra, a.C, a.scal, a.g, a.status);
@@ -1048,7 +1057,7 @@ int launch_gsym_reduce(const LaunchArgs &a, cudaStream_t st) {
     NECG_DISPATCH(a.n, gsym_reduce(a, st));
     return 0;
 }
-int fused_block_warps(int variant) { return variant == 222 || variant == 232 ? 12 : 8; }
+int fused_block_warps(int variant) { return variant == 216 ? 16 : variant == 222 || variant == 232 ? 12 : 8; }
 bool fused_variant_ok(int n, int variant) {
     if (variant < 200) return true;
     if (n < 1 || n > 5) return false;

@@ -349,24 +349,8 @@ NECG_HD bool a_to_vech(const double (&G)[tri(N)], double D, const double (&gS)[3
     return fin;
 }
 
-// The GRADA block of basis k (scaled by sc) from its gradient fields; brak:
+// Sum the nlc partials of basis k and write its GRADA block scaled by sc; brak:
 // field f of its bra record at brak[f * stride].
-template <int N>
-NECG_HD bool fields_to_grad(const double (&o)[Part<N>::size], const double *brak, size_t stride, double sc, double *g,
-                            int k) {
-    using BL = BraLayout<N>;
-    constexpr int blk = tri(N) + 3 * N;
-    double G[tri(N)], gS[3 * N], L[tri(N)];
-#pragma unroll
-    for (int t = 0; t < tri(N); ++t) G[t] = o[t];
-#pragma unroll
-    for (int t = 0; t < 3 * N; ++t) gS[t] = o[tri(N) + 1 + t];
-#pragma unroll
-    for (int t = 0; t < tri(N); ++t) L[t] = brak[(BL::L + t) * stride];
-    return a_to_vech<N>(G, o[tri(N)], gS, L, sc, g + (size_t)k * blk);
-}
-
-// Sum the nlc partials of basis k and write its GRADA block scaled by sc.
 template <int N>
 NECG_HD bool grad_reduce_at(const double *part, int nlc, int K, const double *brak, size_t stride, double sc, double *g,
                             int k) {
@@ -379,7 +363,14 @@ NECG_HD bool grad_reduce_at(const double *part, int nlc, int K, const double *br
 #pragma unroll
         for (int f = 0; f < PS; ++f) o[f] += p[(size_t)f * K];
     }
-    return fields_to_grad<N>(o, brak, stride, sc, g, k);
+    double G[tri(N)], gS[3 * N], L[tri(N)];
+#pragma unroll
+    for (int t = 0; t < tri(N); ++t) G[t] = o[t];
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) gS[t] = o[tri(N) + 1 + t];
+#pragma unroll
+    for (int t = 0; t < tri(N); ++t) L[t] = brak[(BraLayout<N>::L + t) * stride];
+    return a_to_vech<N>(G, o[tri(N)], gS, L, sc, g + (size_t)k * (tri(N) + 3 * N));
 }
 template <int N>
 NECG_HD bool grad_reduce_one(const double *part, int nlc, int K, const double *bra, double sc, double *g, int k) {
@@ -503,38 +494,6 @@ template <int N> struct SumFields {
 // set i of basis k at (i SumFields::size + f) K + k: the bra's H (or, with E
 // known, combined) and S sums, then the ket's.
 constexpr int kSumSets = 4;
-
-// The gradient fields (Part<N>) of basis k from its sums (brak = bra_at(bra, k)),
-// for the gradient of h - E ov; E2 = 2 E, or 0 where the sums are combined already
-// (then there is no S set of the ket).
-template <int N>
-NECG_HD void finish_one(const double *sums, int K, const double *brak, const Consts<N> &cs, int folded, double E2,
-                        int k, double (&o)[Part<N>::size]) {
-    using BL = BraLayout<N>;
-    constexpr int PS = Part<N>::size, PB = SumFields<N>::size;
-    const size_t KK = (size_t)K;
-    const auto sum = [&](int set, int f) { return sums[(set * PB + f) * KK + k]; };
-    double r[PS], kt[PS];
-#pragma unroll
-    for (int f = 0; f < PS; ++f) {
-        r[f] = sum(0, f);
-        kt[f] = sum(2, f);
-        if (E2 != 0.0) {
-            r[f] -= E2 * sum(1, f);
-            kt[f] -= E2 * sum(3, f);
-        }
-        if (!folded) r[f] += kt[f];
-    }
-    const auto sr = [&](int f) { return sum(1, f); };
-    const auto A = [&](int t) { return brak[(BL::A + t) * 32]; };
-    const auto s = [&](int t) { return brak[(BL::S + t) * 32]; };
-    const auto e = [&](int t) { return brak[(BL::AS + t) * 32]; };
-    explicit_tau<N>(sr, A, e, cs, r);
-    fold_raw<N>(FieldsOf<double>{r}, A, s, e, o);
-    if (folded)
-#pragma unroll
-        for (int f = 0; f < PS; ++f) o[f] += kt[f];
-}
 
 // Lane ranges of the two tile kinds (used by the kernels and the emulator).
 // Energy: tile (kb, lc) -> bra k = 32 kb + lane, kets [l0, lend); false if idle.

@@ -15,6 +15,7 @@ from oracle.oracle import Oracle
 
 PASSES = [(0, 4, 8, 1), (1, 3, 8, 1), (1, 1, 12, 1), (2, 2, 118, 1), (2, 1, 122, 2), (2, 2, 12, 1), (2, 3, 228, 1),
           (2, 2, 248, 1), (2, 1, 268, 1)]
+BLOCKS16 = (2, 3, 216, 1)  # 16-warp blocks fit for n <= 3
 
 
 def make(n, K, seed, perms=None):
@@ -50,7 +51,7 @@ def test_every_particle_count(n, K):
     p = make(n, K, 100 * n + K)
     fo, go = Oracle.from_problem(p).outprod(p.x, nthreads=8)
     eng = engine(p)
-    for mode, lc, minw, npc in PASSES:
+    for mode, lc, minw, npc in PASSES + ([BLOCKS16] if n <= 3 else []):
         assert eng.L.necg_set_symmetric(eng.h, mode, lc, minw) == 0
         assert eng.L.necg_set_splits(eng.h, min(npc, p.nst)) == 0
         f, g = eng.outprod(p.x)
@@ -158,3 +159,32 @@ def test_dipole_classes(system, K, keep, shift):
         scale = max(np.max(np.abs(comps_o)), 1e-300)
         assert np.max(np.abs(comps - comps_o)) <= 1e-11 * scale
         assert np.max(np.abs(dip - dip_o)) <= 1e-11 * max(np.max(np.abs(dip_o)), scale)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,K,lc,minw,npc", [(5, 70, 1, 248, 1), (5, 200, 2, 248, 1), (3, 130, 2, 216, 1), (3, 130, 1, 232, 1),
+                                             (2, 90, 3, 118, 2), (4, 33, 2, 12, 1)])
+def test_matrices_and_row_sums_agree(n, K, lc, minw, npc):
+    """H and S written on request (block variants: with their queue's split tail;
+    split symmetry terms) against the oracle, and the same E and gradient, bit for
+    bit, whether they are asked for or not."""
+    import torch
+    from nbo_correlatedgaussians_b200 import _lib, synth
+    system = {2: "He", 3: "H2", 5: "LiH"}.get(n)
+    p = synth.make_problem(system, K, K) if system else make(n, K, K)
+    p.C = np.random.default_rng(K).normal(size=K)
+    fo, go, Ho, So = Oracle.from_problem(p).outprod(p.x, nthreads=8, return_hs=True)
+    eng = engine(p)
+    assert eng.L.necg_set_symmetric(eng.h, 2, lc, minw) == _lib.NECG_OK
+    assert eng.L.necg_set_splits(eng.h, min(npc, p.nst)) == _lib.NECG_OK
+    x = torch.from_numpy(p.x).to(eng.device)
+    H = torch.full((K, K), np.nan, dtype=torch.float64, device=eng.device)
+    S = torch.full_like(H, np.nan)
+    f, g = eng.outprod_device(x, K, H=H, S=S)
+    f2, g2 = eng.outprod_device(x, K)
+    torch.cuda.synchronize()
+    assert float(f) == float(f2) and torch.equal(g, g2)
+    assert abs(float(f) - fo) < TOL_E and normwise(g.cpu().numpy(), go) < TOL_G
+    for M, Mo in ((H, Ho), (S, So)):
+        M = M.cpu().numpy()
+        assert np.array_equal(M, M.T) and np.max(np.abs(M - Mo)) <= 1e-12 * max(1.0, np.max(np.abs(Mo)))
