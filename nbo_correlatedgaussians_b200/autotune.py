@@ -54,7 +54,7 @@ SPLIT_TILES = 2048  # try splits below this many fused tiles
 
 def fused_tiles(K: int, lc: int) -> int:
     """Tiles (32-row block, chunk of lc kets) over the lower triangle of K."""
-    return sum(min(kb * 32 + 31, K - 1) // lc + 1 for kb in range((K + 31) // 32))
+    return sum((K - 1 - 32 * b) // lc + 1 for b in range((K + 31) // 32))
 
 
 def _bucket(K: int) -> int:

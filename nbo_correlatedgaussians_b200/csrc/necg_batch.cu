@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128) batch_prep_kernel(PlanPtrs p) {
             const int q = find_inst(p.pref_bra, ninst, i);
             const InstDesc &d = p.inst[q];
             const int k = i - p.pref_bra[q];
-            BATCH_SWITCH(d.n, prep_bra_at<N>(d.iv + (size_t)k * (tri(N) + 3 * N), consts_of<N>(d), bra_at<N>(d.bra, k), 32));
+            BATCH_SWITCH(d.n, prep_bra_at<N>(d.iv + (size_t)k * (tri(N) + 3 * N), consts_of<N>(d), bra_at<N>(d.bra, d.K, k), 32));
         } else {
             const int j = i - nb;
             const int q = find_inst(p.pref_ket, ninst, j);
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(32) batch_energy_kernel(PlanPtrs p) {
         int k, l0, lend;
         if (energy_lane_range(e.y, e.z, lane, d.lc_e, d.K, k, l0, lend)) {
             int bad = 0, fl = 0;
-            BATCH_SWITCH(d.n, fl = (energy_lane<N, double>(BraRef{bra_at<N>(d.bra, k)}, DevKetB{d.ket}, k,
+            BATCH_SWITCH(d.n, fl = (energy_lane<N, double>(BraRef{bra_at<N>(d.bra, d.K, k)}, DevKetB{d.ket}, k,
                                                            l0, lend, d.K, d.nst, consts_of<N>(d), d.H,
                                                            d.S, nullptr, nullptr, bad)));
             flag_inst(d.status, fl, bad);
@@ -210,7 +210,6 @@ template <int N>
 __device__ __forceinline__ void batch_fused_group(const InstDesc &d, int g, double *smem) {
     constexpr int PB = SumFields<N>::size;
     constexpr int PER_WARP = bfused_warp_smem<N>();
-    constexpr int BS = BraLayout<N>::term;
     constexpr int TBL = ket_table<N>(2);
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
@@ -218,10 +217,8 @@ __device__ __forceinline__ void batch_fused_group(const InstDesc &d, int g, doub
     const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + 64};
     const int2 gr = d.bgroups[g];
     const int K = d.K, kb = gr.x, lc = gr.y + w;
-    const int last = min(kb * 32 + 31, K - 1);
-    const bool idle = lc * d.lc_s > last;
-    const double *bk = bra_at<N>(d.bra, kb * 32);
-    for (int i = threadIdx.x; i < BS * 32; i += 256) sbra[i] = bk[(i & ~31) + min(i & 31, K - 1 - kb * 32)];
+    const bool idle = lc * d.lc_s > row_last(K, kb);
+    stage_bras<N>(sbra, d.bra, K, kb, 256);
     __syncthreads();
     double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * 2 * PB * 32;
     fsym_tile<N, true, true, true, false>(d.stile_start[kb] + lc, make_int2(kb, lc), d.lc_s, K, d.nst,
@@ -231,7 +228,7 @@ __device__ __forceinline__ void batch_fused_group(const InstDesc &d, int g, doub
     // order and written once, to the group's slot
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * PB * 32; i += 256) {
-        if (kb * 32 + (i & 31) >= K) continue;
+        if (kb == 0 && (i & 31) < row_pad(K)) continue;  // no basis
         double v = smem[i];
 #pragma unroll
         for (int q = 1; q < 8; ++q) v += smem[q * PER_WARP + i];
@@ -397,7 +394,7 @@ __global__ void __launch_bounds__(32) batch_grad_kernel(PlanPtrs p) {
             bool ok = true;
             BATCH_SWITCH(d.n, {
                 SmemAcc<N> accH{sacc + lane}, accS{sacc + Part<N>::size * 32 + lane};
-                ok = grad_lane<N, double>(BraRef{bra_at<N>(d.bra, k)}, DevKetB{d.ket}, l0, l1, d.nst,
+                ok = grad_lane<N, double>(BraRef{bra_at<N>(d.bra, d.K, k)}, DevKetB{d.ket}, l0, l1, d.nst,
                                           consts_of<N>(d), 1.0, d.scal[0],
                                           d.part + (size_t)lc * Part<N>::size * d.K + k, (size_t)d.K, accH, accS);
             });
@@ -429,7 +426,7 @@ __global__ void __launch_bounds__(128) batch_reduce_kernel(PlanPtrs p) {
         const int k = i - p.pref_bra[q];
         const double sc = d.scal[1] * d.C[k];
         bool fin = true;
-        BATCH_SWITCH(d.n, fin = grad_reduce_at<N>(d.part, 1, d.K, bra_at<N>(d.bra, k), 32, sc, d.g, k));
+        BATCH_SWITCH(d.n, fin = grad_reduce_at<N>(d.part, 1, d.K, bra_at<N>(d.bra, d.K, k), 32, sc, d.g, k));
         if (!fin) atomicOr(d.status, 2);
     }
 }
@@ -708,7 +705,7 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
         }
         const long long fe = necg_term_flops(n, 4, nullptr), fg = necg_term_flops(n, 5, nullptr);
         for (int kb = 0; kb < nkb; ++kb)
-            for (int lc = 0; lc * d.lc_e <= kb * 32 + 31 && lc * d.lc_e < K; ++lc)
+            for (int lc = 0; lc * d.lc_e <= row_last(K, kb); ++lc)
                 et.push_back({(double)fe * h->nst * d.lc_e, make_int4(q, kb, lc, 0)});
         for (int lc = 0; lc < d.nlc; ++lc)
             for (int kb = 0; kb < nkb; ++kb)

@@ -145,14 +145,13 @@ void free_all(necg_handle *h) {
     for (void *p : ptrs) pool_free(h, p);
 }
 
-// Energy tiles over the lower triangle: (kb, lc) with lc * LC <= kb * 32 + 31.
+// Energy tiles over the lower triangle: (kb, lc) with lc * LC <= row_last(K, kb).
 int ensure_tiles(necg_handle *h, int K, cudaStream_t st) {
     if (h->tiles_K == K && h->tiles_lc == h->lc_e) return NECG_OK;
     std::vector<int2> t;
     const int nkb = (K + 31) / 32;
     for (int kb = 0; kb < nkb; ++kb) {
-        const int kmax = kb * 32 + 31;
-        for (int lc = 0; lc * h->lc_e <= kmax && lc * h->lc_e < K; ++lc) t.push_back(make_int2(kb, lc));
+        for (int lc = 0; lc * h->lc_e <= necg::row_last(K, kb); ++lc) t.push_back(make_int2(kb, lc));
     }
     if ((int)t.size() > h->tiles_cap) {
         pool_free(h, h->d_tiles, st);
@@ -197,8 +196,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
     const int nkb = (K + 31) / 32, LC = h->lc_s;
     for (int kb = 0; kb < nkb; ++kb) {
         start.push_back((int)t.size());
-        const int last = kb * 32 + 31 < K - 1 ? kb * 32 + 31 : K - 1;
-        for (int lc = 0; lc <= last / LC; ++lc) t.push_back(make_int2(kb, lc));
+        for (int lc = 0; lc <= necg::row_last(K, kb) / LC; ++lc) t.push_back(make_int2(kb, lc));
     }
     start.push_back((int)t.size());
     if ((int)t.size() > h->stiles_cap) {

@@ -23,6 +23,15 @@ template <int N> struct SmemAcc {
     __device__ __forceinline__ double &s(int t) { return p[(tri(N) + 1 + t) * 32]; }
 };
 
+// Stage the bra records' term fields of row block kb for BraSmem (by a block of
+// `threads` threads; the caller synchronises).
+template <int N>
+__device__ __forceinline__ void stage_bras(double *sbra, const double *__restrict__ bra, int K, int kb, int threads) {
+    const double *bk = bra + (size_t)kb * (BraLayout<N>::size * 32);
+    const int first = kb == 0 ? row_pad(K) : 0;
+    for (int i = threadIdx.x; i < BraLayout<N>::term * 32; i += threads) sbra[i] = bk[(i & ~31) + max(i & 31, first)];
+}
+
 // Copy a ket record of nd doubles (nd even: records are 16-byte multiples, at
 // 16-byte aligned addresses) from global to shared memory without waiting:
 // 16-byte cp.async per lane, one commit group per record.
@@ -190,7 +199,7 @@ __device__ __noinline__ double fold_slot(const double *slots, double scale, int 
 //        known until those rows are.
 //   KE, the symmetric gradient pass (E = Egiven known): the combined gradient
 //        of h - E ov, and the S fields for the bra only (its explicit share).
-// Tile t = (kb, lc): bras k = 32 kb + lane, kets l in [lc LC, lc LC + LC).  Bra
+// Tile t = (kb, lc): the bras of row block kb, kets l in [lc LC, lc LC + LC).  Bra
 // partials (PB = SumFields::size): part_b[((t * 2 + which) * PB + f) * 32 + lane];
 // ket partials: part_k[((t * LC + l - l0) * 2 + which) * PB + f], which = 0 for H
 // (or the combined gradient) and 1 for S (not written for the ket when KE).
@@ -198,13 +207,12 @@ __device__ __noinline__ double fold_slot(const double *slots, double scale, int 
 // Shared memory per warp must stay under 228 KB / 8 for 8 resident warps, so the
 // ket rows of two lanes are added before they are written (TileOutput) and the
 // table has 16 rows.  The shuffles need the whole warp, so every lane evaluates a
-// term: a lane without a pair (l > k, or k >= K) evaluates the finite pair
+// term: a lane without a pair (l > k, or no basis) evaluates the finite pair
 // (l, l, P) with zero weights, which adds nothing.
 // VKET: ket records re-read at each use (fewer live registers).
 // idle: the warp has no tile (its accumulators are set to zero all the same).
-// SBRA: the block's 32 bras of row block tl.x are staged in shared memory at
-// sbra (field f of lane j at sbra[f * 32 + j]; rows past K hold row K - 1) and
-// read there instead of from global memory.
+// SBRA: the 32 bras of row block tl.x are staged in shared memory at sbra (field f
+// of lane j at sbra[f * 32 + j]; lanes without a basis hold basis 0) and read there instead of from global memory.
 // SKET: each (l, P) ket record is copied by the warp into one of its two
 // buffers at sm.sket and read there; the copy of the next term's record
 // (cp.async) runs while the current term is evaluated.
@@ -231,10 +239,10 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
     static_assert(PS <= 32 && SL <= 32, "the symmetric passes need tri(n) + 1 + 3n <= 32");
     const int lane = threadIdx.x & 31;
     double *krow = sm.krow, *kred = sm.kred;
-    const int k = tl.x * 32 + lane;
+    const int k = tl.x * 32 + lane - row_pad(K);
     const int l0 = tl.y * LC;
-    const int l1 = idle ? l0 : min(l0 + LC, K);
-    const bool kval = k < K && !idle;
+    const int l1 = idle ? l0 : min(l0 + LC, row_last(K, tl.x) + 1);
+    const bool kval = k >= 0 && !idle;
     const double Ck = kval ? C[k] : 0.0;
 #pragma unroll
     for (int f = 0; f < 2 * PB; ++f) sm.sacc[f * 32 + lane] = 0.0;
@@ -263,7 +271,7 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
 #pragma unroll
         for (int q = 0; q < NC; ++q) ak[q] = 0.0;
         const bool active = kval && l <= k;
-        const BraRef b{bra_at<N>(bra, active ? k : l)};
+        const BraRef b{bra_at<N>(bra, K, active ? k : l)};
         for (int P = p0; P < pend; ++P) {
             const double *kr = ket + ((size_t)l * nst + P) * KL::size;
             if constexpr (SKET) {
@@ -422,7 +430,7 @@ __device__ __forceinline__ void sum_partials(const PassParts &p, int kb, int f, 
                                              double (*red)[8][32]) {
     constexpr int PB = SumFields<N>::size;
     const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
-    const int K = p.K, LC = p.LC, m = kb * 32 + lane;
+    const int K = p.K, LC = p.LC, m = kb * 32 + lane - row_pad(K);
     const int ta = p.urange ? p.urange[kb].x : max(p.tstart[kb], p.t0) * p.npc;
     const int tb = p.urange ? p.urange[kb].y : min(p.tstart[kb + 1], p.t1) * p.npc;
     double v[4] = {0.0, 0.0, 0.0, 0.0};
@@ -431,10 +439,10 @@ __device__ __forceinline__ void sum_partials(const PassParts &p, int kb, int f, 
         v[0] += p.part_b[(((size_t)t * 2 + 0) * PB + f) * 32 + lane];
         v[1] += p.part_b[(((size_t)t * 2 + 1) * PB + f) * 32 + lane];
     }
-    if (m < K) {
+    if (m >= 0) {
         const int lc = m / LC, ll = m - lc * LC;
-        const int nkb = (K + 31) >> 5;
-        int kb0 = lc * LC - 31;
+        const int nkb = row_blocks(K);
+        int kb0 = m + row_pad(K) - 31;  // first row block that meets ket m
         kb0 = kb0 > 0 ? (kb0 + 31) >> 5 : 0;
         for (int q = kb0 + seg; q < nkb; q += 8) {
             const int t = p.tstart[q] + lc;
@@ -455,7 +463,7 @@ __device__ __forceinline__ void sum_partials(const PassParts &p, int kb, int f, 
 #pragma unroll
     for (int i = 0; i < 4; ++i) red[i][seg][lane] = v[i];
     __syncthreads();
-    if (seg < 4 && m < K) {  // warp i: set i
+    if (seg < 4 && m >= 0) {  // warp i: set i
         double s = red[seg][0][lane];
 #pragma unroll
         for (int q = 1; q < 8; ++q) s += red[seg][q][lane];
@@ -518,7 +526,7 @@ template <int N> struct FinishSmem {
     static_assert(N > 5 || size * 8 <= 48 * 1024, "shared memory");
 };
 
-// The gradients of the 32 bases of row block kb from their per-basis sums, by one
+// The gradients of the bases 32 kb .. 32 kb + 31 from their per-basis sums, by one
 // block of 256 threads: every step is split over the warps by matrix row, lane =
 // basis, so that the loads of all fields are in flight at once and no thread
 // walks the whole chain (one thread per basis took 11 us at n = 5 for any K).  E2 =
@@ -539,7 +547,7 @@ __device__ __forceinline__ bool finish_block(const double *__restrict__ sums, in
     const int k = min(kb * 32 + lane, K - 1);
     const int nk = min(32, K - kb * 32);
     constexpr int A = FS::rec, S = A + TR * 32, AS = S + 3 * N * 32, L = AS + 3 * N * 32;
-    const double *bk = bra_at<N>(bra, kb * 32) + min(lane, nk - 1);
+    const double *bk = bra_at<N>(bra, K, k);
     auto ket = [&](int f) {  // the kets' combined sum (folded: their gradient)
         const double *q = sums + (size_t)(2 * PB + f) * K + k;
         return E2 != 0.0 ? q[0] - E2 * q[(size_t)PB * K] : q[0];

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(64) prep_kernel(const double *__restrict__ iv,
     }
     if ((int)blockIdx.x < nbb) {
         const int k = blockIdx.x * blockDim.x + threadIdx.x;
-        if (k < K) prep_bra_at<N>(iv + (size_t)k * (tri(N) + 3 * N), cs, bra_at<N>(bra, k), 32);
+        if (k < K) prep_bra_at<N>(iv + (size_t)k * (tri(N) + 3 * N), cs, bra_at<N>(bra, K, k), 32);
         return;
     }
     const int id = (blockIdx.x - nbb) * blockDim.x + threadIdx.x;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(32, MINW) energy_kernel(const int2 *__restrict
     int k, l0, lend;
     if (!energy_lane_range(tl.x, tl.y, lane, LC, K, k, l0, lend)) return;
     int bad = 0;
-    const int fl = energy_lane<N, double>(BraRef{bra_at<N>(bra, k)}, DevKet{ket}, k, l0, lend, K, nst,
+    const int fl = energy_lane<N, double>(BraRef{bra_at<N>(bra, K, k)}, DevKet{ket}, k, l0, lend, K, nst,
                                           cs, H, S, Kin, Pot, bad);
     flag_status(status, fl, bad);
 }
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(32 * W) energy_split_kernel(const int2 *__rest
     const int2 tl = tiles[blockIdx.x];
     int k, l0, lend;
     const bool mine = energy_lane_range(tl.x, tl.y, lane, LC, K, k, l0, lend);
-    const BraRef b{bra_at<N>(bra, mine ? k : 0)};
+    const BraRef b{bra_at<N>(bra, K, mine ? k : 0)};
     const int p0 = w * nst / W, p1 = (w + 1) * nst / W;
     int flags = 0, pair = 0x7fffffff;
     for (int l = tl.y * LC; l < min(tl.y * LC + LC, K); ++l) {
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(32, MINW) grad_kernel(int nkb, int nlc, int LC
     double *out = part + (size_t)lc * Part<N>::size * K + k;
     __shared__ double sacc[2 * Part<N>::size * 32];
     SmemAcc<N> accH{sacc + lane}, accS{sacc + Part<N>::size * 32 + lane};
-    const bool ok = grad_lane<N, double>(BraRef{bra_at<N>(bra, k)}, DevKet{ket}, l0, l1, nst, cs, lam, scal[0],
+    const bool ok = grad_lane<N, double>(BraRef{bra_at<N>(bra, K, k)}, DevKet{ket}, l0, l1, nst, cs, lam, scal[0],
                                          out, (size_t)K, accH, accS);
     if (!ok) flag_status(status, 1, k * K + l0);
 }
@@ -365,11 +365,10 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
     __shared__ int gsh;
     constexpr int PB = SumFields<N>::size;
     constexpr int PER_WARP = fsym_warp_smem<N>();
-    constexpr int BS = BraLayout<N>::term;
     constexpr int TBL = ket_table<N>(2);
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
-    double *sbra = smem + WARPS * PER_WARP;  // BS x 32 doubles after the warps' areas
+    double *sbra = smem + WARPS * PER_WARP;  // after the warps' areas
     const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + 64};
     for (;;) {
         if (threadIdx.x == 0) gsh = atomicAdd(qcount, 1);
@@ -379,8 +378,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
         if (g >= ngroups) break;
         const int2 gr = groups[g];
         const int kb = gr.x, lc = sgroup_lc0(gr) + w;
-        const int last = min(kb * 32 + 31, K - 1);
-        const bool idle = lc * LC > last;  // past this block's triangle
+        const bool idle = lc * LC > row_last(K, kb);  // past this block's triangle
         // a split group of the queue's tail: this unit takes symmetry terms
         // [p0, p1); parts after the first write to their own slots in xsym
         const int part = sgroup_part(gr), parts = sgroup_parts(gr);
@@ -390,10 +388,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
             xo.x = xsym;
             xo.slot = (((g - tail0) / parts) * WARPS + w) * (parts - 1) + (part - 1);
         }
-        // the group's 32 bras, once for all warps (rows past K hold row K - 1)
-        const double *bk = bra_at<N>(bra, kb * 32);
-        for (int i = threadIdx.x; i < BS * 32; i += 32 * WARPS)
-            sbra[i] = bk[(i & ~31) + min(i & 31, K - 1 - kb * 32)];
+        stage_bras<N>(sbra, bra, K, kb, 32 * WARPS);  // the group's bras, once for all warps
         __syncthreads();
         fsym_tile<N, true, true, true, false, KE>(tstart[kb] + lc, make_int2(kb, lc), LC, K, nst, cs, bra, ket, C,
                                                   kmap, H, S, part_b, part_k, status, sm, idle, sbra, p0, p1, xo,
@@ -403,7 +398,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
         // slot of queue unit g
         __syncthreads();
         for (int i = threadIdx.x; i < 2 * PB * 32; i += 32 * WARPS) {
-            if (kb * 32 + (i & 31) >= K) continue;
+            if (kb == 0 && (i & 31) < row_pad(K)) continue;  // no basis
             double v = smem[i];
 #pragma unroll
             for (int q = 1; q < WARPS; ++q) v += smem[q * PER_WARP + i];
@@ -427,12 +422,12 @@ __global__ void __launch_bounds__(256) fsym_tail_fix_kernel(const int2 *__restri
     const int2 gr = groups[tail0 + j * sgroup_parts(groups[tail0])];
     const int parts = sgroup_parts(gr);
     const int kb = gr.x, lc = sgroup_lc0(gr) + w;
-    if (lc * LC > min(kb * 32 + 31, K - 1)) return;
+    if (lc * LC > row_last(K, kb)) return;
     const size_t XS = fsym_tail_slot(PB, LC);
     const double *x0 = xsym + (size_t)(j * W + w) * (parts - 1) * XS + (size_t)LC * 2 * PB;
     for (int i = threadIdx.x; i < LC * 64; i += blockDim.x) {
-        const int l = lc * LC + i / 64, r = i & 63, k = kb * 32 + (r & 31);
-        if (k >= K || l >= K || l > k) continue;
+        const int l = lc * LC + i / 64, r = i & 63, k = kb * 32 + (r & 31) - row_pad(K);
+        if (k < 0 || l > k) continue;
         double *M = r < 32 ? H : S;
         double v = M[(size_t)k * K + l];
         for (int q = 0; q < parts - 1; ++q) v += x0[q * XS + i];
@@ -513,7 +508,7 @@ __global__ void __launch_bounds__(128) grad_reduce_kernel(const double *__restri
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= K) return;
     const double sc = scal[1] * (C ? C[k] : 1.0);
-    if (!grad_reduce_at<N>(part, 1, K, bra_at<N>(bra, k), 32, sc, g, k)) atomicOr(status, 2);
+    if (!grad_reduce_at<N>(part, 1, K, bra_at<N>(bra, K, k), 32, sc, g, k)) atomicOr(status, 2);
 }
 
 // python/rrms.py:21-120 rrms(stfe, stf, ii, jj, n1) per term: terms[5 t ..] =
@@ -627,7 +622,7 @@ __global__ void __launch_bounds__(32) dipole_group_kernel(const int2 *__restrict
     bool ok = true;
     if (energy_lane_range(tl.x, tl.y, lane, LC, K, k, l0, lend)) {
         const double Ck = C[k];
-        const BraRef b{bra_at<N>(bra, k)};
+        const BraRef b{bra_at<N>(bra, K, k)};
         for (int q = q0; q < q1; ++q) {
             double a[3 * N], a0 = 0.0;
 #pragma unroll
@@ -714,7 +709,7 @@ __global__ void __launch_bounds__(128) matel_kernel(const int *__restrict__ term
         return;
     }
     const double *kr = ket + ((size_t)jj * nst + stf) * KetLayout<N>::size;
-    if (!matel_one<N, double>(BraRef{bra_at<N>(bra, ii)}, kr, cs, out + 4 * t))
+    if (!matel_one<N, double>(BraRef{bra_at<N>(bra, K, ii)}, kr, cs, out + 4 * t))
         flag_status(status, 1, ii * K + jj);
 }
 
@@ -737,8 +732,8 @@ __global__ void __launch_bounds__(128) gradel_kernel(const int *__restrict__ ter
     const double *kr = ket + ((size_t)jj * nst + stf) * KetLayout<N>::size;
     double L[tri(N)];
 #pragma unroll
-    for (int q = 0; q < tri(N); ++q) L[q] = bra_at<N>(bra, ii)[(BraLayout<N>::L + q) * 32];
-    if (!gradel_one<N, double>(BraRef{bra_at<N>(bra, ii)}, kr, cs, L, ii == jj,
+    for (int q = 0; q < tri(N); ++q) L[q] = bra_at<N>(bra, K, ii)[(BraLayout<N>::L + q) * 32];
+    if (!gradel_one<N, double>(BraRef{bra_at<N>(bra, K, ii)}, kr, cs, L, ii == jj,
                                tgvl + (size_t)t * blk, tgvls + (size_t)t * blk))
         flag_status(status, 1, ii * K + jj);
 }

@@ -410,9 +410,10 @@ NECG_HD bool gradel_one(const BA &b, const KR &kr, const Consts<N> &cs, const do
     return ok;
 }
 
-// Energy tiles over the lower triangle: tile (kb, lc) covers bra k in
-// [32 kb, 32 kb + 32) and kets l in [lc LC, lc LC + LC) with l <= k; a tile
-// exists when lc LC <= 32 kb + 31 and lc LC < K.
+// Energy tiles over the lower triangle: tile (kb, lc) covers the bras of row block
+// kb and kets l in [lc LC, lc LC + LC) with l <= k; it has pairs when lc LC <=
+// row_last(K, kb).  The count here is of all with lc LC <= 32 kb + 31 and lc LC < K,
+// an upper bound, for lists made without looking at K's remainder.
 NECG_HD int energy_tile_count(int K, int LC) {
     int n = 0;
     for (int kb = 0; kb * 32 < K; ++kb) {
@@ -496,11 +497,11 @@ template <int N> struct SumFields {
 constexpr int kSumSets = 4;
 
 // Lane ranges of the two tile kinds (used by the kernels and the emulator).
-// Energy: tile (kb, lc) -> bra k = 32 kb + lane, kets [l0, lend); false if idle.
+// Energy: tile (kb, lc) -> lane's bra k of row block kb, kets [l0, lend); false if idle.
 NECG_HD bool energy_lane_range(int kb, int lc, int lane, int LC, int K, int &k, int &l0, int &lend) {
-    k = kb * 32 + lane;
+    k = kb * 32 + lane - row_pad(K);
     l0 = lc * LC;
-    if (k >= K || l0 > k) return false;
+    if (k < 0 || k >= K || l0 > k) return false;
     lend = l0 + LC < K ? l0 + LC : K;
     if (lend > k + 1) lend = k + 1;
     return true;

@@ -103,9 +103,8 @@ template <int N> struct KetLayout {
     static constexpr int size = (tMA + 1 + 1) & ~1;  // even, 16-byte records
 };
 
-// Bra record: structure of arrays in blocks of 32 basis functions, field f of
-// basis k at ((k / 32) size + f) 32 + k % 32 (bra_at): a warp's lanes read 256
-// contiguous bytes, and the fields of a lane are a constant distance apart, so a
+// Bra record: structure of arrays by row block, field f of lane j of block kb at
+// (kb size + f) 32 + j (bra_at): a warp's lanes read 256 contiguous bytes, and the fields of a lane are a constant distance apart, so a
 // load needs no address arithmetic of its own (with a stride of K doubles the
 // n = 3 term spent about 60 of its 1480 instructions on addresses).
 template <int N> struct BraLayout {
@@ -122,9 +121,20 @@ template <int N> struct BraLayout {
     static constexpr int size = L + T;
 };
 
+// Rows come in blocks of 32, one per lane: lane j of row block kb is basis
+// 32 kb + j - row_pad(K), so that a K that is not a multiple of 32 leaves its empty
+// lanes in the first block, whose rows meet the fewest kets.  (In the last block
+// they would sit through all K: at K = 101 the blocks' kets add up to 212 instead
+// of 293, and the pair passes take that much less.)
+__host__ __device__ constexpr int row_pad(int K) { return (32 - (K & 31)) & 31; }
+__host__ __device__ constexpr int row_blocks(int K) { return (K + 31) >> 5; }
+// last basis of row block kb
+__host__ __device__ constexpr int row_last(int K, int kb) { return 32 * kb + 31 - row_pad(K); }
+
 // Field 0 of basis k in the blocked layout; further fields are 32 doubles apart.
-template <int N, typename P> __host__ __device__ __forceinline__ P *bra_at(P *bra, int k) {
-    return bra + (size_t)(k >> 5) * (BraLayout<N>::size * 32) + (k & 31);
+template <int N, typename P> __host__ __device__ __forceinline__ P *bra_at(P *bra, int K, int k) {
+    const int p = k + row_pad(K);
+    return bra + (size_t)(p >> 5) * (BraLayout<N>::size * 32) + (p & 31);
 }
 
 // Per-problem constants, passed to kernels by value (constant bank).

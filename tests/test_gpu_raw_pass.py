@@ -188,3 +188,30 @@ def test_matrices_and_row_sums_agree(n, K, lc, minw, npc):
     for M, Mo in ((H, Ho), (S, So)):
         M = M.cpu().numpy()
         assert np.array_equal(M, M.T) and np.max(np.abs(M - Mo)) <= 1e-12 * max(1.0, np.max(np.abs(Mo)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [1, 7, 31, 32, 33, 63, 65, 96, 101])
+@pytest.mark.parametrize("lc", [1, 3, 8])
+def test_row_blocks_of_ragged_sizes(K, lc):
+    """Every remainder class of K against 32 and chunks that do not divide the row
+    blocks' ends: passes, matrices and dipole against the oracle."""
+    from nbo_correlatedgaussians_b200 import synth
+    p = synth.make_problem("H2", K, 9 * K + lc)
+    p.C = np.random.default_rng(K).normal(size=K)
+    o = Oracle.from_problem(p)
+    fo, go, Ho, So = o.outprod(p.x, nthreads=8, return_hs=True)
+    comps_o, _ = o.dipole(p.iv, p.C, nthreads=8)
+    eng = engine(p)
+    for mode, minw, npc in ((0, 8, 1), (1, 8, 1), (2, 12, 1), (2, 122, 3), (2, 248, 1), (2, 216, 1)):
+        assert eng.L.necg_set_symmetric(eng.h, mode, lc, minw) == 0
+        assert eng.L.necg_set_splits(eng.h, npc) == 0
+        f, g = eng.outprod(p.x)
+        assert abs(f - fo) < TOL_E and normwise(g, go) < TOL_G, (mode, minw)
+    eng.set_tiles(lc, 4)
+    H, S, _, _, en = eng.build_matrices(p.iv, p.C)
+    assert abs(float(en[0]) - fo) < TOL_E
+    assert np.max(np.abs(H.cpu().numpy() - Ho)) <= 1e-12 * max(1.0, np.max(np.abs(Ho)))
+    assert np.max(np.abs(S.cpu().numpy() - So)) <= 1e-12 * max(1.0, np.max(np.abs(So)))
+    comps, _ = eng.dipole(p.iv, p.C)
+    assert np.max(np.abs(comps - comps_o)) <= 1e-11 * max(np.max(np.abs(comps_o)), 1e-300)
