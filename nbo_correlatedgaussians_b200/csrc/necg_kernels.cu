@@ -845,13 +845,29 @@ template <int N> struct Launch {
                                                                  a.status);
         }
     }
-    // lockstep blocks when the handle's groups are 8 chunks wide
+    // blocks when the handle's groups are 8 chunks wide, for n > 3 (LiH K = 400, ket
+    // chunk 2: 394 us for the gradient against 528 to 570 of the one-warp tiles; H2
+    // K = 2048, chunk 4: 709 against 653)
     static bool gsym_block(const LaunchArgs &a) {
-        return a.minb_s >= 200 && fused_block_warps(a.minb_s) == 8 && a.sgroups && a.qcount && a.urange;
+        return N > 3 && a.minb_s >= 200 && fused_block_warps(a.minb_s) == 8 && a.sgroups && a.qcount && a.urange;
     }
     static void gsym_tiles(const LaunchArgs &a, cudaStream_t st) {
-        if (gsym_block(a)) {
-            fsym_block<8, true>(a, st);
+        if constexpr (N > 3)
+            if (gsym_block(a)) {
+                fsym_block<8, true>(a, st);
+                return;
+            }
+        // A handle tuned to a block variant at n <= 3 takes one-warp tiles, 16 to the SM
+        // once they are more than 8 to the SM (H2 K = 2048, chunk 4: 653 us for the
+        // gradient, 706 at 8 to the SM; H2 K = 600, chunk 1: 126 and 133), where they
+        // are fewer 8, whose wider register budget has the shorter chain (H2 K = 600,
+        // chunk 8: 130 us, 145 at 16).
+        if (N <= 3 && a.minb_s >= 200) {
+            int dev = 0, sms = 148;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (a.nstiles > 8 * sms) gsym_v<16, false>(a, st);
+            else gsym_v<8, true>(a, st);
             return;
         }
         switch (a.minb_s) {

@@ -215,3 +215,18 @@ def test_row_blocks_of_ragged_sizes(K, lc):
     assert np.max(np.abs(S.cpu().numpy() - So)) <= 1e-12 * max(1.0, np.max(np.abs(So)))
     comps, _ = eng.dipole(p.iv, p.C)
     assert np.max(np.abs(comps - comps_o)) <= 1e-11 * max(np.max(np.abs(comps_o)), 1e-300)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,K,lc", [(2, 290, 1), (3, 290, 1), (3, 290, 5), (1, 290, 1)])
+@pytest.mark.parametrize("minw", [248, 232, 216])
+def test_gradient_with_e_given_of_block_handles(n, K, lc, minw):
+    """n <= 3 handles set to a block variant: one-warp tiles, on both sides of the
+    count where more of them share an SM (chunk 1: 1500 tiles, chunk 5: 300)."""
+    p = make(n, K, 11 * n + lc)
+    fo, go = Oracle.from_problem(p).outprod(p.x, nthreads=8)
+    eng = engine(p)
+    assert eng.L.necg_set_symmetric(eng.h, 2, lc, minw) == 0
+    H, S, _, _, en = eng.build_matrices(p.iv, p.C, parts=False)
+    g = eng.make_grad_dev(p.iv, p.C, H, S, en).cpu().numpy()
+    assert abs(float(en[0]) - fo) < TOL_E and normwise(g, go) < TOL_G
