@@ -5,7 +5,7 @@ device workspace) with tile widths chosen by the autotuner for its (n, K).  A
 ``BatchEngine`` plans a step over any subset of its instances: when every
 instance's symmetry set is closed under inverse, the pair work of all of them
 is one persistent launch of the fused pass over a single queue (instances by
-decreasing tile cost, each over its own tile groups; 8-warp lockstep blocks, or
+decreasing tile cost, each over its own tile groups; 8-warp blocks, or
 one-warp blocks when the plan is too small to fill the SMs); otherwise one
 queue of energy tiles and one of ordered gradient tiles.  The step is a fixed
 sequence of kernels with fixed grids, so each mode's step is captured once as

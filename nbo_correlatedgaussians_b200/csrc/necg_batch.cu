@@ -48,7 +48,7 @@ struct InstDesc {
     int nbgroups;
     int npc;             // one-warp fused kernel: symmetry terms split npc ways per tile
     const int2 *burange; // groups of each row block (their bra partial slots)
-    int groups;          // 1: the bra partials are per group (lockstep kernel)
+    int groups;          // 1: the bra partials are per group (block kernel)
     int general;         // prep: general shift maps
     double *psym;
     RawMap kmap;
@@ -58,7 +58,7 @@ struct InstDesc {
 struct PlanHdr {
     int ninst, ne, ng;
     int qe, qg;  // persistent queue heads
-    int nf, qf;  // fused queue: tile groups (lockstep kernel) or tiles (one-warp kernel)
+    int nf, qf;  // fused queue: tile groups (block kernel) or tiles (one-warp kernel)
     int fine;    // 1: the one-warp fused kernel (few groups for the SMs)
 };
 
@@ -469,7 +469,7 @@ struct necg_batch {
     int cap_inst = 0, cap_tiles = 0;
     int device = 0, sms = 148;
     int occ_energy = 8, occ_grad = 8, occ_fwarp = 8;  // resident one-warp blocks per SM (persistent kernels)
-    int mode = 0;  // of the current plan: 0 ordered, 1 fused lockstep, 2 fused one-warp
+    int mode = 0;  // of the current plan: 0 ordered, 1 fused blocks, 2 fused one-warp
     bool fused = false;  // mode of the current plan
     char *d_plan = nullptr;  // device plan buffer
     char *h_plan = nullptr;  // pinned host staging
@@ -521,7 +521,7 @@ void layout(necg_batch *b, char *base, PlanPtrs &p, size_t *total) {
     if (total) *total = off;
 }
 
-// mode: 0 ordered, 1 fused (lockstep blocks), 2 fused (one-warp blocks)
+// mode: 0 ordered, 1 fused (8-warp blocks), 2 fused (one-warp blocks)
 void launch_step(necg_batch *b, cudaStream_t st, int mode) {
     const PlanPtrs &p = b->ptrs;
     const int g = b->sms;
@@ -587,7 +587,7 @@ int necg_batch_create(int max_instances, int max_tiles, necg_batch **out) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->occ_fwarp, batch_fused_warp_kernel, 32, 0) != cudaSuccess ||
         b->occ_fwarp < 1)
         b->occ_fwarp = 8;
-    // the lockstep fused kernel's shared memory (one 8-warp block per SM) needs the opt-in
+    // the block kernel's shared memory (one 8-warp block per SM) needs the opt-in
     cudaError_t e = cudaFuncSetAttribute(batch_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kBatchFusedSmem);
     if (e == cudaSuccess) e = cudaMalloc((void **)&b->d_plan, b->plan_bytes);

@@ -174,7 +174,7 @@ int ensure_tiles(necg_handle *h, int K, cudaStream_t st) {
 // buffers for H and S.
 int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
     const int PB = necg::part_stride(h->n) + 1;
-    const int gw = necg::fused_block_warps(h->minb_s);  // tiles per group of the lockstep-block pass
+    const int gw = necg::fused_block_warps(h->minb_s);  // tiles per group of the block variants
     const int npc = fused ? necg::fused_splits(h) : 1;
     const size_t hp_need = npc > 1 ? (size_t)npc * K * K : 0;
     if (hp_need > h->hp_cap) {
@@ -233,7 +233,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
         int parts = T > 0 ? sms / T : 1;
         if (parts > 8) parts = 8;
         if (parts > h->nst) parts = h->nst;
-        // the lockstep pass writes bra partials per queue unit into the slots
+        // the block variants write bra partials per queue unit into the slots
         // sized for the tiles: G - T + T parts units must not exceed them
         if (T > 0 && parts > 1 + ((int)t.size() - G) / T) parts = 1 + ((int)t.size() - G) / T;
         h->sg_ntail = 0;

@@ -55,7 +55,7 @@ __device__ __forceinline__ void flag_status(int *status, int flags, int pair) {
     atomicMin(status + 1, pair);
 }
 
-// Where a part of a split tile of the lockstep pass writes instead of the
+// Where a part of a split tile of the block variants writes instead of the
 // main buffers (slot < 0: the main buffers): slot `slot` of x, fsym_tail_slot
 // doubles holding its ket partials, then its LC x 64 H and S sums (H for the 32
 // bras, then S).  The address is formed where it is used, so that

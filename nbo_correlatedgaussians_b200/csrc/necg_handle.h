@@ -40,7 +40,7 @@ struct necg_handle {
     int stiles_cap = 0, stiles_K = -1, stiles_lc = -1, nstiles = 0;
     double *d_psym = nullptr;
     size_t psym_cap = 0;  // doubles
-    int2 *d_sgroups = nullptr;  // groups of 8 fused tiles of one row block (kb, first lc)
+    int2 *d_sgroups = nullptr;  // groups of consecutive fused tiles of one row block (kb, first lc)
     int sgroups_cap = 0, nsgroups = 0, sgroups_w = 0;
     // the queue's tail: its last sg_ntail groups split into sg_parts units from
     // queue index sg_tail0; parts after the first write to d_xsym

@@ -32,7 +32,7 @@ struct LaunchArgs {
     // sums (non-null): write the per-basis sums there and stop before GRADA
     int st_begin, st_end;
     double *sums;
-    // block-synchronised fused pass (variant 208): groups of 8 tiles of one row block
+    // block variants: groups of consecutive tiles of one row block
     const int2 *sgroups;                   // (kb, first lc)
     int nsgroups;
     int *qcount;                           // group queue head (reset before the launch)
@@ -40,19 +40,19 @@ struct LaunchArgs {
     // variants; npc <= 1: no split): split pc writes its H, S sums to Hp, Sp + pc K^2
     int npc;
     double *Hp, *Sp;
-    // lockstep pass: the last sg_ntail groups of the queue are split into
+    // block variants: the last sg_ntail groups of the queue are split into
     // sg_parts units over the symmetry terms, from queue index sg_tail0; parts
     // 1 .. sg_parts - 1 write to xsym (fsym_tail_slot doubles per tile and part)
     double *xsym;
     int sg_tail0, sg_ntail, sg_parts;
-    // lockstep pass: bra partials are written per queue unit; row block kb's
+    // block variants: bra partials are written per queue unit; row block kb's
     // units are [urange[kb].x, urange[kb].y)
     const int2 *urange;
     const int *tslot;                      // first xsym slot of each tile of a split tail group, else -1
     int sms_general, full;                 // prep: general shift maps; whole ket records (else the terms' part)
 };
 
-// A tile group of the lockstep pass: row block kb, first ket chunk lc0 and, for
+// A tile group of the block variants: row block kb, first ket chunk lc0 and, for
 // a split group of the queue's tail, its part and the number of parts (one part
 // per range of symmetry terms).
 __host__ __device__ inline int2 sgroup_pack(int kb, int lc0, int part, int parts) {
@@ -76,7 +76,7 @@ int launch_fsym_sum(const LaunchArgs &a, cudaStream_t st);
 int launch_fsym_finish(const LaunchArgs &a, double *f_out, double *gradc, bool own_e, cudaStream_t st);
 int launch_rows_from_sums(const LaunchArgs &a, double *rows, cudaStream_t st);
 int launch_fsym(const LaunchArgs &a, cudaStream_t st);
-// lockstep-block variants of the fused pass (2xy): warps per block, and
+// block variants of the fused pass (2xy): warps per block, and
 // whether the variant's shared memory fits for n particles
 int fused_block_warps(int variant);
 bool fused_variant_ok(int n, int variant);

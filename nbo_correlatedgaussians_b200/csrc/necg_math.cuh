@@ -85,7 +85,7 @@ __host__ __device__ constexpr int sx(int i, int j) {
 
 // Ket record: one per (l, P), read warp-uniformly by the tile kernels.
 // The pair passes read the first `term` doubles (staged in shared memory by the
-// lockstep blocks); Sp is for the fold of a symmetry term whose shift map is not
+// block variants); Sp is for the fold of a symmetry term whose shift map is not
 // that of its coordinate map, Np8 = -8 A_l' M A_l' and tMA for the energy path.
 template <int N> struct KetLayout {
     static constexpr int T = tri(N);
