@@ -5,7 +5,7 @@
 // gradel(stf, k, l) (python/gradel.py:27-392).  The reference expands every
 // n x n matrix to 3n x 3n with kron(., I3) and inverts with LAPACK; here all
 // work stays in n-space with the shifts viewed as n x 3 matrices, B = A_k + A_l'
-// is factored by Cholesky in registers, and the gradient is formed with respect
+// is inverted in registers (symmetric elimination), and the gradient is formed with respect
 // to A_k = L_k L_k^T (a symmetric n x n matrix) and s_k, then mapped to vech(L_k)
 // once per basis function (dF/dL = 2 G L).
 //
