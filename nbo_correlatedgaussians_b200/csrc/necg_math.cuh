@@ -5,9 +5,9 @@
 // gradel(stf, k, l) (python/gradel.py:27-392).  The reference expands every
 // n x n matrix to 3n x 3n with kron(., I3) and inverts with LAPACK; here all
 // work stays in n-space with the shifts viewed as n x 3 matrices, B = A_k + A_l'
-// is inverted in registers (symmetric elimination), and the gradient is formed with respect
-// to A_k = L_k L_k^T (a symmetric n x n matrix) and s_k, then mapped to vech(L_k)
-// once per basis function (dF/dL = 2 G L).
+// is inverted in registers (symmetric elimination), and the gradient is formed
+// with respect to A_k = L_k L_k^T (a symmetric n x n matrix) and s_k, then mapped
+// to vech(L_k) once per basis function (dF/dL = 2 G L).
 //
 // Notation (n = N particles):
 //   A_k, A_l' = P^T A_l P    symmetric, packed lower (N(N+1)/2)
@@ -104,9 +104,10 @@ template <int N> struct KetLayout {
 };
 
 // Bra record: structure of arrays by row block, field f of lane j of block kb at
-// (kb size + f) 32 + j (bra_at): a warp's lanes read 256 contiguous bytes, and the fields of a lane are a constant distance apart, so a
-// load needs no address arithmetic of its own (with a stride of K doubles the
-// n = 3 term spent about 60 of its 1480 instructions on addresses).
+// (kb size + f) 32 + j (bra_at): a warp's lanes read 256 contiguous bytes, and the
+// fields of a lane are a constant distance apart, so a load needs no address
+// arithmetic of its own (with a stride of K doubles the n = 3 term spent about 60
+// of its 1480 instructions on addresses).
 template <int N> struct BraLayout {
     static constexpr int T = tri(N);
     static constexpr int A = 0;
