@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(128) batch_prep_kernel(PlanPtrs p) {
             const InstDesc &d = p.inst[q];
             const int id = j - p.pref_ket[q];
             BATCH_SWITCH(d.n, prep_ket_one<N>(d.iv, d.C, d.nst, consts_of<N>(d), d.sml, d.sms, d.scvv,
-                                             d.ket, id, d.pinv, d.general, d.kmap.fold));
+                                             d.ket, id, d.pinv, d.general));
         }
     }
 }
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(32) batch_energy_kernel(PlanPtrs p) {
 __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
     __shared__ double sacc[2 * SumFields<kMaxN>::size * 32];
     __shared__ double krow[ket_table<kMaxN>(2)];
-    __shared__ double kred[64];
+    __shared__ double kred[ket_red<kMaxN>()];
     const int lane = threadIdx.x & 31;
     const int nf = p.hdr->nf;
     for (;;) {
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
 // records too, in two buffers (fsym_tile with SBRA, SKET), and the warps meet only
 // at the group's ends.  Shared memory is sized for n = kMaxN.
 template <int N> __host__ __device__ constexpr int bfused_warp_smem() {
-    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
+    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + ket_red<N>() + 2 * KetLayout<N>::size;
 }
 constexpr int kBatchFusedSmem = (8 * bfused_warp_smem<kMaxN>() + BraLayout<kMaxN>::term * 32) * 8;
 
@@ -214,7 +214,7 @@ __device__ __forceinline__ void batch_fused_group(const InstDesc &d, int g, doub
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
     double *sbra = smem + 8 * PER_WARP;
-    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + 64};
+    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + ket_red<N>()};
     const int2 gr = d.bgroups[g];
     const int K = d.K, kb = gr.x, lc = gr.y + w;
     const bool idle = lc * d.lc_s > row_last(K, kb);
@@ -451,7 +451,6 @@ template <int N> void fill_consts(InstDesc &d, const necg_handle *h) {
     static_assert(sizeof(Consts<N>) <= sizeof(d.cs), "constants do not fit");
     Consts<N> c;
     for (int i = 0; i < N * N; ++i) c.M[i] = h->mass[i];
-    c.derive();
     for (int q = 1; q <= N; ++q)
         for (int pp = 0; pp < q; ++pp)
             c.cv[vidx(pp, q)] = 2.0 * h->ncv[pp] * h->ncv[q] / NECG_SQRT_PI;

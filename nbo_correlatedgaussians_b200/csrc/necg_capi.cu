@@ -1016,7 +1016,6 @@ int necg_matel(necg_handle *h, int K, const double *iv_dev, int nterms, const in
     LaunchArgs a = base_args(h, K);
     a.iv = iv_dev;
     a.C = nullptr;
-    a.full = 1;  // matel chooses between the bra's and the ket's A M A
     if (necg::launch_prep(a, st)) return NECG_ERR_UNSUPPORTED;
     if (nterms > 0) necg::launch_matel(a, terms_dev, nterms, out_dev, st);
     return finish_launch();

@@ -69,8 +69,11 @@ struct TileOut {
 // or the symmetric pass (MATS = 1: the combined gradient).
 template <int N> __host__ __device__ constexpr int ket_table(int mats) { return 16 * (mats * KetSlots<N>::SL + 1); }
 
+// Doubles of the reduced ket fields of such a table: one per slot and lane.
+template <int N> __host__ __device__ constexpr int ket_red() { return 2 * KetSlots<N>::SL > 32 ? 64 : 32; }
+
 // Shared memory of one warp's tile: bra accumulators (2 * PB * 32 doubles), the
-// ket table (ket_table) and the reduced ket fields (64).  Sized by the caller
+// ket table (ket_table) and the reduced ket fields (ket_red).  Sized by the caller
 // for its largest n.
 struct FusedSmem {
     double *sacc, *krow, *kred;
@@ -264,7 +267,7 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
     int cur = 0;  // SKET: the buffer that holds the current term's record
     if constexpr (SKET) {
         if (l0 < l1 && p0 < pend)
-            ket_fetch(sm.sket, ket + ((size_t)l0 * nst + p0) * KL::size, KL::term, lane);
+            ket_fetch(sm.sket, ket + ((size_t)l0 * nst + p0) * KL::size, KL::size, lane);
     }
     for (int l = l0; l < l1; ++l) {
         double ak[NC], hsum = 0.0, ssum = 0.0;
@@ -282,9 +285,9 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
                     nP = p0;
                 }
                 if (nl < l1)
-                    ket_fetch(sm.sket + (cur ^ 1) * KL::term, ket + ((size_t)nl * nst + nP) * KL::size, KL::term,
+                    ket_fetch(sm.sket + (cur ^ 1) * KL::size, ket + ((size_t)nl * nst + nP) * KL::size, KL::size,
                               lane);
-                kr = sm.sket + cur * KL::term;
+                kr = sm.sket + cur * KL::size;
                 cur ^= 1;
             }
             out.wb = active ? kr[KL::wC] : 0.0;

@@ -40,7 +40,7 @@ template <int N>
 __global__ void __launch_bounds__(64) prep_kernel(const double *__restrict__ iv, const double *__restrict__ C, int K,
                                                   int nst, int nbb, Consts<N> cs, const double *__restrict__ sml,
                                                   const double *__restrict__ sms, const double *__restrict__ scvv,
-                                                  const int *__restrict__ pinv, int general, int full,
+                                                  const int *__restrict__ pinv, int general,
                                                   double *__restrict__ bra, double *__restrict__ ket, int *status,
                                                   int *qcount) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(64) prep_kernel(const double *__restrict__ iv,
         return;
     }
     const int id = (blockIdx.x - nbb) * blockDim.x + threadIdx.x;
-    if (id < K * nst) prep_ket_one<N>(iv, C, nst, cs, sml, sms, scvv, ket, id, pinv, general, full);
+    if (id < K * nst) prep_ket_one<N>(iv, C, nst, cs, sml, sms, scvv, ket, id, pinv, general);
 }
 
 // Energy tiles over the lower triangle (the loop of python/outprod.py:49-54 and
@@ -278,8 +278,8 @@ __global__ void __launch_bounds__(32, MINW) gsym_kernel(const int2 *__restrict__
                                                    double *__restrict__ part_k, int *status) {
     __shared__ double sacc[2 * SumFields<N>::size * 32];
     __shared__ double krow[ket_table<N>(1)];
-    __shared__ double kred[32];
-    __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::term : 2];
+    __shared__ double kred[ket_red<N>()];
+    __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::size : 2];
     const int t = blockIdx.x;
     if (t >= ntiles) return;
     fsym_tile<N, true, false, SKET, true, true>(t, tiles[t], LC, K, nst, cs, bra, ket, C, kmap, nullptr, nullptr,
@@ -304,8 +304,8 @@ __global__ void __launch_bounds__(32, MINW) fsym_kernel(const int2 *__restrict__
                                                    double *__restrict__ part_k, int *status) {
     __shared__ double sacc[2 * SumFields<N>::size * 32];
     __shared__ double krow[ket_table<N>(2)];
-    __shared__ double kred[64];
-    __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::term : 2];
+    __shared__ double kred[ket_red<N>()];
+    __shared__ __align__(16) double sket[SKET ? 2 * KetLayout<N>::size : 2];
     const int t = t_begin + blockIdx.x;
     if (t >= t_end) return;
     const int pc = blockIdx.y, PC = (nst + npc - 1) / npc;
@@ -339,10 +339,10 @@ __global__ void __launch_bounds__(256) hs_reduce_kernel(const double *__restrict
 // ends: a block barrier per term, which once kept the warps of a scheduler in
 // step, now only costs (LiH K = 1024 on a B200: 2.54 ms with it, 2.76 ms and more
 // with half of the warps taking it in mid-term, 2.34 ms without).  Shared
-// memory (dynamic, 16-byte aligned): per warp 2 PB 32 + ket table + 64 + 2 ket
+// memory (dynamic, 16-byte aligned): per warp 2 PB 32 + ket table + ket_red + 2 ket
 // records doubles, then the bras.  KE: the symmetric pass with E known.
 template <int N> __host__ __device__ constexpr int fsym_warp_smem() {
-    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + 64 + 2 * KetLayout<N>::term;
+    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + ket_red<N>() + 2 * KetLayout<N>::size;
 }
 template <int N> __host__ __device__ constexpr int fsym_block_smem_bytes(int warps) {
     return (warps * fsym_warp_smem<N>() + BraLayout<N>::term * 32) * 8;
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
     const int w = threadIdx.x >> 5;
     double *base = smem + w * PER_WARP;
     double *sbra = smem + WARPS * PER_WARP;  // after the warps' areas
-    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + 64};
+    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + ket_red<N>()};
     for (;;) {
         if (threadIdx.x == 0) gsh = atomicAdd(qcount, 1);
         __syncthreads();
@@ -770,7 +770,6 @@ __global__ void f0_kernel(const double *__restrict__ z, int count, double *__res
 template <int N> Consts<N> make_consts(const double *mass, const double *ncv, double efs) {
     Consts<N> c;
     for (int i = 0; i < N * N; ++i) c.M[i] = mass[i];
-    c.derive();
     for (int q = 1; q <= N; ++q)
         for (int p = 0; p < q; ++p) c.cv[vidx(p, q)] = 2.0 * ncv[p] * ncv[q] / NECG_SQRT_PI;
     for (int i = 0; i < N; ++i) c.q[i] = ncv[i + 1];
@@ -784,7 +783,7 @@ template <int N> struct Launch {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
         const int nbb = (a.K + 63) / 64, nbk = (a.K * a.nst + 63) / 64;
         prep_kernel<N><<<nbb + nbk, 64, 0, st>>>(a.iv, a.C, a.K, a.nst, nbb, cs, a.sml, a.sms, a.scvv, a.pinv,
-                                                 a.sms_general, a.full || a.kmap.fold, a.bra, a.ket, a.status, a.qcount);
+                                                 a.sms_general, a.bra, a.ket, a.status, a.qcount);
     }
     template <int MINW> static void energy_v(const LaunchArgs &a, cudaStream_t st) {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);

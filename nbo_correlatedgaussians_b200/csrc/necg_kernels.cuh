@@ -49,7 +49,7 @@ struct LaunchArgs {
     // units are [urange[kb].x, urange[kb].y)
     const int2 *urange;
     const int *tslot;                      // first xsym slot of each tile of a split tail group, else -1
-    int sms_general, full;                 // prep: general shift maps; whole ket records (else the terms' part)
+    int sms_general;                       // prep: general shift maps
 };
 
 // A tile group of the block variants: row block kb, first ket chunk lc0 and, for

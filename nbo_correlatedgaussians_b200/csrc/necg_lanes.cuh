@@ -100,11 +100,11 @@ template <int N> NECG_HD void prep_bra_one(const double *iv, int K, const Consts
 // Ket record of (l, P) = id / nst, id % nst: python/matel.py:76-87
 // (al <- sml^T al sml, st2 <- sms st2) plus the data the tiles reuse.  general =
 // false: the shift map is kron(m, I3), so that m alone is read (25 instead of 225
-// entries at n = 5).  full = false: only the `term` part of the record.
+// entries at n = 5).
 template <int N>
 NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Consts<N> &cs,
                           const double *sml, const double *sms, const double *scvv, double *ket,
-                          int id, const int *pinv = nullptr, bool general = true, bool full = true) {
+                          int id, const int *pinv = nullptr, bool general = true) {
     using KL = KetLayout<N>;
     constexpr int blk = tri(N) + 3 * N;
     const int l = id / nst, P = id - l * nst;
@@ -175,8 +175,6 @@ NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Cons
     o[KL::w] = scvv[P];
     o[KL::wC] = C ? 2.0 * scvv[P] * C[l] : 0.0;
     o[KL::winv] = pinv ? scvv[pinv[P]] : 0.0;
-    if (KL::term > KL::winv + 1) o[KL::winv + 1] = 0.0;
-    if (!full) return;
     double AM[N * N], AMA[tri(N)], tMA;
     mass_products<N>(Ap, cs.M, AM, AMA, tMA);
 #pragma unroll
@@ -184,7 +182,7 @@ NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Cons
 #pragma unroll
     for (int t = 0; t < tri(N); ++t) o[KL::Np8 + t] = -8.0 * AMA[t];
     o[KL::tMA] = tMA;
-    if (KL::size > KL::tMA + 1) o[KL::tMA + 1] = 0.0;
+    if (KL::size > KL::Sp + 3 * N) o[KL::Sp + 3 * N] = 0.0;
 }
 
 // Sums over the symmetry terms [p0, p1) of one pair: sum[0] = H, [1] = S, [2] =
@@ -380,10 +378,10 @@ NECG_HD bool grad_reduce_one(const double *part, int nlc, int K, const double *b
 // One matel term (python/matel.py:28-210): out = (ov, tk, ert, zht).
 template <int N, typename R, typename BA, typename KR>
 NECG_HD bool matel_one(const BA &b, const KR &kr, const Consts<N> &cs, double *out) {
-    R ov, tau, rho, sig;
-    const bool ok = term_energy<N>(b, kr, cs, ov, tau, rho, sig);
+    R ov, tau2, rho, sig;
+    const bool ok = term_value<N>(b, kr, cs, ov, tau2, rho, sig);
     out[0] = val(ov);
-    out[1] = val(2.0 * ov * tau);
+    out[1] = val(ov * tau2);
     out[2] = val(ov * rho);
     out[3] = val(ov * sig);
     return ok;

@@ -83,10 +83,9 @@ __host__ __device__ constexpr int sx(int i, int j) {
 #define NECG_PI 3.141592653589793
 #define NECG_SQRT_PI 1.7724538509055159
 
-// Ket record: one per (l, P), read warp-uniformly by the tile kernels.
-// The pair passes read the first `term` doubles (staged in shared memory by the
-// block variants); Sp is for the fold of a symmetry term whose shift map is not
-// that of its coordinate map, Np8 = -8 A_l' M A_l' and tMA for the energy path.
+// Ket record: one per (l, P), read warp-uniformly by the tile kernels (staged in
+// shared memory by the block variants).  Np8 = -8 A_l' M A_l', tMA = tr(M A_l') and Sp
+// are for the terms that write the kinetic part with the ket (term_value).
 template <int N> struct KetLayout {
     static constexpr int T = tri(N);
     static constexpr int Ap = 0;
@@ -96,11 +95,10 @@ template <int N> struct KetLayout {
     static constexpr int w = pre + 1;    // symmetry weight scvv[P]
     static constexpr int wC = w + 1;     // 2 scvv[P] C_l (gradient weight)
     static constexpr int winv = wC + 1;  // scvv[P^-1] (ket weight of the symmetric pass)
-    static constexpr int term = (winv + 1 + 1) & ~1;  // even: 16-byte multiples
-    static constexpr int Sp = term;
-    static constexpr int Np8 = Sp + 3 * N;
-    static constexpr int tMA = Np8 + T;  // tr(M A_l')
-    static constexpr int size = (tMA + 1 + 1) & ~1;  // even, 16-byte records
+    static constexpr int tMA = winv + 1;
+    static constexpr int Np8 = tMA + 1;
+    static constexpr int Sp = Np8 + T;
+    static constexpr int size = (Sp + 3 * N + 1) & ~1;  // even, 16-byte records
 };
 
 // Bra record: structure of arrays by row block, field f of lane j of block kb at
@@ -141,16 +139,10 @@ template <int N, typename P> __host__ __device__ __forceinline__ P *bra_at(P *br
 // Per-problem constants, passed to kernels by value (constant bank).
 template <int N> struct Consts {
     double M[N * N];    // inverse-mass tensor, row-major
-    double Mq[tri(N)];  // packed lower: M_ii on the diagonal, M_ik + M_ki below (quadratic forms in M)
     double cv[tri(N)];  // c_v for the n(n+1)/2 Coulomb pairs (p<q, q-major order)
     double q[N];        // ncv[1..n]
     double efs;
     double sqrt8n;      // sqrt(8^n)
-    // Mq from M
-    NECG_HD void derive() {
-        for (int i = 0; i < N; ++i)
-            for (int k = 0; k <= i; ++k) Mq[sx(i, k)] = i == k ? M[i * N + i] : M[i * N + k] + M[k * N + i];
-    }
 };
 
 // Doubles of one part's compact output for one tile of a split group of the
@@ -326,21 +318,6 @@ NECG_HD void symv3(const Acc &S, int off, const R (&x)[3 * N], R (&y)[3 * N]) {
     }
 }
 
-// y += S x for S symmetric (packed, read through an accessor) and x n x 3: the
-// products fuse into y's values
-#pragma nv_exec_check_disable
-template <int N, typename R, typename Acc>
-NECG_HD void symv3_acc(const Acc &S, int off, const R (&x)[3 * N], R (&y)[3 * N]) {
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            const R a = S[off + sx(i, k)];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) y[3 * i + c] += a * x[3 * k + c];
-        }
-}
-
 // Boys-function pieces for one Coulomb pair.  Given a = v^T Bi v and
 // bb = |v^T T|^2 (z = bb / a) returns fs = F0(z) a^{-1/2} and, when GRAD,
 // D2 = 2 F0'(z) / F0(z) (so 2 F0'(z) a^{-1/2} = fs D2) and ia = 1/a.  The Pade branch
@@ -505,55 +482,6 @@ NECG_HD bool term_core(const BA &b, const KA &kr, R (&Bi)[tri(N)], R (&T)[3 * N]
     return ok;
 }
 
-// tau = 3 tr(M X) - 2 <Y, M Y>.  tr(M X) with X = A_k Bi A_l' is written through
-// the matrix with the smaller tr(M A): X = A_s - A_s Bi A_s, which keeps the
-// subtraction free of cancellation.  The choice differs from lane to lane, so
-// both N_s are read and one is selected (no divergent branch).  Y = A_l' (T - S_l').
-#pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA>
-NECG_HD R term_tau(const BA &b, const KA &kr, const Consts<N> &cs, const R (&Bi)[tri(N)],
-                   const R (&T)[3 * N]) {
-    using KL = KetLayout<N>;
-    using BL = BraLayout<N>;
-    R tMX;
-    {
-        const R tl = kr[KL::tMA], tk = b(BL::tMA);
-        const bool use_l = tl <= tk;
-        // -8 tr(Bi N_s): the diagonal and the off-diagonal products summed apart
-        R dg = R(0.0), od = R(0.0);
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-            for (int j = 0; j <= i; ++j) {
-                const R nl = kr[KL::Np8 + sx(i, j)], nk = b(BL::N8 + sx(i, j));
-                const R v = Bi[sx(i, j)] * (use_l ? nl : nk);
-                if (i == j)
-                    dg = (i == 0) ? v : dg + v;
-                else
-                    od = (i == 1) ? v : od + v;
-            }
-        tMX = (use_l ? tl : tk) + 0.125 * (dg + 2.0 * od);
-    }
-    R yMy = R(0.0);
-    {
-        R Y[3 * N];
-        // Y = A_l' (T - S_l') = A_l' T - A_l' S_l', the second product from the ket record
-#pragma unroll
-        for (int t = 0; t < 3 * N; ++t) Y[t] = -kr[KL::ASp + t];
-        symv3_acc<N>(kr, KL::Ap, T, Y);
-        // <Y, M Y> = sum_c sum_i Y_ic (M_ii Y_ic + sum_{k<i} (M_ik + M_ki) Y_kc)
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                R s = cs.Mq[sx(i, i)] * Y[3 * i + c];
-#pragma unroll
-                for (int k = 0; k < i; ++k) s += cs.Mq[sx(i, k)] * Y[3 * k + c];
-                yMy += Y[3 * i + c] * s;
-            }
-    }
-    return 3.0 * tMX - 2.0 * yMy;
-}
 #pragma nv_exec_check_disable
 template <int N, typename R>
 NECG_HD R term_sig(const Consts<N> &cs, const R (&T)[3 * N]) {
@@ -589,21 +517,31 @@ NECG_HD R coulomb_sum(const R (&Bi)[tri(N)], const R (&T)[3 * N], const Consts<N
     return r;
 }
 
-// The matrix passes' value of one term: ov, 2 tau, rho and sig, with tau written
-// with the bra's N and D = T - S_k (as in term_raw: 4 tau = 12 tr(M A_k) +
-// <-8 N, 1.5 Bi + D D^T>), which needs neither the ket's N and S nor a choice
-// between the two.  Returns false if B is not positive definite.
+// The value of one term: ov, 2 tau, rho and sig.  tau = 3 tr(M X) - 2 <A_s D_s, M
+// A_s D_s> with X = A_k Bi A_l' = A_s - A_s Bi A_s, of either side s (D_s = T - S_s, and
+// A_k D_k = -A_l' D_l).  Both subtractions cancel for the tighter side (X and T - S
+// are small there against A and S, by the ratio of the exponents), so each lane
+// takes the side with the smaller tr(M A): 4 tau = 12 tr(M A_s) + <-8 N_s, 1.5 Bi +
+// D_s D_s^T>.  Both sides' N and S are read and one is selected (no divergent branch,
+// no FP64 operation more than with a fixed side).  Returns false if B is not
+// positive definite.
 #pragma nv_exec_check_disable
 template <int N, typename R, typename BA, typename KA>
 NECG_HD bool term_value(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R &tau2, R &rho, R &sig) {
     using BL = BraLayout<N>;
+    using KL = KetLayout<N>;
     R Bi[tri(N)], T[3 * N];
     const bool ok = term_core<N>(b, kr, Bi, T, ov);
     sig = term_sig<N>(cs, T);
     rho = coulomb_sum<N>(Bi, T, cs);
+    const R tl = kr[KL::tMA], tk = b(BL::tMA);
+    const bool use_l = tl <= tk;
     R dg = R(0.0), od = R(0.0);
 #pragma unroll
-    for (int t = 0; t < 3 * N; ++t) T[t] -= b(BL::S + t);
+    for (int t = 0; t < 3 * N; ++t) {
+        const R sl = kr[KL::Sp + t], sk = b(BL::S + t);
+        T[t] -= use_l ? sl : sk;
+    }
 #pragma unroll
     for (int i = 0; i < N; ++i)
 #pragma unroll
@@ -611,27 +549,14 @@ NECG_HD bool term_value(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R
             R u = 1.5 * Bi[sx(i, j)];
 #pragma unroll
             for (int c = 0; c < 3; ++c) u += T[3 * i + c] * T[3 * j + c];
-            const R a = b(BL::N8 + sx(i, j));
+            const R nl = kr[KL::Np8 + sx(i, j)], nk = b(BL::N8 + sx(i, j));
+            const R a = use_l ? nl : nk;
             if (i == j)
                 dg = (i == 0) ? a * u : dg + a * u;
             else
                 od = (i == 1) ? a * u : od + a * u;
         }
-    tau2 = 6.0 * b(BL::tMA) + (0.5 * dg + od);
-    return ok;
-}
-
-// Energy part of a single element (the matel API): returns false if B is not
-// positive definite.  tau through the smaller of the two traces (term_tau).
-#pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA>
-NECG_HD bool term_energy(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R &tau, R &rho,
-                         R &sig) {
-    R Bi[tri(N)], T[3 * N];
-    const bool ok = term_core<N>(b, kr, Bi, T, ov);
-    tau = term_tau<N>(b, kr, cs, Bi, T);
-    sig = term_sig<N>(cs, T);
-    rho = coulomb_sum<N>(Bi, T, cs);
+    tau2 = 6.0 * (use_l ? tl : tk) + (0.5 * dg + od);
     return ok;
 }
 
@@ -710,6 +635,7 @@ template <int N> struct RawPairs {
 template <int N, typename R, typename BA, typename KA, typename OUT>
 NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT &out, R &eta2_out, R &ov_out) {
     using BL = BraLayout<N>;
+    using KL = KetLayout<N>;
     using RP = RawPairs<N>;
     constexpr int TR = tri(N), V = 3 * N;
     R Bi[TR], T[V], ov;
@@ -734,24 +660,30 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
     });
     if constexpr (RP::odd) out.template s2<RP::count - 1>(T[V - 1], R(1.0));
     // tau and the bra's part of Q's right-hand side: V8 = -8 N D, D = T - S_k;
-    // 4 tau = 12 tr(M A_k) + 1.5 <-8 N, Bi> + <D, V8>
+    // 4 tau = 12 tr(M A_s) + 1.5 <-8 N_s, Bi> + <D, V8>.  The trace cancels for the
+    // tighter side (term_value), so it is formed with both and the one of the
+    // smaller tr(M A) taken: tri(N) products more, where selecting N_s would take
+    // twice as many instructions.
     R Z[V], W[TR], eta2;
     {
         R D[V];
 #pragma unroll
         for (int t = 0; t < V; ++t) D[t] = T[t] - b(BL::S + t);
-        R dg = R(0.0), od = R(0.0);
+        R dg = R(0.0), od = R(0.0), dl = R(0.0), ol = R(0.0);
 #pragma unroll
         for (int i = 0; i < N; ++i)
 #pragma unroll
             for (int k = 0; k <= i; ++k) {
                 // each element of N is read once and used for the three columns
-                const R a = b(BL::N8 + sx(i, k));
+                const R a = b(BL::N8 + sx(i, k)), al = kr[KL::Np8 + sx(i, k)];
                 W[sx(i, k)] = -1.5 * a;
-                if (i == k)
+                if (i == k) {
                     dg = (i == 0) ? a * Bi[0] : dg + a * Bi[sx(i, k)];
-                else
+                    dl = (i == 0) ? al * Bi[0] : dl + al * Bi[sx(i, k)];
+                } else {
                     od = (i == 1) ? a * Bi[sx(1, 0)] : od + a * Bi[sx(i, k)];
+                    ol = (i == 1) ? al * Bi[sx(1, 0)] : ol + al * Bi[sx(i, k)];
+                }
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     // element (i, k) is the first of row i when k = 0, and the first of row k when i = k = 0
@@ -769,7 +701,9 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
             e1 += D[3 * i + 1] * Z[3 * i + 1];
             e2 += D[3 * i + 2] * Z[3 * i + 2];
         }
-        eta2 = 12.0 * b(BL::tMA) + (1.5 * (dg + 2.0 * od) + (e0 + e1 + e2));
+        const R tl = kr[KL::tMA], tk = b(BL::tMA);
+        const R xk = 8.0 * tk + (dg + 2.0 * od), xl = 8.0 * tl + (dl + 2.0 * ol);  // 8 tr(M X), of either side
+        eta2 = 1.5 * (tl <= tk ? xl : xk) + (e0 + e1 + e2);
     }
     {
         R sg = R(0.0);

@@ -1,0 +1,84 @@
+"""Accuracy where functions of very different widths meet, element by element,
+against extended precision (tests/extended.py)."""
+import numpy as np
+import pytest
+
+from _util import TOL_ELEM
+from extended import Extended
+from nbo_correlatedgaussians_b200 import synth
+
+SYSTEMS = {"He": (2, 1), "H2": (3, 1), "LiH": (5, 1)}
+
+
+def two_widths(system, K, r, seed=0):
+    """Functions whose L is r times as large for every other one (tight and diffuse in
+    both orders), shifts of about 0.3 widths, so that exp(-s A s) is harmless."""
+    p = synth.make_problem(system, K, 900 + seed)
+    rng = np.random.default_rng([seed, K])
+    n, tri = p.n, p.n * (p.n + 1) // 2
+    b = p.iv.reshape(K, -1)
+    for k in range(K):
+        scale = r if k % 4 in (1, 2) else 1.0
+        L = np.tril(rng.normal(0.0, 0.1, (n, n)))
+        L[np.diag_indices(n)] = rng.uniform(0.7, 1.4, n)
+        b[k, :tri] = scale * np.concatenate([L[j:, j] for j in range(n)])
+        b[k, tri:] = rng.normal(0.0, 0.3 / scale, 3 * n)
+    p.iv, p.C = b.reshape(-1), rng.normal(size=K)
+    return p
+
+
+def check_elements(got, ref, scale, what):
+    """Every element within the suite's bound for elements, against the sum of its terms."""
+    got = np.asarray(got, dtype=np.float64)
+    rel = np.abs(got.astype(np.longdouble) - ref) / np.maximum(scale, np.finfo(np.float64).tiny)
+    assert rel.max() <= TOL_ELEM, (what, float(rel.max()), np.unravel_index(int(rel.argmax()), rel.shape))
+
+
+RATIOS = [1.0, 10.0, 100.0, 1000.0, 1e4]
+
+
+@pytest.mark.parametrize("system", list(SYSTEMS))
+@pytest.mark.parametrize("r", RATIOS)
+def test_elements_between_tight_and_diffuse_functions(system, r):
+    """H of the separate and of the fused pass, and matel, on the host emulation."""
+    from emu import emu
+    p = two_widths(system, 8, r)
+    ref = Extended(p).evaluate()
+    rc, _, _, H, _ = emu.outprod(p)
+    assert rc == 0
+    check_elements(H, ref["H"], ref["aH"], "separate passes")
+    rc, _, _, H, S = emu.outprod_fused(p, 2)
+    assert rc == 0
+    check_elements(H, ref["H"], ref["aH"], "fused pass")
+    terms = [(1 + (i + j) % p.nst, i, j) for i in range(1, 9) for j in range(1, 9)]
+    rc, mat, _, _ = emu.elements(p, terms)
+    m = Extended(p).terms(terms)[0]
+    assert rc == 0
+    check_elements(mat[:, 1], m[:, 1], np.abs(m[:, 1]), "matel kinetic")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("system", list(SYSTEMS))
+@pytest.mark.parametrize("r", RATIOS)
+@pytest.mark.parametrize("K", [8, 40])
+def test_matrices_between_tight_and_diffuse_functions(system, r, K):
+    """Kinetic and H of build_matrices and of necg_matel, and H of the fused pass."""
+    import torch
+    from nbo_correlatedgaussians_b200.engine import Engine
+    p = two_widths(system, K, r)
+    ref = Extended(p).evaluate()
+    eng = Engine(p)
+    for lc in (1, 16):
+        eng.set_tiles(lc, 4)
+        H, S, Kin, Pot, _ = eng.build_matrices(p.iv, p.C)
+        check_elements(Kin.cpu().numpy(), ref["T"], ref["aT"], "kinetic")
+        check_elements(H.cpu().numpy(), ref["H"], ref["aH"], "H")
+    x = torch.from_numpy(p.x).to(eng.device)
+    H, S = (torch.zeros((K, K), dtype=torch.float64, device=eng.device) for _ in range(2))
+    for mode, lc, minw in ((0, 4, 8), (2, 2, 118), (2, 2, 12), (2, 2, 248)):
+        assert eng.L.necg_set_symmetric(eng.h, mode, lc, minw) == 0
+        eng.outprod_device(x, K, H=H, S=S)
+        check_elements(H.cpu().numpy(), ref["H"], ref["aH"], ("outprod", mode, minw))
+    terms = [(1 + (i + j) % p.nst, i, j) for i in range(1, 9) for j in range(1, 9)]
+    m = Extended(p).terms(terms)[0]
+    check_elements(eng.matel(p.iv, terms)[:, 1], m[:, 1], np.abs(m[:, 1]), "matel")
