@@ -393,8 +393,8 @@ template <int N, typename R, typename BA, typename KR>
 NECG_HD bool gradel_one(const BA &b, const KR &kr, const Consts<N> &cs, const double (&L)[tri(N)],
                         bool diag, double *tgvl, double *tgvls) {
     constexpr int PS = Part<N>::size;
-    R bH[PS], bS[PS], h, ov;
-    const bool ok = term_gradients<N, false>(b, kr, cs, bH, bS, bH, bS, h, ov);
+    R bH[PS], bS[PS];
+    const bool ok = term_grad<N>(b, kr, cs, bH, bS);
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
         const R(&v)[PS] = which == 0 ? bH : bS;

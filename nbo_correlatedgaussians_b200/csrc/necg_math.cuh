@@ -517,30 +517,25 @@ NECG_HD R coulomb_sum(const R (&Bi)[tri(N)], const R (&T)[3 * N], const Consts<N
     return r;
 }
 
-// The value of one term: ov, 2 tau, rho and sig.  tau = 3 tr(M X) - 2 <A_s D_s, M
+// 2 tau of one term, tau = 3 tr(M X) - 2 <A_s D_s, M
 // A_s D_s> with X = A_k Bi A_l' = A_s - A_s Bi A_s, of either side s (D_s = T - S_s, and
 // A_k D_k = -A_l' D_l).  Both subtractions cancel for the tighter side (X and T - S
 // are small there against A and S, by the ratio of the exponents), so each lane
 // takes the side with the smaller tr(M A): 4 tau = 12 tr(M A_s) + <-8 N_s, 1.5 Bi +
 // D_s D_s^T>.  Both sides' N and S are read and one is selected (no divergent branch,
-// no FP64 operation more than with a fixed side).  Returns false if B is not
-// positive definite.
+// no FP64 operation more than with a fixed side).
 #pragma nv_exec_check_disable
 template <int N, typename R, typename BA, typename KA>
-NECG_HD bool term_value(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R &tau2, R &rho, R &sig) {
+NECG_HD R term_tau2(const BA &b, const KA &kr, const R (&Bi)[tri(N)], const R (&T)[3 * N]) {
     using BL = BraLayout<N>;
     using KL = KetLayout<N>;
-    R Bi[tri(N)], T[3 * N];
-    const bool ok = term_core<N>(b, kr, Bi, T, ov);
-    sig = term_sig<N>(cs, T);
-    rho = coulomb_sum<N>(Bi, T, cs);
     const R tl = kr[KL::tMA], tk = b(BL::tMA);
     const bool use_l = tl <= tk;
-    R dg = R(0.0), od = R(0.0);
+    R D[3 * N], dg = R(0.0), od = R(0.0);
 #pragma unroll
     for (int t = 0; t < 3 * N; ++t) {
         const R sl = kr[KL::Sp + t], sk = b(BL::S + t);
-        T[t] -= use_l ? sl : sk;
+        D[t] = T[t] - (use_l ? sl : sk);
     }
 #pragma unroll
     for (int i = 0; i < N; ++i)
@@ -548,7 +543,7 @@ NECG_HD bool term_value(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R
         for (int j = 0; j <= i; ++j) {
             R u = 1.5 * Bi[sx(i, j)];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) u += T[3 * i + c] * T[3 * j + c];
+            for (int c = 0; c < 3; ++c) u += D[3 * i + c] * D[3 * j + c];
             const R nl = kr[KL::Np8 + sx(i, j)], nk = b(BL::N8 + sx(i, j));
             const R a = use_l ? nl : nk;
             if (i == j)
@@ -556,7 +551,135 @@ NECG_HD bool term_value(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R
             else
                 od = (i == 1) ? a * u : od + a * u;
         }
-    tau2 = 6.0 * (use_l ? tl : tk) + (0.5 * dg + od);
+    return 6.0 * (use_l ? tl : tk) + (0.5 * dg + od);
+}
+
+// The value of one term: ov, 2 tau, rho and sig; false if B is not positive definite.
+#pragma nv_exec_check_disable
+template <int N, typename R, typename BA, typename KA>
+NECG_HD bool term_value(const BA &b, const KA &kr, const Consts<N> &cs, R &ov, R &tau2, R &rho, R &sig) {
+    R Bi[tri(N)], T[3 * N];
+    const bool ok = term_core<N>(b, kr, Bi, T, ov);
+    sig = term_sig<N>(cs, T);
+    rho = coulomb_sum<N>(Bi, T, cs);
+    tau2 = term_tau2<N>(b, kr, Bi, T);
+    return ok;
+}
+
+// The bra gradient of one term's h and ov (Part<N> fields: dF/dA_k packed without
+// its A_k^-1 part, that part's coefficient, dF/ds_k), in the direct formulation:
+//   dh/dA_k = ov (-eta (1.5 Bi + D_k D_k^T) + Bi (6 N_l' + W) Bi + Q D_k^T + D_k Q^T
+//                 + 0.75 eta A_k^-1),  dh/ds_k = 2 ov (A_k Q - eta Y),
+//   D_k = S_k - T,  Y = A_k D_k = A_l' (T - S_l'),  Q = Bi (Z' - 4 A_l' M Y),
+// and the same of ov with eta = 1 and without W, N_l' and Q.  The other side's N_l'
+// stands where the sums' form (term_raw) has 6 M - 6 (M A_k Bi + Bi A_k M) + 6 Bi N_k Bi,
+// which cancels when the bra is the tighter function; sums over a basis have that
+// function's own term beside it, single elements do not.  Y is formed with the
+// looser side, whose difference of positions does not cancel.
+#pragma nv_exec_check_disable
+template <int N, typename R, typename BA, typename KA>
+NECG_HD bool term_grad(const BA &b, const KA &kr, const Consts<N> &cs, R (&gH)[tri(N) + 1 + 3 * N],
+                       R (&gS)[tri(N) + 1 + 3 * N]) {
+    using BL = BraLayout<N>;
+    using KL = KetLayout<N>;
+    constexpr int TR = tri(N);
+    R Bi[TR], T[3 * N], ov;
+    const bool ok = term_core<N>(b, kr, Bi, T, ov);
+    R Z[3 * N], W[TR];  // 2 Z', 2 W
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) Z[t] = R(0.0);
+#pragma unroll
+    for (int t = 0; t < TR; ++t) W[t] = R(0.0);
+    const R rho = coulomb_grad<N>(Bi, T, cs, Z, W);
+    const R eta = term_tau2<N>(b, kr, Bi, T) + rho - term_sig<N>(cs, T);
+    const bool use_l = kr[KL::tMA] <= b(BL::tMA);
+    R Y[3 * N], p[3 * N];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R yk = R(0.0), yl = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                yk += b(BL::A + sx(i, k)) * (b(BL::S + 3 * k + c) - T[3 * k + c]);
+                yl += kr[KL::Ap + sx(i, k)] * (T[3 * k + c] - kr[KL::Sp + 3 * k + c]);
+            }
+            Y[3 * i + c] = use_l ? yl : yk;
+        }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) v += cs.M[i * N + k] * Y[3 * k + c];
+            p[3 * i + c] = v;  // M Y
+        }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        Z[3 * i + 2] -= cs.efs * cs.q[i];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) v += kr[KL::Ap + sx(i, k)] * p[3 * k + c];
+            Z[3 * i + c] -= 8.0 * v;
+        }
+    }
+    R Q[3 * N];  // 2 Q
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) v += Bi[sx(i, k)] * Z[3 * k + c];
+            Q[3 * i + c] = v;
+        }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) v += b(BL::A + sx(i, k)) * Q[3 * k + c];
+            const R y = 2.0 * (ov * Y[3 * i + c]);
+            gH[TR + 1 + 3 * i + c] = ov * v - eta * y;
+            gS[TR + 1 + 3 * i + c] = -y;
+        }
+#pragma unroll
+    for (int t = 0; t < TR; ++t) W[t] = 0.5 * W[t] - 0.75 * kr[KL::Np8 + t];  // W + 6 N_l'
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) {
+        T[t] = b(BL::S + t) - T[t];  // D_k
+        Q[t] *= 0.5;
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        R col[N];  // column j of (W + 6 N_l') Bi
+#pragma unroll
+        for (int a = 0; a < N; ++a) {
+            R v = W[sx(a, 0)] * Bi[sx(0, j)];
+#pragma unroll
+            for (int k = 1; k < N; ++k) v += W[sx(a, k)] * Bi[sx(k, j)];
+            col[a] = v;
+        }
+#pragma unroll
+        for (int i = j; i < N; ++i) {
+            R v = R(0.0), u = 1.5 * Bi[sx(i, j)];
+#pragma unroll
+            for (int a = 0; a < N; ++a) v += Bi[sx(i, a)] * col[a];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                v += Q[3 * i + c] * T[3 * j + c] + T[3 * i + c] * Q[3 * j + c];
+                u += T[3 * i + c] * T[3 * j + c];
+            }
+            gH[sx(i, j)] = ov * (v - eta * u);
+            gS[sx(i, j)] = -(ov * u);
+        }
+    }
+    gH[TR] = 0.75 * (ov * eta);
+    gS[TR] = 0.75 * ov;
     return ok;
 }
 

@@ -82,3 +82,33 @@ def test_matrices_between_tight_and_diffuse_functions(system, r, K):
     terms = [(1 + (i + j) % p.nst, i, j) for i in range(1, 9) for j in range(1, 9)]
     m = Extended(p).terms(terms)[0]
     check_elements(eng.matel(p.iv, terms)[:, 1], m[:, 1], np.abs(m[:, 1]), "matel")
+
+
+def check_gradel(p, tg, terms):
+    """The L block of every term's dh against its own largest component."""
+    ref = Extended(p).terms(terms)[1][:, :p.svh]
+    err = np.abs(np.asarray(tg)[:, :p.svh] - ref).max(1) / np.abs(ref).max(1)
+    assert err.max() <= TOL_ELEM, (float(err.max()), terms[int(err.argmax())])
+
+
+def all_terms(p, K):
+    return [(1 + (i + j) % p.nst, i, j) for i in range(1, K + 1) for j in range(1, K + 1)]
+
+
+@pytest.mark.parametrize("system", list(SYSTEMS))
+@pytest.mark.parametrize("r", RATIOS)
+def test_gradel_between_tight_and_diffuse_functions(system, r):
+    from emu import emu
+    p = two_widths(system, 8, r)
+    rc, _, tg, _ = emu.elements(p, all_terms(p, 8))
+    assert rc == 0
+    check_gradel(p, tg, all_terms(p, 8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("system", list(SYSTEMS))
+@pytest.mark.parametrize("r", RATIOS)
+def test_device_gradel_between_tight_and_diffuse_functions(system, r):
+    from nbo_correlatedgaussians_b200.engine import Engine
+    p = two_widths(system, 8, r)
+    check_gradel(p, Engine(p).gradel(p.iv, all_terms(p, 8))[0], all_terms(p, 8))
