@@ -682,14 +682,14 @@ int necg_batch_plan(necg_batch *b, int count, necg_handle *const *hs, const int 
             d.lc_s = h->lc_s;
             d.nstiles = h->nstiles;
             d.pinv = h->d_pinv;
-            d.stile_start = h->d_stile_start;
+            d.stile_start = h->lists.start;
             d.psym = h->d_psym;
             d.kmap = RawMap{h->d_kcnt, h->d_ksrc, h->d_kcoef, h->kmaxnz, h->kfold};
-            d.stiles = h->d_stiles;
-            d.bgroups = h->d_bgroups;
+            d.stiles = h->lists.tiles;
+            d.bgroups = h->lists.bgroups;
             d.nbgroups = h->nbgroups;
             d.npc = 1;  // set below for the one-warp kernel
-            d.burange = h->d_burange;
+            d.burange = h->lists.burange;
         }
         d.general = h->sms_general ? 1 : 0;
         const int ps = tri(n) + 1 + 3 * n;

@@ -139,198 +139,106 @@ void free_all(necg_handle *h) {
         if (e) cudaEventDestroy(e);
     void *ptrs[] = {h->d_sml, h->d_sms, h->d_scvv, h->d_bra, h->d_ket, h->d_part, h->d_H,
                     h->d_S, h->d_rows, h->d_scal, h->d_x, h->d_out,
-                    h->d_tiles, h->d_pinv, h->d_kcnt, h->d_ksrc, h->d_kcoef, h->d_stiles,
-                    h->d_stile_start, h->d_psym, h->d_sgroups, h->d_qcount, h->d_bgroups,
-                    h->d_Hp, h->d_Sp, h->d_xsym, h->d_urange, h->d_dipcls, h->d_tslot, h->d_burange};
+                    h->d_tiles, h->d_pinv, h->d_kcnt, h->d_ksrc, h->d_kcoef, h->d_lists,
+                    h->d_psym, h->d_qcount, h->d_Hp, h->d_Sp, h->d_xsym, h->d_dipcls};
     for (void *p : ptrs) pool_free(h, p);
+}
+
+// Lists and buffers change only outside a stream capture (their allocations would
+// belong to the captured graph, and the lists would not be there before a replay).
+int not_capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cap));
+    return cap == cudaStreamCaptureStatusNone ? NECG_OK : NECG_ERR_CUDA;
 }
 
 // Energy tiles over the lower triangle: (kb, lc) with lc * LC <= row_last(K, kb).
 int ensure_tiles(necg_handle *h, int K, cudaStream_t st) {
     if (h->tiles_K == K && h->tiles_lc == h->lc_e) return NECG_OK;
-    std::vector<int2> t;
-    const int nkb = (K + 31) / 32;
-    for (int kb = 0; kb < nkb; ++kb) {
-        for (int lc = 0; lc * h->lc_e <= necg::row_last(K, kb); ++lc) t.push_back(make_int2(kb, lc));
-    }
-    if ((int)t.size() > h->tiles_cap) {
+    int rc = not_capturing(st);
+    if (rc) return rc;
+    const int nt = necg::tiles_before(K, h->lc_e, necg::row_blocks(K));
+    h->tiles_K = -1;
+    if (nt > h->tiles_cap) {
         pool_free(h, h->d_tiles, st);
         h->d_tiles = nullptr;
-        CK(pool_alloc(h, &h->d_tiles, t.size() * sizeof(int2), st));
-        h->tiles_cap = (int)t.size();
+        h->tiles_cap = 0;
+        CK(pool_alloc(h, &h->d_tiles, (size_t)nt * sizeof(int2), st));
+        h->tiles_cap = nt;
     }
-    CK(cudaMemcpyAsync(h->d_tiles, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
-    CK(cudaStreamSynchronize(st));
+    necg::launch_tile_list(h->d_tiles, K, h->lc_e, st);
+    CK(cudaGetLastError());
     h->tiles_K = K;
     ++h->gversion;  // buffers and lists a captured graph may hold changed
     h->tiles_lc = h->lc_e;
-    h->ntiles = (int)t.size();
+    h->ntiles = nt;
     return NECG_OK;
 }
 
-// Lower-triangle tiles of chunk LC for the symmetric pass, plus the first tile
-// of each 32-row block; the partial buffer grows here if this K and LC need more.
-// The fused pass with npc splits needs npc partial slots per tile and npc K x K
-// buffers for H and S.
+// Grow one of the handle's double buffers to `need`.
+int grow(necg_handle *h, double **p, size_t *cap, size_t need, cudaStream_t st) {
+    if (need <= *cap) return NECG_OK;
+    pool_free(h, *p, st);
+    *p = nullptr;
+    h->ws_bytes -= (long long)(*cap * sizeof(double));
+    *cap = 0;
+    ++h->gversion;
+    CK(pool_alloc(h, p, need * sizeof(double), st));
+    h->ws_bytes += (long long)(need * sizeof(double));
+    *cap = need;
+    return NECG_OK;
+}
+
+// Lower-triangle tiles of chunk LC for the symmetric passes and the queue of the
+// block variants (necg_tiles.h); the partial buffers grow here if this K and LC need
+// more.  The fused pass with npc splits needs npc partial slots per tile and npc
+// K x K buffers for H and S.
 int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
-    const int PB = necg::part_stride(h->n) + 1;
+    const int PB = necg::part_stride(h->n) + 1, LC = h->lc_s;
     const int gw = necg::fused_block_warps(h->minb_s);  // tiles per group of the block variants
     const int npc = fused ? necg::fused_splits(h) : 1;
     const size_t hp_need = npc > 1 ? (size_t)npc * K * K : 0;
-    if (hp_need > h->hp_cap) {
-        pool_free(h, h->d_Hp, st);
-        pool_free(h, h->d_Sp, st);
-        h->d_Hp = h->d_Sp = nullptr;
-        h->hp_cap = 0;
-        CK(pool_alloc(h, &h->d_Hp, hp_need * sizeof(double), st));
-        CK(pool_alloc(h, &h->d_Sp, hp_need * sizeof(double), st));
-        ++h->gversion;
-        h->ws_bytes += (long long)(2 * hp_need * sizeof(double));
-        h->hp_cap = hp_need;
-    }
-    if (h->stiles_K == K && h->stiles_lc == h->lc_s && h->sgroups_w == gw &&
-        (size_t)h->nstiles * PB * (32 + h->lc_s) * 2 * npc <= h->psym_cap)
-        return NECG_OK;
-    std::vector<int2> t;
-    std::vector<int> start;
-    const int nkb = (K + 31) / 32, LC = h->lc_s;
-    for (int kb = 0; kb < nkb; ++kb) {
-        start.push_back((int)t.size());
-        for (int lc = 0; lc <= necg::row_last(K, kb) / LC; ++lc) t.push_back(make_int2(kb, lc));
-    }
-    start.push_back((int)t.size());
-    if ((int)t.size() > h->stiles_cap) {
-        pool_free(h, h->d_stiles, st);
-        h->d_stiles = nullptr;
-        CK(pool_alloc(h, &h->d_stiles, t.size() * sizeof(int2), st));
-        h->stiles_cap = (int)t.size();
-    }
-    if (!h->d_stile_start) CK(pool_alloc(h, &h->d_stile_start, ((h->K_max + 31) / 32 + 2) * sizeof(int), st));
-    const size_t need = t.size() * (size_t)PB * (32 + LC) * 2 * npc;
-    if (need > h->psym_cap) {
-        pool_free(h, h->d_psym, st);
-        h->d_psym = nullptr;
-        CK(pool_alloc(h, &h->d_psym, need * sizeof(double), st));
-        h->ws_bytes += (long long)((need - h->psym_cap) * sizeof(double));
-        h->psym_cap = need;
-    }
-    std::vector<int2> groups;  // gw consecutive ket chunks of one row block, largest blocks first
-    for (int kb = nkb - 1; kb >= 0; --kb) {
-        const int ntk = start[kb + 1] - start[kb];
-        for (int lc0 = 0; lc0 < ntk; lc0 += gw) groups.push_back(necg::sgroup_pack(kb, lc0, 0, 1));
-    }
-    // The groups are equal work, one block per SM takes them from the queue, so
-    // the last round runs G mod SMs groups while the other SMs idle: split each
-    // of those groups into `parts` units over the symmetry terms (as many as
-    // keep the round within one unit per SM, at most 8; the kernel gives the
-    // parts balanced ranges of terms), so the last round is a part of a group
-    // long.
-    {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-        const int G = (int)groups.size();
-        const int T = G % sms;
-        int parts = T > 0 ? sms / T : 1;
-        if (parts > 8) parts = 8;
-        if (parts > h->nst) parts = h->nst;
-        // the block variants write bra partials per queue unit into the slots
-        // sized for the tiles: G - T + T parts units must not exceed them
-        if (T > 0 && parts > 1 + ((int)t.size() - G) / T) parts = 1 + ((int)t.size() - G) / T;
-        h->sg_ntail = 0;
-        h->sg_parts = 1;
-        h->sg_tail0 = G;
-        if (parts >= 2) {
-            std::vector<int2> tail(groups.end() - T, groups.end());
-            groups.resize(G - T);
-            for (const int2 &g : tail)
-                for (int q = 0; q < parts; ++q)
-                    groups.push_back(necg::sgroup_pack(g.x, necg::sgroup_lc0(g), q, parts));
-            h->sg_tail0 = G - T;
-            h->sg_ntail = T;
-            h->sg_parts = parts;
-            const size_t xneed = (size_t)T * gw * (parts - 1) * necg::fsym_tail_slot(PB, LC);
-            if (xneed > h->xsym_cap) {
-                pool_free(h, h->d_xsym, st);
-                h->d_xsym = nullptr;
-                h->xsym_cap = 0;
-                CK(pool_alloc(h, &h->d_xsym, xneed * sizeof(double), st));
-                h->ws_bytes += (long long)(xneed * sizeof(double));
-                h->xsym_cap = xneed;
-            }
-        }
-    }
-    if ((int)groups.size() > h->sgroups_cap) {
-        pool_free(h, h->d_sgroups, st);
-        h->d_sgroups = nullptr;
-        CK(pool_alloc(h, &h->d_sgroups, groups.size() * sizeof(int2), st));
-        h->sgroups_cap = (int)groups.size();
+    const bool same = h->stiles_K == K && h->stiles_lc == LC && h->sgroups_w == gw;
+    if (same && hp_need <= h->hp_cap && (size_t)h->nstiles * PB * (32 + LC) * 2 * npc <= h->psym_cap) return NECG_OK;
+    int rc = not_capturing(st);
+    if (rc) return rc;
+    size_t cap = h->hp_cap;
+    if ((rc = grow(h, &h->d_Hp, &cap, hp_need, st)) || (rc = grow(h, &h->d_Sp, &h->hp_cap, hp_need, st))) return rc;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+    const necg::SymQueue q = necg::sym_queue(K, LC, gw, h->nst, sms);
+    if ((rc = grow(h, &h->d_psym, &h->psym_cap, (size_t)q.ntiles * PB * (32 + LC) * 2 * npc, st))) return rc;
+    if (q.ntail && (rc = grow(h, &h->d_xsym, &h->xsym_cap, (size_t)q.ntail * gw * (q.parts - 1) * necg::fsym_tail_slot(PB, LC), st))) return rc;
+    if (same) return NECG_OK;
+    // one buffer for all lists: the int2 lists, then the int lists
+    const int nkb = necg::row_blocks(K), nb = necg::groups_before(K, LC, 8, -1), nu = q.units();
+    const size_t n2 = (size_t)q.ntiles + nu + nb + 2 * nkb, need = n2 + (q.ntiles + nkb + 1 + 1) / 2;
+    h->stiles_K = -1;
+    if (need > h->lists_cap) {
+        pool_free(h, h->d_lists, st);
+        h->d_lists = nullptr;
+        h->lists_cap = 0;
+        CK(pool_alloc(h, &h->d_lists, need * sizeof(int2), st));
+        h->lists_cap = need;
     }
     if (!h->d_qcount) CK(pool_alloc(h, &h->d_qcount, sizeof(int), st));
-    // each row block's queue units are contiguous (blocks in decreasing order,
-    // a split group's parts next to each other)
-    std::vector<int2> urange(nkb, make_int2(0, 0));
-    for (int u = 0; u < (int)groups.size(); ++u) {
-        int2 &r = urange[groups[u].x];
-        if (r.y == 0) r.x = u;
-        r.y = u + 1;
-    }
-    if (nkb > h->urange_cap) {
-        pool_free(h, h->d_urange, st);
-        h->d_urange = nullptr;
-        CK(pool_alloc(h, &h->d_urange, nkb * sizeof(int2), st));
-        h->urange_cap = nkb;
-    }
-    // the tiles of the split tail groups: warp w of tail group j has slots
-    // (j gw + w)(parts - 1) .. of xsym
-    std::vector<int> tslot(t.size(), -1);
-    for (int j = 0; j < h->sg_ntail; ++j) {
-        const int2 g = groups[h->sg_tail0 + j * h->sg_parts];
-        for (int w = 0; w < gw; ++w) {
-            const int lc = necg::sgroup_lc0(g) + w;
-            if (start[g.x] + lc < start[g.x + 1]) tslot[start[g.x] + lc] = (j * gw + w) * (h->sg_parts - 1);
-        }
-    }
-    if ((int)t.size() > h->tslot_cap) {
-        pool_free(h, h->d_tslot, st);
-        h->d_tslot = nullptr;
-        CK(pool_alloc(h, &h->d_tslot, t.size() * sizeof(int), st));
-        h->tslot_cap = (int)t.size();
-    }
-    CK(cudaMemcpyAsync(h->d_tslot, tslot.data(), tslot.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(h->d_urange, urange.data(), nkb * sizeof(int2), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(h->d_sgroups, groups.data(), groups.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
-    h->nsgroups = (int)groups.size();
+    necg::SymLists &o = h->lists;
+    o.tiles = h->d_lists;
+    o.groups = o.tiles + q.ntiles;
+    o.bgroups = o.groups + nu;
+    o.urange = o.bgroups + nb;
+    o.burange = o.urange + nkb;
+    o.tslot = (int *)(o.burange + nkb);
+    o.start = o.tslot + q.ntiles;
+    necg::launch_sym_lists(q, o, st);
+    CK(cudaGetLastError());
+    h->queue = q;
+    h->nbgroups = nb;
+    h->nstiles = q.ntiles;
     h->sgroups_w = gw;
-    std::vector<int2> bgroups;  // width 8, for the batched step
-    std::vector<int2> burange(nkb);
-    for (int kb = nkb - 1; kb >= 0; --kb) {
-        const int ntk = start[kb + 1] - start[kb];
-        burange[kb].x = (int)bgroups.size();
-        for (int lc0 = 0; lc0 < ntk; lc0 += 8) bgroups.push_back(make_int2(kb, lc0));
-        burange[kb].y = (int)bgroups.size();
-    }
-    if (nkb > h->burange_cap) {
-        pool_free(h, h->d_burange, st);
-        h->d_burange = nullptr;
-        CK(pool_alloc(h, &h->d_burange, nkb * sizeof(int2), st));
-        h->burange_cap = nkb;
-    }
-    CK(cudaMemcpyAsync(h->d_burange, burange.data(), nkb * sizeof(int2), cudaMemcpyHostToDevice, st));
-    if ((int)bgroups.size() > h->bgroups_cap) {
-        pool_free(h, h->d_bgroups, st);
-        h->d_bgroups = nullptr;
-        CK(pool_alloc(h, &h->d_bgroups, bgroups.size() * sizeof(int2), st));
-        h->bgroups_cap = (int)bgroups.size();
-    }
-    CK(cudaMemcpyAsync(h->d_bgroups, bgroups.data(), bgroups.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
-    h->nbgroups = (int)bgroups.size();
-    CK(cudaMemcpyAsync(h->d_stiles, t.data(), t.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(h->d_stile_start, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-    CK(cudaStreamSynchronize(st));
+    h->stiles_lc = LC;
     h->stiles_K = K;
     ++h->gversion;
-    h->stiles_lc = LC;
-    h->nstiles = (int)t.size();
     return NECG_OK;
 }
 
@@ -533,20 +441,20 @@ LaunchArgs base_args(necg_handle *h, int K) {
 
 // The tile lists and buffers of the symmetric passes, as ensure_sym_tiles left them.
 void sym_args(const necg_handle *h, LaunchArgs &a) {
-    a.stiles = h->d_stiles;
-    a.stile_start = h->d_stile_start;
+    a.stiles = h->lists.tiles;
+    a.stile_start = h->lists.start;
     a.nstiles = h->nstiles;
     a.LC_s = h->lc_s;
     a.psym = h->d_psym;
-    a.sgroups = h->d_sgroups;
-    a.nsgroups = h->nsgroups;
+    a.sgroups = h->lists.groups;
+    a.nsgroups = h->queue.units();
     a.qcount = h->d_qcount;
     a.xsym = h->d_xsym;
-    a.sg_tail0 = h->sg_tail0;
-    a.sg_ntail = h->sg_ntail;
-    a.sg_parts = h->sg_parts;
-    a.urange = h->d_urange;
-    a.tslot = h->d_tslot;
+    a.sg_tail0 = h->queue.tail0;
+    a.sg_ntail = h->queue.ntail;
+    a.sg_parts = h->queue.parts;
+    a.urange = h->lists.urange;
+    a.tslot = h->lists.tslot;
 }
 
 // The gradient passes after E and norm are in scal: symmetric (unordered pairs)
@@ -797,7 +705,7 @@ int necg_outprod(necg_handle *h, int K, const double *x_dev, double *f_dev, doub
     } else if ((rc = begin(h, st))) {
         return rc;
     }
-    if ((rc = ensure_tiles(h, K, st))) return rc;
+    if (!fused && (rc = ensure_tiles(h, K, st))) return rc;
     const size_t siv = (size_t)K * (h->n * (h->n + 1) / 2 + 3 * h->n);
     LaunchArgs a = base_args(h, K);
     a.iv = x_dev;
@@ -874,9 +782,7 @@ int necg_shard_tiles(necg_handle *h, int K, int *ntiles) {
     int rc = check_K(h, K);
     if (rc) return rc;
     if (!h->sym_ok) return NECG_ERR_UNSUPPORTED;
-    CK(cudaSetDevice(h->device));
-    if ((rc = ensure_sym_tiles(h, K, h->last_stream, true))) return rc;
-    *ntiles = h->nstiles;
+    *ntiles = necg::tiles_before(K, h->lc_s, necg::row_blocks(K));
     return NECG_OK;
 }
 

@@ -5,6 +5,7 @@
 
 #include <vector>
 
+#include "necg_tiles.h"
 #include "../../include/necg.h"
 
 struct necg_handle {
@@ -35,28 +36,19 @@ struct necg_handle {
     int *d_kcnt = nullptr, *d_ksrc = nullptr;
     double *d_kcoef = nullptr;
     int kmaxnz = 0, kfold = 0;  // the ket frame map (RawMap)
-    int2 *d_stiles = nullptr;
-    int *d_stile_start = nullptr;
-    int stiles_cap = 0, stiles_K = -1, stiles_lc = -1, nstiles = 0;
+    // tile lists of the symmetric passes and the queue of the block variants, in one
+    // buffer (lists points into it)
+    int2 *d_lists = nullptr;
+    size_t lists_cap = 0;  // int2
+    necg::SymLists lists = {};
+    necg::SymQueue queue = {};
+    int stiles_K = -1, stiles_lc = -1, nstiles = 0, nbgroups = 0, sgroups_w = 0;
     double *d_psym = nullptr;
     size_t psym_cap = 0;  // doubles
-    int2 *d_sgroups = nullptr;  // groups of consecutive fused tiles of one row block (kb, first lc)
-    int sgroups_cap = 0, nsgroups = 0, sgroups_w = 0;
-    // the queue's tail: its last sg_ntail groups split into sg_parts units from
-    // queue index sg_tail0; parts after the first write to d_xsym
-    int sg_tail0 = 0, sg_ntail = 0, sg_parts = 1;
-    double *d_xsym = nullptr;
+    double *d_xsym = nullptr;  // parts after the first of the queue's split tail groups
     size_t xsym_cap = 0;  // doubles
-    int2 *d_urange = nullptr;  // queue units of each row block (bra partial slots)
-    int urange_cap = 0;
-    int *d_tslot = nullptr;    // per tile: its slots in d_xsym, or -1
-    int tslot_cap = 0;
     bool sms_general = true;   // some shift map is not kron(m, I3)
     int *d_qcount = nullptr;    // queue head of the block-synchronised fused pass
-    int2 *d_bgroups = nullptr;  // the same groups with 8 chunks each (the batched step's blocks)
-    int bgroups_cap = 0, nbgroups = 0;
-    int2 *d_burange = nullptr;  // groups of each row block in d_bgroups
-    int burange_cap = 0;
     // fused pass with one-warp tiles: symmetry terms split over npc warps per tile
     int npc = 1;
     double *d_Hp = nullptr, *d_Sp = nullptr;  // npc K x K sums each

@@ -57,8 +57,18 @@ __global__ void __launch_bounds__(64) prep_kernel(const double *__restrict__ iv,
     if (id < K * nst) prep_ket_one<N>(iv, C, nst, cs, sml, sms, scvv, ket, id, pinv, general);
 }
 
+// The tile lists: block kb writes row block kb's entries.  A few microseconds, once
+// per size and setting.
+__global__ void __launch_bounds__(128) tile_list_kernel(int2 *tiles, int K, int LC) {
+    const int kb = blockIdx.x, t0 = tiles_before(K, LC, kb), nt = block_tiles(K, LC, kb);
+    for (int lc = threadIdx.x; lc < nt; lc += blockDim.x) tiles[t0 + lc] = make_int2(kb, lc);
+}
+__global__ void __launch_bounds__(128) sym_lists_kernel(SymQueue q, SymLists o) {
+    fill_sym_lists(q, o, blockIdx.x, threadIdx.x, blockDim.x);
+}
+
 // Energy tiles over the lower triangle (the loop of python/outprod.py:49-54 and
-// python/necg.py:43-50); tile list built by the host (energy_tile_count order).
+// python/necg.py:43-50), in the order of tile_list_kernel.
 // One warp per block; MINW = minimum resident warps per SM the kernel is
 // compiled for (register budget 65536 / (32 MINW) per thread).
 template <int N, int MINW>
@@ -1037,6 +1047,12 @@ template <int N> struct Launch {
     default: return -1;             \
     }
 
+void launch_tile_list(int2 *tiles, int K, int LC, cudaStream_t st) {
+    tile_list_kernel<<<row_blocks(K), 128, 0, st>>>(tiles, K, LC);
+}
+void launch_sym_lists(const SymQueue &q, const SymLists &o, cudaStream_t st) {
+    sym_lists_kernel<<<row_blocks(q.K), 128, 0, st>>>(q, o);
+}
 int launch_prep(const LaunchArgs &a, cudaStream_t st) {
     NECG_DISPATCH(a.n, prep(a, st));
     return 0;

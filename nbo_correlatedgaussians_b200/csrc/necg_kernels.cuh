@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include "necg_lanes.cuh"
+#include "necg_tiles.h"
 
 namespace necg {
 
@@ -52,17 +53,9 @@ struct LaunchArgs {
     int sms_general;                       // prep: general shift maps
 };
 
-// A tile group of the block variants: row block kb, first ket chunk lc0 and, for
-// a split group of the queue's tail, its part and the number of parts (one part
-// per range of symmetry terms).
-__host__ __device__ inline int2 sgroup_pack(int kb, int lc0, int part, int parts) {
-    return make_int2(kb, lc0 | (part << 20) | (parts << 24));
-}
-__host__ __device__ inline int sgroup_lc0(int2 g) { return g.y & 0xFFFFF; }
-__host__ __device__ inline int sgroup_part(int2 g) { return (g.y >> 20) & 0xF; }
-__host__ __device__ inline int sgroup_parts(int2 g) { return ((g.y >> 24) & 0xF) > 1 ? ((g.y >> 24) & 0xF) : 1; }
-
-
+// the tile lists (necg_tiles.h): energy tiles (kb, lc), and those of the symmetric passes
+void launch_tile_list(int2 *tiles, int K, int LC, cudaStream_t st);
+void launch_sym_lists(const SymQueue &q, const SymLists &o, cudaStream_t st);
 int launch_prep(const LaunchArgs &a, cudaStream_t st);
 int launch_energy(const LaunchArgs &a, cudaStream_t st);
 int launch_grad(const LaunchArgs &a, cudaStream_t st);

@@ -101,20 +101,6 @@ Carve carve(int n, int nst, int K) {
     return c;
 }
 
-// Energy tile list (the order of the handle path): thread per 32-row block kb
-// writes its tiles (kb, 0 .. last / LC) after the tiles of all earlier blocks.
-__global__ void noalloc_tiles_kernel(int2 *tiles, int K, int LC) {
-    const int kb = blockIdx.x * blockDim.x + threadIdx.x;
-    if (kb * 32 >= K) return;
-    int start = 0;
-    for (int b = 0; b < kb; ++b) {
-        const int last = b * 32 + 31 < K - 1 ? b * 32 + 31 : K - 1;
-        start += last / LC + 1;
-    }
-    const int last = kb * 32 + 31 < K - 1 ? kb * 32 + 31 : K - 1;
-    for (int lc = 0; lc <= last / LC; ++lc) tiles[start + lc] = make_int2(kb, lc);
-}
-
 }  // namespace
 
 extern "C" int necg_outprod_noalloc(int n, int nst, int K, double efs, const double *mass_host,
@@ -138,8 +124,7 @@ extern "C" int necg_outprod_noalloc(int n, int nst, int K, double efs, const dou
         cudaMemcpyAsync(base + c.sms, sms_host, sizeof(double) * nst * 9 * n * n, cudaMemcpyHostToDevice, st) ||
         cudaMemcpyAsync(base + c.scvv, scvv_host, sizeof(double) * nst, cudaMemcpyHostToDevice, st))
         return NECG_ERR_CUDA;
-    const int nkb = (K + 31) / 32;
-    noalloc_tiles_kernel<<<(nkb + 127) / 128, 128, 0, st>>>(tiles, K, kLcEnergy);
+    necg::launch_tile_list(tiles, K, kLcEnergy, st);
 
     necg::LaunchArgs a;
     memset(&a, 0, sizeof(a));
@@ -158,7 +143,7 @@ extern "C" int necg_outprod_noalloc(int n, int nst, int K, double efs, const dou
     a.bra = base + c.bra;
     a.ket = base + c.ket;
     a.tiles = tiles;
-    a.ntiles = necg::energy_tile_count(K, kLcEnergy);
+    a.ntiles = necg::tiles_before(K, kLcEnergy, necg::row_blocks(K));
     a.LC_e = kLcEnergy;
     a.LC_g = kLcGrad;
     a.minb_e = 16;

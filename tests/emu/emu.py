@@ -18,7 +18,7 @@ _lib = None
 
 
 def build() -> str:
-    deps = [SRC] + [os.path.join(CSRC, f) for f in ("necg_lanes.cuh", "necg_math.cuh", "necg_hostscalar.cuh")]
+    deps = [SRC] + [os.path.join(CSRC, f) for f in ("necg_lanes.cuh", "necg_math.cuh", "necg_tiles.h", "necg_hostscalar.cuh")]
     if os.path.exists(LIB) and all(os.path.getmtime(LIB) >= os.path.getmtime(d) for d in deps):
         return LIB
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
@@ -136,6 +136,23 @@ def elements(p, terms):
             ctypes.c_int(len(t)), ctypes.c_void_p(_p(t)), ctypes.c_void_p(_p(mat)), ctypes.c_void_p(_p(tg)),
             ctypes.c_void_p(_p(tgs)))
     return rc, mat, tg, tgs
+
+
+def sym_lists(K, lc, w, nst, sms, nj=7):
+    """The tile lists of the symmetric passes: dict of counts and arrays."""
+    L = lib()
+    head = np.zeros(6, np.int32)
+    none = [None] * 7
+    L.emu_sym_lists(K, lc, w, nst, sms, nj, ctypes.c_void_p(_p(head)), *none)
+    out = dict(zip(("ntiles", "units", "nb", "tail0", "ntail", "parts"), head.tolist()))
+    nkb = (K + 31) // 32
+    out.update(tiles=np.full((out["ntiles"], 2), -9, np.int32), start=np.full(nkb + 1, -9, np.int32),
+               groups=np.full((out["units"], 2), -9, np.int32), urange=np.full((nkb, 2), -9, np.int32),
+               tslot=np.full(out["ntiles"], -9, np.int32), bgroups=np.full((out["nb"], 2), -9, np.int32),
+               burange=np.full((nkb, 2), -9, np.int32))
+    L.emu_sym_lists(K, lc, w, nst, sms, nj, ctypes.c_void_p(_p(head)),
+                    *[ctypes.c_void_p(_p(out[k])) for k in ("tiles", "start", "groups", "urange", "tslot", "bgroups", "burange")])
+    return out
 
 
 class EmuShardOps:

@@ -12,6 +12,7 @@
 
 #include "../../nbo_correlatedgaussians_b200/csrc/necg_hostscalar.cuh"
 #include "../../nbo_correlatedgaussians_b200/csrc/necg_lanes.cuh"
+#include "../../nbo_correlatedgaussians_b200/csrc/necg_tiles.h"
 
 using namespace necg;
 
@@ -763,4 +764,18 @@ extern "C" int emu_elements(int n, int nst, int K, double efs, const double *mas
                             int nterms, const int *terms, double *mat, double *tg, double *tgs) {
     Args a{nst, K, efs, mass, ncv, scvv, sml, sms};
     EMU_DISPATCH(n, (elements<N>(a, iv, nterms, terms, mat, tg, tgs)));
+}
+
+// The tile lists of the symmetric passes, filled row block by row block with nj
+// threads each; head: ntiles, units, groups of 8, tail0, ntail, parts.  Null lists: head only.
+extern "C" int emu_sym_lists(int K, int LC, int w, int nst, int sms, int nj, int *head, int *tiles, int *start,
+                             int *groups, int *urange, int *tslot, int *bgroups, int *burange) {
+    const SymQueue q = sym_queue(K, LC, w, nst, sms);
+    const int h[6] = {q.ntiles, q.units(), groups_before(K, LC, 8, -1), q.tail0, q.ntail, q.parts};
+    for (int i = 0; i < 6; ++i) head[i] = h[i];
+    if (!tiles) return 0;
+    const SymLists o{(int2 *)tiles, start, (int2 *)groups, (int2 *)urange, tslot, (int2 *)bgroups, (int2 *)burange};
+    for (int kb = 0; kb < row_blocks(K); ++kb)
+        for (int j = 0; j < nj; ++j) fill_sym_lists(q, o, kb, j, nj);
+    return 0;
 }
