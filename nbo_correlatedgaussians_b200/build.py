@@ -18,7 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libnecg_b200.so")
 SOURCES = ["necg_kernels.cu", "necg_capi.cu", "necg_count.cu", "necg_batch.cu", "necg_noalloc.cu"]
 HEADERS = ["necg_math.cuh", "necg_kernels.cuh", "necg_lanes.cuh", "necg_handle.h", "necg_hostscalar.cuh",
-           "necg_device.cuh", "necg_tiles.h", "necg_trace.h"]
+           "necg_device.cuh", "necg_tiles.h", "necg_maps.h", "necg_trace.h"]
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMPILE_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]

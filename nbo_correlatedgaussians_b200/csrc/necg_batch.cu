@@ -201,40 +201,13 @@ __global__ void __launch_bounds__(32, 8) batch_fused_warp_kernel(PlanPtrs p) {
 // bras; the group's bras are staged in shared memory once, each warp's ket
 // records too, in two buffers (fsym_tile with SBRA, SKET), and the warps meet only
 // at the group's ends.  Shared memory is sized for n = kMaxN.
-template <int N> __host__ __device__ constexpr int bfused_warp_smem() {
-    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + ket_red<N>() + 2 * KetLayout<N>::size;
-}
-constexpr int kBatchFusedSmem = (8 * bfused_warp_smem<kMaxN>() + BraLayout<kMaxN>::term * 32) * 8;
+constexpr int kBatchFusedSmem = fsym_block_smem_bytes<kMaxN>(8);
 
 template <int N>
 __device__ __forceinline__ void batch_fused_group(const InstDesc &d, int g, double *smem) {
-    constexpr int PB = SumFields<N>::size;
-    constexpr int PER_WARP = bfused_warp_smem<N>();
-    constexpr int TBL = ket_table<N>(2);
-    const int w = threadIdx.x >> 5;
-    double *base = smem + w * PER_WARP;
-    double *sbra = smem + 8 * PER_WARP;
-    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + ket_red<N>()};
-    const int2 gr = d.bgroups[g];
-    const int K = d.K, kb = gr.x, lc = gr.y + w;
-    const bool idle = lc * d.lc_s > row_last(K, kb);
-    stage_bras<N>(sbra, d.bra, K, kb, 256);
-    __syncthreads();
-    double *part_b = d.psym, *part_k = d.psym + (size_t)d.nstiles * 2 * PB * 32;
-    fsym_tile<N, true, true, true, false>(d.stile_start[kb] + lc, make_int2(kb, lc), d.lc_s, K, d.nst,
-                                          consts_of<N>(d), d.bra, d.ket, d.C, d.kmap, nullptr, nullptr, part_b,
-                                          part_k, d.status, sm, idle, sbra);
-    // the warps share the group's bras: their accumulators are summed in warp
-    // order and written once, to the group's slot
-    __syncthreads();
-    for (int i = threadIdx.x; i < 2 * PB * 32; i += 256) {
-        if (kb == 0 && (i & 31) < row_pad(K)) continue;  // no basis
-        double v = smem[i];
-#pragma unroll
-        for (int q = 1; q < 8; ++q) v += smem[q * PER_WARP + i];
-        part_b[(size_t)g * 2 * PB * 32 + i] = v;
-    }
-    __syncthreads();  // sbra and the warps' areas are reused by the next group
+    fsym_group<N, 8, false>(g, d.bgroups[g], 0, d.stile_start, d.lc_s, d.K, d.nst, consts_of<N>(d), d.bra, d.ket, d.C,
+                            d.kmap, nullptr, nullptr, d.psym,
+                            d.psym + (size_t)d.nstiles * 2 * SumFields<N>::size * 32, d.status, nullptr, 0.0, smem);
 }
 
 __global__ void __launch_bounds__(256, 1) batch_fused_kernel(PlanPtrs p) {

@@ -29,6 +29,7 @@
 
 #include "necg_handle.h"
 #include "necg_kernels.cuh"
+#include "necg_maps.h"
 #include "necg_math.cuh"
 #include "necg_trace.h"
 
@@ -256,92 +257,26 @@ namespace {
 // ket gradient from P's frame to the basis function's frame.  Sets sym_ok
 // when every term's inverse is in the set and n <= 5.
 int setup_symmetric(necg_handle *h) {
-    const int n = h->n, nst = h->nst, m = 3 * n;
+    const int n = h->n, nst = h->nst;
     if (n > 5) return NECG_OK;
-    std::vector<int> pinv(nst, -1);
-    for (int p = 0; p < nst; ++p)
-        for (int q = 0; q < nst && pinv[p] < 0; ++q) {
-            bool ok = true;
-            for (int i = 0; i < n && ok; ++i)
-                for (int j = 0; j < n && ok; ++j) {
-                    double s = 0.0;
-                    for (int k = 0; k < n; ++k) s += h->sml[(size_t)p * n * n + i * n + k] * h->sml[(size_t)q * n * n + k * n + j];
-                    ok = fabs(s - (i == j ? 1.0 : 0.0)) < 1e-12;
-                }
-            for (int i = 0; i < m && ok; ++i)
-                for (int j = 0; j < m && ok; ++j) {
-                    double s = 0.0;
-                    for (int k = 0; k < m; ++k) s += h->sms[(size_t)p * m * m + i * m + k] * h->sms[(size_t)q * m * m + k * m + j];
-                    ok = fabs(s - (i == j ? 1.0 : 0.0)) < 1e-12;
-                }
-            if (ok) pinv[p] = q;
-        }
-    for (int p = 0; p < nst; ++p)
-        if (pinv[p] < 0) return NECG_OK;  // not closed under inverse: ordered pass only
-    // e' = A' s' maps as e = A s does when each shift map is that of its coordinate
-    // map, sms = kron(sml^-1, I3), i.e. sms kron(sml, I3) = 1; the kets' raw sums
-    // are then mapped and summed as they are, else folded in P's frame first
-    bool fold = false;
-    for (int p = 0; p < nst && !fold; ++p)
-        for (int r = 0; r < m && !fold; ++r)
-            for (int j = 0; j < n && !fold; ++j)
-                for (int c = 0; c < 3 && !fold; ++c) {  // column (j, c) of sms kron(sml, I3)
-                    double v = 0.0;
-                    for (int k = 0; k < n; ++k) v += h->sms[(size_t)p * m * m + r * m + 3 * k + c] * h->sml[(size_t)p * n * n + k * n + j];
-                    fold = fabs(v - (r == 3 * j + c ? 1.0 : 0.0)) > 1e-12;
-                }
-    const int T = n * (n + 1) / 2, SL = necg::ket_slots(n);
-    std::vector<std::vector<std::pair<int, double>>> rows((size_t)nst * SL);
-    auto slot = [n](int f) { return necg::ket_slot(n, f); };
-    for (int p = 0; p < nst; ++p) {
-        const double *P = &h->sml[(size_t)p * n * n];
-        const double *Sm = &h->sms[(size_t)p * m * m];
-        for (int a = 0; a < n; ++a)
-            for (int b = 0; b <= a; ++b) {  // (sml G' sml^T)_ab
-                std::vector<double> coef(T, 0.0);
-                for (int cc = 0; cc < n; ++cc)
-                    for (int d = 0; d < n; ++d) coef[necg::sx(cc, d)] += P[a * n + cc] * P[b * n + d];
-                auto &row = rows[(size_t)p * SL + slot(necg::sx(a, b))];
-                for (int s = 0; s < T; ++s)
-                    if (coef[s] != 0.0) row.push_back({slot(s), coef[s]});
-            }
-        rows[(size_t)p * SL + slot(T)].push_back({slot(T), 1.0});
-        for (int r = 0; r < m; ++r) {
-            auto &row = rows[(size_t)p * SL + slot(T + 1 + r)];
-            if (fold) {  // dF/ds: (sms^T g')_r
-                for (int cc = 0; cc < m; ++cc)
-                    if (Sm[cc * m + r] != 0.0) row.push_back({slot(T + 1 + cc), Sm[cc * m + r]});
-            } else {  // dF/de: (sml g')_r
-                for (int k = 0; k < n; ++k)
-                    if (P[(r / 3) * n + k] != 0.0) row.push_back({slot(T + 1 + 3 * k + r % 3), P[(r / 3) * n + k]});
-            }
-        }
-    }
-    int maxnz = 1;
-    for (auto &r : rows) maxnz = (int)r.size() > maxnz ? (int)r.size() : maxnz;
-    std::vector<int> cnt(rows.size()), src(rows.size() * maxnz, 0);
-    std::vector<double> coef(rows.size() * maxnz, 0.0);
-    for (size_t e = 0; e < rows.size(); ++e) {
-        cnt[e] = (int)rows[e].size();
-        for (size_t i = 0; i < rows[e].size(); ++i) {
-            src[e * maxnz + i] = rows[e][i].first;
-            coef[e * maxnz + i] = rows[e][i].second;
-        }
-    }
+    std::vector<int> pinv;
+    if (!necg::inverse_terms(n, nst, h->sml.data(), h->sms.data(), pinv)) return NECG_OK;  // ordered pass only
+    const necg::RawMapTable t = necg::raw_map_table(n, nst, h->sml.data(), h->sms.data(), necg::ket_slots(n),
+                                                    [n](int f) { return necg::ket_slot(n, f); });
     int rc = NECG_OK;
     if (!rc) rc = dalloc(h, &h->d_pinv, (size_t)nst);
-    if (!rc) rc = dalloc(h, &h->d_kcnt, cnt.size());
-    if (!rc) rc = dalloc(h, &h->d_ksrc, src.size());
-    if (!rc) rc = dalloc(h, &h->d_kcoef, coef.size());
+    if (!rc) rc = dalloc(h, &h->d_kcnt, t.cnt.size());
+    if (!rc) rc = dalloc(h, &h->d_ksrc, t.src.size());
+    if (!rc) rc = dalloc(h, &h->d_kcoef, t.coef.size());
     if (rc) return rc;
     cudaStream_t ls = lib_stream(h);
     CK(cudaMemcpyAsync(h->d_pinv, pinv.data(), nst * sizeof(int), cudaMemcpyHostToDevice, ls));
-    CK(cudaMemcpyAsync(h->d_kcnt, cnt.data(), cnt.size() * sizeof(int), cudaMemcpyHostToDevice, ls));
-    CK(cudaMemcpyAsync(h->d_ksrc, src.data(), src.size() * sizeof(int), cudaMemcpyHostToDevice, ls));
-    CK(cudaMemcpyAsync(h->d_kcoef, coef.data(), coef.size() * sizeof(double), cudaMemcpyHostToDevice, ls));
+    CK(cudaMemcpyAsync(h->d_kcnt, t.cnt.data(), t.cnt.size() * sizeof(int), cudaMemcpyHostToDevice, ls));
+    CK(cudaMemcpyAsync(h->d_ksrc, t.src.data(), t.src.size() * sizeof(int), cudaMemcpyHostToDevice, ls));
+    CK(cudaMemcpyAsync(h->d_kcoef, t.coef.data(), t.coef.size() * sizeof(double), cudaMemcpyHostToDevice, ls));
     CK(cudaStreamSynchronize(ls));  // the host vectors above end with this scope
-    h->kmaxnz = maxnz;
-    h->kfold = fold ? 1 : 0;
+    h->kmaxnz = t.maxnz;
+    h->kfold = t.fold;
     h->sym_ok = true;
     h->grad_mode = 1;
     return NECG_OK;

@@ -7,6 +7,7 @@
 
 #include "necg_lanes.cuh"
 #include "necg_math.cuh"
+#include "necg_tiles.h"
 
 namespace necg {
 
@@ -37,14 +38,24 @@ __device__ __forceinline__ void stage_bras(double *sbra, const double *__restric
 // 16-byte cp.async per lane, one commit group per record.
 __device__ __forceinline__ void ket_fetch(double *dst, const double *src, int nd, int lane) {
     for (int i = lane; 2 * i < nd; i += 32) {
+#ifdef __CUDACC__
         const unsigned d = (unsigned)__cvta_generic_to_shared(dst + 2 * i);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + 2 * i) : "memory");
+#else
+        simt::copy16(dst + 2 * i, src + 2 * i);
+#endif
     }
+#ifdef __CUDACC__
     asm volatile("cp.async.commit_group;" ::: "memory");
+#endif
 }
 // Wait for this lane's copies and make the warp's copies visible to the warp.
 __device__ __forceinline__ void ket_wait() {
+#ifdef __CUDACC__
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+#else
+    simt::copies_wait();
+#endif
     __syncwarp();
 }
 
@@ -407,6 +418,82 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
     if (!ok) flags |= 1;
     flag_status(status, flags, bad);
     __syncwarp();
+}
+
+// Dynamic shared memory of a block of warps (doubles, 16-byte aligned): per warp its
+// tile's areas (FusedSmem), then the bras that the warps share.
+template <int N> __host__ __device__ constexpr int fsym_warp_smem() {
+    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + ket_red<N>() + 2 * KetLayout<N>::size;
+}
+template <int N> __host__ __device__ constexpr int fsym_block_smem_bytes(int warps) {
+    return (warps * fsym_warp_smem<N>() + BraLayout<N>::term * 32) * 8;
+}
+
+// One unit of a queue of tile groups by a block of WARPS warps: unit g = row block
+// kb and ket chunks lc0 .. lc0 + WARPS - 1 (or one part of their symmetry terms),
+// one per warp.  The unit's bras are staged in shared memory once for all warps, each
+// warp stages its ket records, and the warps meet only at the unit's ends.  Parts
+// after the first of a split group write to their own slots in xsym (groups split
+// from unit tail0 on); KE: the symmetric pass with E known.
+template <int N, int WARPS, bool KE>
+__device__ __forceinline__ void fsym_group(int g, int2 gr, int tail0, const int *__restrict__ tstart, int LC, int K,
+                                           int nst, const Consts<N> &cs, const double *__restrict__ bra,
+                                           const double *__restrict__ ket, const double *__restrict__ C,
+                                           const RawMap &kmap, double *__restrict__ H, double *__restrict__ S,
+                                           double *__restrict__ part_b, double *__restrict__ part_k, int *status,
+                                           double *__restrict__ xsym, double E, double *smem) {
+    constexpr int PB = SumFields<N>::size, PER_WARP = fsym_warp_smem<N>(), TBL = ket_table<N>(2);
+    const int w = threadIdx.x >> 5;
+    double *base = smem + w * PER_WARP;
+    double *sbra = smem + WARPS * PER_WARP;  // after the warps' areas
+    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + ket_red<N>()};
+    const int kb = gr.x, lc = sgroup_lc0(gr) + w;
+    const bool idle = lc * LC > row_last(K, kb);  // past this block's triangle
+    const int part = sgroup_part(gr), parts = sgroup_parts(gr);
+    const int p0 = part * nst / parts, p1 = (part + 1) * nst / parts;  // balanced ranges
+    TileOut xo;
+    if (part > 0) {
+        xo.x = xsym;
+        xo.slot = (((g - tail0) / parts) * WARPS + w) * (parts - 1) + (part - 1);
+    }
+    stage_bras<N>(sbra, bra, K, kb, 32 * WARPS);
+    __syncthreads();
+    fsym_tile<N, true, true, true, false, KE>(tstart[kb] + lc, make_int2(kb, lc), LC, K, nst, cs, bra, ket, C, kmap,
+                                              H, S, part_b, part_k, status, sm, idle, sbra, p0, p1, xo, E);
+    // the unit's bra partials: its warps share the 32 bras, so their accumulators
+    // are summed (in warp order) and written once, to the slot of unit g
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * PB * 32; i += 32 * WARPS) {
+        if (kb == 0 && (i & 31) < row_pad(K)) continue;  // no basis
+        double v = smem[i];
+#pragma unroll
+        for (int q = 1; q < WARPS; ++q) v += smem[q * PER_WARP + i];
+        part_b[(size_t)g * 2 * PB * 32 + i] = v;
+    }
+    __syncthreads();  // sbra and the warps' areas are rewritten for the next unit
+}
+
+// H and S of one tile (warp w) of tail group j, when the caller wants them: add parts
+// 1 .. parts - 1 (their slots in xsym, in part order) to what part 0 wrote, by a block
+// of any size.  Entries that no part wrote (kets past K or above the diagonal, tiles
+// past the block's triangle) are left alone.
+template <int N>
+__device__ __forceinline__ void fix_tail_tile(int2 gr, int j, int w, int W, int LC, int K, const double *__restrict__ xsym,
+                                              double *__restrict__ H, double *__restrict__ S) {
+    constexpr int PB = SumFields<N>::size;
+    const int parts = sgroup_parts(gr), kb = gr.x, lc = sgroup_lc0(gr) + w;
+    if (lc * LC > row_last(K, kb)) return;
+    const size_t XS = fsym_tail_slot(PB, LC);
+    const double *x0 = xsym + (size_t)(j * W + w) * (parts - 1) * XS + (size_t)LC * 2 * PB;
+    for (int i = threadIdx.x; i < LC * 64; i += blockDim.x) {
+        const int l = lc * LC + i / 64, r = i & 63, k = kb * 32 + (r & 31) - row_pad(K);
+        if (k < 0 || l > k) continue;
+        double *M = r < 32 ? H : S;
+        double v = M[(size_t)k * K + l];
+        for (int q = 0; q < parts - 1; ++q) v += x0[q * XS + i];
+        M[(size_t)k * K + l] = v;
+        M[(size_t)l * K + k] = v;
+    }
 }
 
 // Where the partials of a symmetric pass are and which of them count: tiles

@@ -342,22 +342,11 @@ __global__ void __launch_bounds__(256) hs_reduce_kernel(const double *__restrict
 }
 
 // The fused pass with W-warp blocks (W = 8, 12 or 16), one per SM, persistent over
-// a queue of tile groups: group g = row block kb and ket chunks lc0 .. lc0 + W
-// - 1, one per warp.  The group's bras are staged in shared memory once for all
-// warps, each warp stages its ket records in two buffers (the next term's copied
-// while the current one is evaluated), and the warps meet only at the group's
-// ends: a block barrier per term, which once kept the warps of a scheduler in
-// step, now only costs (LiH K = 1024 on a B200: 2.54 ms with it, 2.76 ms and more
-// with half of the warps taking it in mid-term, 2.34 ms without).  Shared
-// memory (dynamic, 16-byte aligned): per warp 2 PB 32 + ket table + ket_red + 2 ket
-// records doubles, then the bras.  KE: the symmetric pass with E known.
-template <int N> __host__ __device__ constexpr int fsym_warp_smem() {
-    return 2 * SumFields<N>::size * 32 + ket_table<N>(2) + ket_red<N>() + 2 * KetLayout<N>::size;
-}
-template <int N> __host__ __device__ constexpr int fsym_block_smem_bytes(int warps) {
-    return (warps * fsym_warp_smem<N>() + BraLayout<N>::term * 32) * 8;
-}
-
+// the queue of tile groups (fsym_group).  The warps of a block meet only at the
+// ends of a unit: a block barrier per term, which once kept the warps of a scheduler
+// in step, now only costs (LiH K = 1024 on a B200, an earlier form of the term: 2.54
+// ms with it, 2.76 ms and more with half of the warps taking it in mid-term, 2.34
+// ms without).  KE: the symmetric pass with E known.
 template <int N, int WARPS, bool KE = false>
 __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *__restrict__ groups, int ngroups,
                                                                 int *__restrict__ qcount,
@@ -373,77 +362,25 @@ __global__ void __launch_bounds__(32 * WARPS, 1) fsym_block_kernel(const int2 *_
                                                                 const double *__restrict__ scal) {
     extern __shared__ __align__(16) double smem[];
     __shared__ int gsh;
-    constexpr int PB = SumFields<N>::size;
-    constexpr int PER_WARP = fsym_warp_smem<N>();
-    constexpr int TBL = ket_table<N>(2);
-    const int w = threadIdx.x >> 5;
-    double *base = smem + w * PER_WARP;
-    double *sbra = smem + WARPS * PER_WARP;  // after the warps' areas
-    const FusedSmem sm{base, base + 2 * PB * 32, base + 2 * PB * 32 + TBL, base + 2 * PB * 32 + TBL + ket_red<N>()};
     for (;;) {
         if (threadIdx.x == 0) gsh = atomicAdd(qcount, 1);
         __syncthreads();
         const int g = gsh;
         __syncthreads();  // every thread has read gsh before it changes
         if (g >= ngroups) break;
-        const int2 gr = groups[g];
-        const int kb = gr.x, lc = sgroup_lc0(gr) + w;
-        const bool idle = lc * LC > row_last(K, kb);  // past this block's triangle
-        // a split group of the queue's tail: this unit takes symmetry terms
-        // [p0, p1); parts after the first write to their own slots in xsym
-        const int part = sgroup_part(gr), parts = sgroup_parts(gr);
-        const int p0 = part * nst / parts, p1 = (part + 1) * nst / parts;  // balanced ranges
-        TileOut xo;
-        if (part > 0) {
-            xo.x = xsym;
-            xo.slot = (((g - tail0) / parts) * WARPS + w) * (parts - 1) + (part - 1);
-        }
-        stage_bras<N>(sbra, bra, K, kb, 32 * WARPS);  // the group's bras, once for all warps
-        __syncthreads();
-        fsym_tile<N, true, true, true, false, KE>(tstart[kb] + lc, make_int2(kb, lc), LC, K, nst, cs, bra, ket, C,
-                                                  kmap, H, S, part_b, part_k, status, sm, idle, sbra, p0, p1, xo,
-                                                  KE ? scal[0] : 0.0);
-        // the group's bra partials: its warps share the 32 bras, so their
-        // accumulators are summed (in warp order) and written once, to the
-        // slot of queue unit g
-        __syncthreads();
-        for (int i = threadIdx.x; i < 2 * PB * 32; i += 32 * WARPS) {
-            if (kb == 0 && (i & 31) < row_pad(K)) continue;  // no basis
-            double v = smem[i];
-#pragma unroll
-            for (int q = 1; q < WARPS; ++q) v += smem[q * PER_WARP + i];
-            part_b[(size_t)g * 2 * PB * 32 + i] = v;
-        }
-        __syncthreads();  // sbra and the warps' areas are rewritten for the next group
+        fsym_group<N, WARPS, KE>(g, groups[g], tail0, tstart, LC, K, nst, cs, bra, ket, C, kmap, H, S, part_b, part_k,
+                                 status, xsym, KE ? scal[0] : 0.0, smem);
     }
 }
 
-// H and S of the tiles of the block variants' split tail, when the caller wants
-// them: add parts 1 .. parts - 1 of each tile (their compact slots in xsym, in
-// part order) to what part 0 wrote.  Block = one tile (tail group j, warp w);
-// entries that no part wrote (kets past K or above the diagonal, tiles past the
-// block's triangle) are left alone.
+// H and S of the tiles of the block variants' split tail: block = one tile (tail
+// group j, warp w).
 template <int N>
 __global__ void __launch_bounds__(256) fsym_tail_fix_kernel(const int2 *__restrict__ groups, int tail0, int W,
                                                             int LC, int K, const double *__restrict__ xsym,
                                                             double *__restrict__ H, double *__restrict__ S) {
-    constexpr int PB = SumFields<N>::size;
     const int j = blockIdx.x / W, w = blockIdx.x - j * W;
-    const int2 gr = groups[tail0 + j * sgroup_parts(groups[tail0])];
-    const int parts = sgroup_parts(gr);
-    const int kb = gr.x, lc = sgroup_lc0(gr) + w;
-    if (lc * LC > row_last(K, kb)) return;
-    const size_t XS = fsym_tail_slot(PB, LC);
-    const double *x0 = xsym + (size_t)(j * W + w) * (parts - 1) * XS + (size_t)LC * 2 * PB;
-    for (int i = threadIdx.x; i < LC * 64; i += blockDim.x) {
-        const int l = lc * LC + i / 64, r = i & 63, k = kb * 32 + (r & 31) - row_pad(K);
-        if (k < 0 || l > k) continue;
-        double *M = r < 32 ? H : S;
-        double v = M[(size_t)k * K + l];
-        for (int q = 0; q < parts - 1; ++q) v += x0[q * XS + i];
-        M[(size_t)k * K + l] = v;
-        M[(size_t)l * K + k] = v;
-    }
+    fix_tail_tile<N>(groups[tail0 + j * sgroup_parts(groups[tail0])], j, w, W, LC, K, xsym, H, S);
 }
 
 // Partials of the fused (KE = false) or the symmetric pass into the per-basis

@@ -19,7 +19,7 @@ struct LaunchArgs {
     int minb_e, minb_g;                    // kernel variants: min resident blocks per SM
     double *H, *S, *Kin, *Pot;             // device outputs (Kin/Pot optional)
     double *rows, *scal, *part, *g;        // device workspace / outputs
-    double lam, scale_override;
+    double lam;
     int *status;
     const double *dip_cls;                 // dipole classes of a group (c_Q, R_Q), null: general set
     // symmetric gradient pass

@@ -92,11 +92,6 @@ NECG_HD void prep_bra_at(const double *b, const Consts<N> &cs, double *bra, size
     for (int t = 0; t < tri(N); ++t) bra[(BL::L + t) * stride] = L[t];
 }
 
-// The same for basis k of a buffer with field f at f * K + k (the host emulation).
-template <int N> NECG_HD void prep_bra_one(const double *iv, int K, const Consts<N> &cs, double *bra, int k) {
-    prep_bra_at<N>(iv + (size_t)k * (tri(N) + 3 * N), cs, bra + k, (size_t)K);
-}
-
 // Ket record of (l, P) = id / nst, id % nst: python/matel.py:76-87
 // (al <- sml^T al sml, st2 <- sms st2) plus the data the tiles reuse.  general =
 // false: the shift map is kron(m, I3), so that m alone is read (25 instead of 225
@@ -308,13 +303,6 @@ NECG_HD bool grad_lane(const BA &b, const KB &ket, int l0, int l1, int nst, cons
     return ok;
 }
 
-template <int N, typename R, typename BA, typename KB>
-NECG_HD bool grad_lane(const BA &b, const KB &ket, int l0, int l1, int nst, const Consts<N> &cs,
-                       R lam, R E, double *part, size_t stride) {
-    RegAcc<N, R> accH, accS;
-    return grad_lane<N, R>(b, ket, l0, l1, nst, cs, lam, E, part, stride, accH, accS);
-}
-
 // Map an A-space gradient dF/dA = G + D A^-1 (G packed symmetric, D the
 // scalar coefficient of A^-1) and dF/ds = gS to the reference's parameter
 // block [vech(dF/dL), dF/ds]: dF/dL = 2 (G + D A^-1) L = 2 G L + 2 D L^-T, whose
@@ -370,11 +358,6 @@ NECG_HD bool grad_reduce_at(const double *part, int nlc, int K, const double *br
     for (int t = 0; t < tri(N); ++t) L[t] = brak[(BraLayout<N>::L + t) * stride];
     return a_to_vech<N>(G, o[tri(N)], gS, L, sc, g + (size_t)k * (tri(N) + 3 * N));
 }
-template <int N>
-NECG_HD bool grad_reduce_one(const double *part, int nlc, int K, const double *bra, double sc, double *g, int k) {
-    return grad_reduce_at<N>(part, nlc, K, bra + k, (size_t)K, sc, g, k);
-}
-
 // One matel term (python/matel.py:28-210): out = (ov, tk, ert, zht).
 template <int N, typename R, typename BA, typename KR>
 NECG_HD bool matel_one(const BA &b, const KR &kr, const Consts<N> &cs, double *out) {
@@ -420,41 +403,6 @@ NECG_HD int energy_tile_count(int K, int LC) {
         n += last / LC + 1;
     }
     return n;
-}
-
-// Sparse linear map taking a ket gradient from P's transformed frame to the
-// basis function's own frame: dF/dA_l = sml dF/dA_l' sml^T (packed), the A^-1
-// coefficient unchanged, dF/ds_l = sms^T dF/ds_l'.  Entry (P, f): cnt values
-// at src/coef[(P * PS + f) * maxnz + i].
-struct KetMap {
-    const int *cnt, *src;
-    const double *coef;
-    int maxnz;
-};
-
-NECG_HD double ket_map_apply(const KetMap &m, int P, int f, int PS, const double *in) {
-    const int e = P * PS + f;
-    const int n = m.cnt[e];
-    double v = 0.0;
-    for (int i = 0; i < n; ++i) v += m.coef[(size_t)e * m.maxnz + i] * in[m.src[(size_t)e * m.maxnz + i]];
-    return v;
-}
-
-// The same map applied to two inputs (the H and S ket gradients), reading the
-// map entries once.
-NECG_HD void ket_map_apply2(const KetMap &m, int P, int f, int PS, const double *in0, const double *in1,
-                            double &out0, double &out1) {
-    const int e = P * PS + f;
-    const int n = m.cnt[e];
-    double v0 = 0.0, v1 = 0.0;
-    for (int i = 0; i < n; ++i) {
-        const double c = m.coef[(size_t)e * m.maxnz + i];
-        const int s = m.src[(size_t)e * m.maxnz + i];
-        v0 += c * in0[s];
-        v1 += c * in1[s];
-    }
-    out0 = v0;
-    out1 = v1;
 }
 
 // Where the pair passes keep the ket's raw fields of a term: field f of matrix

@@ -155,65 +155,50 @@ __host__ __device__ inline size_t fsym_tail_slot(int pb, int lc) {
 __host__ __device__ constexpr int vidx(int p, int q) { return q * (q - 1) / 2 + p; }
 
 // ---------------------------------------------------------------------------
-// Device accessors
-#ifdef __CUDACC__
-// Bra fields are per-lane and invariant over a tile's ket loops; holding them in
-// registers would cost 2 (6N + 2 tri(N)) registers, so they are re-read from the
-// (L1-resident) structure-of-arrays at the point of use.  The volatile asm keeps
-// the compiler from hoisting the loads out of the ket loops.
+// Accessors.  Bra fields are per-lane and invariant over a tile's ket loops; holding
+// them in registers would cost 2 (6N + 2 tri(N)) registers, so they are re-read from
+// the (L1-resident) structure-of-arrays at the point of use.  The volatile asm keeps
+// the compiler from hoisting the loads out of the ket loops.  (Compiled for the host
+// by the emulation of the kernels, these are plain loads.)
 __device__ __forceinline__ double ldv(const double *p) {
+#ifdef __CUDACC__
     double v;
     asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
     return v;
+#else
+    return *p;
+#endif
+}
+// The same from shared memory.
+__device__ __forceinline__ double lds(const double *p) {
+#ifdef __CUDACC__
+    double v;
+    const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+#else
+    return *p;
+#endif
 }
 struct BraRef {
     const double *p;  // bra_at(bra, k)
     __device__ __forceinline__ double operator()(int f) const { return ldv(p + f * 32); }
 };
-// Bra record staged in shared memory (field f of this lane at p[f * 32]), read
-// at the point of use through a volatile shared load (not hoisted into registers).
+// Bra record staged in shared memory (field f of this lane at p[f * 32]).
 struct BraSmem {
     const double *p;  // shared base + lane
-    __device__ __forceinline__ double operator()(int f) const {
-        double v;
-        const unsigned a = (unsigned)__cvta_generic_to_shared(p + f * 32);
-        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
-        return v;
-    }
+    __device__ __forceinline__ double operator()(int f) const { return lds(p + f * 32); }
 };
-// Ket record staged in shared memory by its warp, read at the point of use
-// (a broadcast shared load, not hoisted into registers).
+// Ket record staged in shared memory by its warp (a broadcast load).
 struct KetSmem {
     const double *p;
-    __device__ __forceinline__ double operator[](int i) const {
-        double v;
-        const unsigned a = (unsigned)__cvta_generic_to_shared(p + i);
-        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
-        return v;
-    }
+    __device__ __forceinline__ double operator[](int i) const { return lds(p + i); }
 };
 // Ket record read at the point of use (warp-uniform, L1 broadcast), so its
 // fields do not stay live in registers between their uses within a term.
 struct KetRefV {
     const double *p;
     __device__ __forceinline__ double operator[](int i) const { return ldv(p + i); }
-};
-#endif
-
-// Register accumulators of one bra gradient (see term_grad).
-template <int N, typename R> struct RegAcc {
-    R G[tri(N)], D, S[3 * N];
-#pragma nv_exec_check_disable
-    NECG_HD void zero() {
-#pragma unroll
-        for (int t = 0; t < tri(N); ++t) G[t] = R(0.0);
-        D = R(0.0);
-#pragma unroll
-        for (int t = 0; t < 3 * N; ++t) S[t] = R(0.0);
-    }
-    NECG_HD R &g(int t) { return G[t]; }
-    NECG_HD R &d() { return D; }
-    NECG_HD R &s(int t) { return S[t]; }
 };
 
 // ---------------------------------------------------------------------------
@@ -986,105 +971,6 @@ template <typename R> struct FieldsOf {
     const R *p;
     NECG_HD const R &operator()(int f) const { return p[f]; }
 };
-
-// Raw values of one term kept in arrays (unit weight: ov included).
-template <int N, typename R> struct RawValues {
-    static constexpr int PS = tri(N) + 1 + 3 * N;
-    R h[PS], s[PS], ov;
-    NECG_HD void begin(R o) { ov = o; }
-    template <int I> NECG_HD void s2(R va, R vb) {
-        s[RawPairs<N>::fa(I)] = ov * va;
-        s[RawPairs<N>::fb(I)] = ov * vb;
-    }
-    template <int I> NECG_HD void h2(R va, R vb) {
-        h[RawPairs<N>::fa(I)] = ov * va;
-        h[RawPairs<N>::fb(I)] = ov * vb;
-    }
-    NECG_HD void s1(int f, R v) { s[f] = ov * v; }
-    NECG_HD void h1(int f, R v) { h[f] = ov * v; }
-    NECG_HD void scalar(R e2) {
-        h[tri(N)] = ov * e2;
-        s[tri(N)] = ov;
-    }
-};
-
-// Gradients of h and of ov of one term, with respect to the bra (oH, oS; Part<N>
-// fields) and, when KET, to the transformed ket (A_l', s_l').
-#pragma nv_exec_check_disable
-template <int N, bool KET, typename R, typename BA, typename KA>
-NECG_HD bool term_gradients(const BA &b, const KA &kr, const Consts<N> &cs, R (&bH)[tri(N) + 1 + 3 * N],
-                            R (&bS)[tri(N) + 1 + 3 * N], R (&kH)[tri(N) + 1 + 3 * N],
-                            R (&kS)[tri(N) + 1 + 3 * N], R &h, R &ov) {
-    using BL = BraLayout<N>;
-    using KL = KetLayout<N>;
-    constexpr int PS = tri(N) + 1 + 3 * N;
-    RawValues<N, R> v;
-    R eta2;
-    const bool ok = term_raw<N>(b, kr, cs, R(0.0), v, eta2, ov);
-    h = 0.5 * ov * eta2;
-    const auto A = [&](int t) { return b(BL::A + t); };
-    const auto s = [&](int t) { return b(BL::S + t); };
-    const auto e = [&](int t) { return b(BL::AS + t); };
-    R s2[PS];  // the raw fields of ov alone in the scale of H's (twice G and scalar, once g): 2 S
-#pragma unroll
-    for (int f = 0; f < PS; ++f) s2[f] = 2.0 * v.s[f];
-    if (KET) {
-        const auto Ak = [&](int t) { return kr[KL::Ap + t]; };
-        const auto sk = [&](int t) { return kr[KL::Sp + t]; };
-        const auto ek = [&](int t) { return kr[KL::ASp + t]; };
-        fold_raw<N>(FieldsOf<R>{v.h}, Ak, sk, ek, kH);
-        fold_raw<N>(FieldsOf<R>{s2}, Ak, sk, ek, kS);
-    }
-    explicit_tau<N>(FieldsOf<R>{v.s}, A, e, cs, v.h);
-    fold_raw<N>(FieldsOf<R>{v.h}, A, s, e, bH);
-    fold_raw<N>(FieldsOf<R>{s2}, A, s, e, bS);
-    return ok;
-}
-
-// One unordered term of the fused pass with both gradients folded per term: the
-// bra's into the accumulators (weight wb), the ket's out through ko.put(f, vH,
-// vS) (weight wk), for callers that keep gradients and not raw sums (the
-// host emulation of the passes).
-#pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA, typename ACC, typename KOUT>
-NECG_HD bool term_fused(const BA &b, const KA &kr, const Consts<N> &cs, R wb, R wk, ACC &accH, ACC &accS,
-                        KOUT &ko, R &h, R &ov) {
-    constexpr int TR = tri(N), PS = TR + 1 + 3 * N;
-    R bH[PS], bS[PS], kH[PS], kS[PS];
-    const bool ok = term_gradients<N, true>(b, kr, cs, bH, bS, kH, kS, h, ov);
-#pragma unroll
-    for (int t = 0; t < TR; ++t) {
-        accH.g(t) += wb * bH[t];
-        accS.g(t) += wb * bS[t];
-    }
-    accH.d() += wb * bH[TR];
-    accS.d() += wb * bS[TR];
-#pragma unroll
-    for (int t = 0; t < 3 * N; ++t) {
-        accH.s(t) += wb * bH[TR + 1 + t];
-        accS.s(t) += wb * bS[TR + 1 + t];
-    }
-#pragma unroll
-    for (int f = 0; f < PS; ++f) ko.put(f, wk * kH[f], wk * kS[f]);
-    return ok;
-}
-
-// The same for the gradient of h - E ov.
-#pragma nv_exec_check_disable
-template <int N, typename R, typename BA, typename KA, typename ACC, typename KOUT>
-NECG_HD bool term_sym(const BA &b, const KA &kr, const Consts<N> &cs, R E, R wb, R wk, ACC &acc, KOUT &ko) {
-    constexpr int TR = tri(N), PS = TR + 1 + 3 * N;
-    R bH[PS], bS[PS], kH[PS], kS[PS], h, ov;
-    const bool ok = term_gradients<N, true>(b, kr, cs, bH, bS, kH, kS, h, ov);
-#pragma unroll
-    for (int t = 0; t < TR; ++t) acc.g(t) += wb * (bH[t] - E * bS[t]);
-    acc.d() += wb * (bH[TR] - E * bS[TR]);
-#pragma unroll
-    for (int t = 0; t < 3 * N; ++t) acc.s(t) += wb * (bH[TR + 1 + t] - E * bS[TR + 1 + t]);
-#pragma unroll
-    for (int f = 0; f < PS; ++f) ko.put(f, wk * (kH[f] - E * kS[f]));
-    return ok;
-}
 
 // One term of the dipole element of python/rrms.py:21-120 for the bra record
 // (k, Pe) and the ket record (l, P) (both in KetLayout: symmetry applied to both

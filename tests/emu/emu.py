@@ -1,6 +1,6 @@
-"""TEST INFRASTRUCTURE: ctypes wrapper of libnecg_emu.so, the host emulator that
-runs the kernels' per-thread bodies (necg_lanes.cuh) tile by tile and lane by
-lane on the CPU."""
+"""TEST INFRASTRUCTURE: ctypes wrappers of the host emulators of the kernels:
+libnecg_emu.so runs the per-thread bodies of necg_lanes.cuh tile by tile and lane by
+lane, libnecg_simt.so the warps and blocks of necg_device.cuh thread by thread."""
 from __future__ import annotations
 
 import ctypes
@@ -27,6 +27,32 @@ def build() -> str:
                            "-Wno-deprecated-gpu-targets", "-o", tmp, SRC])
     os.replace(tmp, LIB)
     return LIB
+
+
+SIMT_LIB = os.path.join(HERE, "libnecg_simt.so")
+_simt = None
+
+
+def simt():
+    """The emulation of the passes over unordered pairs (simt_emu.cpp)."""
+    global _simt
+    if _simt is None:
+        deps = [os.path.join(HERE, f) for f in ("simt_emu.cpp", "simt.h", os.path.join("stub", "cuda_runtime.h"))]
+        deps += [os.path.join(CSRC, f) for f in ("necg_device.cuh", "necg_lanes.cuh", "necg_math.cuh", "necg_tiles.h", "necg_maps.h")]
+        if not os.path.exists(SIMT_LIB) or any(os.path.getmtime(SIMT_LIB) < os.path.getmtime(d) for d in deps):
+            tmp = f"{SIMT_LIB}.{os.getpid()}.tmp"
+            subprocess.check_call(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-U_FORTIFY_SOURCE", "-Wno-unknown-pragmas",
+                                   "-I", os.path.join(HERE, "stub"), "-o", tmp, deps[0]])
+            os.replace(tmp, SIMT_LIB)
+        _simt = ctypes.CDLL(SIMT_LIB)
+    return _simt
+
+
+def _problem(p):
+    """The arguments every entry of the emulation starts with (and the arrays behind them)."""
+    c = _consts(p)
+    return [ctypes.c_int(p.n), ctypes.c_int(p.nst), ctypes.c_int(p.K), ctypes.c_double(p.efs),
+            *[ctypes.c_void_p(_p(a)) for a in c]], c
 
 
 def lib():
@@ -61,38 +87,27 @@ def outprod(p, lc_e=4, lc_g=4):
     return rc, float(f[0]), g, H, S
 
 
-def outprod_sym(p, lc_e=4, lc_s=4):
-    """The symmetric gradient pass (unordered pairs) emulated on the host."""
-    L = lib()
-    c = _consts(p)
+def _pass(p, mode, variant, lc, npc, sms):
+    args, keep = _problem(p)
     x = np.ascontiguousarray(p.x)
-    f = np.zeros(1)
-    g = np.zeros(x.size)
-    H = np.zeros((p.K, p.K))
-    S = np.zeros((p.K, p.K))
-    fn = L.emu_outprod_sym
-    fn.restype = ctypes.c_int
-    rc = fn(ctypes.c_int(p.n), ctypes.c_int(p.nst), ctypes.c_int(p.K), ctypes.c_double(p.efs),
-            *[ctypes.c_void_p(_p(a)) for a in c], ctypes.c_void_p(_p(x)), ctypes.c_int(lc_e), ctypes.c_int(lc_s),
-            ctypes.c_void_p(_p(f)), ctypes.c_void_p(_p(g)), ctypes.c_void_p(_p(H)), ctypes.c_void_p(_p(S)))
+    f, g = np.zeros(1), np.full(x.size, np.nan)
+    H, S = np.zeros((p.K, p.K)), np.zeros((p.K, p.K))
+    rc = simt().simt_outprod(*args, ctypes.c_void_p(_p(x)), *[ctypes.c_int(v) for v in (mode, variant, lc, npc, sms)],
+                             *[ctypes.c_void_p(_p(a)) for a in (f, g, H, S)])
     return rc, float(f[0]), g, H, S
 
 
-def outprod_fused(p, lc_s=4):
-    """The fused energy + symmetric gradient pass emulated on the host."""
-    L = lib()
-    c = _consts(p)
-    x = np.ascontiguousarray(p.x)
-    f = np.zeros(1)
-    g = np.zeros(x.size)
-    H = np.zeros((p.K, p.K))
-    S = np.zeros((p.K, p.K))
-    fn = L.emu_outprod_fused
-    fn.restype = ctypes.c_int
-    rc = fn(ctypes.c_int(p.n), ctypes.c_int(p.nst), ctypes.c_int(p.K), ctypes.c_double(p.efs),
-            *[ctypes.c_void_p(_p(a)) for a in c], ctypes.c_void_p(_p(x)), ctypes.c_int(lc_s),
-            ctypes.c_void_p(_p(f)), ctypes.c_void_p(_p(g)), ctypes.c_void_p(_p(H)), ctypes.c_void_p(_p(S)))
-    return rc, float(f[0]), g, H, S
+def outprod_sym(p, lc_e=4, lc_s=4, variant=2, sms=148):
+    """The symmetric gradient pass (unordered pairs, E known) emulated on the host.
+    variant: 0 one-warp tiles, 1 with ket records re-read, 2 staged, 8 / 12 / 16 blocks of
+    that many warps on a GPU of `sms` SMs."""
+    return _pass(p, 1, variant, lc_s, 1, sms)
+
+
+def outprod_fused(p, lc_s=4, variant=2, npc=1, sms=148):
+    """The fused energy + symmetric gradient pass emulated on the host; npc: splits of
+    the symmetry terms of one-warp tiles."""
+    return _pass(p, 2, variant, lc_s, npc, sms)
 
 
 def rrms(p, terms):
@@ -169,40 +184,33 @@ class EmuShardOps:
         self.n, self.blk = p.n, p.blk
         self.ps = p.n * (p.n + 1) // 2 + 1 + 3 * p.n
         self.device = torch.device("cpu")
-        self._sumH = self._sumS = None
+        self._sums = None
         self._status = 0
 
     def _call_pairs(self, x, K, t0, t1):
-        L = lib()
-        c = _consts(self.p)
-        rows = np.zeros(2 * K)
-        sH = np.zeros(self.ps * K)
-        sS = np.zeros(self.ps * K)
-        nt = ctypes.c_int(0)
-        fn = L.emu_shard_pairs
-        fn.restype = ctypes.c_int
-        rc = fn(ctypes.c_int(self.p.n), ctypes.c_int(self.p.nst), ctypes.c_int(K), ctypes.c_double(self.p.efs),
-                *[ctypes.c_void_p(_p(a)) for a in c], ctypes.c_void_p(_p(x)), ctypes.c_int(self.lc),
-                ctypes.c_int(t0), ctypes.c_int(t1), ctypes.c_void_p(_p(rows)), ctypes.c_void_p(_p(sH)),
-                ctypes.c_void_p(_p(sS)), ctypes.byref(nt))
-        return rc, rows, sH, sS, nt.value
+        args, keep = _problem(self.p)
+        rows, nt = np.zeros(2 * K), ctypes.c_int(0)
+        sums = np.zeros(4 * (self.ps + 1) * K)
+        rc = simt().simt_shard_pairs(*args, ctypes.c_void_p(_p(x)), ctypes.c_int(self.lc), ctypes.c_int(t0), ctypes.c_int(t1),
+                                     ctypes.c_void_p(_p(rows)), ctypes.c_void_p(_p(sums)), ctypes.byref(nt))
+        return rc, rows, sums, nt.value
 
     def tiles(self, K):
         x = np.ascontiguousarray(self.p.x)
-        rc, _, _, _, nt = self._call_pairs(x, K, 0, 0)
+        rc, _, _, nt = self._call_pairs(x, K, 0, 0)
         assert rc >= 0
         return nt
 
     def pairs(self, x, K, t0, t1):
         xn = np.ascontiguousarray(x.numpy())
-        rc, rows, self._sumH, self._sumS, _ = self._call_pairs(xn, K, t0, t1)
+        rc, rows, self._sums, _ = self._call_pairs(xn, K, t0, t1)
         assert rc >= 0
         self._status = 2 if rc & 1 else (3 if rc & 2 else 0)
         return self.torch.from_numpy(rows)
 
     def grad(self, x, K, rows, t0, t1):
         # the finalize kernel: E, norm and GRADC from the summed rows
-        xn = x.numpy()
+        xn = np.ascontiguousarray(x.numpy())
         C = xn[K * self.blk:]
         r = rows.numpy()
         cHc, cSc = float(C @ r[:K]), float(C @ r[K:])
@@ -210,20 +218,20 @@ class EmuShardOps:
         g = np.zeros(K * self.blk + K)
         g[K * self.blk:] = 2.0 * norm * (r[:K] - E * r[K:])
         self._norm = norm
-        sums = self._sumH - E * self._sumS
+        args, keep = _problem(self.p)
+        fields = np.zeros(self.ps * K)
+        rc = simt().simt_shard_fields(*args, ctypes.c_void_p(_p(xn)), ctypes.c_void_p(_p(self._sums)), ctypes.c_double(E),
+                                      ctypes.c_double(norm), ctypes.c_void_p(_p(fields)))
+        assert rc == 0
         return (self.torch.tensor([E], dtype=self.torch.float64), self.torch.from_numpy(g),
-                self.torch.from_numpy(sums))
+                self.torch.from_numpy(fields))
 
     def finish(self, x, K, sums, g):
-        L = lib()
-        c = _consts(self.p)
+        args, keep = _problem(self.p)
         gn = np.ascontiguousarray(g.numpy()).copy()
-        fn = L.emu_shard_finish
-        fn.restype = ctypes.c_int
-        fn(ctypes.c_int(self.p.n), ctypes.c_int(self.p.nst), ctypes.c_int(K), ctypes.c_double(self.p.efs),
-           *[ctypes.c_void_p(_p(a)) for a in c], ctypes.c_void_p(_p(np.ascontiguousarray(x.numpy()))),
-           ctypes.c_void_p(_p(np.ascontiguousarray(sums.numpy()))), ctypes.c_double(self._norm),
-           ctypes.c_void_p(_p(gn)))
+        xn, sn = np.ascontiguousarray(x.numpy()), np.ascontiguousarray(sums.numpy())
+        simt().simt_shard_finish(*args, ctypes.c_void_p(_p(xn)), ctypes.c_void_p(_p(sn)), ctypes.c_double(self._norm),
+                                 ctypes.c_void_p(_p(gn)))
         return self.torch.from_numpy(gn)
 
     def status(self):
