@@ -91,14 +91,15 @@ struct FusedSmem {
     double *sket;  // SKET: two ket-record buffers of this warp (16-byte aligned)
 };
 
-// term_raw's output in a tile: the weighted raw values are added to the lane's
-// bra accumulators and, for the ket, summed over lane pairs into the warp's
-// table.  Lanes 2i and 2i+1 exchange one value per pair of fields: lane 2i keeps
-// the first field, lane 2i+1 the second, each adds its partner's, and both store
-// to row i (one select-and-shuffle per two fields, and half the rows to sum).
+// term_raw's output in a tile: the bra's weighted raw values are added to the lane's
+// accumulators, the ket's summed over lane pairs into the warp's table.  Lanes 2i and
+// 2i+1 exchange one value per pair of fields: lane 2i keeps the first field, lane
+// 2i+1 the second, each adds its partner's, and both store to row i (one
+// select-and-shuffle per two fields, and half the rows to sum).
 // KE (E known): the S fields go to the bra only, and H's are the combined ones.
 template <int N, bool KE> struct TileOutput {
     using RP = RawPairs<N>;
+    static constexpr bool kets = true, ket_s = !KE;
     static constexpr int PB = SumFields<N>::size, SL = KetSlots<N>::SL;
     double *acc;  // this lane's accumulators: H fields, then S fields, 32 doubles apart
     double *row;  // the lane pair's row, + 8 for the odd lane
@@ -108,52 +109,25 @@ template <int N, bool KE> struct TileOutput {
         wob = wb * ov;
         wok = wk * ov;
     }
-    // The accumulators and the table row are read and written BATCH pairs at a
-    // time: the loads of a batch are issued together, ahead of its arithmetic,
-    // and do not wait for the stores of the pair before (the compiler cannot tell
-    // that a row and an accumulator never alias).
     __device__ __forceinline__ void bra(int f, double v) { acc[f * 32] = fma(wob, v, acc[f * 32]); }
     __device__ __forceinline__ double exchange(double va, double vb) {
         const double send = wok * (odd ? va : vb);
         return fma(wok, odd ? vb : va, __shfl_xor_sync(0xffffffffu, send, 1));
     }
-    // n <= 3: the accumulators and the table row are read and written BATCH pairs at
-    // a time, so that the loads of a batch are issued together, ahead of its
-    // arithmetic, and do not wait for the stores of the pair before (the compiler
-    // cannot tell that rows and accumulators never alias).  H2 K = 2048 on a B200,
-    // 16 warps per SM: 761 us pair by pair, 740 in batches of 5; at n = 5 the
-    // registers a batch holds cost more (2336 us pair by pair, 2364 to 2450).
-    static constexpr int BATCH = N > 3 ? 1 : 5;
-    double av[2 * BATCH], rv[BATCH];
-    template <bool H, int E> __device__ __forceinline__ void put(double va, double vb) {
-        constexpr int off = H ? 0 : PB, b = E % BATCH, e0 = E - b, base = H ? 0 : SL;
-        constexpr bool ket = H || !KE;
-        if constexpr (BATCH == 1) {
-            constexpr int i = H ? RP::h_pair(E) : E;
-            if constexpr (ket) row[base + KetSlots<N>::of_pair(i)] = exchange(va, vb);
-            bra(off + RP::fa(i), va);
-            bra(off + RP::fb(i), vb);
-        } else {
-            if constexpr (b == 0)
-                unrolled<e0, (e0 + BATCH < RP::paired ? e0 + BATCH : RP::paired)>([&](auto q) {
-                    constexpr int e = decltype(q)::value, i = H ? RP::h_pair(e) : e;
-                    av[2 * (e - e0)] = acc[(off + RP::fa(i)) * 32];
-                    av[2 * (e - e0) + 1] = acc[(off + RP::fb(i)) * 32];
-                });
-            av[2 * b] = fma(wob, va, av[2 * b]);
-            av[2 * b + 1] = fma(wob, vb, av[2 * b + 1]);
-            if constexpr (ket) rv[b] = exchange(va, vb);
-            if constexpr (b == BATCH - 1 || E == RP::paired - 1)
-                unrolled<e0, E + 1>([&](auto q) {
-                    constexpr int e = decltype(q)::value, i = H ? RP::h_pair(e) : e;
-                    acc[(off + RP::fa(i)) * 32] = av[2 * (e - e0)];
-                    acc[(off + RP::fb(i)) * 32] = av[2 * (e - e0) + 1];
-                    if constexpr (ket) row[base + KetSlots<N>::of_pair(i)] = rv[e - e0];
-                });
-        }
+    template <int I> __device__ __forceinline__ void sb(double va, double vb) {
+        bra(PB + RP::fa(I), va);
+        bra(PB + RP::fb(I), vb);
     }
-    template <int I> __device__ __forceinline__ void s2(double va, double vb) { put<false, I>(va, vb); }
-    template <int I> __device__ __forceinline__ void h2(double va, double vb) { put<true, RP::h_seq(I)>(va, vb); }
+    template <int I> __device__ __forceinline__ void hb(double va, double vb) {
+        bra(RP::fa(I), va);
+        bra(RP::fb(I), vb);
+    }
+    template <int I> __device__ __forceinline__ void sk(double va, double vb) {
+        row[SL + KetSlots<N>::of_pair(I)] = exchange(va, vb);
+    }
+    template <int I> __device__ __forceinline__ void hk(double va, double vb) {
+        row[KetSlots<N>::of_pair(I)] = exchange(va, vb);
+    }
     __device__ __forceinline__ void scalar(double e2) {
         constexpr int p = KetSlots<N>::of_pair(RP::count - 1);
         bra(RP::scalar, e2);
@@ -166,14 +140,13 @@ template <int N, bool KE> struct TileOutput {
             row[odd ? SL + p - 8 : p] = (odd ? wok : vh) + __shfl_xor_sync(0xffffffffu, send, 1);
         }
     }
-    __device__ __forceinline__ void s1(int, double) {}  // n = 6 has no symmetric passes
-    __device__ __forceinline__ void h1(int, double) {}
+    __device__ __forceinline__ void sb1(int, double) {}  // n = 6 has no symmetric passes
+    __device__ __forceinline__ void hb1(int, double) {}
 };
 
-// One field of fold_raw at run time, from the reduced slots of one matrix (scale 1
-// for H and the combined gradient, 2 for S).
+// One field of fold_raw at run time, from the reduced slots of one matrix.
 template <int N>
-__device__ __noinline__ double fold_slot(const double *slots, double scale, int f, const double *kr) {
+__device__ __noinline__ double fold_slot(const double *slots, int f, const double *kr) {
     using KL = KetLayout<N>;
     constexpr int TR = tri(N);
     auto r = [&](int q) {
@@ -181,32 +154,20 @@ __device__ __noinline__ double fold_slot(const double *slots, double scale, int 
 #pragma unroll
         for (int u = 0; u < Part<N>::size; ++u)
             if (u == q) v = slots[KetSlots<N>::slot(u)];
-        return scale * v;
+        return v;
     };
-    const double F = 0.5 * r(TR);
-    if (f == TR) return 0.75 * F;
-    if (f < TR) {
-        int i = 0;
-        while ((i + 1) * (i + 2) / 2 <= f) ++i;
-        const int j = f - i * (i + 1) / 2;
-        double v = r(f);
-        for (int c = 0; c < 3; ++c) {
-            const double si = kr[KL::Sp + 3 * i + c], sj = kr[KL::Sp + 3 * j + c];
-            v += r(TR + 1 + 3 * i + c) * sj + si * r(TR + 1 + 3 * j + c) - 2.0 * F * si * sj;
-        }
-        return 0.5 * v;
-    }
+    if (f == TR) return 0.375 * r(TR);
+    if (f < TR) return 0.5 * r(f);
     const int i = (f - TR - 1) / 3, c = (f - TR - 1) - 3 * i;
-    double v = -2.0 * F * kr[KL::ASp + 3 * i + c];
+    double v = 0.0;
     for (int k = 0; k < N; ++k) v += kr[KL::Ap + (i >= k ? i * (i + 1) / 2 + k : k * (k + 1) / 2 + i)] * r(TR + 1 + 3 * k + c);
     return v;
 }
 
 // One tile of the pair passes over unordered pairs (k >= l).  Each term gives
-// the raw values of term_raw (h, ov and their derivatives with respect to B and
-// e, the same for the bra and the ket); the bra's weighted sums stay in the
-// lane's accumulators, the ket's are summed over the warp per (l, P), mapped to
-// l's frame and summed over P.
+// the raw values of term_raw (h, ov and their derivatives for the bra and for the
+// ket); the bra's weighted sums stay in the lane's accumulators, the ket's are
+// summed over the warp per (l, P), mapped to l's frame and summed over P.
 //   !KE, the fused pass: H_kl = H_lk and S_kl are the sums over P of h and ov,
 //        written when H is not null and always summed into the rows of H C and
 //        S C (SumFields::row); the H and S fields are kept apart, since E is not
@@ -351,7 +312,7 @@ __device__ __forceinline__ void fsym_tile(int t, int2 tl, int LC, int K, int nst
 #pragma unroll
                 for (int q = 0; q < NC; ++q) {
                     const int wq = which + q;
-                    v[q] = mine ? (wq ? 0.5 : 1.0) * fold_slot<N>(kred + wq * SL, wq ? 2.0 : 1.0, fld, krg) : 0.0;
+                    v[q] = mine ? fold_slot<N>(kred + wq * SL, fld, krg) : 0.0;
                 }
                 __syncwarp();
 #pragma unroll
@@ -605,10 +566,9 @@ template <int N> struct FinishSmem {
     static constexpr int r = 0;                    // combined raw sums, then the gradient fields
     static constexpr int s = r + PS * 32;          // the bra's S sums, then the output
     static constexpr int out = s;                  // blk x 32, basis-major with an odd stride (<= PS)
-    static constexpr int rec = s + PS * 32;        // A, S, AS and L of the 32 bases
-    static constexpr int y = rec + (tri(N) + 6 * N + tri(N)) * 32;
-    static constexpr int p = y + 3 * N * 32;
-    static constexpr int MA = p + 3 * N * 32;
+    static constexpr int rec = s + PS * 32;        // A and L of the 32 bases
+    static constexpr int y = rec + 2 * tri(N) * 32;
+    static constexpr int MA = y + 3 * N * 32;
     static constexpr int size = MA + N * N * 32;
     static_assert((blk | 1) <= PS, "the output fits where the S sums were");
     // more than 48 KB would need the opt-in and another split of the SM's L1 (n = 5
@@ -636,7 +596,7 @@ __device__ __forceinline__ bool finish_block(const double *__restrict__ sums, in
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k = min(kb * 32 + lane, K - 1);
     const int nk = min(32, K - kb * 32);
-    constexpr int A = FS::rec, S = A + TR * 32, AS = S + 3 * N * 32, L = AS + 3 * N * 32;
+    constexpr int A = FS::rec, L = A + TR * 32;
     const double *bk = bra_at<N>(bra, K, k);
     auto ket = [&](int f) {  // the kets' combined sum (folded: their gradient)
         const double *q = sums + (size_t)(2 * PB + f) * K + k;
@@ -653,26 +613,20 @@ __device__ __forceinline__ bool finish_block(const double *__restrict__ sums, in
         sm[FS::s + f * 32 + lane] = bs;
     }
 #pragma unroll
-    for (int f = w; f < TR + 6 * N; f += 8) {  // A, S, AS are fields 0 .. of the record
-        static_assert(BL::A == 0 && BL::S == TR && BL::AS == TR + 3 * N, "record order");
-        sm[A + f * 32 + lane] = bk[f * 32];
+    for (int f = w; f < TR; f += 8) {
+        sm[A + f * 32 + lane] = bk[(BL::A + f) * 32];
+        sm[L + f * 32 + lane] = bk[(BL::L + f) * 32];
     }
-#pragma unroll
-    for (int f = w; f < TR; f += 8) sm[L + f * 32 + lane] = bk[(BL::L + f) * 32];
     __syncthreads();
     auto at = [&](int base, int f) -> double & { return sm[base + f * 32 + lane]; };
     const int i = w;  // this warp's matrix row
     if (i < N) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            double v = at(AS, 3 * i + c) * at(FS::s, TR), p = 0.0;
+            double v = 0.0;
 #pragma unroll
-            for (int q = 0; q < N; ++q) {
-                v -= at(A, sx(i, q)) * at(FS::s, TR + 1 + 3 * q + c);
-                p += cs.M[i * N + q] * at(AS, 3 * q + c);
-            }
+            for (int q = 0; q < N; ++q) v += at(A, sx(i, q)) * at(FS::s, TR + 1 + 3 * q + c);
             at(FS::y, 3 * i + c) = v;
-            at(FS::p, 3 * i + c) = p;
         }
 #pragma unroll
         for (int j = 0; j < N; ++j) {
@@ -689,17 +643,13 @@ __device__ __forceinline__ bool finish_block(const double *__restrict__ sums, in
             double v = 0.0;
 #pragma unroll
             for (int q = 0; q < N; ++q) v += cs.M[i * N + q] * at(FS::y, 3 * q + c);
-            at(FS::r, TR + 1 + 3 * i + c) -= 8.0 * v;
+            at(FS::r, TR + 1 + 3 * i + c) += 8.0 * v;
         }
         for (int j = 0; j <= i; ++j) {
             double v = 3.0 * cs.M[i * N + j] * at(FS::s, TR);
 #pragma unroll
             for (int q = 0; q < N; ++q)
                 v += 2.0 * (at(FS::MA, i * N + q) * at(FS::s, sx(q, j)) + at(FS::s, sx(i, q)) * at(FS::MA, j * N + q));
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                v += 2.0 * (at(FS::s, TR + 1 + 3 * i + c) * at(FS::p, 3 * j + c) +
-                            at(FS::p, 3 * i + c) * at(FS::s, TR + 1 + 3 * j + c));
             at(FS::r, sx(i, j)) += 4.0 * v;
         }
     }
@@ -709,20 +659,14 @@ __device__ __forceinline__ bool finish_block(const double *__restrict__ sums, in
     double gs[3];
     if (i < N) {
         for (int j = 0; j <= i; ++j) {
-            double v = 0.0;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const double si = at(S, 3 * i + c), sj = at(S, 3 * j + c);
-                v += at(FS::r, TR + 1 + 3 * i + c) * sj + si * at(FS::r, TR + 1 + 3 * j + c) - 2.0 * F * si * sj;
-            }
-            v = 0.5 * (at(FS::r, sx(i, j)) + v);
+            const double v = 0.5 * at(FS::r, sx(i, j));
             at(FS::r, sx(i, j)) = folded ? v + ket(sx(i, j)) : v;
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            double v = -2.0 * F * at(AS, 3 * i + c);
+            double v = at(A, sx(i, 0)) * at(FS::r, TR + 1 + c);
 #pragma unroll
-            for (int q = 0; q < N; ++q) v += at(A, sx(i, q)) * at(FS::r, TR + 1 + 3 * q + c);
+            for (int q = 1; q < N; ++q) v += at(A, sx(i, q)) * at(FS::r, TR + 1 + 3 * q + c);
             gs[c] = folded ? v + ket(TR + 1 + 3 * i + c) : v;
         }
     }

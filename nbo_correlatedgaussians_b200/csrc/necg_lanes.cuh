@@ -247,19 +247,20 @@ template <int N> struct Part {
 // Raw sums of one bra over its terms (term_raw's `out`): H and S fields into two
 // accumulators (g(t), d(), s(t)), weight w ov.
 template <int N, typename R, typename ACC> struct BraSums {
+    static constexpr bool kets = false, ket_s = false;
     ACC &H, &S;
     R w, wo;
     NECG_HD static R &at(ACC &a, int f) { return f < tri(N) ? a.g(f) : f == tri(N) ? a.d() : a.s(f - tri(N) - 1); }
     NECG_HD void begin(R ov) { wo = w * ov; }
-    NECG_HD void s1(int f, R v) { at(S, f) += wo * v; }
-    NECG_HD void h1(int f, R v) { at(H, f) += wo * v; }
-    template <int I> NECG_HD void s2(R va, R vb) {
-        s1(RawPairs<N>::fa(I), va);
-        s1(RawPairs<N>::fb(I), vb);
+    NECG_HD void sb1(int f, R v) { at(S, f) += wo * v; }
+    NECG_HD void hb1(int f, R v) { at(H, f) += wo * v; }
+    template <int I> NECG_HD void sb(R va, R vb) {
+        sb1(RawPairs<N>::fa(I), va);
+        sb1(RawPairs<N>::fb(I), vb);
     }
-    template <int I> NECG_HD void h2(R va, R vb) {
-        h1(RawPairs<N>::fa(I), va);
-        h1(RawPairs<N>::fb(I), vb);
+    template <int I> NECG_HD void hb(R va, R vb) {
+        hb1(RawPairs<N>::fa(I), va);
+        hb1(RawPairs<N>::fb(I), vb);
     }
     NECG_HD void scalar(R e2) {
         H.d() += wo * e2;
@@ -290,14 +291,12 @@ NECG_HD bool grad_lane(const BA &b, const KB &ket, int l0, int l1, int nst, cons
     R r[PS], o[PS];
     const auto sr = [&](int f) { return BraSums<N, R, ACC>::at(accS, f); };
     const auto A = [&](int t) { return b(BL::A + t); };
-    const auto s = [&](int t) { return b(BL::S + t); };
-    const auto e = [&](int t) { return b(BL::AS + t); };
 #pragma unroll
     for (int f = 0; f < PS; ++f) r[f] = BraSums<N, R, ACC>::at(accH, f);
-    explicit_tau<N>(sr, A, e, cs, r);
+    explicit_tau<N>(sr, A, cs, r);
 #pragma unroll
     for (int f = 0; f < PS; ++f) r[f] = lam * r[f] - 2.0 * E * sr(f);
-    fold_raw<N>(FieldsOf<R>{r}, A, s, e, o);
+    fold_raw<N>(FieldsOf<R>{r}, A, o);
 #pragma unroll
     for (int f = 0; f < PS; ++f) part[f * stride] = val(o[f]);
     return ok;

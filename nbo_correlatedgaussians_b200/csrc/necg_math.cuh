@@ -13,9 +13,9 @@
 //   A_k, A_l' = P^T A_l P    symmetric, packed lower (N(N+1)/2)
 //   S_k, S_l' = sms s_l      n x 3 (row = particle, column = x, y, z)
 //   B = A_k + A_l', Bi = B^-1, e = A_k S_k + A_l' S_l', T = Bi e   (st in the reference)
-//   D = T - S_k, N = A_k M A_k, U = 1.5 Bi + T T^T
+//   D_k = T - S_k, D_l = T - S_l', N = A_k M A_k, U_s = 1.5 Bi + D_s D_s^T
 //   ov  = sqrt(8^n) (|L_k| |L_l|)^{3/2} / |B|^{3/2} exp(<e,T> - i1 - i2)
-//   tau = 3 tr(M A_k) - 3 <N, Bi> - 2 <D, N D>,   tk = 2 ov tau
+//   tau = 3 tr(M A_k) - 3 <N, Bi> - 2 <D_k, N D_k>,   tk = 2 ov tau
 //   rho = sum_v c_v F0(|v^T T|^2 / v^T Bi v) (v^T Bi v)^{-1/2}, ert = ov rho
 //   sig = efs sum_i q_i T[i,z],  zht = ov sig
 //   eta = 2 tau + rho - sig,  h = tk + ert - zht = ov eta
@@ -24,22 +24,23 @@
 //
 // Gradient.  h and ov depend on the pair through B and e alone, apart from
 // factors of one side only: |L_k|^{3/2} exp(-i1) of each side, and tau, which is
-// written with the bra's A_k and e_k = A_k S_k.  With F0's derivative pieces
+// written with the bra's A_k and s_k.  With F0's derivative pieces
 //   Z' = sum_v alpha_v v b_v^T - (efs/2) q e_z^T,  W = sum_v beta_v v v^T,
 //   alpha_v = c_v F0'(z) a^{-3/2},  beta_v = c_v a^{-3/2} (z F0'(z) + F0(z)/2),
-//   Q = Bi (Z' - 4 N D)
-// the derivatives with respect to B and e are
-//   dh/dB = ov (Bi (6 N + W) Bi - Q T^T - T Q^T - eta U),  dh/de = 2 ov (Q + eta T)
-//   dS/dB = -ov U,                                         dS/de = 2 ov T
-// and serve the bra and the ket alike (term_raw).  A basis function sums them
-// over its terms as they are; what depends on its own A, s and e (the chain
-// from e = A s, its prefactors, and the bra's explicit share of tau) multiplies
-// only those sums, once per basis function (fold_raw, explicit_tau).  That
-// takes the products with A_k, A_l', S_k and S_l', the second sandwich and the
-// second outer products out of the term: 2816 instead of 4374 FLOP at n = 5 and
-// 1075 instead of 1626 at n = 3.  The FP64 pipe bounds the pair passes; whole
-// evaluations on a B200 went from 3.53 to 2.35 ms (LiH K = 1024), 1.06 to 0.76 ms
-// (H2 K = 2048) and 0.34 to 0.27 ms (He K = 2032).
+//   Q = Bi (Z' - 4 N D_k)
+// the derivatives with respect to A_s and e_s = A_s S_s of side s = k, l through B
+// and e, with the origin moved to that side's S_s, are
+//   dh:  ov (Bi (6 N + W) Bi - Q D_s^T - D_s Q^T - eta U_s),  2 ov (Q + eta D_s)
+//   dS: -ov U_s,                                               2 ov D_s
+// (term_raw).  A basis function sums them over its terms as they are; what depends
+// on its own A (the chain from e = A s, and the bra's explicit share of tau)
+// multiplies only those sums, once per basis function (fold_raw, explicit_tau).
+// That takes the products with A_k and A_l' and the second sandwich out of the term:
+// fewer operations than a term that forms its own gradients by a third (n = 5).
+// The origin: with T in the place of D_s both sides would share all values, 180
+// operations less at n = 5, but the sums of a function away from the origin would
+// hold differences |s|^2 A times as large as themselves (components of dF/dL of tight
+// functions lost 10 to 50 times the rounding error).
 // The A^-1 term (coefficient D = 0.75 F) maps to vech(dF/dL) as 2 D / L_ii
 // on the diagonal only, so it is kept as one scalar per basis function.
 //
@@ -681,10 +682,10 @@ template <int A, int END, typename F> NECG_HD void unrolled(F &&f) {
 
 // Fields of the raw sums of one basis function (Part<N>::size of them, the same
 // count and order as the partial buffers): G[tri] (derivative with respect to
-// B), one scalar, g[3N] (derivative with respect to e).  Raw values of one term,
-// before the weight w ov:
-//   H:  X = 2 (Bi (6 N + W) Bi - Q T^T - T Q^T - eta U),  2 eta,  2 (Q + eta T)
-//   S:  -U,                                               1,      T
+// A through B and e), one scalar, g[3N] (derivative with respect to e).  Raw values of
+// one term for side s, before the weight w ov:
+//   H:  X = 2 (Bi (6 N + W) Bi - Q D_s^T - D_s Q^T - eta U_s),  2 eta,  2 (Q + eta D_s)
+//   S:  -U_s,                                                   1,      D_s
 // so that H - 2 E S holds twice the G, twice the scalar and once the g of the
 // gradient of h - E ov.  term_raw hands the fields out in pairs, for outputs
 // that combine two values at a time: pair i < tri holds G_i and g_i, the
@@ -701,22 +702,6 @@ template <int N> struct RawPairs {
     __host__ __device__ static constexpr int pair_of(int f) {
         return f < T ? f : f == T ? count - 1 : f - T - 1 < lead ? f - T - 1 : lead + (f - T - 1 - lead) / 2;
     }
-    // the pairs in the order in which the H values are formed (X by columns)
-    __host__ __device__ static constexpr int h_pair(int e) {
-        if (e >= lead) return e;
-        int j = 0, n = N;
-        while (e >= n) {
-            e -= n;
-            --n;
-            ++j;
-        }
-        return sx(j + e, j);
-    }
-    __host__ __device__ static constexpr int h_seq(int i) {
-        int e = 0;
-        while (h_pair(e) != i) ++e;
-        return e;
-    }
     // fields of pair i
     __host__ __device__ static constexpr int fa(int i) { return i < lead ? i : T + 1 + lead + 2 * (i - lead); }
     __host__ __device__ static constexpr int fb(int i) {
@@ -728,17 +713,90 @@ template <int N> struct RawPairs {
     }
 };
 
+// The raw values of one side (KET: the ket's) handed to `out`, pair by pair.
+template <int N, bool KET, int I, typename R, typename OUT> NECG_HD void put_s(OUT &out, R va, R vb) {
+    if constexpr (KET) out.template sk<I>(va, vb);
+    else out.template sb<I>(va, vb);
+}
+template <int N, bool KET, int I, typename R, typename OUT> NECG_HD void put_h(OUT &out, R va, R vb) {
+    if constexpr (KET) out.template hk<I>(va, vb);
+    else out.template hb<I>(va, vb);
+}
+// S: -U = -(1.5 Bi + D D^T), D, 1
+#pragma nv_exec_check_disable
+template <int N, bool KET, typename R, typename OUT>
+NECG_HD void raw_s(const R (&Bi)[tri(N)], const R (&D)[3 * N], OUT &out) {
+    using RP = RawPairs<N>;
+    unrolled<0, N>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        unrolled<0, i + 1>([&](auto jc) {
+            constexpr int j = decltype(jc)::value, t = sx(i, j);
+            R u = 1.5 * Bi[t];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) u += D[3 * i + c] * D[3 * j + c];
+            if constexpr (t < RP::lead) put_s<N, KET, t, R>(out, -u, D[t]);
+            else if constexpr (!KET) out.sb1(t, -u);
+        });
+    });
+    unrolled<0, RP::left / 2>([&](auto qc) {
+        constexpr int q = decltype(qc)::value;
+        put_s<N, KET, RP::lead + q, R>(out, D[RP::lead + 2 * q], D[RP::lead + 2 * q + 1]);
+    });
+    if constexpr (RP::odd) put_s<N, KET, RP::count - 1, R>(out, D[3 * N - 1], R(1.0));
+}
+// H's entry (i, j): x = (Bi W Bi - 1.5 et Bi)_ij less Q' D^T + D Q'^T, and its g = Q' + et D / 2
+#pragma nv_exec_check_disable
+template <int N, bool KET, int I, int J, typename R, typename OUT>
+NECG_HD void raw_h(R x, const R (&D)[3 * N], const R (&Q)[3 * N], R eh, OUT &out) {
+    constexpr int t = sx(I, J);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        x -= Q[3 * I + c] * D[3 * J + c];
+        x -= D[3 * I + c] * Q[3 * J + c];
+    }
+    if constexpr (t < RawPairs<N>::lead) put_h<N, KET, t, R>(out, x, Q[t] + eh * D[t]);
+    else if constexpr (!KET) out.hb1(t, x);
+}
+// the remaining g
+#pragma nv_exec_check_disable
+template <int N, bool KET, typename R, typename OUT>
+NECG_HD void raw_h_rest(const R (&D)[3 * N], const R (&Q)[3 * N], R eh, R et, OUT &out) {
+    using RP = RawPairs<N>;
+    unrolled<0, RP::left / 2>([&](auto qc) {
+        constexpr int q = decltype(qc)::value, u = RP::lead + 2 * q;
+        put_h<N, KET, RP::lead + q, R>(out, Q[u] + eh * D[u], Q[u + 1] + eh * D[u + 1]);
+    });
+    if constexpr (RP::odd) put_h<N, KET, RP::count - 1, R>(out, Q[3 * N - 1] + eh * D[3 * N - 1], et);
+}
+// all of one side's H values from X = Bi W Bi - 1.5 et Bi and Q
+#pragma nv_exec_check_disable
+template <int N, bool KET, typename R, typename OUT>
+NECG_HD void raw_h_side(const R (&X)[tri(N)], const R (&D)[3 * N], const R (&Q)[3 * N], R eh, R et, OUT &out) {
+    R Qs[3 * N];
+#pragma unroll
+    for (int t = 0; t < 3 * N; ++t) Qs[t] = Q[t] + eh * D[t];
+    unrolled<0, N>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        unrolled<0, i + 1>([&](auto jc) {
+            constexpr int j = decltype(jc)::value;
+            raw_h<N, KET, i, j, R>(X[sx(i, j)], D, Qs, eh, out);
+        });
+    });
+    raw_h_rest<N, KET, R>(D, Qs, eh, et, out);
+}
 // One (k, l, P) term: the overlap and the raw values above, handed to `out`:
 //   out.begin(ov)              once, first
-//   out.s2<i>(va, vb)          pair i of the S values, i = 0, 1, ...
-//   out.h2<i>(va, vb)          pair i of the H values (in the order h_pair), with
-//                              eta - E2 / 2 in the place of eta (E2 = 2 E gives the
-//                              gradient of h - E ov)
+//   out.sb<i>(va, vb), sk<i>   pair i of the bra's / the ket's S values
+//   out.hb<i>(va, vb), hk<i>   pair i of the bra's / the ket's H values, with eta - E2 / 2
+//                              in the place of eta (E2 = 2 E gives the gradient of h - E ov)
 //   out.scalar(eta2)           the scalar pair when it holds nothing else
-//   out.s1 / out.h1(f, v)      single fields (n = 6 only)
+//   out.sb1 / out.hb1(f, v)    single fields (n = 6 only, which has no ket side)
+// OUT::kets: the ket's values are wanted; OUT::ket_s: its S values too.
 // eta2_out = 2 eta (so h = ov eta2_out / 2).  The S values leave before the
-// Coulomb sum, so that U is not live across it (n = 5, 255 registers: 15 FP64
-// operations fewer with U kept, but 64 bytes of spill, 2.37 against 2.34 ms).
+// Coulomb sum, so that U is not live across it, and D_k and D_l are formed again
+// after it for the same reason.  One side's values leave after the other's: side by
+// side saves a few operations and costs registers (LiH K = 1024 on a B200: 2.50 ms,
+// 2.52 with H's and 2.53 with S's two sides in one loop).
 #pragma nv_exec_check_disable
 template <int N, typename R, typename BA, typename KA, typename OUT>
 NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT &out, R &eta2_out, R &ov_out) {
@@ -750,26 +808,15 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
     const bool ok = term_core<N>(b, kr, Bi, T, ov);
     ov_out = ov;
     out.begin(ov);
-    // S: -U = -(1.5 Bi + T T^T), T, 1
-    unrolled<0, N>([&](auto ic) {
-        constexpr int i = decltype(ic)::value;
-        unrolled<0, i + 1>([&](auto jc) {
-            constexpr int j = decltype(jc)::value, t = sx(i, j);
-            R u = 1.5 * Bi[t];
+    if constexpr (OUT::ket_s) {
+        R D[V];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) u += T[3 * i + c] * T[3 * j + c];
-            if constexpr (t < RP::lead) out.template s2<t>(-u, T[t]);
-            else out.s1(t, -u);
-        });
-    });
-    unrolled<0, RP::left / 2>([&](auto qc) {
-        constexpr int q = decltype(qc)::value;
-        out.template s2<RP::lead + q>(T[RP::lead + 2 * q], T[RP::lead + 2 * q + 1]);
-    });
-    if constexpr (RP::odd) out.template s2<RP::count - 1>(T[V - 1], R(1.0));
-    // tau and the bra's part of Q's right-hand side: V8 = -8 N D, D = T - S_k;
+        for (int t = 0; t < V; ++t) D[t] = T[t] - kr[KL::Sp + t];
+        raw_s<N, true, R>(Bi, D, out);
+    }
+    // tau and the bra's part of Q's right-hand side: V8 = -8 N D, D = D_k;
     // 4 tau = 12 tr(M A_s) + 1.5 <-8 N_s, Bi> + <D, V8>.  The trace cancels for the
-    // tighter side (term_value), so it is formed with both and the one of the
+    // tighter side (term_tau2), so it is formed with both and the one of the
     // smaller tr(M A) taken: tri(N) products more, where selecting N_s would take
     // twice as many instructions.
     R Z[V], W[TR], eta2;
@@ -777,6 +824,7 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
         R D[V];
 #pragma unroll
         for (int t = 0; t < V; ++t) D[t] = T[t] - b(BL::S + t);
+        raw_s<N, false, R>(Bi, D, out);
         R dg = R(0.0), od = R(0.0), dl = R(0.0), ol = R(0.0);
 #pragma unroll
         for (int i = 0; i < N; ++i)
@@ -826,24 +874,24 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
     const R rho = coulomb_grad<N>(Bi, T, cs, Z, W);
     eta2 += 2.0 * rho;
     eta2_out = eta2;
-    const R et = eta2 - E2;
+    const R et = eta2 - E2, eh = 0.5 * et, e15 = 1.5 * et;
     if (!RP::odd) out.scalar(et);
-    // X = Bi W Bi - 1.5 et Bi - Q' T^T - T Q'^T with Q' = Q + et T / 2 (the T T^T
-    // part of et U folded into the outer products); g = Q' + et T / 2
+    // X = Bi W Bi - 1.5 et Bi - Q' D^T - D Q'^T with Q' = Q + et D / 2 (the D D^T
+    // part of et U folded into the outer products); g = Q' + et D / 2.  Up to the
+    // outer products it is the same for both sides.
     R Q[V];
-    const R eh = 0.5 * et;
 #pragma unroll
     for (int i = 0; i < N; ++i)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            R s = eh * T[3 * i + c];
+            R s = Bi[sx(i, 0)] * Z[c];
 #pragma unroll
-            for (int k = 0; k < N; ++k) s += Bi[sx(i, k)] * Z[3 * k + c];
+            for (int k = 1; k < N; ++k) s += Bi[sx(i, k)] * Z[3 * k + c];
             Q[3 * i + c] = s;
         }
-    const R e15 = 1.5 * et;
-    unrolled<0, N>([&](auto jc) {
-        constexpr int j = decltype(jc)::value;
+    R X[TR];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
         R col[N];  // column j of W Bi
 #pragma unroll
         for (int a = 0; a < N; ++a) {
@@ -852,86 +900,70 @@ NECG_HD bool term_raw(const BA &b, const KA &kr, const Consts<N> &cs, R E2, OUT 
             for (int k = 1; k < N; ++k) s += W[sx(a, k)] * Bi[sx(k, j)];
             col[a] = s;
         }
-        unrolled<j, N>([&](auto ic) {
-            constexpr int i = decltype(ic)::value, t = sx(i, j);
-            R s = -(e15 * Bi[t]);
+#pragma unroll
+        for (int i = j; i < N; ++i) {
+            R s = -(e15 * Bi[sx(i, j)]);
 #pragma unroll
             for (int a = 0; a < N; ++a) s += Bi[sx(i, a)] * col[a];
+            X[sx(i, j)] = s;
+        }
+    }
+    {
+        R D[V];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                s -= Q[3 * i + c] * T[3 * j + c];
-                s -= T[3 * i + c] * Q[3 * j + c];
-            }
-            if constexpr (t < RP::lead) out.template h2<t>(s, Q[t] + eh * T[t]);
-            else out.h1(t, s);
-        });
-    });
-    unrolled<0, RP::left / 2>([&](auto qc) {
-        constexpr int q = decltype(qc)::value, u = RP::lead + 2 * q;
-        out.template h2<RP::lead + q>(Q[u] + eh * T[u], Q[u + 1] + eh * T[u + 1]);
-    });
-    if constexpr (RP::odd) out.template h2<RP::count - 1>(Q[V - 1] + eh * T[V - 1], et);
+        for (int t = 0; t < V; ++t) D[t] = T[t] - b(BL::S + t);
+        raw_h_side<N, false, R>(X, D, Q, eh, et, out);
+    }
+    if constexpr (OUT::kets) {
+        R D[V];
+#pragma unroll
+        for (int t = 0; t < V; ++t) D[t] = T[t] - kr[KL::Sp + t];
+        raw_h_side<N, true, R>(X, D, Q, eh, et, out);
+    }
     return ok;
 }
 
-// The gradient of one side from its raw sums.  r: raw fields (H, 2 S, or their
-// combination H - 2 E S), A, s, e = A s of the function in the frame of the sums:
-//   dF/dA = G + (g s^T + s g^T) / 2 - F s s^T + 0.75 F A^-1,   dF/ds = A g - 2 F e
-// with G = r_G / 2, F = r_scalar / 2 and g = r_g.  o: Part<N> fields.
+// The gradient of one side from its raw sums r (H, 2 S, or their combination H - 2 E
+// S) and its A, in the frame of the sums: dF/dA = r_G / 2 + 0.75 F A^-1, F = r_scalar /
+// 2, and dF/ds = A r_g.  o: Part<N> fields.
 #pragma nv_exec_check_disable
-template <int N, typename R, typename RAW, typename FA, typename FS, typename FE>
-NECG_HD void fold_raw(const RAW &r, const FA &A, const FS &s, const FE &e, R (&o)[tri(N) + 1 + 3 * N]) {
+template <int N, typename R, typename RAW, typename FA>
+NECG_HD void fold_raw(const RAW &r, const FA &A, R (&o)[tri(N) + 1 + 3 * N]) {
     constexpr int TR = tri(N);
-    const R F = 0.5 * r(TR);
 #pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int j = 0; j <= i; ++j) {
-            R v = R(0.0);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const R si = s(3 * i + c), sj = s(3 * j + c);
-                v += r(TR + 1 + 3 * i + c) * sj + si * r(TR + 1 + 3 * j + c) - 2.0 * F * si * sj;
-            }
-            o[sx(i, j)] = 0.5 * (r(sx(i, j)) + v);
-        }
-    o[TR] = 0.75 * F;
+    for (int t = 0; t < TR; ++t) o[t] = 0.5 * r(t);
+    o[TR] = 0.375 * r(TR);
 #pragma unroll
     for (int i = 0; i < N; ++i)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            R v = -2.0 * F * e(3 * i + c);
+            R v = A(sx(i, 0)) * r(TR + 1 + c);
 #pragma unroll
-            for (int k = 0; k < N; ++k) v += A(sx(i, k)) * r(TR + 1 + 3 * k + c);
+            for (int k = 1; k < N; ++k) v += A(sx(i, k)) * r(TR + 1 + 3 * k + c);
             o[TR + 1 + 3 * i + c] = v;
         }
 }
 
 // The bra's explicit share of dh through tau, added to its combined raw sums r:
-// tau depends on A_k and e_k = A_k S_k directly (not through B and e), so that
-// with the bra's raw S sums s = (-U, 1, T) and p = M e_k
-//   dh/dA_k |_{e_k} += 2 (3 M s_1 + 2 (M A s_U + s_U A M) + 2 (s_T p^T + p s_T^T))
-//   dh/de_k         += -8 M (e_k s_1 - A s_T)
+// tau depends on A_k and s_k directly (not through B and e).  With the bra's raw S
+// sums s = (-U_k, 1, D_k)
+//   dh/dA_k += 2 (3 M s_1 + 2 (M A s_U + s_U A M)),   dh/de_k += 8 M A s_D
 // (r's G is held twice).
 #pragma nv_exec_check_disable
-template <int N, typename R, typename SRAW, typename FA, typename FE>
-NECG_HD void explicit_tau(const SRAW &sr, const FA &A, const FE &e, const Consts<N> &cs,
-                          R (&r)[tri(N) + 1 + 3 * N]) {
+template <int N, typename R, typename SRAW, typename FA>
+NECG_HD void explicit_tau(const SRAW &sr, const FA &A, const Consts<N> &cs, R (&r)[tri(N) + 1 + 3 * N]) {
     constexpr int TR = tri(N);
     const R s1 = sr(TR);
-    R y[3 * N];  // e s_1 - A s_T
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R v = e(3 * i + c) * s1;
-#pragma unroll
-            for (int k = 0; k < N; ++k) v -= A(sx(i, k)) * sr(TR + 1 + 3 * k + c);
-            y[3 * i + c] = v;
-        }
-    R MA[N * N], p[3 * N];
+    R y[3 * N], MA[N * N];  // A s_D, M A
 #pragma unroll
     for (int i = 0; i < N; ++i) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) v += A(sx(i, k)) * sr(TR + 1 + 3 * k + c);
+            y[3 * i + c] = v;
+        }
 #pragma unroll
         for (int j = 0; j < N; ++j) {
             R v = R(0.0);
@@ -939,31 +971,25 @@ NECG_HD void explicit_tau(const SRAW &sr, const FA &A, const FE &e, const Consts
             for (int k = 0; k < N; ++k) v += cs.M[i * N + k] * A(sx(k, j));
             MA[i * N + j] = v;
         }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            R v = R(0.0), g = R(0.0);
-#pragma unroll
-            for (int k = 0; k < N; ++k) {
-                v += cs.M[i * N + k] * e(3 * k + c);
-                g += cs.M[i * N + k] * y[3 * k + c];
-            }
-            p[3 * i + c] = v;
-            r[TR + 1 + 3 * i + c] -= 8.0 * g;
-        }
     }
 #pragma unroll
-    for (int i = 0; i < N; ++i)
+    for (int i = 0; i < N; ++i) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            R v = R(0.0);
+#pragma unroll
+            for (int k = 0; k < N; ++k) v += cs.M[i * N + k] * y[3 * k + c];
+            r[TR + 1 + 3 * i + c] += 8.0 * v;
+        }
 #pragma unroll
         for (int j = 0; j <= i; ++j) {
             R v = 3.0 * cs.M[i * N + j] * s1;
 #pragma unroll
             for (int k = 0; k < N; ++k)
                 v += 2.0 * (MA[i * N + k] * sr(sx(k, j)) + sr(sx(i, k)) * MA[j * N + k]);
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                v += 2.0 * (sr(TR + 1 + 3 * i + c) * p[3 * j + c] + p[3 * i + c] * sr(TR + 1 + 3 * j + c));
             r[sx(i, j)] += 4.0 * v;
         }
+    }
 }
 
 // One side's fields in an array, read as a functor.

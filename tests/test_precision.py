@@ -3,7 +3,7 @@ against extended precision (tests/extended.py)."""
 import numpy as np
 import pytest
 
-from _util import TOL_ELEM
+from _util import TOL_ELEM, TOL_G
 from extended import Extended
 from nbo_correlatedgaussians_b200 import synth
 
@@ -112,3 +112,58 @@ def test_device_gradel_between_tight_and_diffuse_functions(system, r):
     from nbo_correlatedgaussians_b200.engine import Engine
     p = two_widths(system, 8, r)
     check_gradel(p, Engine(p).gradel(p.iv, all_terms(p, 8))[0], all_terms(p, 8))
+
+
+def away_from_origin(system, K, lo, hi, shift, seed=0):
+    """Tight functions (L diagonal lo .. hi) whose centres are spread by `shift`."""
+    p = synth.make_problem(system, K, 70 + seed)
+    rng = np.random.default_rng([seed, K])
+    n, b = p.n, p.iv.reshape(K, -1)
+    diagonal = [sum(n - q for q in range(j)) for j in range(n)]
+    b[:, diagonal] = rng.uniform(lo, hi, (K, n))
+    b[:, p.svh:] = rng.normal(0.0, shift, (K, 3 * n))
+    p.iv, p.C = b.reshape(-1), rng.normal(size=K)
+    return p
+
+
+def check_components(p, g, ref, hi, shift, what):
+    """The median relative error of GRADA's components: the suite's bound for gradients
+    at 180 widths from the origin, where the differences of positions that the gradient is
+    made of have lost that many digits, and by the square of that distance less nearer."""
+    g = np.asarray(g)[:p.siv].reshape(p.K, -1)
+    err = float(np.median(np.abs(g - ref) / np.abs(ref)))
+    assert err <= TOL_G * (hi * shift / 180.0) ** 2, (what, err)
+
+
+FAR = [("He", 40), ("H2", 40), ("LiH", 12)]
+
+
+@pytest.mark.parametrize("system,K", FAR)
+@pytest.mark.parametrize("lo,hi,shift", [(5.0, 60.0, 3.0), (2.0, 30.0, 1.0)])
+def test_gradient_components_away_from_the_origin(system, K, lo, hi, shift):
+    from emu import emu
+    p = away_from_origin(system, K, lo, hi, shift)
+    ref = Extended(p).evaluate()["g"]
+    for what, out in (("ordered", emu.outprod(p)), ("fused", emu.outprod_fused(p, 2)), ("symmetric", emu.outprod_sym(p, 4, 2)),
+                      ("blocks", emu.outprod_fused(p, 1, 8, 1, 3))):
+        assert out[0] == 0
+        check_components(p, out[2], ref, hi, shift, what)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("system,K", FAR)
+@pytest.mark.parametrize("lo,hi,shift", [(5.0, 60.0, 3.0), (2.0, 30.0, 1.0)])
+def test_device_gradient_components_away_from_the_origin(system, K, lo, hi, shift):
+    from nbo_correlatedgaussians_b200.batch import BatchEngine
+    from nbo_correlatedgaussians_b200.engine import Engine
+    p = away_from_origin(system, K, lo, hi, shift)
+    ref = Extended(p).evaluate()["g"]
+    eng = Engine(p)
+    for mode, lc, minw in ((0, 4, 8), (1, 2, 8), (2, 2, 118), (2, 2, 12), (2, 1, 248)):
+        assert eng.L.necg_set_symmetric(eng.h, mode, lc, minw) == 0
+        check_components(p, eng.outprod(p.x)[1], ref, hi, shift, (mode, minw))
+    be = BatchEngine([p, p], tune=False)
+    be.plan()
+    be.step()
+    be.check()
+    check_components(p, be.results(0)[1], ref, hi, shift, "batch")
