@@ -82,9 +82,11 @@ DEFAULT_TILES = {"lc_e": 2, "minb_e": 16, "lc_g": 4, "minb_g": 8, "sym": 2, "lc_
 # the fused-pass variant measured fastest for other n (n = 3: one-warp blocks, 16 per SM)
 DEFAULT_FUSED = {3: {"lc_s": 4, "minw_s": 16}}
 PASS_MODE = {"ordered": 0, "symmetric": 1, "fused": 2}
-# FP64 FLOPs per (k, l, P) term (FMA = 2; each div/sqrt/rsqrt/exp = 1), frozen at
-# the counts the kernels' own templates gave when the fused pass was first
-# measured; the roofline fraction is reported at these and at the current count
+# FP64 operations per (k, l, P) term (FMA = 2; each div/sqrt/rsqrt/exp = 1) of the
+# formulation the fused pass was first measured with, which formed whole gradients in
+# every term: a fixed measure of the work asked for, by which rates of different
+# versions compare ("direct_equivalent").  It is more than the kernels execute, so
+# the roofline fraction is not taken at it
 FROZEN_FLOPS = {5: {"energy": 1339, "grad": 3337, "sym": 4362, "fused": 4639},
                 3: {"energy": 511, "grad": 1236, "sym": 1586, "fused": 1710},
                 2: {"energy": 253, "grad": 598, "sym": 762, "fused": 832}}
@@ -382,29 +384,24 @@ def run_engine(args):
     unordered = (K * (K + 1) // 2) * nst
     ph = np.array(phases)
     ph_mean = ph.mean(axis=0)
-    energy_flops = unordered * tf["energy"]
+    energy_flops = unordered * tf["energy_executed"]
     if mode == 2:  # one pass over unordered pairs: H, S and both gradients
         block = int(tiles.get("minw_s", 8)) >= 200  # blocks of warps
         kname, per_term = (f"fsym_block_kernel<{n}>" if block else f"fsym_kernel<{n}>"), "fused"
-        kern_flops, kern_ms = unordered * tf["fused"], float(ph_mean[1])
-        eval_flops = kern_flops
+        terms_launch, kern_ms = unordered, float(ph_mean[1])
     elif mode == 1:  # energy pass + unordered pairs with bra and ket gradients
         kname, per_term = f"gsym_kernel<{n}>", "sym"
-        kern_flops, kern_ms = unordered * tf["sym"], float(ph_mean[3])
-        eval_flops = kern_flops + energy_flops
+        terms_launch, kern_ms = unordered, float(ph_mean[3])
     else:  # energy pass + ordered pairs (the reference's loop structure)
         kname, per_term = f"grad_kernel<{n}>", "grad"
-        kern_flops, kern_ms = K * K * nst * tf["grad"], float(ph_mean[3])
-        eval_flops = kern_flops + energy_flops
-    ordered_equiv = K * K * nst * tf["grad"] + energy_flops
-    # the roofline's FLOPs: the frozen per-term count of the direct formulation; the
-    # operations the kernels execute per term (fewer) are reported beside it
-    per_frozen = frozen.get(per_term, tf[per_term])
-    terms_launch = kern_flops // tf[per_term]
+        terms_launch, kern_ms = K * K * nst, float(ph_mean[3])
+    # the roofline's operations are those the kernels execute
     executed = tf[per_term + "_executed"]
-    achieved_executed = terms_launch * executed / (kern_ms * 1e-3) / 1e12
-    kern_flops_frozen = terms_launch * per_frozen
-    achieved = kern_flops_frozen / (kern_ms * 1e-3) / 1e12
+    kern_flops = terms_launch * executed
+    eval_flops = kern_flops + (0 if mode == 2 else energy_flops)
+    achieved = kern_flops / (kern_ms * 1e-3) / 1e12
+    per_frozen = frozen.get(per_term, tf[per_term])
+    ordered_equiv = K * K * nst * tf["grad"] + unordered * tf["energy"]
     traffic, traffic_src = None, None
     tpath = os.path.join(HERE, "profiles", "traffic.json")
     if os.path.exists(tpath):
@@ -445,15 +442,14 @@ def run_engine(args):
         "roofline": {"bound": "fp64", "kernel": kname, "achieved": achieved, "peak": peak.value,
                      "unit": "TFLOP/s", "frac": achieved / peak.value, "traffic": traffic,
                      "traffic_source": traffic_src,
-                     "flops_per_term_frozen": per_frozen,
-                     "flops_per_term_executed": executed,
-                     "achieved_executed": achieved_executed,
-                     "frac_executed": achieved_executed / peak.value,
                      "kernel_ms": kern_ms,
                      "peak_source": "measured now by the FP64 FMA probe (necg_fp64_peak); "
                                     "MEASURED_PEAKS.json has no FP64 figure; nominal B200 FP64 = 37 TFLOP/s",
-                     "flops_per_launch": kern_flops_frozen, "flops_per_term": tf[per_term],
+                     "flops_per_launch": kern_flops, "flops_per_term": executed,
                      "special_per_term": tf[per_term + "_special"],
+                     "direct_equivalent": {"flops_per_term": per_frozen,
+                                           "tflops": terms_launch * per_frozen / (kern_ms * 1e-3) / 1e12,
+                                           "ratio_to_peak": terms_launch * per_frozen / (kern_ms * 1e-3) / 1e12 / peak.value},
                      "energy_kernel": (None if mode == 2 else
                                        {"achieved": energy_flops / (float(ph_mean[1]) * 1e-3) / 1e12,
                                         "flops_per_launch": energy_flops}),
