@@ -717,7 +717,12 @@ int necg_shard_tiles(necg_handle *h, int K, int *ntiles) {
     int rc = check_K(h, K);
     if (rc) return rc;
     if (!h->sym_ok) return NECG_ERR_UNSUPPORTED;
-    *ntiles = necg::tiles_before(K, h->lc_s, necg::row_blocks(K));
+    // builds the lists and buffers now, for callers that keep that out of their first
+    // step, on whatever stream that will be
+    CK(cudaSetDevice(h->device));
+    if ((rc = ensure_sym_tiles(h, K, h->last_stream, true))) return rc;
+    CK(cudaStreamSynchronize(h->last_stream));
+    *ntiles = h->nstiles;
     return NECG_OK;
 }
 
