@@ -45,6 +45,7 @@ MINW_SYM = (8, 12)
 MINW_FUSED = (8, 12, 16, 108, 112, 118, 122, 248, 232, 216)
 SPLITS = (1, 2, 3, 4, 6, 8, 12, 24)
 SPLIT_TILES = 2048  # try splits below this many fused tiles
+SPLIT_SLOTS = 8192  # and at most this many (tile, split) slots: 3 and more rounds of 16 warps on each of 148 SMs
 # 100 + w: ket records re-read at each use (118 / 122: staged in shared memory,
 # 8 / 12 warps); 248 / 232 / 216: blocks of 8 / 12 / 16 warps with bras and ket
 # records in shared memory (the library also takes the codes 208 .. 268 of earlier block
@@ -55,6 +56,12 @@ SPLIT_TILES = 2048  # try splits below this many fused tiles
 def fused_tiles(K: int, lc: int) -> int:
     """Tiles (32-row block, chunk of lc kets) over the lower triangle of K."""
     return sum((K - 1 - 32 * b) // lc + 1 for b in range((K + 31) // 32))
+
+
+def splits(K: int, lc: int, nst: int) -> list[int]:
+    """The numbers of splits tried for one-warp tiles of chunk lc."""
+    tiles = fused_tiles(K, lc)
+    return [s for s in SPLITS if s == 1 or (s <= nst and tiles < SPLIT_TILES and s * tiles <= SPLIT_SLOTS)]
 
 
 def _bucket(K: int) -> int:
@@ -141,10 +148,7 @@ def tune(eng: Engine, x, K: int, reps: int = 3, report: bool = False) -> dict:
             for lc in LC_S:
                 if L.necg_set_symmetric(eng.h, 2, lc, minw) != _lib.NECG_OK:
                     continue
-                splits = [1]
-                if minw < 200 and fused_tiles(K, lc) < SPLIT_TILES:
-                    splits = [s for s in SPLITS if s <= eng.nst]
-                for npc in splits:
+                for npc in splits(K, lc, eng.nst) if minw < 200 else [1]:
                     _lib.check(L.necg_set_splits(eng.h, npc), "necg_set_splits")
                     _phase_times(eng, x, K, 1)
                     t = _phase_times(eng, x, K, reps).min(axis=0)

@@ -147,10 +147,26 @@ void free_all(necg_handle *h) {
 
 // Lists and buffers change only outside a stream capture (their allocations would
 // belong to the captured graph, and the lists would not be there before a replay).
-int not_capturing(cudaStream_t st) {
+bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(st, &cap));
-    return cap == cudaStreamCaptureStatusNone ? NECG_OK : NECG_ERR_CUDA;
+    return cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+int not_capturing(cudaStream_t st) { return capturing(st) ? NECG_ERR_CUDA : NECG_OK; }
+
+// Make one of the handle's buffers hold `need` entries: grown when too small, and
+// given back in part when the settings have changed since (h->refit) and it is larger.
+template <typename T> int fit(necg_handle *h, T **p, size_t *cap, size_t need, cudaStream_t st) {
+    if (need <= *cap && !(h->refit && need < *cap)) return NECG_OK;
+    pool_free(h, *p, st);
+    *p = nullptr;
+    h->ws_bytes -= (long long)(*cap * sizeof(T));
+    *cap = 0;
+    ++h->gversion;  // buffers and lists a captured graph may hold changed
+    if (!need) return NECG_OK;
+    CK(pool_alloc(h, p, need * sizeof(T), st));
+    h->ws_bytes += (long long)(need * sizeof(T));
+    *cap = need;
+    return NECG_OK;
 }
 
 // Energy tiles over the lower triangle: (kb, lc) with lc * LC <= row_last(K, kb).
@@ -160,13 +176,7 @@ int ensure_tiles(necg_handle *h, int K, cudaStream_t st) {
     if (rc) return rc;
     const int nt = necg::tiles_before(K, h->lc_e, necg::row_blocks(K));
     h->tiles_K = -1;
-    if (nt > h->tiles_cap) {
-        pool_free(h, h->d_tiles, st);
-        h->d_tiles = nullptr;
-        h->tiles_cap = 0;
-        CK(pool_alloc(h, &h->d_tiles, (size_t)nt * sizeof(int2), st));
-        h->tiles_cap = nt;
-    }
+    if ((rc = fit(h, &h->d_tiles, &h->tiles_cap, (size_t)nt, st))) return rc;
     necg::launch_tile_list(h->d_tiles, K, h->lc_e, st);
     CK(cudaGetLastError());
     h->tiles_K = K;
@@ -176,52 +186,50 @@ int ensure_tiles(necg_handle *h, int K, cudaStream_t st) {
     return NECG_OK;
 }
 
-// Grow one of the handle's double buffers to `need`.
-int grow(necg_handle *h, double **p, size_t *cap, size_t need, cudaStream_t st) {
-    if (need <= *cap) return NECG_OK;
-    pool_free(h, *p, st);
-    *p = nullptr;
-    h->ws_bytes -= (long long)(*cap * sizeof(double));
-    *cap = 0;
-    ++h->gversion;
-    CK(pool_alloc(h, p, need * sizeof(double), st));
-    h->ws_bytes += (long long)(need * sizeof(double));
-    *cap = need;
-    return NECG_OK;
-}
-
-// Lower-triangle tiles of chunk LC for the symmetric passes and the queue of the
-// block variants (necg_tiles.h); the partial buffers grow here if this K and LC need
-// more.  The fused pass with npc splits needs npc partial slots per tile and npc
-// K x K buffers for H and S.
-int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
-    const int PB = necg::part_stride(h->n) + 1, LC = h->lc_s;
-    const int gw = necg::fused_block_warps(h->minb_s);  // tiles per group of the block variants
-    const int npc = fused ? necg::fused_splits(h) : 1;
-    const size_t hp_need = npc > 1 ? (size_t)npc * K * K : 0;
-    const bool same = h->stiles_K == K && h->stiles_lc == LC && h->sgroups_w == gw;
-    if (same && hp_need <= h->hp_cap && (size_t)h->nstiles * PB * (32 + LC) * 2 * npc <= h->psym_cap) return NECG_OK;
+// The K x K buffers of a fused pass with split terms whose caller wants H and S.
+int ensure_split_matrices(necg_handle *h, int K, int npc, cudaStream_t st) {
+    const size_t need = npc > 1 ? (size_t)npc * K * K : 0;
+    if (need <= h->hp_cap) return NECG_OK;
     int rc = not_capturing(st);
     if (rc) return rc;
     size_t cap = h->hp_cap;
-    if ((rc = grow(h, &h->d_Hp, &cap, hp_need, st)) || (rc = grow(h, &h->d_Sp, &h->hp_cap, hp_need, st))) return rc;
+    if ((rc = fit(h, &h->d_Hp, &cap, need, st))) h->hp_cap = 0;
+    else rc = fit(h, &h->d_Sp, &h->hp_cap, need, st);
+    return rc;
+}
+
+// Lower-triangle tiles of chunk LC for the symmetric passes and the queue of the
+// block variants (necg_tiles.h), and the partial buffers for this K and LC with npc
+// slots per tile.
+int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, int npc) {
+    const int PB = necg::part_stride(h->n) + 1, LC = h->lc_s;
+    const int gw = necg::fused_block_warps(h->minb_s);  // tiles per group of the block variants
+    const bool same = h->stiles_K == K && h->stiles_lc == LC && h->sgroups_w == gw;
+    const bool enough = same && (size_t)h->nstiles * PB * (32 + LC) * 2 * npc <= h->psym_cap;
+    if (enough && (!h->refit || capturing(st))) return NECG_OK;
+    int rc = not_capturing(st);
+    if (rc) return rc;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     const necg::SymQueue q = necg::sym_queue(K, LC, gw, h->nst, sms);
-    if ((rc = grow(h, &h->d_psym, &h->psym_cap, (size_t)q.ntiles * PB * (32 + LC) * 2 * npc, st))) return rc;
-    if (q.ntail && (rc = grow(h, &h->d_xsym, &h->xsym_cap, (size_t)q.ntail * gw * (q.parts - 1) * necg::fsym_tail_slot(PB, LC), st))) return rc;
-    if (same) return NECG_OK;
+    const size_t xneed = q.ntail ? (size_t)q.ntail * gw * (q.parts - 1) * necg::fsym_tail_slot(PB, LC) : 0;
+    if ((rc = fit(h, &h->d_psym, &h->psym_cap, (size_t)q.ntiles * PB * (32 + LC) * 2 * npc, st))) return rc;
+    if ((rc = fit(h, &h->d_xsym, &h->xsym_cap, xneed, st))) return rc;
+    if (h->refit && h->hp_cap) {  // ensure_split_matrices makes them again if they are wanted
+        size_t cap = h->hp_cap;
+        fit(h, &h->d_Hp, &cap, 0, st);
+        fit(h, &h->d_Sp, &h->hp_cap, 0, st);
+    }
+    if (same) {
+        h->refit = false;
+        return NECG_OK;
+    }
     // one buffer for all lists: the int2 lists, then the int lists
     const int nkb = necg::row_blocks(K), nb = necg::groups_before(K, LC, 8, -1), nu = q.units();
     const size_t n2 = (size_t)q.ntiles + nu + nb + 2 * nkb, need = n2 + (q.ntiles + nkb + 1 + 1) / 2;
     h->stiles_K = -1;
-    if (need > h->lists_cap) {
-        pool_free(h, h->d_lists, st);
-        h->d_lists = nullptr;
-        h->lists_cap = 0;
-        CK(pool_alloc(h, &h->d_lists, need * sizeof(int2), st));
-        h->lists_cap = need;
-    }
+    if ((rc = fit(h, &h->d_lists, &h->lists_cap, need, st))) return rc;
+    h->refit = false;
     if (!h->d_qcount) CK(pool_alloc(h, &h->d_qcount, sizeof(int), st));
     necg::SymLists &o = h->lists;
     o.tiles = h->d_lists;
@@ -248,7 +256,7 @@ int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, bool fused) {
 int necg::prepare_fused(necg_handle *h, int K, cudaStream_t st) {
     if (!h || !h->sym_ok) return NECG_ERR_UNSUPPORTED;
     CK(cudaSetDevice(h->device));
-    return ensure_sym_tiles(h, K, st, true);
+    return ensure_sym_tiles(h, K, st, fused_splits(h));
 }
 
 namespace {
@@ -398,7 +406,7 @@ void sym_args(const necg_handle *h, LaunchArgs &a) {
 // symmetric pass alone is used.)
 int launch_gradient(necg_handle *h, LaunchArgs &a, cudaStream_t st) {
     if (h->grad_mode >= 1) {
-        int rc = ensure_sym_tiles(h, a.K, st, h->grad_mode == 2);
+        int rc = ensure_sym_tiles(h, a.K, st, 1);
         if (rc) return rc;
         sym_args(h, a);
         mark(h, 3, st);
@@ -580,6 +588,7 @@ int necg_set_symmetric(necg_handle *h, int mode, int lc, int minw) {
     if (!h || mode < 0 || mode > 2 || lc < 1 || lc > 64 || !okw) return NECG_ERR_ARG;
     if (blockv && !necg::fused_variant_ok(h->n, minw)) return NECG_ERR_UNSUPPORTED;  // shared memory
     if (mode && !h->sym_ok) return NECG_ERR_UNSUPPORTED;
+    h->refit = h->refit || h->grad_mode != mode || h->lc_s != lc || h->minb_s != minw;
     h->grad_mode = mode;
     h->lc_s = lc;
     h->minb_s = minw;
@@ -589,6 +598,7 @@ int necg_set_symmetric(necg_handle *h, int mode, int lc, int minw) {
 
 int necg_set_splits(necg_handle *h, int npc) {
     if (!h || npc < 1 || npc > h->nst) return NECG_ERR_ARG;
+    h->refit = h->refit || h->npc != npc;
     h->npc = npc;
     ++h->gversion;
     return NECG_OK;
@@ -648,13 +658,15 @@ int necg_outprod(necg_handle *h, int K, const double *x_dev, double *f_dev, doub
     a.H = H_dev ? H_dev : h->d_H;
     a.S = S_dev ? S_dev : h->d_S;
     a.g = g_dev;
-    if (h->grad_mode >= 1 && (rc = ensure_sym_tiles(h, K, st, h->grad_mode == 2))) return rc;
+    const int npc = necg::fused_splits(h);
+    if (h->grad_mode >= 1 && (rc = ensure_sym_tiles(h, K, st, npc))) return rc;
     if (fused) {
         // fused: one pass over unordered pairs writes H, S and the split gradients
         sym_args(h, a);
         // H and S are written only for a caller that wants one of them
         if (!H_dev && !S_dev) a.H = a.S = nullptr;
-        a.npc = necg::fused_splits(h);
+        else if ((rc = ensure_split_matrices(h, K, npc, st))) return rc;
+        a.npc = npc;
         a.Hp = h->d_Hp;
         a.Sp = h->d_Sp;
         // A call that repeats the previous call's buffers, K and settings
@@ -693,7 +705,7 @@ int shard_args(necg_handle *h, int K, const double *x_dev, int t0, int t1, cudaS
     if (!x_dev) return NECG_ERR_ARG;
     if (!h->sym_ok) return NECG_ERR_UNSUPPORTED;
     CK(cudaSetDevice(h->device));
-    if ((rc = ensure_sym_tiles(h, K, st, true))) return rc;
+    if ((rc = ensure_sym_tiles(h, K, st, 1))) return rc;
     if (t0 < 0 || t1 < t0 || t1 > h->nstiles) return NECG_ERR_ARG;
     a = base_args(h, K);
     const size_t siv = (size_t)K * (h->n * (h->n + 1) / 2 + 3 * h->n);
@@ -720,7 +732,7 @@ int necg_shard_tiles(necg_handle *h, int K, int *ntiles) {
     // builds the lists and buffers now, for callers that keep that out of their first
     // step, on whatever stream that will be
     CK(cudaSetDevice(h->device));
-    if ((rc = ensure_sym_tiles(h, K, h->last_stream, true))) return rc;
+    if ((rc = ensure_sym_tiles(h, K, h->last_stream, necg::fused_splits(h)))) return rc;
     CK(cudaStreamSynchronize(h->last_stream));
     *ntiles = h->nstiles;
     return NECG_OK;

@@ -18,7 +18,8 @@ struct necg_handle {
     double *d_x = nullptr, *d_g = nullptr, *d_f = nullptr;
     int *d_status = nullptr;
     int2 *d_tiles = nullptr;
-    int tiles_cap = 0, tiles_K = -1, tiles_lc = -1, ntiles = 0;
+    size_t tiles_cap = 0;
+    int tiles_K = -1, tiles_lc = -1, ntiles = 0;
     int lc_e = 8, lc_g = 8;
     int minb_e = 16, minb_g = 8;
     int device = 0;
@@ -51,7 +52,8 @@ struct necg_handle {
     int *d_qcount = nullptr;    // queue head of the block-synchronised fused pass
     // fused pass with one-warp tiles: symmetry terms split over npc warps per tile
     int npc = 1;
-    double *d_Hp = nullptr, *d_Sp = nullptr;  // npc K x K sums each
+    bool refit = false;  // the pass's settings changed: its buffers are made to measure at the next use
+    double *d_Hp = nullptr, *d_Sp = nullptr;  // npc K x K sums each, when the caller wants H and S
     size_t hp_cap = 0;                        // doubles per buffer
     double *d_out = nullptr;  // f, the status words and g (d_f, d_status and d_g point into it)
     double *h_out = nullptr;  // its pinned copy, of the host entry point

@@ -38,28 +38,34 @@ import torch
 
 from . import _lib
 from .clients import OP_CLOSE, OP_EVAL, OP_OPEN, REPLY_OK, encode_error
-from .autotune import tuned
+from .autotune import LC_S, fused_tiles, splits, tuned
 from .batch import Batch
 from .engine import Engine
 from .problem import Problem
 
 
 def workspace_estimate(p: Problem, K_max: int | None = None) -> int:
-    """Device bytes a run's Engine allocates (mirror of necg_create's sizes)."""
+    """Device bytes a run's Engine holds at most, whatever the tuner sets: necg_create's
+    buffers, and the largest lists and partials of the tuner's settings."""
     K, n, nst = int(K_max or p.K), p.n, p.nst
-    tri = n * (n + 1) // 2
-    ket = (((tri + 3 * n + 6) & ~1) + 3 * n + tri + 2) & ~1
-    bra = tri + 6 * n + tri + 3 + tri
-    Kb = (K + 31) // 32 * 32
-    ps = tri + 1 + 3 * n
-    blk = tri + 3 * n
-    # symmetric-pass partials at the tuner's narrowest ket chunk (2), doubled
-    # for the fused pass (H and S partials kept apart)
-    ntiles = sum(min(kb * 32 + 31, K - 1) // 2 + 1 for kb in range((K + 31) // 32))
-    sym = 2 * ntiles * ps * (32 + 2) if n <= 5 else 0
-    doubles = (bra * Kb + ket * K * nst + ps * K * max((K + 3) // 4, 3) + 2 * K * K + 2 * K + 4
-               + 2 * (K * blk + K) + 2 + nst * (n * n + 9 * n * n + 1) + sym)
-    return 8 * doubles + 3 * 8 * (K * blk + K) + 4096
+    tri, blk = n * (n + 1) // 2, n * (n + 1) // 2 + 3 * n
+    ket = (2 * tri + 6 * n + 6 + 1) & ~1
+    bra = 3 * tri + 6 * n + 3
+    ps, nkb = tri + 1 + 3 * n, (K + 31) // 32
+    pb = ps + 1
+    fixed = (bra * 32 * nkb + ket * K * nst + max(ps * K * ((K + 3) // 4), 4 * pb * K) + 2 * K * K + 2 * K + 8
+             + 2 * (K * blk + K) + nst * (n * n + 9 * n * n + 1))
+    tables = nst * (1 + n * n) + nst * (1 + 32 * (1 + 2 * max(n * n, 3 * n)))  # dipole classes, ket map
+    tiles = fused_tiles(K, 1)
+    lists = 4 * (tiles + 8 * nkb)  # energy tiles; tiles, units, groups of 8, their ranges and slots
+    part = tail = 0
+    if n <= 5:
+        part = max(fused_tiles(K, lc) * s * pb * (32 + lc) * 2 for lc in LC_S for s in splits(K, lc, nst))
+        for lc in LC_S:  # at most 7 more parts of the last groups, fewer than there are SMs
+            for warps in (8, 12, 16):
+                groups = sum(-(-((K - 1 - 32 * b) // lc + 1) // warps) for b in range(nkb))
+                tail = max(tail, min(7 * groups, 148) * warps * lc * (2 * pb + 64))
+    return 8 * (fixed + tables + lists + part + tail) + 3 * 8 * (K * blk + K) + 4096
 
 
 class Run:
