@@ -3,8 +3,9 @@
 For one (n, nst, K) it times, with the library's phase events, the energy
 tiles over (ket-chunk width LC_e, register variant minb_e) and the gradient
 tiles over (LC_g, minb_g) -- the two are independent -- and keeps the fastest
-of each.  Results are cached in a JSON file keyed by GPU name, n, nst and a K
-bucket (powers of two), so a run pays for tuning once.
+of each.  Results are cached in a JSON file keyed by GPU name, n, nst, a K bucket
+(powers of two) and the kernels' sources, so a run pays for tuning once and not with
+choices timed on other kernels.
 
 The search space:
   LC_e   ket chunk of an energy tile (kets per warp per tile)
@@ -12,7 +13,10 @@ The search space:
   minw   minimum resident warps per SM the kernel is compiled for (one warp
          per block): 8 -> up to 255 registers per thread, 12 -> 168, 16 -> 128,
          20 -> 96 (the register file is split between the four schedulers, so
-         these are the only distinct budgets)
+         these are the only distinct budgets).  Energy tiles that several warps
+         share (few tiles, energy_warps) have one kernel whatever minb_e says, and the
+         ordered gradient is compiled for 8 and 12 warps, and 16 for n <= 3: only
+         these are tried
   sym    gradient pass over unordered pairs (bra and ket gradient per term,
          when the symmetry set is closed under inverse) instead of ordered
          pairs, with its own ket chunk lc_s and variant minw_s; sym = 2 fuses
@@ -25,6 +29,9 @@ The search space:
 from __future__ import annotations
 
 import ctypes
+import functools
+import glob
+import hashlib
 import json
 import os
 
@@ -39,7 +46,6 @@ CACHE = os.environ.get("NECG_TUNE_CACHE", os.path.join(os.path.dirname(os.path.a
 LC_E = (1, 2, 4, 8, 16)
 LC_G = (4, 8, 16, 32, 64)
 MINB = (8, 12, 16, 20)
-MINB_GRAD_EXTRA = (112, 116)  # gradient kernel with shared-memory accumulators
 LC_S = (1, 2, 4, 8, 16)       # kets per tile of the symmetric gradient pass
 MINW_SYM = (8, 12)
 MINW_FUSED = (8, 12, 16, 108, 112, 118, 122, 248, 232, 216)
@@ -64,6 +70,37 @@ def splits(K: int, lc: int, nst: int) -> list[int]:
     return [s for s in SPLITS if s == 1 or (s <= nst and tiles < SPLIT_TILES and s * tiles <= SPLIT_SLOTS)]
 
 
+def energy_warps(nst: int, tiles: int, sms: int) -> int:
+    """Warps that share an energy tile (csrc/necg_tiles.h)."""
+    w = 1
+    while 2 * w <= nst and w < 8 and tiles * w < 12 * sms:
+        w *= 2
+    return w
+
+
+def separate_candidates(n: int, nst: int, K: int, sms: int) -> list[tuple]:
+    """(minb, lc_e, lc_g, energy, grad) of the separate passes' search: whether the energy
+    and the gradient kernel of this setting are ones that no earlier setting ran."""
+    out = []
+    for minb in MINB:
+        for lc_e, lc_g in zip(LC_E, LC_G):
+            energy = minb == MINB[0] or energy_warps(nst, fused_tiles(K, lc_e), sms) == 1
+            grad = minb in ((8, 12, 16) if n <= 3 else (8, 12))
+            if energy or grad:
+                out.append((minb, lc_e, lc_g, energy, grad))
+    return out
+
+
+@functools.cache
+def kernels() -> str:
+    """A digest of the kernels' sources."""
+    h = hashlib.sha256()
+    for f in sorted(glob.glob(os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc", "*"))):
+        with open(f, "rb") as fh:
+            h.update(os.path.basename(f).encode() + b"\0" + fh.read())
+    return h.hexdigest()[:12]
+
+
 def _bucket(K: int) -> int:
     b = 16
     while b < K:
@@ -73,7 +110,7 @@ def _bucket(K: int) -> int:
 
 def _key(n: int, nst: int, K: int) -> str:
     name = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
-    return f"{name}|n{n}|nst{nst}|K{_bucket(K)}"
+    return f"{name}|n{n}|nst{nst}|K{_bucket(K)}|{kernels()}"
 
 
 def load_cache() -> dict:
@@ -114,18 +151,18 @@ def tune(eng: Engine, x, K: int, reps: int = 3, report: bool = False) -> dict:
     rows = []
     best_e = (float("inf"), None)
     best_g = (float("inf"), None)
-    for minb in MINB + MINB_GRAD_EXTRA:
-        for lc_e, lc_g in zip(LC_E, LC_G):
-            _lib.check(L.necg_set_tiles(eng.h, lc_e, lc_g), "necg_set_tiles")
-            _lib.check(L.necg_set_variant(eng.h, minb if minb < 100 else 8, minb), "necg_set_variant")
-            _phase_times(eng, x, K, 1)  # warm-up (also builds the energy tile list)
-            t = _phase_times(eng, x, K, reps).min(axis=0)
-            e_ms, g_ms = float(t[1]), float(t[3] + t[4])
-            rows.append({"minb": minb, "lc_e": lc_e, "lc_g": lc_g, "energy_ms": e_ms, "grad_ms": g_ms})
-            if e_ms < best_e[0] and minb < 100:
-                best_e = (e_ms, (lc_e, minb))
-            if g_ms < best_g[0]:
-                best_g = (g_ms, (lc_g, minb))
+    sms = torch.cuda.get_device_properties(eng.device).multi_processor_count
+    for minb, lc_e, lc_g, energy, grad in separate_candidates(eng.n, eng.nst, K, sms):
+        _lib.check(L.necg_set_tiles(eng.h, lc_e, lc_g), "necg_set_tiles")
+        _lib.check(L.necg_set_variant(eng.h, minb, minb), "necg_set_variant")
+        _phase_times(eng, x, K, 1)  # warm-up (also builds the energy tile list)
+        t = _phase_times(eng, x, K, reps).min(axis=0)
+        e_ms, g_ms = float(t[1]), float(t[3] + t[4])
+        rows.append({"minb": minb, "lc_e": lc_e, "lc_g": lc_g, "energy_ms": e_ms, "grad_ms": g_ms})
+        if energy and e_ms < best_e[0]:
+            best_e = (e_ms, (lc_e, minb))
+        if grad and g_ms < best_g[0]:
+            best_g = (g_ms, (lc_g, minb))
     res = {"lc_e": best_e[1][0], "minb_e": best_e[1][1], "lc_g": best_g[1][0], "minb_g": best_g[1][1],
            "energy_ms": best_e[0], "grad_ms": best_g[0], "sym": 0, "lc_s": 4, "minw_s": 8}
     # the symmetric gradient pass (unordered pairs), when the symmetry set allows it
@@ -176,13 +213,15 @@ def apply(eng: Engine, cfg: dict) -> None:
 
 
 def tuned(eng: Engine, x, K: int, retune: bool = False) -> dict:
-    """Apply the cached setting for (GPU, n, nst, K bucket), tuning on a miss."""
+    """Apply the cached setting for (GPU, n, nst, K bucket) of these kernels, tuning on a
+    miss; settings of other kernels leave the cache with the next one that is kept."""
     cache = load_cache()
     key = _key(eng.n, eng.nst, K)
     if key in cache and not retune:
         apply(eng, cache[key])
         return cache[key]
     res = tune(eng, x, K)
+    cache = {k: v for k, v in cache.items() if k.endswith("|" + kernels())}
     cache[key] = {k: v for k, v in res.items() if k != "table"}
     try:
         save_cache(cache)

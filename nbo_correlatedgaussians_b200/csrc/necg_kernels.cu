@@ -725,6 +725,14 @@ template <int N> Consts<N> make_consts(const double *mass, const double *ncv, do
     return c;
 }
 
+// SMs of the current device.
+int device_sms() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 template <int N> struct Launch {
     static void prep(const LaunchArgs &a, cudaStream_t st) {
         Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
@@ -743,11 +751,7 @@ template <int N> struct Launch {
                                                                a.Kin, a.Pot, a.status);
     }
     static void energy(const LaunchArgs &a, cudaStream_t st) {
-        // warps per tile: enough for about 12 warps per SM of a 148-SM GPU, at
-        // most one per symmetry term
-        int w = 1;
-        while (2 * w <= a.nst && w < 8 && a.ntiles * w < 148 * 12) w *= 2;
-        switch (w) {
+        switch (energy_warps(a.nst, a.ntiles, device_sms())) {
         case 2: energy_split<2>(a, st); return;
         case 4: energy_split<4>(a, st); return;
         case 8: energy_split<8>(a, st); return;
@@ -809,10 +813,7 @@ template <int N> struct Launch {
         // are fewer 8, whose wider register budget has the shorter chain (H2 K = 600,
         // chunk 8: 130 us, 145 at 16).
         if (N <= 3 && a.minb_s >= 200) {
-            int dev = 0, sms = 148;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (a.nstiles > 8 * sms) gsym_v<16, false>(a, st);
+            if (a.nstiles > 8 * device_sms()) gsym_v<16, false>(a, st);
             else gsym_v<8, true>(a, st);
             return;
         }
@@ -864,7 +865,7 @@ template <int N> struct Launch {
             constexpr int smem = fsym_block_smem_bytes<N>(WARPS);
             if constexpr (smem <= 232448) {
                 auto kern = fsym_block_kernel<N, WARPS, KE>;
-                int dev = 0, sms = 148;
+                int dev = 0;
                 cudaGetDevice(&dev);
                 // the shared-memory opt-in is per device: once per instantiation and device
                 static bool attr[64] = {};
@@ -872,7 +873,7 @@ template <int N> struct Launch {
                     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
                     if (dev >= 0 && dev < 64) attr[dev] = true;
                 }
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+                const int sms = device_sms();
                 Consts<N> cs = make_consts<N>(a.mass_h, a.ncv_h, a.efs);
                 // the fused sequence's prep has reset the queue; the gradient alone comes later
                 if (KE) cudaMemsetAsync(a.qcount, 0, sizeof(int), st);
@@ -939,10 +940,7 @@ template <int N> struct Launch {
         if (a.dip_cls) {
             // classes split so that there are about 16 one-warp blocks per SM (the
             // partials must fit the workspace)
-            int dev = 0, sms = 148;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            int split = (16 * sms + a.ntiles - 1) / a.ntiles;
+            int split = (16 * device_sms() + a.ntiles - 1) / a.ntiles;
             const size_t fit = cap / ((size_t)a.ntiles * (3 * N + 1));
             if (split > a.nst) split = a.nst;
             if ((size_t)split > fit) split = (int)fit;

@@ -24,6 +24,15 @@ NECG_HD int groups_before(int K, int LC, int w, int kb) {
     return n;
 }
 
+// Warps per energy tile: one, or for bases with few tiles up to 8 that share a tile's
+// symmetry terms, until there are 12 per SM (matrices of LiH K = 301 on a B200, chunk
+// 2: 170 us with 8 per SM, 158 with 12, 157 with 16).
+NECG_HD int energy_warps(int nst, int ntiles, int sms) {
+    int w = 1;
+    while (2 * w <= nst && w < 8 && ntiles * w < 12 * sms) w *= 2;
+    return w;
+}
+
 // A tile group of the block variants: row block kb, first ket chunk lc0 and, for
 // a split group of the queue's tail, its part and the number of parts (one part
 // per range of symmetry terms).
