@@ -803,16 +803,19 @@ int necg_outprod_host(necg_handle *h, int K, const double *x_host, double *f_hos
     rc = necg_outprod(h, K, h->d_x, h->d_f, h->d_g, nullptr, nullptr, stream);
     if (rc) return rc;
     // f, the status words and g come back in one copy into a pinned buffer of the
-    // handle, and the stream is waited for once; a pinned g_host gets its copy
-    // straight (a copy into pageable memory would go through the driver's own
-    // staging, one more wait)
+    // handle, and the stream is waited for once; a g_host that is not ordinary
+    // memory of the process (pinned, managed, or a device address, for which the
+    // runtime decides) gets its copy straight, since a copy into pageable memory
+    // would go through the driver's own staging, one more wait
     if (!h->h_out) CK(cudaMallocHost((void **)&h->h_out, (kOutHead + (size_t)h->K_max * (len / K)) * sizeof(double)));
     cudaPointerAttributes at;
-    const bool pinned = cudaPointerGetAttributes(&at, g_host) == cudaSuccess && at.type == cudaMemoryTypeHost;
-    CK(cudaMemcpyAsync(h->h_out, h->d_out, (kOutHead + (pinned ? 0 : len)) * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (pinned) CK(cudaMemcpyAsync(g_host, h->d_g, len * sizeof(double), cudaMemcpyDeviceToHost, st));
+    const cudaError_t known = cudaPointerGetAttributes(&at, g_host);
+    if (known != cudaSuccess) cudaGetLastError();
+    const bool direct = known == cudaSuccess && at.type != cudaMemoryTypeUnregistered;
+    CK(cudaMemcpyAsync(h->h_out, h->d_out, (kOutHead + (direct ? 0 : len)) * sizeof(double), cudaMemcpyDeviceToHost, st));
+    if (direct) CK(cudaMemcpyAsync(g_host, h->d_g, len * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (!pinned) memcpy(g_host, h->h_out + kOutHead, len * sizeof(double));
+    if (!direct) memcpy(g_host, h->h_out + kOutHead, len * sizeof(double));
     if (f_host) *f_host = h->h_out[0];
     int sw[2];
     memcpy(sw, h->h_out + 1, sizeof(sw));
