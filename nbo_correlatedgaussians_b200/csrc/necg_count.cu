@@ -64,30 +64,30 @@ template <int N> void host_records(std::vector<double> &bra, std::vector<double>
 template <int N, bool KET, bool KE> struct CountOut {
     static constexpr bool kets = KET, ket_s = KET && !KE;
     CD acc[2][64], ket[2][64], wb = CD(1.0), wk = CD(1.0), wob, wok;
-    void begin(CD ov) {
+    NECG_HD void begin(CD ov) {
         wob = wb * ov;
         if (KET) wok = wk * ov;
     }
-    void put(int m, int f, CD v) { acc[m][f] += wob * v; }
-    void sb1(int f, CD v) { put(1, f, v); }
-    void hb1(int f, CD v) { put(0, f, v); }
-    template <int I> void sb(CD va, CD vb) {
+    NECG_HD void put(int m, int f, CD v) { acc[m][f] += wob * v; }
+    NECG_HD void sb1(int f, CD v) { put(1, f, v); }
+    NECG_HD void hb1(int f, CD v) { put(0, f, v); }
+    template <int I> NECG_HD void sb(CD va, CD vb) {
         put(1, RawPairs<N>::fa(I), va);
         put(1, RawPairs<N>::fb(I), vb);
     }
-    template <int I> void hb(CD va, CD vb) {
+    template <int I> NECG_HD void hb(CD va, CD vb) {
         put(0, RawPairs<N>::fa(I), va);
         put(0, RawPairs<N>::fb(I), vb);
     }
-    template <int I> void sk(CD va, CD vb) {
+    template <int I> NECG_HD void sk(CD va, CD vb) {
         ket[1][RawPairs<N>::fa(I)] = wok * va;
         ket[1][RawPairs<N>::fb(I)] = wok * vb;
     }
-    template <int I> void hk(CD va, CD vb) {
+    template <int I> NECG_HD void hk(CD va, CD vb) {
         ket[0][RawPairs<N>::fa(I)] = wok * va;
         ket[0][RawPairs<N>::fb(I)] = wok * vb;
     }
-    void scalar(CD e2) {
+    NECG_HD void scalar(CD e2) {
         put(0, tri(N), e2);
         acc[1][tri(N)] += wob;
         if (KET) ket[0][tri(N)] = wok * e2;

@@ -6,6 +6,8 @@
 #include <math.h>
 #include <stddef.h>
 
+#include "necg_math.cuh"
+
 namespace necg {
 
 struct CountCtx {
@@ -16,48 +18,51 @@ inline CountCtx &count_ctx() {
     return c;
 }
 
+// (Host and device for the templates' sake, which are: only the host runs them.)
 struct CD {
     double v;
-    CD() : v(0.0) {}
-    CD(double x) : v(x) {}
-    CD &operator+=(const CD &o) { ++count_ctx().flops; v += o.v; return *this; }
-    CD &operator-=(const CD &o) { ++count_ctx().flops; v -= o.v; return *this; }
-    CD &operator*=(const CD &o) { ++count_ctx().flops; v *= o.v; return *this; }
+    NECG_HD CD() : v(0.0) {}
+    NECG_HD CD(double x) : v(x) {}
+    NECG_HD CD &operator+=(const CD &o) { v += o.v; return flop(); }
+    NECG_HD CD &operator-=(const CD &o) { v -= o.v; return flop(); }
+    NECG_HD CD &operator*=(const CD &o) { v *= o.v; return flop(); }
+#pragma nv_exec_check_disable
+    NECG_HD CD &flop() { ++count_ctx().flops; return *this; }
+#pragma nv_exec_check_disable
+    NECG_HD CD &spec() { ++count_ctx().special; return *this; }
 };
-inline CD operator+(CD a, CD b) { ++count_ctx().flops; return CD(a.v + b.v); }
-inline CD operator-(CD a, CD b) { ++count_ctx().flops; return CD(a.v - b.v); }
-inline CD operator*(CD a, CD b) { ++count_ctx().flops; return CD(a.v * b.v); }
-inline CD operator/(CD a, CD b) { ++count_ctx().special; return CD(a.v / b.v); }
-inline CD operator+(double a, CD b) { return CD(a) + b; }
-inline CD operator+(CD a, double b) { return a + CD(b); }
-inline CD operator-(double a, CD b) { return CD(a) - b; }
-inline CD operator-(CD a, double b) { return a - CD(b); }
-inline CD operator*(double a, CD b) { return CD(a) * b; }
-inline CD operator*(CD a, double b) { return a * CD(b); }
-inline CD operator-(CD a) { return CD(-a.v); }
-inline bool operator>(CD a, double b) { return a.v > b; }
-inline bool operator<=(CD a, double b) { return a.v <= b; }
-inline bool operator<=(CD a, CD b) { return a.v <= b.v; }
-inline CD sqrt(CD a) { ++count_ctx().special; return CD(::sqrt(a.v)); }
-inline CD rsqrt(CD a) { ++count_ctx().special; return CD(1.0 / ::sqrt(a.v)); }
-inline CD rsq(CD a) { return rsqrt(a); }
-inline CD rcp(CD a) { return CD(1.0) / a; }
-inline CD exp(CD a) { ++count_ctx().special; return CD(::exp(a.v)); }
-inline double val(CD x) { return x.v; }
+NECG_HD CD operator+(CD a, CD b) { return CD(a.v + b.v).flop(); }
+NECG_HD CD operator-(CD a, CD b) { return CD(a.v - b.v).flop(); }
+NECG_HD CD operator*(CD a, CD b) { return CD(a.v * b.v).flop(); }
+NECG_HD CD operator/(CD a, CD b) { return CD(a.v / b.v).spec(); }
+NECG_HD CD operator+(double a, CD b) { return CD(a) + b; }
+NECG_HD CD operator+(CD a, double b) { return a + CD(b); }
+NECG_HD CD operator-(double a, CD b) { return CD(a) - b; }
+NECG_HD CD operator-(CD a, double b) { return a - CD(b); }
+NECG_HD CD operator*(double a, CD b) { return CD(a) * b; }
+NECG_HD CD operator*(CD a, double b) { return a * CD(b); }
+NECG_HD CD operator-(CD a) { return CD(-a.v); }
+NECG_HD bool operator>(CD a, double b) { return a.v > b; }
+NECG_HD bool operator<=(CD a, double b) { return a.v <= b; }
+NECG_HD bool operator<=(CD a, CD b) { return a.v <= b.v; }
+NECG_HD CD rsq(CD a) { return CD(1.0 / ::sqrt(a.v)).spec(); }
+NECG_HD CD rcp(CD a) { return CD(1.0) / a; }
+NECG_HD CD exp(CD a) { return CD(::exp(a.v)).spec(); }
+NECG_HD double val(CD x) { return x.v; }
 
 // bra record field f of basis k in a structure-of-arrays buffer
 struct HostBra {
     const double *p;  // bra + k
     size_t K;
-    CD operator()(int f) const { return CD(p[(size_t)f * K]); }
+    NECG_HD CD operator()(int f) const { return CD(p[(size_t)f * K]); }
 };
 struct HostKet {
     const double *p;
-    CD operator[](int i) const { return CD(p[i]); }
+    NECG_HD CD operator[](int i) const { return CD(p[i]); }
 };
 struct HostKetBase {
     const double *p;
-    HostKet at(size_t off) const { return HostKet{p + off}; }
+    NECG_HD HostKet at(size_t off) const { return HostKet{p + off}; }
 };
 
 }  // namespace necg

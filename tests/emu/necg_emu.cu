@@ -32,14 +32,14 @@ template <int N> Consts<N> consts(const double *mass, const double *ncv, double 
 // Accumulators of one bra gradient (SmemAcc on the device).
 template <int N> struct RegAcc {
     CD G[tri(N)], D, S[3 * N];
-    void zero() {
+    NECG_HD void zero() {
         for (CD &v : G) v = CD(0.0);
         D = CD(0.0);
         for (CD &v : S) v = CD(0.0);
     }
-    CD &g(int t) { return G[t]; }
-    CD &d() { return D; }
-    CD &s(int t) { return S[t]; }
+    NECG_HD CD &g(int t) { return G[t]; }
+    NECG_HD CD &d() { return D; }
+    NECG_HD CD &s(int t) { return S[t]; }
 };
 
 struct Args {
