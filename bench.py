@@ -79,8 +79,8 @@ def parse():
 
 
 DEFAULT_TILES = {"lc_e": 2, "minb_e": 16, "lc_g": 4, "minb_g": 8, "sym": 2, "lc_s": 2, "minw_s": 248}
-# the fused-pass variant measured fastest for other n (n = 3: one-warp blocks, 16 per SM)
-DEFAULT_FUSED = {3: {"lc_s": 4, "minw_s": 16}}
+# the fused-pass variant measured fastest for other n (n = 3: one-warp blocks with staged ket records, 12 per SM)
+DEFAULT_FUSED = {3: {"lc_s": 4, "minw_s": 122}}
 PASS_MODE = {"ordered": 0, "symmetric": 1, "fused": 2}
 # FP64 operations per (k, l, P) term (FMA = 2; each div/sqrt/rsqrt/exp = 1) of the
 # formulation the fused pass was first measured with, which formed whole gradients in

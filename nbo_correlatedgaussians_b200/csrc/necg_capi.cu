@@ -5,11 +5,15 @@
 // K_max functions:
 //   bra   BraLayout<n>::size * K_max       per-basis data (K_max rounded up to 32)
 //   ket   KetLayout<n>::size * K_max * nst per-(l, P) ket records
-//   part  part_stride(n) * K_max * ceil(K_max / lc_grad)   gradient tile partials
+//   part  part_doubles(n, K_max)           tile partials of the ordered gradient, or
+//                                          the symmetric passes' per-basis sums
 //   H, S  K_max^2 each (used when the caller passes no H/S)
 //   rows  2 K_max, scal 4, x/g staging for the host-pointer entry point
-// Nothing is allocated after necg_create, so every device-pointer entry point
-// is stream-ordered and capturable in a CUDA graph once tiles for K exist.
+// The tile lists and the partial buffers of the symmetric passes, whose sizes follow
+// from K and the settings, are made when a call first needs them (as are the dipole's
+// classes and the host entry point's pinned buffer): every device-pointer entry
+// point is stream-ordered, and capturable in a CUDA graph once a call with the same
+// K and settings has run.
 //
 // Handle memory comes from one stream-ordered pool per device (cudaMemPool_t,
 // blocks kept for reuse), allocated and freed on the library's own
@@ -661,7 +665,8 @@ int necg_outprod(necg_handle *h, int K, const double *x_dev, double *f_dev, doub
     const int npc = necg::fused_splits(h);
     if (h->grad_mode >= 1 && (rc = ensure_sym_tiles(h, K, st, npc))) return rc;
     if (fused) {
-        // fused: one pass over unordered pairs writes H, S and the split gradients
+        // fused: one pass over unordered pairs: row sums, both gradients' raw sums of H
+        // and of S and, on request, H and S
         sym_args(h, a);
         // H and S are written only for a caller that wants one of them
         if (!H_dev && !S_dev) a.H = a.S = nullptr;

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(32, MINW) energy_kernel(const int2 *__restrict
 // bases with too few tiles to fill the GPU (a tile is a chain of LC nst terms):
 // the warps' sums of a pair meet in shared memory and are added in warp order.
 // FP64 latency bounds it.  LiH K = 301 with H, S, Kinetic and Potential on a
-// B200: 222 us one warp per tile, 145 us with 2 and the shorter term.
+// B200: 222 us one warp per tile (with an earlier term), 154 us with 2.
 template <int N, int W>
 __global__ void __launch_bounds__(32 * W) energy_split_kernel(const int2 *__restrict__ tiles, int LC, int K, int nst,
                                                               Consts<N> cs, const double *__restrict__ bra,
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(32) dipole_kernel(const int2 *__restrict__ til
 // (cls: c_Q and R_Q, N x N row-major, per class).  R_Q multiplies the sums over
 // the tile's kets.  FP64-latency bound at small K, so the classes are split over
 // blockIdx.y until the GPU is full; partials at slot t gridDim.y + blockIdx.y.
-// LiH K = 160 on a B200: the whole call 836 -> 154 us (24 instead of 576 terms per pair).
+// LiH K = 160 on a B200: the whole call 829 -> 106 us (24 instead of 576 terms per pair).
 template <int N>
 __global__ void __launch_bounds__(32) dipole_group_kernel(const int2 *__restrict__ tiles, int ntiles, int LC, int K,
                                                           int nst, Consts<N> cs, const double *__restrict__ bra,
@@ -770,8 +770,8 @@ template <int N> struct Launch {
                                                        a.part, a.status);
     }
     // variant codes: warps per SM the kernel is compiled for (100 + w: the same
-    // as w); 128 registers spill the n > 3 term (LiH K = 700: 4.07 ms at 16 warps
-    // per SM, 3.32 at 12, 2.76 at 8), so 16 and 20 run 12 there
+    // as w); 168 registers spill the n > 3 term (LiH K = 700, chunk 4: 2.00 ms at 8
+    // warps per SM, 2.61 at 12) and 128 more so: 16 and 20 run 12 there
     static void grad_tiles(const LaunchArgs &a, cudaStream_t st) {
         const int w = a.minb_g % 100;
         if (w == 8) grad_v<8>(a, st);
@@ -796,8 +796,8 @@ template <int N> struct Launch {
         }
     }
     // blocks when the handle's groups are 8 chunks wide, for n > 3 (LiH K = 400, ket
-    // chunk 2: 394 us for the gradient against 528 to 570 of the one-warp tiles; H2
-    // K = 2048, chunk 4: 709 against 653)
+    // chunk 2: 434 us for the gradient against 578 to 621 of the one-warp tiles; H2
+    // K = 2048, chunk 4, measured with an earlier term: 709 against 653)
     static bool gsym_block(const LaunchArgs &a) {
         return N > 3 && a.minb_s >= 200 && fused_block_warps(a.minb_s) == 8 && a.sgroups && a.qcount && a.urange;
     }
@@ -807,13 +807,14 @@ template <int N> struct Launch {
                 fsym_block<8, true>(a, st);
                 return;
             }
-        // A handle tuned to a block variant at n <= 3 takes one-warp tiles, 16 to the SM
-        // once they are more than 8 to the SM (H2 K = 2048, chunk 4: 653 us for the
-        // gradient, 706 at 8 to the SM; H2 K = 600, chunk 1: 126 and 133), where they
-        // are fewer 8, whose wider register budget has the shorter chain (H2 K = 600,
-        // chunk 8: 130 us, 145 at 16).
+        // A handle tuned to a block variant at n <= 3 takes one-warp tiles with staged ket
+        // records, 12 to the SM once they are more than 8 to the SM (the gradient of H2 K =
+        // 2048, chunk 4: 716 us, 756 at 8 to the SM, 734 at 16; H2 K = 300, chunk 1: 63.5,
+        // 67.8 and 65.5; He K = 2032, chunk 8: 250, 249 and 254), where they are fewer 8,
+        // whose wider register budget has the shorter chain (H2 K = 600, chunk 8: 139 us,
+        // 143 at 12; H2 K = 300, chunk 4: 76 and 82).
         if (N <= 3 && a.minb_s >= 200) {
-            if (a.nstiles > 8 * device_sms()) gsym_v<16, false>(a, st);
+            if (a.nstiles > 8 * device_sms()) gsym_v<12, true>(a, st);
             else gsym_v<8, true>(a, st);
             return;
         }

@@ -36,9 +36,12 @@
 // on its own A (the chain from e = A s, and the bra's explicit share of tau)
 // multiplies only those sums, once per basis function (fold_raw, explicit_tau).
 // That takes the products with A_k and A_l' and the second sandwich out of the term:
-// fewer operations than a term that forms its own gradients by a third (n = 5).
-// The origin: with T in the place of D_s both sides would share all values, 180
-// operations less at n = 5, but the sums of a function away from the origin would
+// 3238 instead of 4374 FLOP at n = 5 and 1266 instead of 1626 at n = 3.  The FP64 pipe
+// bounds the pair passes; whole evaluations on a B200 went from 3.53 to 2.49 ms (LiH K
+// = 1024), 1.06 to 0.72 ms (H2 K = 2048) and 0.34 to 0.22 ms (He K = 2032), the
+// launches around the passes included.
+// The origin: with T in the place of D_s both sides would share all values, some 400
+// FLOP less at n = 5 (2.29 ms), but the sums of a function away from the origin would
 // hold differences |s|^2 A times as large as themselves (components of dF/dL of tight
 // functions lost 10 to 50 times the rounding error).
 // The A^-1 term (coefficient D = 0.75 F) maps to vech(dF/dL) as 2 D / L_ii
