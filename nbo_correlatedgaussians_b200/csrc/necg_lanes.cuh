@@ -170,12 +170,51 @@ NECG_HD void prep_ket_one(const double *iv, const double *C, int nst, const Cons
     o[KL::w] = scvv[P];
     o[KL::wC] = C ? 2.0 * scvv[P] * C[l] : 0.0;
     o[KL::winv] = pinv ? scvv[pinv[P]] : 0.0;
-    double AM[N * N], AMA[tri(N)], tMA;
-    mass_products<N>(Ap, cs.M, AM, AMA, tMA);
+    // A' M A' = pm^T (A (pm M pm^T) A) pm, and the trace likewise: where M is
+    // unchanged by pm, as in a permutation of equal particles, these are the bra's own
+    // values in another order, with the same rounding for every P, which then
+    // cancels in an antisymmetric sum over P as the terms do (E of LiH K = 512: 1e-14
+    // relative with A' M A' formed from A', 1e-15 so)
+    double Mp[N * N], AM[N * N], AMA[tri(N)], tMA;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        double r[N];  // row i of pm M
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < N; ++k) s += pm[i * N + k] * cs.M[k * N + j];
+            r[j] = s;
+        }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < N; ++k) s += r[k] * pm[j * N + k];
+            Mp[i * N + j] = s;
+        }
+    }
+    mass_products<N>(A, Mp, AM, AMA, tMA);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < N; ++k) s += AMA[sx(i, k)] * pm[k * N + j];
+            AM[i * N + j] = s;  // A Mp A pm
+        }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < N; ++k) s += pm[k * N + i] * AM[k * N + j];
+            o[KL::Np8 + sx(i, j)] = -8.0 * s;
+        }
 #pragma unroll
     for (int t = 0; t < 3 * N; ++t) o[KL::Sp + t] = Sp[t];
-#pragma unroll
-    for (int t = 0; t < tri(N); ++t) o[KL::Np8 + t] = -8.0 * AMA[t];
     o[KL::tMA] = tMA;
     if (KL::size > KL::Sp + 3 * N) o[KL::Sp + 3 * N] = 0.0;
 }

@@ -153,6 +153,15 @@ def elements(p, terms):
     return rc, mat, tg, tgs
 
 
+def mass_records(p):
+    """-8 A M A (packed lower) and tr(M A): of the bras (K, tri + 1) and kets (K, nst, tri + 1)."""
+    args, keep = _problem(p)
+    ob, ok = np.zeros((p.K, p.svh + 1)), np.zeros((p.K, p.nst, p.svh + 1))
+    iv = np.ascontiguousarray(p.iv)
+    assert lib().emu_mass_records(*args, *[ctypes.c_void_p(_p(a)) for a in (iv, ob, ok)]) == 0
+    return ob, ok
+
+
 def sym_lists(K, lc, w, nst, sms, nj=7):
     """The tile lists of the symmetric passes: dict of counts and arrays."""
     L = lib()

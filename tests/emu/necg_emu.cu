@@ -263,6 +263,30 @@ extern "C" int emu_elements(int n, int nst, int K, double efs, const double *mas
     EMU_DISPATCH(n, (elements<N>(a, iv, nterms, terms, mat, tg, tgs)));
 }
 
+// A M A (packed lower) and tr(M A) of every function as the bra's and as the kets'
+// records hold them: bra K x (tri + 1), ket K x nst x (tri + 1).
+namespace {
+template <int N> int mass_records(const Args &a, const double *iv, double *ob, double *ok) {
+    std::vector<double> bra, ket;
+    Consts<N> cs = consts<N>(a.mass, a.ncv, a.efs);
+    prep<N>(a, iv, nullptr, bra, ket, cs);
+    for (int k = 0; k < a.K; ++k)
+        for (int t = 0; t <= tri(N); ++t) {
+            ob[k * (tri(N) + 1) + t] = bra[(size_t)(t < tri(N) ? BraLayout<N>::N8 + t : BraLayout<N>::tMA) * a.K + k];
+            for (int P = 0; P < a.nst; ++P)
+                ok[((size_t)k * a.nst + P) * (tri(N) + 1) + t] =
+                    ket[((size_t)k * a.nst + P) * KetLayout<N>::size + (t < tri(N) ? KetLayout<N>::Np8 + t : KetLayout<N>::tMA)];
+        }
+    return 0;
+}
+}  // namespace
+extern "C" int emu_mass_records(int n, int nst, int K, double efs, const double *mass, const double *ncv,
+                                const double *scvv, const double *sml, const double *sms, const double *iv, double *ob,
+                                double *ok) {
+    Args a{nst, K, efs, mass, ncv, scvv, sml, sms};
+    EMU_DISPATCH(n, (mass_records<N>(a, iv, ob, ok)));
+}
+
 // The tile lists of the symmetric passes, filled row block by row block with nj
 // threads each; head: ntiles, units, groups of 8, tail0, ntail, parts.  Null lists: head only.
 extern "C" int emu_sym_lists(int K, int LC, int w, int nst, int sms, int nj, int *head, int *tiles, int *start,

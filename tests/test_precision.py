@@ -167,3 +167,36 @@ def test_device_gradient_components_away_from_the_origin(system, K, lo, hi, shif
     be.step()
     be.check()
     check_components(p, be.results(0)[1], ref, hi, shift, "batch")
+
+
+@pytest.mark.parametrize("system", ["He", "LiH"])
+def test_permuted_kets_hold_the_permuted_values_of_the_bra(system):
+    """A M A and tr(M A) of a function in the frame of a permutation that leaves M as it is
+    are its own, bit for bit, so that their rounding cancels in an antisymmetric sum."""
+    from emu import emu
+    p = synth.make_problem(system, 9, 4)
+    bra, ket = emu.mass_records(p)
+    low = [(i, j) for i in range(p.n) for j in range(i + 1)]
+    for P in range(p.nst):
+        m = p.sml[P]
+        assert np.array_equal(m @ p.mass @ m.T, p.mass)
+        for k in range(p.K):
+            full = np.zeros((p.n, p.n))
+            for t, (i, j) in enumerate(low):
+                full[i, j] = full[j, i] = bra[k, t]
+            moved = m.T @ full @ m
+            assert np.array_equal(ket[k, P, :-1], [moved[i, j] for i, j in low]) and ket[k, P, -1] == bra[k, -1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,lc,minw", [(0, 4, 8), (2, 2, 118), (2, 2, 248)])
+def test_energy_of_antisymmetric_sums(mode, lc, minw):
+    """E of LiH bases of K = 512 (the synthetic workloads' seeds 1 to 3), against 80-bit sums
+    of the same terms: 30 roundings of E."""
+    from nbo_correlatedgaussians_b200.engine import Engine
+    for seed, E in ((1, "4.6758029388500884573"), (2, "7.1651162402481331"), (3, "3.8932810772307178317")):
+        p = synth.make_problem("LiH", 512, seed)
+        eng = Engine(p)
+        assert eng.L.necg_set_symmetric(eng.h, mode, lc, minw) == 0
+        f, _ = eng.outprod(p.x)
+        assert abs(np.longdouble(f) - np.longdouble(E)) <= 30 * np.finfo(np.float64).eps / 2 * np.longdouble(E), seed
