@@ -654,7 +654,8 @@ int necg_outprod(necg_handle *h, int K, const double *x_dev, double *f_dev, doub
     } else if ((rc = begin(h, st))) {
         return rc;
     }
-    if (!fused && (rc = ensure_tiles(h, K, st))) return rc;
+    // in fused mode too, which does not read them: a later call that does may be captured
+    if ((rc = ensure_tiles(h, K, st))) return rc;
     const size_t siv = (size_t)K * (h->n * (h->n + 1) / 2 + 3 * h->n);
     LaunchArgs a = base_args(h, K);
     a.iv = x_dev;
@@ -662,7 +663,7 @@ int necg_outprod(necg_handle *h, int K, const double *x_dev, double *f_dev, doub
     a.H = H_dev ? H_dev : h->d_H;
     a.S = S_dev ? S_dev : h->d_S;
     a.g = g_dev;
-    const int npc = necg::fused_splits(h);
+    int npc = necg::fused_splits(h);
     if (h->grad_mode >= 1 && (rc = ensure_sym_tiles(h, K, st, npc))) return rc;
     if (fused) {
         // fused: one pass over unordered pairs: row sums, both gradients' raw sums of H
@@ -670,6 +671,7 @@ int necg_outprod(necg_handle *h, int K, const double *x_dev, double *f_dev, doub
         sym_args(h, a);
         // H and S are written only for a caller that wants one of them
         if (!H_dev && !S_dev) a.H = a.S = nullptr;
+        else if (npc > 1 && (size_t)npc * K * K > h->hp_cap && capturing(st)) npc = 1;  // no buffers for split H and S
         else if ((rc = ensure_split_matrices(h, K, npc, st))) return rc;
         a.npc = npc;
         a.Hp = h->d_Hp;
@@ -737,6 +739,7 @@ int necg_shard_tiles(necg_handle *h, int K, int *ntiles) {
     // builds the lists and buffers now, for callers that keep that out of their first
     // step, on whatever stream that will be
     CK(cudaSetDevice(h->device));
+    if ((rc = ensure_tiles(h, K, h->last_stream))) return rc;
     if ((rc = ensure_sym_tiles(h, K, h->last_stream, necg::fused_splits(h)))) return rc;
     CK(cudaStreamSynchronize(h->last_stream));
     *ntiles = h->nstiles;

@@ -99,3 +99,26 @@ def test_prepared_engines_allocate_nothing_in_their_first_step():
     ready = eng.workspace_bytes()
     eng.outprod_device(x, p.K)
     assert before < ready == eng.workspace_bytes()
+
+
+def test_captures_after_a_plain_evaluation():
+    """A fused evaluation without H and S makes what a capture of the other calls at its
+    size needs: the matrices, and the evaluation with H and S of split terms."""
+    import torch
+    p, eng, x = _engine("H2", 40)
+    assert eng.L.necg_set_symmetric(eng.h, 2, 2, 12) == 0 and eng.L.necg_set_splits(eng.h, 4) == 0
+    f, g = eng.outprod_device(x, p.K)
+    iv, C = x[:p.siv].clone(), x[p.siv:].clone()
+    H, S = (torch.zeros((p.K, p.K), dtype=torch.float64, device=eng.device) for _ in range(2))
+    f1, g1 = torch.zeros_like(f), torch.zeros_like(g)
+    torch.cuda.synchronize()
+    graphs = [torch.cuda.CUDAGraph() for _ in range(2)]
+    with torch.cuda.graph(graphs[0]):
+        Hm, Sm, _, _, en = eng.build_matrices(iv, C, K=p.K, check=False)
+    with torch.cuda.graph(graphs[1]):
+        eng.outprod_device(x, p.K, f=f1, g=g1, H=H, S=S)
+    for graph in graphs:
+        graph.replay()
+    torch.cuda.synchronize()
+    for a, b in ((f1, f), (g1, g), (H, Hm), (S, Sm), (en[:1], f)):
+        assert float((a - b).abs().max()) <= 1e-12 * float(b.abs().max())
