@@ -157,10 +157,9 @@ bool capturing(cudaStream_t st) {
 }
 int not_capturing(cudaStream_t st) { return capturing(st) ? NECG_ERR_CUDA : NECG_OK; }
 
-// Make one of the handle's buffers hold `need` entries: grown when too small, and
-// given back in part when the settings have changed since (h->refit) and it is larger.
-template <typename T> int fit(necg_handle *h, T **p, size_t *cap, size_t need, cudaStream_t st) {
-    if (need <= *cap && !(h->refit && need < *cap)) return NECG_OK;
+// Make one of the handle's buffers hold `need` entries, or (exact) just those.
+template <typename T> int fit(necg_handle *h, T **p, size_t *cap, size_t need, cudaStream_t st, bool exact = false) {
+    if (exact ? need == *cap : need <= *cap) return NECG_OK;
     pool_free(h, *p, st);
     *p = nullptr;
     h->ws_bytes -= (long long)(*cap * sizeof(T));
@@ -204,35 +203,34 @@ int ensure_split_matrices(necg_handle *h, int K, int npc, cudaStream_t st) {
 
 // Lower-triangle tiles of chunk LC for the symmetric passes and the queue of the
 // block variants (necg_tiles.h), and the partial buffers for this K and LC with npc
-// slots per tile.
+// slots per tile.  Settings that have changed since the lists were made give back what
+// they need less (while the lists stay as they are, so do the buffers: a caller's own
+// captured graphs hold them).
 int ensure_sym_tiles(necg_handle *h, int K, cudaStream_t st, int npc) {
     const int PB = necg::part_stride(h->n) + 1, LC = h->lc_s;
     const int gw = necg::fused_block_warps(h->minb_s);  // tiles per group of the block variants
     const bool same = h->stiles_K == K && h->stiles_lc == LC && h->sgroups_w == gw;
-    const bool enough = same && (size_t)h->nstiles * PB * (32 + LC) * 2 * npc <= h->psym_cap;
-    if (enough && (!h->refit || capturing(st))) return NECG_OK;
+    if (same && (size_t)h->nstiles * PB * (32 + LC) * 2 * npc <= h->psym_cap) return NECG_OK;
+    const bool exact = !same && h->refit;
     int rc = not_capturing(st);
     if (rc) return rc;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     const necg::SymQueue q = necg::sym_queue(K, LC, gw, h->nst, sms);
     const size_t xneed = q.ntail ? (size_t)q.ntail * gw * (q.parts - 1) * necg::fsym_tail_slot(PB, LC) : 0;
-    if ((rc = fit(h, &h->d_psym, &h->psym_cap, (size_t)q.ntiles * PB * (32 + LC) * 2 * npc, st))) return rc;
-    if ((rc = fit(h, &h->d_xsym, &h->xsym_cap, xneed, st))) return rc;
-    if (h->refit && h->hp_cap) {  // ensure_split_matrices makes them again if they are wanted
+    if ((rc = fit(h, &h->d_psym, &h->psym_cap, (size_t)q.ntiles * PB * (32 + LC) * 2 * npc, st, exact))) return rc;
+    if ((rc = fit(h, &h->d_xsym, &h->xsym_cap, xneed, st, exact))) return rc;
+    if (exact && h->hp_cap) {  // ensure_split_matrices makes them again if they are wanted
         size_t cap = h->hp_cap;
-        fit(h, &h->d_Hp, &cap, 0, st);
-        fit(h, &h->d_Sp, &h->hp_cap, 0, st);
+        fit(h, &h->d_Hp, &cap, 0, st, true);
+        fit(h, &h->d_Sp, &h->hp_cap, 0, st, true);
     }
-    if (same) {
-        h->refit = false;
-        return NECG_OK;
-    }
+    if (same) return NECG_OK;
     // one buffer for all lists: the int2 lists, then the int lists
     const int nkb = necg::row_blocks(K), nb = necg::groups_before(K, LC, 8, -1), nu = q.units();
     const size_t n2 = (size_t)q.ntiles + nu + nb + 2 * nkb, need = n2 + (q.ntiles + nkb + 1 + 1) / 2;
     h->stiles_K = -1;
-    if ((rc = fit(h, &h->d_lists, &h->lists_cap, need, st))) return rc;
+    if ((rc = fit(h, &h->d_lists, &h->lists_cap, need, st, exact))) return rc;
     h->refit = false;
     if (!h->d_qcount) CK(pool_alloc(h, &h->d_qcount, sizeof(int), st));
     necg::SymLists &o = h->lists;

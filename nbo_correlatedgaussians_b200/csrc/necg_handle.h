@@ -52,7 +52,7 @@ struct necg_handle {
     int *d_qcount = nullptr;    // queue head of the block-synchronised fused pass
     // fused pass with one-warp tiles: symmetry terms split over npc warps per tile
     int npc = 1;
-    bool refit = false;  // the pass's settings changed: its buffers are made to measure at the next use
+    bool refit = false;  // the pass's settings changed: its buffers are made to measure with the next lists
     double *d_Hp = nullptr, *d_Sp = nullptr;  // npc K x K sums each, when the caller wants H and S
     size_t hp_cap = 0;                        // doubles per buffer
     double *d_out = nullptr;  // f, the status words and g (d_f, d_status and d_g point into it)

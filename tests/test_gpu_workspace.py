@@ -122,3 +122,26 @@ def test_captures_after_a_plain_evaluation():
     torch.cuda.synchronize()
     for a, b in ((f1, f), (g1, g), (H, Hm), (S, Sm), (en[:1], f)):
         assert float((a - b).abs().max()) <= 1e-12 * float(b.abs().max())
+
+
+def test_a_callers_graph_outlives_a_change_of_splits():
+    """Fewer splits with the same lists leave the buffers that a captured graph holds."""
+    import torch
+    p, eng, x = _engine("H2", 40)
+    f, g = torch.empty(1, dtype=torch.float64, device=eng.device), torch.empty_like(x)
+    assert eng.L.necg_set_symmetric(eng.h, 2, 2, 12) == 0 and eng.L.necg_set_splits(eng.h, 4) == 0
+    eng.outprod_device(x, p.K, f=f, g=g)
+    ref = f.clone(), g.clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        eng.outprod_device(x, p.K, f=f, g=g)
+    held = eng.workspace_bytes()
+    assert eng.L.necg_set_splits(eng.h, 1) == 0
+    eng.outprod_device(x, p.K)
+    assert eng.workspace_bytes() == held
+    f.zero_()
+    g.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(f, ref[0]) and torch.equal(g, ref[1])
